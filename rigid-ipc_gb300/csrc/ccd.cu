@@ -14,6 +14,8 @@
 //    becomes the new earliest root; otherwise it is split at the midpoint of
 //    the dimension with the largest width / tolerance, second half pushed
 //    first.
+// The pruned search (the earliest time of impact alone) runs in single
+// precision first and here only where that cannot decide: ccd_filter.cuh.
 // The time of impact of a candidate (the t.lo of its earliest root box) does
 // not depend on the order boxes are visited, so boxes whose t.lo is not below
 // the running minimum over all candidates can be skipped too: that never
@@ -57,6 +59,8 @@ constexpr int kMaxLaunches = 32;
 constexpr int kWindowLog2 = 6;
 constexpr int64_t kWindowMinCandidates = 1 << 16;
 constexpr unsigned long long kWindowCap = 1ull << 22;
+// box budgets from which the single-precision front is used (the default)
+constexpr int64_t kFilterMinBudget = int64_t(1) << 22;
 
 struct CCDArgs {
     const double* rest;
@@ -99,6 +103,13 @@ struct CCDArgs {
     // seeds, so the deep searches of the tail spread over the whole GPU.
     const struct Piece* pieces_in;
     long long n_pieces;         // pieces in pieces_in (launch 0: none, seeds)
+    const unsigned long long* n_pieces_dev;  // their number on the device instead, or null
+    // records for the single-precision front of the search (ccd_filter.cuh),
+    // written by the set-up kernel; null: none
+    struct FilterRec* rec;
+    const double* ref;
+    const float* frames32;
+    const float* bodies32;
     struct Piece* pieces_out;
     unsigned long long* n_out;
     unsigned long long out_cap;
@@ -562,38 +573,6 @@ __device__ __forceinline__ void load_candidate(const CCDArgs& a, int64_t i, Quer
     q.ct0 = q.ct1 = __longlong_as_double(0x7ff8000000000000ll);
 }
 
-// Per-candidate set-up, one thread per candidate: the tolerances (length
-// tolerances 1e-4 / edge length; the time tolerance divided by 100 when f
-// over [0, toi_tol] x [0, tol_a] x [0, tol_b] contains zero).
-__global__ void __launch_bounds__(128) k_ccd_prepare(CCDArgs a)
-{
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= a.nee + a.nfv) return;
-    Query q;
-    load_candidate(a, i, q);
-    double tol[3];
-    if (i < a.nee) {
-        tol[1] = RDIV(1e-4, a.edge_len[a.ee[i].x]);
-        tol[2] = RDIV(1e-4, a.edge_len[a.ee[i].y]);
-    } else {
-        int f = a.fv[i - a.nee].x;
-        tol[1] = RDIV(1e-4, a.edge_len[a.f2e[3 * f]]);
-        tol[2] = RDIV(1e-4, a.edge_len[a.f2e[3 * f + 1]]);
-    }
-    tol[0] = a.toi_tol;
-    Box xt { 0.0, tol[0], 0.0, tol[1], 0.0, tol[2] };
-    Itv R[9], p[3];
-    const int na = q.fv ? 1 : 2;
-    frame_load(a.table + ((size_t)q.body_a * kTableSlots + kTableNodes) * kTableEntry, R, p);
-    for (int k = 0; k < na; k++) iworld_vertex(R, p, q.v[k], q.P[k]);
-    frame_load(a.table + ((size_t)q.body_b * kTableSlots + kTableNodes) * kTableEntry, R, p);
-    for (int k = na; k < 4; k++) iworld_vertex(R, p, q.v[k], q.P[k]);
-    if (f_zero(q, xt)) tol[0] = RDIV(tol[0], 1e2);
-    a.ctol[3 * i] = tol[0];
-    a.ctol[3 * i + 1] = tol[1];
-    a.ctol[3 * i + 2] = tol[2];
-}
-
 // a <= b for non-negative doubles (+0 and +inf included), on the bit pattern
 __device__ __forceinline__ bool le_nn(double a, double b)
 {
@@ -683,6 +662,50 @@ __device__ __forceinline__ int split_dim_keys(const Node& c, const TolKeys& K, c
         }
     }
     return split;
+}
+
+} // namespace rigc
+
+#include "ccd_filter.cuh"
+
+namespace rigc {
+
+// Per-candidate set-up, one thread per candidate: the tolerances (length
+// tolerances 1e-4 / edge length; the time tolerance divided by 100 when f
+// over [0, toi_tol] x [0, tol_a] x [0, tol_b] contains zero), and the record of
+// the search's single-precision front.
+__global__ void __launch_bounds__(128) k_ccd_prepare(CCDArgs a)
+{
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= a.nee + a.nfv) return;
+    Query q;
+    load_candidate(a, i, q);
+    double tol[3];
+    if (i < a.nee) {
+        tol[1] = RDIV(1e-4, a.edge_len[a.ee[i].x]);
+        tol[2] = RDIV(1e-4, a.edge_len[a.ee[i].y]);
+    } else {
+        int f = a.fv[i - a.nee].x;
+        tol[1] = RDIV(1e-4, a.edge_len[a.f2e[3 * f]]);
+        tol[2] = RDIV(1e-4, a.edge_len[a.f2e[3 * f + 1]]);
+    }
+    tol[0] = a.toi_tol;
+    Box xt { 0.0, tol[0], 0.0, tol[1], 0.0, tol[2] };
+    Itv R[9], p[3];
+    const int na = q.fv ? 1 : 2;
+    frame_load(a.table + ((size_t)q.body_a * kTableSlots + kTableNodes) * kTableEntry, R, p);
+    for (int k = 0; k < na; k++) iworld_vertex(R, p, q.v[k], q.P[k]);
+    frame_load(a.table + ((size_t)q.body_b * kTableSlots + kTableNodes) * kTableEntry, R, p);
+    for (int k = na; k < 4; k++) iworld_vertex(R, p, q.v[k], q.P[k]);
+    if (f_zero(q, xt)) tol[0] = RDIV(tol[0], 1e2);
+    a.ctol[3 * i] = tol[0];
+    a.ctol[3 * i + 1] = tol[1];
+    a.ctol[3 * i + 2] = tol[2];
+    if (a.rec) {
+        FilterRec r;
+        filter_record(q, tol, a.ref, a.frames32, a.bodies32, r);
+        a.rec[i] = r;
+    }
 }
 
 // The node of the candidate's subdivision tree at depth d reached by the
@@ -794,6 +817,13 @@ static __device__ __noinline__ double earliest_unexplored(const Node& cn, u128 m
     return m;
 }
 
+// work items of a launch: pieces, or the candidates' seeds
+__device__ __forceinline__ int64_t work_items(const CCDArgs& a)
+{
+    if (a.n_pieces_dev) return (int64_t)(*a.n_pieces_dev < a.out_cap ? *a.n_pieces_dev : a.out_cap);
+    return a.pieces_in ? a.n_pieces : ((a.nee + a.nfv) << a.seeds_log2);
+}
+
 // Persistent kernel: each lane takes the next unprocessed candidate from a
 // global counter whenever its search runs out of boxes.  Every iteration each
 // lane pops boxes until one survives the cheap tests (or takes a new
@@ -804,6 +834,7 @@ __global__ void __launch_bounds__(kCCDThreads)
 k_ccd(CCDArgs a)
 {
     const int64_t n = a.nee + a.nfv;
+    const int64_t nwork = work_items(a);
     unsigned long long tot_boxes = 0, tot_hits = 0, pops = 0;
     Query q;
     double tol[3] = { 0, 0, 0 };
@@ -970,7 +1001,7 @@ k_ccd(CCDArgs a)
                 // work item w: seed w / n of candidate w % n (seed-major, so
                 // early times of every candidate come first), or piece w
                 const int64_t w = (int64_t)atomicAdd(a.next, 1ull);
-                if (w >= (a.pieces_in ? a.n_pieces : (n << a.seeds_log2))) {
+                if (w >= nwork) {
                     done = true;
                 } else if (a.pieces_in) {
                     // the piece's node is popped (and tested) in the next iteration
@@ -1189,7 +1220,7 @@ k_ccd_group(CCDArgs a)
 {
     static_assert(W == 32 || W == 16, "a warp or a half-warp per search");
     const int64_t n = a.nee + a.nfv;
-    const int64_t nwork = a.pieces_in ? a.n_pieces : (n << a.seeds_log2);
+    const int64_t nwork = work_items(a);
     const int lane = threadIdx.x & 31;
     const int gl = lane & (W - 1);  // lane within the group
     const unsigned gmask = W == 32 ? 0xffffffffu : (0xffffu << (lane & 16));
@@ -1502,20 +1533,20 @@ k_ccd_group(CCDArgs a)
 }
 
 // The pieces of the last launch (out, *n_out of them, at most cap) and those
-// kept for later windows (kept, n_kept): the ones that start before `window`
+// kept for later windows (kept, *n_kept, at most cap): the ones that start before `window`
 // go to `now`, the others to `later`, the ones that start at or after the
 // running minimum `gmin` (single scene; null: none) nowhere.  A list that is
 // full takes the piece into the other (their capacities sum to at least
-// the pieces given); counts[0] / counts[1] end as the appends to now / later
+// the pieces given); *n_now / *n_later end as the appends to now / later
 // (above cap: only the first cap slots were written).
 __global__ void __launch_bounds__(256) k_split_pieces(
     const Piece* __restrict__ out, const unsigned long long* __restrict__ n_out, unsigned long long cap,
-    const Piece* __restrict__ kept, unsigned long long n_kept, double window,
+    const Piece* __restrict__ kept, const unsigned long long* __restrict__ n_kept, double window,
     const unsigned long long* __restrict__ gmin, Piece* __restrict__ now, Piece* __restrict__ later,
-    unsigned long long* __restrict__ counts)
+    unsigned long long* __restrict__ n_now, unsigned long long* __restrict__ n_later)
 {
     const unsigned long long n0 = n_out ? (*n_out < cap ? *n_out : cap) : 0ull;
-    const unsigned long long total = n0 + n_kept;
+    const unsigned long long total = n0 + (*n_kept < cap ? *n_kept : cap);
     const double g = gmin ? __longlong_as_double((long long)*gmin) : INFINITY;
     const int lane = threadIdx.x & 31;
     const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
@@ -1536,8 +1567,8 @@ __global__ void __launch_bounds__(256) k_split_pieces(
         const unsigned m_later = __ballot_sync(0xffffffffu, keep && !soon);
         unsigned long long b_now = 0, b_later = 0;
         if (lane == 0) {
-            if (m_now) b_now = atomicAdd(counts, (unsigned long long)__popc(m_now));
-            if (m_later) b_later = atomicAdd(counts + 1, (unsigned long long)__popc(m_later));
+            if (m_now) b_now = atomicAdd(n_now, (unsigned long long)__popc(m_now));
+            if (m_later) b_later = atomicAdd(n_later, (unsigned long long)__popc(m_later));
         }
         b_now = __shfl_sync(0xffffffffu, b_now, 0);
         b_later = __shfl_sync(0xffffffffu, b_later, 0);
@@ -1548,7 +1579,7 @@ __global__ void __launch_bounds__(256) k_split_pieces(
         if (slot >= cap) {
             // that list is full: the other one
             to_now = !soon;
-            slot = atomicAdd(counts + (to_now ? 0 : 1), 1ull);
+            slot = atomicAdd(to_now ? n_now : n_later, 1ull);
         }
         if (slot < cap) (to_now ? now : later)[slot] = pc;
     }
@@ -1604,14 +1635,20 @@ int reserve_rot_table(Ctx& c)
 
 // counters layout in the context's device scalars (byte offset 256):
 // [0] gmin bits, [1] boxes, [2] hits, [3] status, [4] next work item,
-// [5] search pieces handed off
-int run_ccd(Ctx& c, const double* x0, const double* x1, double toi_tol, int flags,
-            double* toi_host, double* per)
+// [5] search pieces handed off, [6] pieces of the next launch, [7] / [8] of
+// later windows, [9] the filter's next work item, [10] the pieces of the
+// launch behind it
+constexpr int kCCDCounters = 11;
+
+// filter: with the single-precision front; *redo is set (and no result
+// given) when its pieces did not fit their buffers
+static int run_search(Ctx& c, const double* x0, const double* x1, double toi_tol, int flags,
+                      double* toi_host, double* per, bool filter, bool* redo)
 {
     cudaStream_t st = c.stream;
     const int64_t n = c.cand.num_ee + c.cand.num_fv;
     unsigned long long* cnt = reinterpret_cast<unsigned long long*>(c.d_scalars.as<char>() + 256);
-    unsigned long long init[6] = { (unsigned long long)0x7ff0000000000000ull, 0, 0, 0, 0, 0 };
+    unsigned long long init[kCCDCounters] = { (unsigned long long)0x7ff0000000000000ull };
     RIGC_CUDA(cudaMemcpyAsync(cnt, init, sizeof(init), cudaMemcpyHostToDevice, st));
     if (n > 0) {
         CCDArgs a;
@@ -1680,6 +1717,25 @@ int run_ccd(Ctx& c, const double* x0, const double* x1, double toi_tol, int flag
         a.fkeys = c.frame_keys.as<unsigned long long>();
         a.fvals = c.frame_vals.as<double>();
         a.fmask = slots - 1;
+        a.rec = nullptr;
+        a.ref = nullptr;
+        a.frames32 = nullptr;
+        a.bodies32 = nullptr;
+        if (filter) {
+            const size_t ref_bytes = (size_t)c.s.nb * kRef64 * sizeof(double);
+            const size_t body_bytes = (size_t)c.s.nb * kBody32 * sizeof(float);
+            RIGC_TRY(c.ccd_frames32.reserve(ref_bytes + body_bytes
+                                            + (size_t)c.s.nb * kTableSlots * kFrame32 * sizeof(float)));
+            RIGC_TRY(c.ccd_rec.reserve((size_t)n * sizeof(FilterRec)));
+            a.rec = c.ccd_rec.as<FilterRec>();
+            a.ref = c.ccd_frames32.as<double>();
+            a.bodies32 = reinterpret_cast<const float*>(c.ccd_frames32.as<char>() + ref_bytes);
+            a.frames32 = reinterpret_cast<const float*>(c.ccd_frames32.as<char>() + ref_bytes + body_bytes);
+            RIGC_COUNT_LAUNCH();
+            k_filter_bodies<<<(unsigned)c.s.nb, kTableSlots, 0, st>>>(
+                a.table, x0, a.traj, const_cast<double*>(a.ref), const_cast<float*>(a.frames32),
+                const_cast<float*>(a.bodies32));
+        }
         RIGC_COUNT_LAUNCH();
         k_ccd_prepare<<<grid_for(n, 128), 128, 0, st>>>(a);
         if (per) {
@@ -1699,40 +1755,48 @@ int run_ccd(Ctx& c, const double* x0, const double* x1, double toi_tol, int flag
                                                      : blocks_per_sm;
         int64_t full = (int64_t)sms * bps;
         // few candidates: start each search from 2^d boxes of its tree so
-        // that the searches fill the GPU (prune mode; at most 32 per candidate)
+        // that the searches fill the GPU (prune mode; at most 32 per
+        // candidate): a box per lane of 16 warps per SM in the filter, four
+        // searches per resident one without it
         a.seeds_log2 = 0;
         if (a.prune) {
+            const int64_t fill = filter ? (int64_t)sms * 16 * 32 : (full * per_block + 3) / 4;
             if (c.tune.ccd_seeds_log2 >= 0) a.seeds_log2 = std::min(c.tune.ccd_seeds_log2, 5);
             else
-                while (a.seeds_log2 < 5 && (n << a.seeds_log2) * 4 < full * per_block) a.seeds_log2++;
+                while (a.seeds_log2 < 5 && (n << a.seeds_log2) < fill) a.seeds_log2++;
         }
-        // search pieces (prune mode): launch 0 searches the seeds; a search
-        // that reaches hand_off boxes once the work list has run dry hands its
-        // pending boxes on, and boxes after the launch's time window are
-        // deferred; k_split_pieces then gives the next launch those that
-        // start before its window and keeps the others for later ones; the
-        // last launch hands nothing on
+        // search pieces (prune mode): the filter, or launch 0 without it,
+        // searches the seeds; a search that reaches hand_off boxes once the
+        // work list has run dry hands its pending boxes on, and boxes after
+        // the launch's time window are deferred; k_split_pieces then gives
+        // the next launch those that start before its window and keeps the
+        // others for later ones; the last launch hands nothing on
         a.pieces_in = nullptr;
         a.n_pieces = 0;
+        a.n_pieces_dev = nullptr;
         a.hand_off = 0;
         a.n_out = cnt + 5;
         a.out_cap = 0;
         a.pieces_out = nullptr;
         a.window = INFINITY;
+        int window_log2 = 0;
         if (a.prune) {
             const int ho = c.tune.ccd_hand_off >= 0 ? c.tune.ccd_hand_off : kHandOff;
-            const int wl = mode == 0                     ? 0
+            const int wl = mode == 0 && !filter          ? 0
                            : c.tune.ccd_window_log2 >= 0 ? c.tune.ccd_window_log2
+                           : filter                      ? kWindowLog2
                            : n >= kWindowMinCandidates   ? kWindowLog2
                                                          : 0;
-            unsigned long long cap = ho > 0 ? kPiecesCap : 0;
+            window_log2 = wl;
+            unsigned long long cap = ho > 0 || filter ? kPiecesCap : 0;
             if (wl > 0) {
                 // deferred boxes: a few per candidate whose search goes deeper
                 // than its root box
                 if (!cap) cap = kPiecesCap;
-                while (cap < kWindowCap && cap < (unsigned long long)(n << a.seeds_log2) * 2) cap *= 2;
                 a.window = std::ldexp(1.0, -wl);
             }
+            if (wl > 0 || filter)
+                while (cap < kWindowCap && cap < (unsigned long long)(n << a.seeds_log2) * 2) cap *= 2;
             if (cap > 0) {
                 for (int b = 0; b < 4; b++) RIGC_TRY(c.ccd_pieces[b].reserve(cap * sizeof(Piece)));
                 a.hand_off = (unsigned long long)std::max(ho, 0);
@@ -1742,19 +1806,46 @@ int run_ccd(Ctx& c, const double* x0, const double* x1, double toi_tol, int flag
         }
         // pieces: [0] a launch's output, [1] the next launch's input, [2] / [3]
         // those after its window (ping-pong)
-        unsigned long long* split_n = cnt + 6;
-        unsigned long long n_later = 0;
+        unsigned long long* n_now_dev = cnt + 6;
+        unsigned long long* n_later_dev = cnt + 5;  // + later (2 or 3)
         int later = 2;
-        int dev_sms = kNumSMs;
-        {
-            int dv = 0;
-            RIGC_CUDA(cudaGetDevice(&dv));
-            RIGC_CUDA(cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, dv));
-        }
+        // the filter appends its pieces to the first launch's
+        FilterArgs f;
+        f.rec = a.rec;
+        f.frames = a.frames32;
+        f.bodies = a.bodies32;
+        f.n = n;
+        f.seeds_log2 = a.seeds_log2;
+        f.window_log2 = window_log2;
+        f.out = c.ccd_pieces[1].as<Piece>();
+        f.n_out = n_now_dev;
+        f.cap = a.out_cap;
+        f.next = cnt + 9;
+        f.boxes = a.boxes;
+        f.hits = a.hits;
+        f.gmin = a.gmin;
+        f.scene_gmin = a.scene_gmin;
+        f.bscene = a.bscene;
+        if (filter) a.pieces_in = c.ccd_pieces[1].as<Piece>();
         int64_t want = ((n << a.seeds_log2) + per_block - 1) / per_block;
         c.stats.ccd_launches = 0;
         c.stats.ccd_pieces = 0;
         for (int launch = 0;; launch++) {
+            const bool front = filter && launch == 0;
+            if (front) {
+                const unsigned blocks = (unsigned)std::min<int64_t>(grid_for(n << f.seeds_log2, kFilterThreads),
+                                                                    (int64_t)sms * kFilterBlocks);
+                // later boxes: up to four per candidate and list
+                f.later_cap = 256;
+                while (f.later_cap < 4096 && (int64_t)f.later_cap * blocks < 4 * n) f.later_cap *= 2;
+                RIGC_TRY(c.ccd_later.reserve((size_t)blocks * kFilterLists * f.later_cap * sizeof(FNode)));
+                f.later = c.ccd_later.as<FNode>();
+                RIGC_COUNT_LAUNCH();
+                k_ccd_filter<<<blocks, kFilterThreads, 0, st>>>(f);
+                RIGC_CUDA(cudaGetLastError());
+                a.n_pieces_dev = n_now_dev;
+                want = full;
+            }
             RIGC_COUNT_LAUNCH();
             const unsigned grid = (unsigned)std::min(want, full);
             switch (mode) {
@@ -1776,30 +1867,45 @@ int run_ccd(Ctx& c, const double* x0, const double* x1, double toi_tol, int flag
             bool from_out = true;
             for (;;) {
                 const double next_window = last_launch || !(a.window < 0.5) ? INFINITY : 2 * a.window;
-                RIGC_CUDA(cudaMemsetAsync(split_n, 0, 2 * sizeof(unsigned long long), st));
+                const int other = 5 - later;
+                if (front && from_out) {
+                    // read before the split reuses it
+                    RIGC_CUDA(cudaMemcpyAsync(cnt + 10, n_now_dev, sizeof(unsigned long long),
+                                              cudaMemcpyDeviceToDevice, st));
+                }
+                RIGC_CUDA(cudaMemsetAsync(n_now_dev, 0, sizeof(unsigned long long), st));
+                RIGC_CUDA(cudaMemsetAsync(n_later_dev + other, 0, sizeof(unsigned long long), st));
                 RIGC_COUNT_LAUNCH();
-                k_split_pieces<<<4 * dev_sms, 256, 0, st>>>(
+                k_split_pieces<<<4 * sms, 256, 0, st>>>(
                     c.ccd_pieces[0].as<Piece>(), from_out ? a.n_out : nullptr, a.out_cap,
-                    c.ccd_pieces[later].as<Piece>(), n_later, next_window,
+                    c.ccd_pieces[later].as<Piece>(), n_later_dev + later, next_window,
                     c.s.nscenes > 1 ? nullptr : a.gmin, c.ccd_pieces[1].as<Piece>(),
-                    c.ccd_pieces[5 - later].as<Piece>(), split_n);
+                    c.ccd_pieces[other].as<Piece>(), n_now_dev, n_later_dev + other);
                 RIGC_CUDA(cudaGetLastError());
-                unsigned long long h[2];
-                RIGC_CUDA(cudaMemcpyAsync(h, split_n, sizeof(h), cudaMemcpyDeviceToHost, st));
+                unsigned long long h[kCCDCounters];
+                RIGC_CUDA(cudaMemcpyAsync(h, cnt, sizeof(h), cudaMemcpyDeviceToHost, st));
                 RIGC_CUDA(cudaStreamSynchronize(st));
-                n_now = std::min(h[0], a.out_cap);
-                n_later = std::min(h[1], a.out_cap);
-                later = 5 - later;
-                a.window = next_window;
+                if (front && from_out) {
+                    if (h[10] > a.out_cap) {
+                        *redo = true;
+                        return RIGC_OK;
+                    }
+                    c.stats.ccd_pieces += (int64_t)h[10];
+                }
+                n_now = std::min(h[6], a.out_cap);
+                const unsigned long long n_later = std::min(h[5 + other], a.out_cap);
+                later = other;
                 from_out = false;
+                a.window = next_window;
                 if (n_now > 0 || n_later == 0) break;
             }
             if (n_now == 0) break;
-            const unsigned long long zero[2] = { 0, 0 };
-            RIGC_CUDA(cudaMemcpyAsync(a.next, zero, sizeof(zero), cudaMemcpyHostToDevice, st));
+            // the next work items and the handed-off pieces
+            RIGC_CUDA(cudaMemsetAsync(a.next, 0, 2 * sizeof(unsigned long long), st));
             a.pieces_in = c.ccd_pieces[1].as<Piece>();
             a.n_pieces = (long long)n_now;
-            c.stats.ccd_pieces += (int64_t)n_now;
+            a.n_pieces_dev = nullptr;
+            if (!filter) c.stats.ccd_pieces += (int64_t)n_now;
             if (last_launch) a.hand_off = 0;
             want = ((int64_t)n_now + per_block - 1) / per_block;
         }
@@ -1825,6 +1931,21 @@ int run_ccd(Ctx& c, const double* x0, const double* x1, double toi_tol, int flag
     int status = (int)(out[3] & 0xffffffffu);
     c.stats.last_status = status;
     return status;
+}
+
+// The pruned search runs behind the single-precision front unless it has to
+// report per-candidate times (every box is then the double-precision
+// search's) or its box budget is below the default: a search that ends at
+// its budget reports a bound that depends on the boxes it has counted.
+int run_ccd(Ctx& c, const double* x0, const double* x1, double toi_tol, int flags,
+            double* toi_host, double* per)
+{
+    const bool filter = !(flags & RIGC_TOI_NO_PRUNE) && !per && c.ccd_max_boxes >= kFilterMinBudget
+        && c.cand.num_ee + c.cand.num_fv < (int64_t(1) << 31);
+    bool redo = false;
+    const int s = run_search(c, x0, x1, toi_tol, flags, toi_host, per, filter, &redo);
+    if (!redo) return s;
+    return run_search(c, x0, x1, toi_tol, flags, toi_host, per, false, &redo);
 }
 
 } // namespace rigc

@@ -190,6 +190,8 @@ struct Ctx {
     DevBuf frame_keys, frame_vals;  // CCD frame cache (hash table)
     DevBuf pl_table;  // piecewise-linear CCD: per-body piece frames and point rotations
     DevBuf ccd_pieces[4];           // CCD search pieces: a launch's input and output, the later windows' (two)
+    // CCD filter: candidates' records, start and single-precision frames, boxes of later windows
+    DevBuf ccd_rec, ccd_frames32, ccd_later;
     Friction fric;
     int64_t ccd_max_boxes = int64_t(1) << 22;  // per-candidate CCD box budget
     // launch shapes chosen by rigc_autotune (0: the built-in choice)
