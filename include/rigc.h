@@ -226,9 +226,10 @@ int rigc_earliest_toi_piecewise_linear(rigc_ctx* ctx, const double* x0,
                                        const double* x1, double dmin,
                                        double* toi_host, double* per_candidate);
 
-/* How the piecewise-linear CCD spreads its searches: 0 one candidate per
- * warp (the warp evaluates each box's corners together; the default, also
- * for -1), 1 one per lane.  The results are the same bits. */
+/* How the piecewise-linear CCD spreads its searches: 1 pieces and boxes of
+ * all candidates one per lane (the default, also for -1), 0 one candidate per
+ * warp (the warp evaluates each box's corners together).  The results are the
+ * same bits. */
 int rigc_set_pl_search(rigc_ctx* ctx, int32_t per_lane);
 
 /* Time windows of the rigid CCD's pruned searches (the earliest time of

@@ -188,6 +188,7 @@ struct Ctx {
     DevBuf rot_table;
     DevBuf cand_tol;  // CCD: per-candidate tolerances
     DevBuf frame_keys, frame_vals;  // CCD frame cache (hash table)
+    DevBuf pl_work;   // piecewise-linear CCD: per-candidate state, pieces whose boxes are searched
     DevBuf pl_table;  // piecewise-linear CCD: per-body piece frames and point rotations
     DevBuf ccd_pieces[4];           // CCD search pieces: a launch's input and output, the later windows' (two)
     // CCD filter: candidates' records, start and single-precision frames, boxes of later windows
@@ -203,7 +204,7 @@ struct Ctx {
         int ccd_hand_off = -1;         // CCD boxes per search piece before a hand-off (-1: default, 0: never)
         int ccd_window_log2 = -1;      // CCD first time window 2^-k (-1: built-in, 0: no windows)
         int ccd_warp = -1;             // CCD search per lane (0) or per warp (1); -1: by candidate count
-        int pl_per_lane = -1;          // piecewise-linear CCD: a candidate per lane (1) or per warp (0, -1)
+        int pl_per_lane = -1;          // piecewise-linear CCD: pieces and boxes per thread (1, -1) or a candidate per warp (0)
     } tune;
     Sim* sim = nullptr;
     // batched contexts: per-scene results of the last calls

@@ -239,8 +239,8 @@ class Context:
         return toi.value
 
     def set_pl_search(self, per_lane=-1):
-        """Piecewise-linear CCD: a candidate per lane (1) or per warp (0, and
-        -1: the default)."""
+        """Piecewise-linear CCD: pieces and boxes one per lane (1, and -1: the
+        default) or a candidate per warp (0)."""
         L.check(self.lib.rigc_set_pl_search(self.h, int(per_lane)), "rigc_set_pl_search")
 
     def set_ccd_window(self, window_log2=-1):
