@@ -23,9 +23,8 @@
 // f = weight * m(D) * b(d - dmin^2) (m = 1 except mollified EE), so the body
 // Hessian is  sum of outer products of the body-space gradients of the basic
 // scalars + Gram terms + skew pair blocks + the curvature term
-// sum_i grad_Xi f . d2X_i/dtheta2.  It is then projected to the PSD cone by
-// a warp-parallel Jacobi eigensolver (a matrix with no negative eigenvalue is
-// returned unchanged, as project_to_psd does), V max(L, 0) V^T otherwise.
+// sum_i grad_Xi f . d2X_i/dtheta2.  It is then projected to the PSD cone,
+// V max(L, 0) V^T (local_terms.cuh).
 #include <algorithm>
 
 #include "common.cuh"
@@ -103,8 +102,8 @@ __device__ __forceinline__ int local_body_of(int type, int i)
 }
 
 // H += J_i^T Hb J_j (+ its transpose when i and j are different vertices),
-// J_i = [I | D_i], on the upper triangle
-__device__ __forceinline__ void add_vertex_block(SMat H, const Vtx& Vi, int oi, const Vtx& Vj, int oj,
+// J_i = [I | D_i]
+__device__ __forceinline__ void add_vertex_block(SMat H, const Vtx& Vi, int bi, const Vtx& Vj, int bj,
                                                  const double (*Hb)[3], bool same_vertex)
 {
     double HD[3][3], DH[3][3], DHD[3][3];
@@ -116,17 +115,21 @@ __device__ __forceinline__ void add_vertex_block(SMat H, const Vtx& Vi, int oi, 
     for (int r = 0; r < 3; r++)
         for (int c = 0; c < 3; c++)
             DHD[r][c] = Vi.D[0][r] * HD[0][c] + Vi.D[1][r] * HD[1][c] + Vi.D[2][r] * HD[2][c];
-    for (int r = 0; r < 6; r++)
-        for (int c = 0; c < 6; c++) {
-            double v = r < 3 ? (c < 3 ? Hb[r][c] : HD[r][c - 3])
-                             : (c < 3 ? DH[r - 3][c] : DHD[r - 3][c - 3]);
-            int R = oi + r, C = oj + c;
-            if (same_vertex) {
-                if (R <= C) H.at(R, C) += v;
-            } else {
-                if (R <= C) H.at(R, C) += v;
-                if (C <= R) H.at(C, R) += v;
+    if (!same_vertex) {
+        double tt[3][3];
+        for (int r = 0; r < 3; r++)
+            for (int c = 0; c < 3; c++) tt[r][c] = Hb[r][c] + Hb[c][r];
+        add_pair_blocks(H, bi, bj, tt, HD, DH, DHD);
+        return;
+    }
+    const int o = red_rot(bi);
+    for (int r = 0; r < 3; r++)
+        for (int c = 0; c < 3; c++) {
+            if (bi == 0) {
+                if (r <= c) H.at(r, c) += Hb[r][c];
+                H.at(r, o + c) += HD[r][c];
             }
+            if (r <= c) H.at(o + r, o + c) += DHD[r][c];
         }
 }
 
@@ -254,8 +257,7 @@ static __device__ __noinline__ bool ee_endpoint_build(const BarrierArgs& a, int6
         for (int k = 0; k < 12; k++) a.grad[ci * 12 + k] = G[k];
     if (!want_h) return false;
 
-    for (int r = 0; r < 12; r++)
-        for (int cc = r; cc < 12; cc++) H.at(r, cc) = 0;
+    H.clear();
     // M_i = alpha_i (-[B]x) + beta_i [A]x (dn/dX_i), C_i likewise for c = a x b
     auto skew_of = [](double sa, const double* Bv, double sb, const double* Av, double (*M)[3]) {
         double v0 = -sa * Bv[0] + sb * Av[0], v1 = -sa * Bv[1] + sb * Av[1],
@@ -300,14 +302,14 @@ static __device__ __noinline__ bool ee_endpoint_build(const BarrierArgs& a, int6
                                           + m1 * b1 * (gd[i][r] * gD[j][q2] + gD[i][r] * gd[j][q2])
                                           + bv * m2 * gD[i][r] * gD[j][q2] + bv * m1 * hD);
                 }
-            add_vertex_block(H, V[i], 6 * lbody[i], V[j], 6 * lbody[j], Hb, i == j);
+            add_vertex_block(H, V[i], lbody[i], V[j], lbody[j], Hb, i == j);
         }
     for (int i = 0; i < 4; i++) add_curvature(H, fr[lbody[i]], lbody[i], vrest[i], gv[i]);
     return true;
 }
 
-// Energy, gradient and (upper triangle of the) unprojected body Hessian of
-// constraint ci into H; returns true when H holds a Hessian to project and
+// Energy, gradient and (reduced) unprojected body Hessian of constraint ci
+// into H; returns true when H holds a Hessian to project and
 // write, false when every output of the constraint is already written.
 static __device__ __noinline__ bool barrier_build(const BarrierArgs& a, int64_t ci, SMat H)
 {
@@ -482,11 +484,12 @@ static __device__ __noinline__ bool barrier_build(const BarrierArgs& a, int64_t 
     if (!want_h) return false;
 
     // ---- Hessian
-    for (int r = 0; r < 12; r++)
-        for (int c = r; c < 12; c++) H.at(r, c) = 0;
-    double G1[12], G2[12];
-    to_body(V, lbody, nvc, g1v, G1);
-    to_body(V, lbody, nvc, g2v, G2);
+    H.clear();
+    double G1[kRed], G2[kRed];
+    to_body(V, lbody, nvc, g1v, G);
+    reduce12(G, G1);
+    to_body(V, lbody, nvc, g2v, G);
+    reduce12(G, G2);
     // second-derivative coefficients of d in terms of (g1, g2) and the
     // Hessians of the basic scalars:
     //  PT/EE: hess d = (2/D) g1g1 + c1 H_u - (2u/D^2)(g1g2 + g2g1) + (2u^2/D^3) g2g2 + c2 H_D
@@ -544,7 +547,7 @@ static __device__ __noinline__ bool barrier_build(const BarrierArgs& a, int64_t 
                     sv[k] = bu * su + bD * sD;
                 }
                 if (sv[0] == 0 && sv[1] == 0 && sv[2] == 0) continue;
-                add_skew_pair(H, V[i], 6 * lbody[i], V[j], 6 * lbody[j], sv);
+                add_skew_pair(H, V[i], lbody[i], V[j], lbody[j], sv);
             }
     } else if (type == 1) {
         // H_N = 2 (dc)^T(dc) + skew(c); H_e = 2 (de)^T(de)
@@ -569,7 +572,7 @@ static __device__ __noinline__ bool barrier_build(const BarrierArgs& a, int64_t 
                 for (int k = 0; k < 3; k++)
                     sv[k] = bu * 2 * (-al[i] * be[j] * n[k] + al[j] * be[i] * n[k]);
                 if (sv[0] == 0 && sv[1] == 0 && sv[2] == 0) continue;
-                add_skew_pair(H, V[i], 6 * lbody[i], V[j], 6 * lbody[j], sv);
+                add_skew_pair(H, V[i], lbody[i], V[j], lbody[j], sv);
             }
     } else {
         // d = |w|^2: hess = 2 (dw)^T (dw), coefficient P2 (c1 = 1)
@@ -586,43 +589,44 @@ static __device__ __noinline__ bool barrier_build(const BarrierArgs& a, int64_t 
 }
 
 
-// One warp per block.  Lanes 0 .. per_warp-1 each build one constraint's
-// terms (a thread per constraint); then the whole warp projects the built
-// Hessians one after another.  per_warp is chosen by the host so that small
-// constraint sets still spread over the SMs.
-__global__ void __launch_bounds__(kBarrierTPB)
-k_barrier_local(BarrierArgs a, int per_warp)
+template <int W>
+__global__ void __launch_bounds__(kBarrierTPB) k_barrier_local(BarrierArgs a, int per_warp)
 {
     extern __shared__ double smem[];
-    const int lane = threadIdx.x;
-    const int64_t ci = (int64_t)blockIdx.x * per_warp + lane;
-    const bool mine = lane < per_warp && ci < a.n;
-    SMat H { smem + lane };
-    bool built = mine && barrier_build(a, ci, H);
-    if (!(a.flags & RIGC_HESS)) return;  // uniform over the block
-    if (a.flags & RIGC_PROJECT_PSD) {
-        double* work = smem + kSymEntries * kBarrierTPB;
-        unsigned todo = __ballot_sync(0xffffffffu, built);
-        while (todo) {
-            int t = __ffs(todo) - 1;
-            todo &= todo - 1;
-            warp_psd_project(SMat { smem + t }, work, lane);
-        }
+    local_terms<W>(a.n, per_warp, a.flags, a.hess, a.blocks, smem,
+                   [&](int64_t ci, SMat H) { return barrier_build(a, ci, H); });
+}
+
+size_t local_terms_smem_bytes(int per_warp)
+{
+    return (size_t)(kRed * kRed) * (per_warp | 1) * sizeof(double);
+}
+
+// Constraints per warp: a thread per constraint (32) once they give every SM
+// eight warps, fewer for small sets, down to 2 (16 lanes to each).  A power of
+// two; tuned > 0: at most that.
+int local_terms_per_warp(int64_t n, int tuned)
+{
+    const int64_t w = tuned > 0 ? tuned : (n + kNumSMs * 8 - 1) / (kNumSMs * 8);
+    int p = 2;
+    while (p < kBarrierTPB && p < w) p *= 2;
+    return p;
+}
+
+static int launch_barrier(const BarrierArgs& a, int per_warp, cudaStream_t st)
+{
+    const unsigned grid = grid_for(a.n, per_warp);
+    const size_t smem = local_terms_smem_bytes(per_warp);
+    RIGC_COUNT_LAUNCH();
+    switch (per_warp) {
+    case 2: k_barrier_local<16><<<grid, kBarrierTPB, smem, st>>>(a, per_warp); break;
+    case 4: k_barrier_local<8><<<grid, kBarrierTPB, smem, st>>>(a, per_warp); break;
+    case 8: k_barrier_local<4><<<grid, kBarrierTPB, smem, st>>>(a, per_warp); break;
+    case 16: k_barrier_local<2><<<grid, kBarrierTPB, smem, st>>>(a, per_warp); break;
+    default: k_barrier_local<1><<<grid, kBarrierTPB, smem, st>>>(a, per_warp);
     }
-    if (built) write_local_hessian(H, ci, a.hess, a.blocks);
-}
-
-size_t local_terms_smem_bytes()
-{
-    return (size_t)(kSymEntries * kBarrierTPB + kWorkDoubles) * sizeof(double);
-}
-
-// constraints per warp: a thread per constraint once there are enough of
-// them to fill the GPU, fewer (down to one) for small sets
-int local_terms_per_warp(int64_t n)
-{
-    int64_t w = (n + kNumSMs * 8 - 1) / (kNumSMs * 8);
-    return (int)std::max<int64_t>(1, std::min<int64_t>(kBarrierTPB, w));
+    RIGC_CUDA(cudaGetLastError());
+    return RIGC_OK;
 }
 
 int launch_body_frames(Ctx& c, const double* x)
@@ -639,12 +643,6 @@ int launch_barrier_local(Ctx& c, const double* x, double dhat, double dmin, int 
 {
     RIGC_TRY(launch_body_frames(c, x));
     if (c.cons.num == 0) return RIGC_OK;
-    static bool attr = false;
-    if (!attr) {
-        RIGC_CUDA(cudaFuncSetAttribute(k_barrier_local, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)local_terms_smem_bytes()));
-        attr = true;
-    }
     BarrierArgs a;
     a.rest = c.s.rest;
     a.frames = c.frames.as<double>();
@@ -661,12 +659,7 @@ int launch_barrier_local(Ctx& c, const double* x, double dhat, double dmin, int 
     a.grad = grad;
     a.blocks = blocks;
     a.hess = hess;
-    const int pw = c.tune.barrier_per_warp > 0 ? std::min(c.tune.barrier_per_warp, kBarrierTPB)
-                                               : local_terms_per_warp(c.cons.num);
-    RIGC_COUNT_LAUNCH();
-    k_barrier_local<<<grid_for(c.cons.num, pw), kBarrierTPB, local_terms_smem_bytes(), c.stream>>>(a, pw);
-    RIGC_CUDA(cudaGetLastError());
-    return RIGC_OK;
+    return launch_barrier(a, local_terms_per_warp(c.cons.num, c.tune.barrier_per_warp), c.stream);
 }
 
 // Frames and per-constraint terms with every buffer supplied by the caller
@@ -682,8 +675,6 @@ int launch_barrier_local_raw(const double* rest, int64_t nv, int nb, const doubl
     k_body_frames<<<grid_for(nb, 128), 128, 0, stream>>>(x, nb, frames);
     RIGC_CUDA(cudaGetLastError());
     if (n == 0) return RIGC_OK;
-    RIGC_CUDA(cudaFuncSetAttribute(k_barrier_local, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)local_terms_smem_bytes()));
     BarrierArgs a;
     a.rest = rest;
     a.frames = frames;
@@ -702,11 +693,7 @@ int launch_barrier_local_raw(const double* rest, int64_t nv, int nb, const doubl
     a.hess = hess;
     a.check_nb = nb;
     a.check_nv = nv;
-    const int pw = local_terms_per_warp(n);
-    RIGC_COUNT_LAUNCH();
-    k_barrier_local<<<grid_for(n, pw), kBarrierTPB, local_terms_smem_bytes(), stream>>>(a, pw);
-    RIGC_CUDA(cudaGetLastError());
-    return RIGC_OK;
+    return launch_barrier(a, local_terms_per_warp(n, 0), stream);
 }
 
 // ---------------------------------------------------------------------------
@@ -750,50 +737,73 @@ __global__ void k_seg_starts(const int32_t* __restrict__ head, const int32_t* __
     if (head[i]) seg_start[segid[i]] = (int32_t)i;
 }
 
-// one thread per (unique block, entry): sequential sum in slot order
-__global__ void k_block_sums(const uint64_t* __restrict__ keys, const uint32_t* __restrict__ slots,
-                             const int32_t* __restrict__ seg_start,
-                             const int32_t* __restrict__ nseg_ptr, int64_t m,
-                             const double* __restrict__ blocks, int nb,
-                             int32_t* __restrict__ col, double* __restrict__ val,
-                             int32_t* __restrict__ row_count)
+// Sum of a segment's items by a block, one thread per (slice, entry): slice s
+// takes items s, s + S, ... in order, then the slices are added in order, so
+// the sum depends on the segment's items alone and one of at most S items is
+// the sequential sum.  A few bodies in face-to-face contact give segments of
+// 10^4 items (172 k constraints between 33 bodies: one thread per entry took
+// 4.3 ms for the blocks and 2.4 ms for the gradient, the latency of a chain of
+// adds; the slices take 0.22 and 0.1 ms).
+template <int E, int S, class Load>
+__device__ __forceinline__ double segment_sum(int64_t s0, int64_t s1, double* part, Load load)
 {
-    int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int32_t nseg = *nseg_ptr;
-    if (t >= (int64_t)nseg * 36) return;
-    int32_t sgi = (int32_t)(t / 36);
-    int e = (int)(t % 36);
-    int64_t s0 = seg_start[sgi];
-    int64_t s1 = sgi + 1 < nseg ? seg_start[sgi + 1] : m;
+    const int e = threadIdx.x % E, s = threadIdx.x / E;
     double acc = 0;
-    for (int64_t i = s0; i < s1; i++) acc += blocks[(size_t)slots[i] * 36 + e];
-    val[(size_t)sgi * 36 + e] = acc;
-    if (e == 0) {
-        uint64_t k = keys[s0];
-        int32_t r = (int32_t)(k / (uint64_t)nb);
-        col[sgi] = (int32_t)(k % (uint64_t)nb);
-        atomicAdd(&row_count[r], 1);
+    int64_t i = s0 + s;
+    for (; i + 3 * S < s1; i += 4 * S) {
+        const double a = load(i, e), b = load(i + S, e), c = load(i + 2 * S, e), d = load(i + 3 * S, e);
+        acc = (((acc + a) + b) + c) + d;
+    }
+    for (; i < s1; i += S) acc += load(i, e);
+    part[s * E + e] = acc;
+    __syncthreads();
+    double sum = 0;
+    if (s == 0) {
+        const int64_t used = s1 - s0 < S ? s1 - s0 : S;
+        for (int k = 0; k < used; k++) sum += part[k * E + e];
+    }
+    __syncthreads();
+    return sum;
+}
+
+constexpr int kBlockSlices = 16, kGradSlices = 64;
+
+// blocks over the unique Hessian blocks
+__global__ void __launch_bounds__(36 * kBlockSlices) k_block_sums(
+    const uint64_t* __restrict__ keys, const uint32_t* __restrict__ slots, const int32_t* __restrict__ seg_start,
+    const int32_t* __restrict__ nseg_ptr, int64_t m, const double* __restrict__ blocks, int nb,
+    int32_t* __restrict__ col, double* __restrict__ val, int32_t* __restrict__ row_count)
+{
+    __shared__ double part[36 * kBlockSlices];
+    const int32_t nseg = *nseg_ptr;
+    for (int32_t sgi = blockIdx.x; sgi < nseg; sgi += gridDim.x) {
+        const int64_t s0 = seg_start[sgi], s1 = sgi + 1 < nseg ? seg_start[sgi + 1] : m;
+        const double sum = segment_sum<36, kBlockSlices>(
+            s0, s1, part, [&](int64_t i, int e) { return blocks[(size_t)slots[i] * 36 + e]; });
+        if (threadIdx.x < 36) val[(size_t)sgi * 36 + threadIdx.x] = sum;
+        if (threadIdx.x == 0) {
+            const uint64_t k = keys[s0];
+            col[sgi] = (int32_t)(k % (uint64_t)nb);
+            atomicAdd(&row_count[(int32_t)(k / (uint64_t)nb)], 1);
+        }
     }
 }
 
-__global__ void k_grad_sums(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ slots,
-                            const int32_t* __restrict__ seg_start,
-                            const int32_t* __restrict__ nseg_ptr, int64_t m,
-                            const double* __restrict__ cgrad, double* __restrict__ grad)
+// blocks over the bodies with a gradient
+__global__ void __launch_bounds__(6 * kGradSlices) k_grad_sums(
+    const uint32_t* __restrict__ keys, const uint32_t* __restrict__ slots, const int32_t* __restrict__ seg_start,
+    const int32_t* __restrict__ nseg_ptr, int64_t m, const double* __restrict__ cgrad, double* __restrict__ grad)
 {
-    int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    __shared__ double part[6 * kGradSlices];
     const int32_t nseg = *nseg_ptr;
-    if (t >= (int64_t)nseg * 6) return;
-    int32_t sgi = (int32_t)(t / 6);
-    int e = (int)(t % 6);
-    int64_t s0 = seg_start[sgi];
-    int64_t s1 = sgi + 1 < nseg ? seg_start[sgi + 1] : m;
-    double acc = 0;
-    for (int64_t i = s0; i < s1; i++) {
-        uint32_t slot = slots[i];  // = 2 c + side
-        acc += cgrad[(size_t)(slot >> 1) * 12 + 6 * (slot & 1) + e];
+    for (int32_t sgi = blockIdx.x; sgi < nseg; sgi += gridDim.x) {
+        const int64_t s0 = seg_start[sgi], s1 = sgi + 1 < nseg ? seg_start[sgi + 1] : m;
+        const double sum = segment_sum<6, kGradSlices>(s0, s1, part, [&](int64_t i, int e) {
+            const uint32_t slot = slots[i];  // = 2 c + side
+            return cgrad[(size_t)(slot >> 1) * 12 + 6 * (slot & 1) + e];
+        });
+        if (threadIdx.x < 6) grad[(size_t)keys[s0] * 6 + threadIdx.x] = sum;
     }
-    grad[(size_t)keys[s0] * 6 + e] = acc;
 }
 
 int assemble_terms(Ctx& c, const int* bodies, int64_t n, const double* cgrad,
@@ -835,7 +845,7 @@ int assemble_terms(Ctx& c, const int* bodies, int64_t n, const double* cgrad,
         k_seg_starts<<<grid_for(m, 256), 256, 0, st>>>(head, segid, m, segst);
         // at most m segments; the kernel reads the true count on the device
         RIGC_COUNT_LAUNCH();
-        k_grad_sums<<<grid_for(m * 6, 256), 256, 0, st>>>(
+        k_grad_sums<<<(unsigned)std::min<int64_t>(m, kNumSMs * 4), 6 * kGradSlices, 0, st>>>(
             S[2].as<uint32_t>(), S[3].as<uint32_t>(), segst, nseg_dev, m, cgrad,
             grad.as<double>());
     }
@@ -867,7 +877,7 @@ int assemble_terms(Ctx& c, const int* bodies, int64_t n, const double* cgrad,
         RIGC_TRY(col.reserve((size_t)m * sizeof(int32_t)));
         RIGC_TRY(val.reserve((size_t)m * 36 * sizeof(double)));
         RIGC_COUNT_LAUNCH();
-        k_block_sums<<<grid_for(m * 36, 256), 256, 0, st>>>(
+        k_block_sums<<<(unsigned)std::min<int64_t>(m, kNumSMs * 3), 36 * kBlockSlices, 0, st>>>(
             S[2].as<uint64_t>(), S[3].as<uint32_t>(), segst, nseg_dev, m, cblocks, nb,
             col.as<int32_t>(), val.as<double>(), row_ptr.as<int32_t>() + 1);
         // row counts -> row_ptr (exclusive scan of counts shifted by one)

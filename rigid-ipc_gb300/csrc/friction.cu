@@ -245,16 +245,17 @@ static __device__ __noinline__ bool friction_build(const FrictionArgs& a, int64_
     if (a.grad)
         for (int k = 0; k < 12; k++) a.grad[ci * 12 + k] = G[k];
     if (!want_h) return false;
-    for (int r = 0; r < 12; r++)
-        for (int c = r; c < 12; c++) H.at(r, c) = 0;
-    double A0[4][3], A1[4][3], G0[12], G1[12];
+    H.clear();
+    double A0[4][3], A1[4][3], G0[kRed], G1[kRed];
     for (int i = 0; i < nvc; i++)
         for (int j = 0; j < 3; j++) {
             A0[i][j] = g[i] * t1[j];
             A1[i][j] = g[i] * t2[j];
         }
-    to_body(V, lbody, nvc, A0, G0);
-    to_body(V, lbody, nvc, A1, G1);
+    to_body(V, lbody, nvc, A0, G);
+    reduce12(G, G0);
+    to_body(V, lbody, nvc, A1, G);
+    reduce12(G, G1);
     add_outer(H, ml * h00, G0);
     add_sym_outer(H, ml * h01, G0, G1);
     add_outer(H, ml * h11, G1);
@@ -262,28 +263,12 @@ static __device__ __noinline__ bool friction_build(const FrictionArgs& a, int64_
     return true;
 }
 
-// one warp per block, per_warp constraints built by lanes, then projected
-// by the warp (the layout of the barrier kernel)
-__global__ void __launch_bounds__(kBarrierTPB)
-k_friction_local(FrictionArgs a, int per_warp)
+template <int W>
+__global__ void __launch_bounds__(kBarrierTPB) k_friction_local(FrictionArgs a, int per_warp)
 {
     extern __shared__ double smem[];
-    const int lane = threadIdx.x;
-    const int64_t ci = (int64_t)blockIdx.x * per_warp + lane;
-    const bool mine = lane < per_warp && ci < a.n;
-    SMat H { smem + lane };
-    bool built = mine && friction_build(a, ci, H);
-    if (!(a.flags & RIGC_HESS)) return;  // uniform over the block
-    if (a.flags & RIGC_PROJECT_PSD) {
-        double* work = smem + kSymEntries * kBarrierTPB;
-        unsigned todo = __ballot_sync(0xffffffffu, built);
-        while (todo) {
-            int t = __ffs(todo) - 1;
-            todo &= todo - 1;
-            warp_psd_project(SMat { smem + t }, work, lane);
-        }
-    }
-    if (built) write_local_hessian(H, ci, a.hess, a.blocks);
+    local_terms<W>(a.n, per_warp, a.flags, a.hess, a.blocks, smem,
+                   [&](int64_t ci, SMat H) { return friction_build(a, ci, H); });
 }
 
 // ---------------------------------------------------------------------------
@@ -331,12 +316,6 @@ int launch_friction_local(Ctx& c, const double* x, double epsvh, int flags, doub
     Friction& F = c.fric;
     RIGC_TRY(launch_body_frames(c, x));
     if (F.num == 0) return RIGC_OK;
-    static bool attr = false;
-    if (!attr) {
-        RIGC_CUDA(cudaFuncSetAttribute(k_friction_local, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)local_terms_smem_bytes()));
-        attr = true;
-    }
     FrictionArgs a;
     a.rest = c.s.rest;
     a.frames = c.frames.as<double>();
@@ -353,9 +332,17 @@ int launch_friction_local(Ctx& c, const double* x, double epsvh, int flags, doub
     a.grad = grad;
     a.blocks = blocks;
     a.hess = hess;
-    const int pw = local_terms_per_warp(F.num);
+    const int pw = local_terms_per_warp(F.num, 0);
+    const unsigned grid = grid_for(F.num, pw);
+    const size_t smem = local_terms_smem_bytes(pw);
     RIGC_COUNT_LAUNCH();
-    k_friction_local<<<grid_for(F.num, pw), kBarrierTPB, local_terms_smem_bytes(), c.stream>>>(a, pw);
+    switch (pw) {
+    case 2: k_friction_local<16><<<grid, kBarrierTPB, smem, c.stream>>>(a, pw); break;
+    case 4: k_friction_local<8><<<grid, kBarrierTPB, smem, c.stream>>>(a, pw); break;
+    case 8: k_friction_local<4><<<grid, kBarrierTPB, smem, c.stream>>>(a, pw); break;
+    case 16: k_friction_local<2><<<grid, kBarrierTPB, smem, c.stream>>>(a, pw); break;
+    default: k_friction_local<1><<<grid, kBarrierTPB, smem, c.stream>>>(a, pw);
+    }
     RIGC_CUDA(cudaGetLastError());
     return RIGC_OK;
 }

@@ -1,9 +1,17 @@
 // Device helpers shared by the per-constraint local terms (barrier and
 // friction): vertex positions with their rotation derivatives, body-space
-// images of vertex-space vectors, shared-memory 12x12 accumulators, the rigid
-// curvature term of apply_chain_rule
-// (src/problems/distance_barrier_rb_problem.cpp:1182-1248) and the
-// warp-parallel PSD projection.
+// images of vertex-space vectors, shared-memory Hessian accumulators, the
+// rigid curvature term of apply_chain_rule
+// (src/problems/distance_barrier_rb_problem.cpp:1182-1248) and the PSD
+// projection.
+//
+// A constraint's energy depends on its bodies' translations through their
+// difference t_a - t_b only, so its 12x12 Hessian over (t_a, theta_a, t_b,
+// theta_b) is that over (t_a, theta_a, theta_b) with the rows and columns of
+// t_b the negatives of t_a's.  The kernels accumulate those 9 rows (45
+// entries).  In the orthonormal basis with (t_a - t_b) / sqrt 2 in the place
+// of the translations the Hessian is the 9x9 with its t_a rows and columns
+// times sqrt 2 (and zero on t_a + t_b), so the projection is that of the 9x9.
 #pragma once
 
 #include "common.cuh"
@@ -31,30 +39,49 @@ __device__ __forceinline__ double dot(const double* a, const double* b)
     return a[0] * b[0] + a[1] * b[1] + a[2] * b[2];
 }
 
-// shared-memory symmetric 12x12 accumulator: the upper triangle (r <= c)
-// packed row by row (78 entries), entry-major / thread-minor
-constexpr int kSymEntries = 78;
+// reduced index (t_a 0-2, theta_a 3-5, theta_b 6-8) of body lb's rotation
+__device__ __forceinline__ int red_rot(int lb) { return 3 + 3 * lb; }
+
+// shared-memory symmetric 9x9 of one constraint: element (r, c), r >= c, in
+// the lower triangle of a full row-major 9x9 whose entries are `stride`
+// doubles apart (the constraints of a warp interleaved, the stride odd so that
+// both a warp over constraints and a warp over entries meet all banks)
+constexpr int kRed = 9;
 struct SMat {
     double* base;
-    __device__ __forceinline__ double& at(int r, int c) const
+    int stride;
+    __device__ __forceinline__ double& full(int r, int c) const { return base[(r * kRed + c) * stride]; }
+    // entry (r, c) of the upper triangle, r <= c
+    __device__ __forceinline__ double& at(int r, int c) const { return full(c, r); }
+    __device__ __forceinline__ void clear() const
     {
-        return base[(r * (23 - r) / 2 + c) * kBarrierTPB];
+        for (int r = 0; r < kRed; r++)
+            for (int c = 0; c <= r; c++) full(r, c) = 0;
     }
 };
 
-// H += coef * (a b^T + b a^T) on the upper triangle (a, b in body space)
+// the reduced entries of a body-space 12-vector
+__device__ __forceinline__ void reduce12(const double* g, double* r)
+{
+#pragma unroll
+    for (int k = 0; k < 6; k++) r[k] = g[k];
+#pragma unroll
+    for (int k = 6; k < 9; k++) r[k] = g[k + 3];
+}
+
+// H += coef * (a b^T + b a^T) (a, b reduced)
 __device__ __forceinline__ void add_sym_outer(SMat H, double coef, const double* a, const double* b)
 {
-    for (int r = 0; r < 12; r++) {
+    for (int r = 0; r < kRed; r++) {
         double ar = coef * a[r], br = coef * b[r];
-        for (int c = r; c < 12; c++) H.at(r, c) += ar * b[c] + br * a[c];
+        for (int c = r; c < kRed; c++) H.at(r, c) += ar * b[c] + br * a[c];
     }
 }
 __device__ __forceinline__ void add_outer(SMat H, double coef, const double* a)
 {
-    for (int r = 0; r < 12; r++) {
+    for (int r = 0; r < kRed; r++) {
         double ar = coef * a[r];
-        for (int c = r; c < 12; c++) H.at(r, c) += ar * a[c];
+        for (int c = r; c < kRed; c++) H.at(r, c) += ar * a[c];
     }
 }
 
@@ -72,56 +99,75 @@ __device__ __forceinline__ void to_body(const Vtx* V, const int* lbody, int nvc,
     }
 }
 
-// Gram term H += coef * JM^T JM where JM (3 x 12) = sum_i M_i J_i and
+// Gram term H += coef * JM^T JM where JM (3 x 9) = sum_i M_i J_i and
 // M_i = m_i * I + (skew parts): here M_i given as full 3x3 per vertex.
 __device__ __forceinline__ void add_gram(SMat H, double coef, const Vtx* V, const int* lbody,
                                          int nvc, const double (*M)[9])
 {
-    double JM[3][12];
+    double JM[3][kRed];
     for (int r = 0; r < 3; r++)
-        for (int c = 0; c < 12; c++) JM[r][c] = 0;
+        for (int c = 0; c < kRed; c++) JM[r][c] = 0;
     for (int i = 0; i < nvc; i++) {
-        int o = 6 * lbody[i];
+        const int o = red_rot(lbody[i]);
         for (int r = 0; r < 3; r++) {
-            for (int j = 0; j < 3; j++) JM[r][o + j] += M[i][3 * r + j];
+            if (lbody[i] == 0)
+                for (int j = 0; j < 3; j++) JM[r][j] += M[i][3 * r + j];
             for (int k = 0; k < 3; k++)
-                JM[r][o + 3 + k] += M[i][3 * r] * V[i].D[0][k] + M[i][3 * r + 1] * V[i].D[1][k]
+                JM[r][o + k] += M[i][3 * r] * V[i].D[0][k] + M[i][3 * r + 1] * V[i].D[1][k]
                     + M[i][3 * r + 2] * V[i].D[2][k];
         }
     }
-    for (int r = 0; r < 12; r++) {
+    for (int r = 0; r < kRed; r++) {
         double a0 = coef * JM[0][r], a1 = coef * JM[1][r], a2 = coef * JM[2][r];
-        for (int c = r; c < 12; c++) H.at(r, c) += a0 * JM[0][c] + a1 * JM[1][c] + a2 * JM[2][c];
+        for (int c = r; c < kRed; c++) H.at(r, c) += a0 * JM[0][c] + a1 * JM[1][c] + a2 * JM[2][c];
     }
 }
 
-// skew pair block: H(i-part, j-part) += J_i^T [s]x J_j, and its transpose
-__device__ __forceinline__ void add_skew_pair(SMat H, const Vtx& Vi, int oi, const Vtx& Vj,
-                                              int oj, const double* s)
+// J_i^T B J_j for different vertices i, j (bodies bi <= bj) and its
+// transpose: KD = B D_j, DK = D_i^T B (rows), DKD = D_i^T B D_j; tt = B + B^T
+// (null: zero)
+__device__ __forceinline__ void add_pair_blocks(SMat H, int bi, int bj, const double (*tt)[3],
+                                                const double (*KD)[3], const double (*DK)[3],
+                                                const double (*DKD)[3])
 {
-    // K = [s]x
-    const double K[3][3] = { { 0, -s[2], s[1] }, { s[2], 0, -s[0] }, { -s[1], s[0], 0 } };
-    // blocks: [K, K Dj ; Di^T K, Di^T K Dj]
+    const int oi = red_rot(bi), oj = red_rot(bj);
+    if (bi == 0 && bj == 0 && tt)
+        for (int r = 0; r < 3; r++)
+            for (int c = r; c < 3; c++) H.at(r, c) += tt[r][c];
+    // rows t_a: B D_j where vertex i is body a's, (D_i^T B)^T where j is
+    if (bi == 0)
+        for (int r = 0; r < 3; r++)
+            for (int c = 0; c < 3; c++) H.at(r, oj + c) += KD[r][c];
+    if (bj == 0)
+        for (int r = 0; r < 3; r++)
+            for (int c = 0; c < 3; c++) H.at(r, oi + c) += DK[c][r];
+    if (bi == bj) {
+        for (int r = 0; r < 3; r++)
+            for (int c = r; c < 3; c++) H.at(oi + r, oi + c) += DKD[r][c] + DKD[c][r];
+    } else {
+        for (int r = 0; r < 3; r++)
+            for (int c = 0; c < 3; c++) H.at(oi + r, oj + c) += DKD[r][c];
+    }
+}
+
+// skew pair block: J_i^T [s]x J_j and its transpose ([s]x + [s]x^T = 0)
+__device__ __forceinline__ void add_skew_pair(SMat H, const Vtx& Vi, int bi, const Vtx& Vj, int bj,
+                                              const double* s)
+{
     double KD[3][3], DK[3][3], DKD[3][3];
-    for (int r = 0; r < 3; r++)
-        for (int c = 0; c < 3; c++) {
-            KD[r][c] = K[r][0] * Vj.D[0][c] + K[r][1] * Vj.D[1][c] + K[r][2] * Vj.D[2][c];
-            DK[r][c] = Vi.D[0][r] * K[0][c] + Vi.D[1][r] * K[1][c] + Vi.D[2][r] * K[2][c];
-        }
+    for (int c = 0; c < 3; c++) {
+        // columns s x D_j[:, c]; rows (D_i^T [s]x)[c, :] = D_i[:, c] x s
+        KD[0][c] = s[1] * Vj.D[2][c] - s[2] * Vj.D[1][c];
+        KD[1][c] = s[2] * Vj.D[0][c] - s[0] * Vj.D[2][c];
+        KD[2][c] = s[0] * Vj.D[1][c] - s[1] * Vj.D[0][c];
+        DK[c][0] = Vi.D[1][c] * s[2] - Vi.D[2][c] * s[1];
+        DK[c][1] = Vi.D[2][c] * s[0] - Vi.D[0][c] * s[2];
+        DK[c][2] = Vi.D[0][c] * s[1] - Vi.D[1][c] * s[0];
+    }
     for (int r = 0; r < 3; r++)
         for (int c = 0; c < 3; c++)
             DKD[r][c] = Vi.D[0][r] * KD[0][c] + Vi.D[1][r] * KD[1][c] + Vi.D[2][r] * KD[2][c];
-    // B (6x6) = [[K, KD], [DK, DKD]] goes to rows oi.., cols oj..; its
-    // transpose to rows oj.., cols oi..; accumulate into the upper triangle.
-    for (int r = 0; r < 6; r++)
-        for (int c = 0; c < 6; c++) {
-            double v = r < 3 ? (c < 3 ? K[r][c] : KD[r][c - 3])
-                             : (c < 3 ? DK[r - 3][c] : DKD[r - 3][c - 3]);
-            int R = oi + r, C = oj + c;
-            // entry (R, C) of B and entry (C, R) of B^T are both v
-            if (R <= C) H.at(R, C) += v;
-            if (C <= R) H.at(C, R) += v;
-        }
+    add_pair_blocks(H, bi, bj, nullptr, KD, DK, DKD);
 }
 
 // curvature term: H(rot lb, rot lb) += sum_j g_j (d2R_kl v)_j
@@ -129,7 +175,7 @@ __device__ __forceinline__ void add_curvature(SMat H, const double* frame, int l
                                               const double* v, const double* g)
 {
     const double* d2 = frame + 36;
-    int o = 6 * lb + 3;
+    const int o = red_rot(lb);
     for (int k = 0; k < 3; k++)
         for (int l = k; l < 3; l++) {
             const double* M = d2 + 9 * sym_index(k, l);
@@ -141,246 +187,298 @@ __device__ __forceinline__ void add_curvature(SMat H, const double* frame, int l
 }
 
 // ---------------------------------------------------------------------------
-// PSD projection of one 12x12 (upper triangle filled, in the packed layout
-// of its owner thread) by the whole warp: V max(L, 0) V^T from the
-// eigen-decomposition A = V L V^T.  As project_to_psd does, a matrix whose
-// eigenvalues are all >= 0 is left as it is.
+// PSD projection of one 9x9 (lower triangle filled): A + V max(-L, 0) V^T from
+// the eigen-decomposition A = V L V^T (as project_to_psd does, a matrix with
+// no negative eigenvalue is left as it is), by Householder tridiagonalisation and the
+// implicit symmetric QR algorithm with Wilkinson shifts (Golub & Van Loan,
+// Matrix Computations, algorithms 8.3.1 - 8.3.3), in double throughout.
 //
-// The decomposition is a parallel cyclic Jacobi in round-robin order (each
-// round rotates six disjoint (p, q) planes at once, eleven rounds visit all
-// 66 pairs), run twice:
-//  1. in single precision on A rounded to float, to convergence: it gives
-//     eigenvectors V32 accurate to single precision;
-//  2. in double precision on B = Q^T A Q, Q being V32 orthonormalised in
-//     double; B is diagonal up to the single-precision error, so the Jacobi
-//     sweeps converge quadratically from there (two or three sweeps where
-//     seven or eight were needed from A itself), the rotations accumulated
-//     into Q.
-// An FP64 warp instruction costs this GPU's FP64 unit 64 cycles whatever its
-// active lanes, a single-precision one one cycle of issue, so the sweeps of
-// step 1 are nearly free and the FP64 work drops to a few 12 x 12 products
-// and the refining sweeps.  The double-precision stopping rule is the one-step
-// method's (off-diagonal sum of squares <= 1e-30 of the diagonal's), so the
-// result is the same decomposition to rounding.  (A double-precision
-// refinement of V32 by matrix products alone, with no rotations, does not
-// reach double precision when the eigenvalues span more decades than single
-// precision resolves, as these Hessians' do.)
-// Rotation (c, s) per plane follows the textbook symmetric Schur step:
-// theta = (a_qq - a_pp) / (2 a_pq), t = sign(theta) / (|theta| +
-// sqrt(theta^2 + 1)), c = 1 / sqrt(t^2 + 1), s = t c; the single-precision
-// sweeps take it with the fast reciprocal and reciprocal square root (they
-// only seed step 2).
+// W lanes share one matrix, each taking every W-th row (or column): W = 1 for
+// many constraints (a thread per constraint: every FP64 instruction of a warp
+// works on 32 matrices; an FP64 warp instruction takes this GPU's FP64 unit 64
+// cycles whatever its active lanes), more for few (a shorter chain per
+// matrix).  Every W computes each number by the same operations in the same
+// order (products that feed sums are rounded explicitly, so that no
+// instantiation contracts them), so the results are the same bits.  The scalars of a step (rotations,
+// shifts, the tridiagonal matrix) are computed by every lane of the matrix
+// for itself; V stays in the matrix's shared memory.
+// Measured against a parallel Jacobi of the 12x12 by a warp (single-precision
+// seed, double refinement), building included: 172 k barrier constraints 41.8
+// -> 4.1 ms (FP64 issue), 98 k friction constraints 25.9 -> 1.4 ms, 180 barrier
+// constraints (16 lanes each) 0.50 -> 0.34 ms (the chain of one matrix).
 
-constexpr int kLd = 13;  // padded row stride of the warp's work matrices
-// doubles: A, Q, T, U (12 x kLd each), 6 (c, s) + 4; then floats A32, V32
-// (12 x kLd each), 6 (c, s) + 4
-constexpr int kWorkDoubles = 4 * 12 * kLd + 16 + (2 * 12 * kLd + 16) / 2;
-
-// round-robin schedule over 12 indices: round r pairs (r, 11) and
-// (pos_k, pos_{11-k}) for k = 1 .. 5, pos_k = (k + r) mod 11; (p, q) with p < q
-__device__ __forceinline__ void round_pair(int round, int k, int& p, int& q)
+// 1 / sqrt(h) for normal h: the hardware approximation (about 20 bits) and one
+// third-order step
+__device__ __forceinline__ double rsqrt_refined(double h)
 {
-    if (k == 0) {
-        p = round;
-        q = 11;
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(h));
+    const double e = fma(-h * y, y, 1.0);
+    return fma(y * e, fma(0.375, e, 0.5), y);
+}
+
+template <int W>
+__device__ __forceinline__ void group_sync(unsigned mask)
+{
+    if (W > 1) __syncwarp(mask);
+}
+
+constexpr int kQRSteps = 30 * kRed;  // bound of the QR iteration (converges in about 1.7 per row)
+
+// g: this lane's number in the matrix's group of W lanes, mask: the group's
+template <int W>
+static __device__ void psd_project(SMat H, int g, unsigned mask)
+{
+    double d[kRed], e[kRed];
+    const double kSqrt2 = 1.4142135623730951;
+    double keep[(kRed + W - 1) / W][kRed];  // the matrix as given
+#pragma unroll
+    for (int i = 0; i < (kRed + W - 1) / W; i++)
+#pragma unroll
+        for (int c = 0; c < kRed; c++)
+            if (g + i * W < kRed && c <= g + i * W) keep[i][c] = H.full(g + i * W, c);
+    group_sync<W>(mask);
+    // (t_a - t_b) / sqrt 2 in the place of t_a
+    for (int r = g; r < kRed; r += W)
+        for (int c = 0; c < 3 && c <= r; c++) H.full(r, c) *= r < 3 ? 2.0 : kSqrt2;
+    group_sync<W>(mask);
+    // ---- tridiagonalisation: v_k in column k below the diagonal, its factor
+    // beta_k on the diagonal, the update vector in row k above it
+#pragma unroll 1
+    for (int k = 0; k < kRed - 2; k++) {
+        const double x1 = H.full(k + 1, k);
+        double sg = 0;
+        for (int i = k + 2; i < kRed; i++) sg = fma(H.full(i, k), H.full(i, k), sg);
+        d[k] = H.full(k, k);
+        group_sync<W>(mask);
+        const double h = fma(x1, x1, sg);
+        if (!(sg > 0.0) || h < 1e-290) {
+            e[k] = x1;
+            if (g == 0) H.full(k, k) = 0;
+            group_sync<W>(mask);
+            continue;
+        }
+        const double r = __dmul_rn(h, rsqrt_refined(h));
+        e[k] = x1 > 0 ? -r : r;
+        const double v1 = x1 - e[k];
+        const double beta = 1.0 / fma(fabs(x1), r, h);
+        if (g == 0) {
+            H.full(k + 1, k) = v1;
+            H.full(k, k) = beta;
+        }
+        group_sync<W>(mask);
+        // p = beta A v, then w = p - (beta / 2 v^T p) v
+        for (int i = k + 1 + g; i < kRed; i += W) {
+            double a = 0;
+            for (int j = k + 1; j < kRed; j++) a = fma(i >= j ? H.full(i, j) : H.full(j, i), H.full(j, k), a);
+            H.full(k, i) = beta * a;
+        }
+        group_sync<W>(mask);
+        double vp = 0;
+        for (int i = k + 1; i < kRed; i++) vp = fma(H.full(i, k), H.full(k, i), vp);
+        group_sync<W>(mask);
+        const double K = 0.5 * beta * vp;
+        for (int i = k + 1 + g; i < kRed; i += W) H.full(k, i) = fma(-K, H.full(i, k), H.full(k, i));
+        group_sync<W>(mask);
+        for (int i = k + 1 + g; i < kRed; i += W) {
+            const double vi = H.full(i, k), wi = H.full(k, i);
+            for (int j = k + 1; j <= i; j++)
+                H.full(i, j) = fma(-vi, H.full(k, j), fma(-wi, H.full(j, k), H.full(i, j)));
+        }
+        group_sync<W>(mask);
+    }
+    d[kRed - 2] = H.full(kRed - 2, kRed - 2);
+    d[kRed - 1] = H.full(kRed - 1, kRed - 1);
+    e[kRed - 2] = H.full(kRed - 1, kRed - 2);
+    e[kRed - 1] = 0;
+    group_sync<W>(mask);
+    // ---- V = H_0 H_1 ... from the last reflection back, growing a row and
+    // a column at a time; lanes take columns
+    for (int r = kRed - 2 + g; r < kRed; r += W)
+        for (int c = kRed - 2; c < kRed; c++) H.full(r, c) = r == c ? 1.0 : 0.0;
+    group_sync<W>(mask);
+#pragma unroll 1
+    for (int k = kRed - 3; k >= 0; k--) {
+        const double beta = H.full(k, k);
+        for (int c = k + 1 + g; c < kRed; c += W) {
+            double a = 0;
+            for (int i = k + 1; i < kRed; i++) a = fma(H.full(i, k), H.full(i, c), a);
+            a *= beta;
+            for (int i = k + 1; i < kRed; i++) H.full(i, c) = fma(-a, H.full(i, k), H.full(i, c));
+        }
+        group_sync<W>(mask);
+        // row and column k become the identity's
+        for (int c = k + g; c < kRed; c += W) {
+            H.full(k, c) = c == k ? 1.0 : 0.0;
+            H.full(c, k) = c == k ? 1.0 : 0.0;
+        }
+        group_sync<W>(mask);
+    }
+    // ---- implicit QR on (d, e); an off-diagonal below rounding is set to
+    // zero; lanes rotate their rows of V
+    double norm = 0;
+    for (int k = 0; k < kRed; k++) norm += fabs(d[k]) + fabs(e[k]);
+    if (!(norm < INFINITY)) {
+        for (int r = g; r < kRed; r += W)
+            for (int c = 0; c <= r; c++) H.full(r, c) = norm - norm;  // NaN
+        group_sync<W>(mask);
         return;
     }
-    int a = k + round, b = 11 - k + round;
-    a = a >= 11 ? a - 11 : a;
-    b = b >= 11 ? b - 11 : b;
-    p = min(a, b);
-    q = max(a, b);
-}
-
-// row and column of upper-triangle entry u (row-major, 0 <= u < 78)
-__device__ __forceinline__ void upper_rc(int u, int& r, int& c)
-{
-    r = 0;
-    int start = 0;
-    while (u >= start + 12 - r) {
-        start += 12 - r;
-        r++;
+    // scaled by a power of two to a norm of [1, 2): the shifts are single
+    // precision; off-diagonals below 1e-17 of the norm are zero
+    const long long ex = (__double_as_longlong(norm) >> 52) & 0x7ff;
+    const bool scaled = ex > 0 && ex < 2046;
+    const double scale = scaled ? __longlong_as_double((2046 - ex) << 52) : 1.0;
+    const double unscale = scaled ? __longlong_as_double(ex << 52) : 1.0;
+    for (int k = 0; k < kRed; k++) {
+        d[k] *= scale;
+        e[k] *= scale;
     }
-    c = r + (u - start);
-}
-
-template <class T> __device__ __forceinline__ T warp_sum(T v)
-{
+    const double tiny = norm * scale * 1e-17;
+    for (int k = 0; k + 1 < kRed; k++)
+        if (fabs(e[k]) <= fma(1.1102230246251565e-16, fabs(d[k]) + fabs(d[k + 1]), tiny)) e[k] = 0;
+#pragma unroll 1
+    for (int step = 0; step < kQRSteps; step++) {
+        int q = kRed - 1;
+        while (q > 0 && (__double_as_longlong(e[q - 1]) << 1) == 0) q--;
+        if (q == 0) break;
+        int p = q - 1;
+        while (p > 0 && (__double_as_longlong(e[p - 1]) << 1) != 0) p--;
+        // the shift only steers the convergence: single precision
+        const float eq = (float)e[q - 1], dl = 0.5f * (float)(d[q - 1] - d[q]);
+        const float rt = sqrtf(fmaf(dl, dl, eq * eq));
+        const float den = dl + (dl >= 0.0f ? rt : -rt);
+        const double mu = d[q] - (double)(den != 0.0f ? __fdividef(eq, den) * eq : 0.0f);
+        double x = d[p] - mu, z = e[p];
+        double dk = d[p], ek = e[p];
+#pragma unroll 1
+        for (int k = p; k < q; k++) {
+            // rotation of (k, k + 1) that takes (x, z) to (r, 0)
+            const double h = fma(x, x, z * z);
+            double c = 1, s = 0;
+            if (h > 1e-290) {
+                const double ir = rsqrt_refined(h);
+                c = x * ir;
+                s = z * ir;
+                if (k > p) {
+                    const double r = h * ir;
+                    e[k - 1] = fabs(r) <= fma(1.1102230246251565e-16, fabs(d[k - 1]) + fabs(dk), tiny) ? 0.0 : r;
+                }
+            } else if (k > p) {
+                e[k - 1] = 0;
+            }
+            const double d1 = d[k + 1];
+            const double t = __dmul_rn(fma(s, dk - d1, -2.0 * c * ek), s);  // dk - new dk
+            const double cs = c * s, c2s2 = fma(c, c, -s * s);
+            const double en = fma(cs, d1 - dk, c2s2 * ek);
+            d[k] = dk - t;
+            dk = d1 + t;
+            d[k + 1] = dk;
+            if (k + 1 < q) {
+                z = s * e[k + 1];
+                ek = c * e[k + 1];
+                e[k + 1] = ek;
+            }
+            x = en;
+            e[k] = en;
+            for (int r = g; r < kRed; r += W) {
+                const double a = H.full(r, k), b = H.full(r, k + 1);
+                H.full(r, k) = fma(s, b, c * a);
+                H.full(r, k + 1) = fma(c, b, -s * a);
+            }
+        }
+        if (fabs(e[q - 1]) <= fma(1.1102230246251565e-16, fabs(d[q - 1]) + fabs(d[q]), tiny)) e[q - 1] = 0;
+    }
+    group_sync<W>(mask);
+    // ---- the matrix minus its negative part, A + V max(-L, 0) V^T, lower
+    // triangle: rounds relative to the negative part, and leaves a matrix
+    // with no negative eigenvalue as it is
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-
-__device__ __forceinline__ void jacobi_angle(float app, float aqq, float apq, float& c, float& s)
-{
-    const float theta = __fdividef(aqq - app, 2.0f * apq);
-    const float at = fabsf(theta);
-    // |theta| > 2^40: t = 1 / (2 theta) to single precision (and theta^2 is
-    // not formed)
-    float t;
-    if (at > 1.0995116e12f) {
-        t = __fdividef(0.5f, at);
-    } else {
-        const float h = fmaf(theta, theta, 1.0f);
-        t = __frcp_rn(at + h * rsqrtf(h));
-    }
-    t = theta >= 0.0f ? t : -t;
-    c = rsqrtf(fmaf(t, t, 1.0f));
-    s = t * c;
-}
-__device__ __forceinline__ void jacobi_angle(double app, double aqq, double apq, double& c, double& s)
-{
-    const double theta = (aqq - app) / (2 * apq);
-    const double t = (theta >= 0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(theta * theta + 1));
-    c = 1.0 / sqrt(t * t + 1);
-    s = t * c;
-}
-
-// Cyclic Jacobi on the warp's A (12 x kLd, symmetric) accumulating the
-// rotations into V, until the off-diagonal sum of squares is <= tol of the
-// diagonal's (or max_sweeps); cs holds 12 scalars of scratch.
-template <class T>
-__device__ void warp_jacobi(T* A, T* V, T* cs, int lane, T tol, int max_sweeps)
-{
-    for (int sweep = 0; sweep < max_sweeps; sweep++) {
-        T off = 0, diag = 0;
-        for (int e = lane; e < 144; e += 32) {
-            int r = e / 12, c = e % 12;
-            T v = A[r * kLd + c];
-            if (r == c) diag += v * v;
-            else if (r < c) off += v * v;
-        }
-        off = warp_sum(off);
-        diag = warp_sum(diag);
-        if (off <= tol * diag || off == T(0)) break;
-        for (int round = 0; round < 11; round++) {
-            if (lane < 6) {
-                int p, q;
-                round_pair(round, lane, p, q);
-                T apq = A[p * kLd + q];
-                T c = 1, sn = 0;
-                if (apq != T(0)) jacobi_angle(A[p * kLd + p], A[q * kLd + q], apq, c, sn);
-                cs[2 * lane] = c;
-                cs[2 * lane + 1] = sn;
-            }
-            __syncwarp();
-            // columns of A and V: 2 x 6 planes x 12 rows
-            for (int it = lane; it < 144; it += 32) {
-                T* M = it < 72 ? A : V;
-                int j = it < 72 ? it : it - 72;
-                int pr = j % 6, k = j / 6;
-                int p, q;
-                round_pair(round, pr, p, q);
-                T c = cs[2 * pr], sn = cs[2 * pr + 1];
-                T mkp = M[k * kLd + p], mkq = M[k * kLd + q];
-                M[k * kLd + p] = c * mkp - sn * mkq;
-                M[k * kLd + q] = sn * mkp + c * mkq;
-            }
-            __syncwarp();
-            // rows of A: 6 planes x 12 columns
-            for (int it = lane; it < 72; it += 32) {
-                int pr = it % 6, k = it / 6;
-                int p, q;
-                round_pair(round, pr, p, q);
-                T c = cs[2 * pr], sn = cs[2 * pr + 1];
-                T apk = A[p * kLd + k], aqk = A[q * kLd + k];
-                A[p * kLd + k] = c * apk - sn * aqk;
-                A[q * kLd + k] = sn * apk + c * aqk;
-            }
-            __syncwarp();
-        }
-    }
-}
-
-// C = op(X) Y for 12 x 12 matrices with row stride kLd (op(X) = X or X^T),
-// by the warp, entry-strided over the lanes
-__device__ __forceinline__ void warp_mm(const double* X, bool xt, const double* Y, double* C, int lane)
-{
-    for (int e = lane; e < 144; e += 32) {
-        const int r = e / 12, c = e % 12;
-        double acc = 0;
-        for (int k = 0; k < 12; k++) acc += (xt ? X[k * kLd + r] : X[r * kLd + k]) * Y[k * kLd + c];
-        C[r * kLd + c] = acc;
-    }
-    __syncwarp();
-}
-
-static __device__ void warp_psd_project(SMat H, double* work, int lane)
-{
-    double* A = work;               // the matrix
-    double* Q = work + 12 * kLd;    // eigenvectors
-    double* T = work + 24 * kLd;    // scratch, then B = Q^T A Q
-    double* U = work + 36 * kLd;    // scratch
-    double* cs = work + 48 * kLd;   // 6 x (c, s)
-    float* A32 = reinterpret_cast<float*>(work + 48 * kLd + 16);
-    float* V32 = A32 + 12 * kLd;
-    float* cs32 = V32 + 12 * kLd;
-    // 1. single-precision eigenvectors
-    for (int e = lane; e < 144; e += 32) {
-        int r = e / 12, c = e % 12;
-        const double a = r <= c ? H.at(r, c) : H.at(c, r);
-        A[r * kLd + c] = a;
-        A32[r * kLd + c] = (float)a;
-        V32[r * kLd + c] = r == c ? 1.0f : 0.0f;
-    }
-    __syncwarp();
-    warp_jacobi<float>(A32, V32, cs32, lane, 1e-14f, 12);
-    // 2. orthonormalise them in double (two Newton-Schulz steps
-    // Q <- Q (3 I - Q^T Q) / 2: the single-precision rotations leave them
-    // orthogonal to ~1e-6, each step squares that)
-    for (int e = lane; e < 144; e += 32) Q[(e / 12) * kLd + e % 12] = (double)V32[(e / 12) * kLd + e % 12];
-    __syncwarp();
-    for (int step = 0; step < 2; step++) {
-        warp_mm(Q, true, Q, T, lane);
-        for (int e = lane; e < 144; e += 32) {
-            const int r = e / 12, c = e % 12;
-            T[r * kLd + c] = (r == c ? 1.5 : 0.0) - 0.5 * T[r * kLd + c];
-        }
-        __syncwarp();
-        warp_mm(Q, false, T, U, lane);
-        for (int e = lane; e < 144; e += 32) Q[(e / 12) * kLd + e % 12] = U[(e / 12) * kLd + e % 12];
-        __syncwarp();
-    }
-    // 3. B = Q^T A Q (symmetric: the upper triangle, mirrored), then the
-    // double-precision Jacobi from there, the rotations accumulated into Q
-    warp_mm(A, false, Q, U, lane);
-    warp_mm(Q, true, U, T, lane);
-    for (int e = lane; e < 144; e += 32) {
-        const int r = e / 12, c = e % 12;
-        if (r > c) T[r * kLd + c] = T[c * kLd + r];
-    }
-    __syncwarp();
-    warp_jacobi<double>(T, Q, cs, lane, 1e-30, 30);
-    double wmin = INFINITY;
+    for (int i = 0; i < (kRed + W - 1) / W; i++) {
+        const int r = g + i * W;
+        if (r >= kRed) break;
+        double wz[kRed];
 #pragma unroll
-    for (int i = 0; i < 12; i++) wmin = fmin(wmin, T[i * kLd + i]);
-    if (wmin >= 0.0) return;  // already PSD: keep the matrix as it is
-    // rebuild the upper triangle: sum over positive eigenvalues
-    for (int u = lane; u < kSymEntries; u += 32) {
-        int r, c;
-        upper_rc(u, r, c);
-        double acc = 0;
-        for (int k = 0; k < 12; k++) {
-            const double w = T[k * kLd + k];
-            if (w > 0) acc += Q[r * kLd + k] * w * Q[c * kLd + k];
+        for (int k = 0; k < kRed; k++) wz[k] = fmax(-d[k] * unscale, 0.0) * H.full(r, k);
+#pragma unroll
+        for (int c = 0; c < kRed; c++) {
+            if (c > r) break;
+            double a = 0;
+#pragma unroll
+            for (int k = 0; k < kRed; k++) a = fma(wz[k], H.full(c, k), a);
+            keep[i][c] = fma(a, c >= 3 ? 1.0 : r < 3 ? 0.5 : 0.70710678118654757, keep[i][c]);
         }
-        H.at(r, c) = acc;
     }
-    __syncwarp();
+    group_sync<W>(mask);
+#pragma unroll
+    for (int i = 0; i < (kRed + W - 1) / W; i++) {
+        const int r = g + i * W;
+        if (r >= kRed) break;
+#pragma unroll
+        for (int c = 0; c < kRed; c++)
+            if (c <= r) H.full(r, c) = keep[i][c];
+    }
 }
 
-// local Hessian (symmetric from the upper triangle) to the outputs
-__device__ __forceinline__ void write_local_hessian(SMat H, int64_t ci, double* hess, double* blocks)
+// reduced index and sign of a row of the full 12x12
+__device__ __forceinline__ void full_row(int r, int& i, bool& neg)
 {
-    for (int r = 0; r < 12; r++)
-        for (int c = 0; c < 12; c++) {
-            double v = r <= c ? H.at(r, c) : H.at(c, r);
-            if (hess) hess[ci * 144 + 12 * r + c] = v;
-            if (blocks) {
-                int blk = (r / 6) * 2 + (c / 6);
-                blocks[ci * 144 + blk * 36 + (r % 6) * 6 + (c % 6)] = v;
+    neg = r >= 6 && r < 9;
+    i = r < 6 ? r : r < 9 ? r - 6 : r - 3;
+}
+
+// The warp writes the local Hessians of its `count` constraints from ci0 on
+// (slots 0 .. count - 1 of base; bit s of built: slot s holds one), 144
+// coalesced doubles each, to the full and the blocked output.
+__device__ __forceinline__ void write_local_hessians(const double* base, int stride, unsigned built, int64_t ci0,
+                                                     double* hess, double* blocks)
+{
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int o = 0; o < 2; o++) {
+        double* dst = o ? blocks : hess;
+        if (!dst) continue;
+        for (int k = lane; k < 144; k += 32) {
+            const int r = o ? (k / 72) * 6 + (k % 36) / 6 : k / 12;
+            const int c = o ? ((k / 36) & 1) * 6 + k % 6 : k % 12;
+            int i, j;
+            bool ni, nj;
+            full_row(r, i, ni);
+            full_row(c, j, nj);
+            const double* src = base + (size_t)(max(i, j) * kRed + min(i, j)) * stride;
+            for (unsigned b = built; b; b &= b - 1) {
+                const int s = __ffs(b) - 1;
+                const double v = src[s];
+                dst[(ci0 + s) * 144 + k] = ni != nj ? -v : v;
             }
         }
+    }
+}
+
+// One warp per block and per_warp constraints (a power of two) per warp: W =
+// min(16, 32 / per_warp) lanes to each.  The first lane of a group builds its
+// constraint's terms (build(ci, H): true when H holds a Hessian to project
+// and write), the group projects it, the warp writes it.
+template <int W, class Build>
+__device__ __forceinline__ void local_terms(int64_t n, int per_warp, int flags, double* hess, double* blocks,
+                                            double* smem, Build build)
+{
+    const int lane = threadIdx.x, slot = lane / W, g = lane % W;
+    const int64_t ci0 = (int64_t)blockIdx.x * per_warp, ci = ci0 + slot;
+    const int stride = per_warp | 1;
+    SMat H { smem + slot, stride };
+    const bool mine = g == 0 && slot < per_warp && ci < n;
+    const bool built = mine && build(ci, H);
+    if (!(flags & RIGC_HESS)) return;  // uniform over the block
+    const unsigned leaders = __ballot_sync(0xffffffffu, built);
+    const unsigned group = W == 32 ? 0xffffffffu : ((1u << (W & 31)) - 1u) << (slot * W);
+    __syncwarp();
+    if ((flags & RIGC_PROJECT_PSD) && ((leaders >> (slot * W)) & 1u)) psd_project<W>(H, g, group);
+    __syncwarp();
+    unsigned slots = 0;
+#pragma unroll
+    for (int s = 0; s < 32 / W; s++) slots |= ((leaders >> (s * W)) & 1u) << s;
+    write_local_hessians(smem, stride, slots, ci0, hess, blocks);
 }
 
 // Generic deterministic assembly of per-constraint body-space terms: cgrad
@@ -392,8 +490,8 @@ int assemble_terms(Ctx& c, const int* bodies, int64_t n, const double* cgrad,
                    const double* cblocks, DevBuf& grad, DevBuf& row_ptr, DevBuf& col,
                    DevBuf& val, int32_t* nseg_dev, bool with_hess);
 
-size_t local_terms_smem_bytes();
-int local_terms_per_warp(int64_t n);
+size_t local_terms_smem_bytes(int per_warp);
+int local_terms_per_warp(int64_t n, int tuned);
 int launch_body_frames(Ctx& c, const double* x);
 
 } // namespace rigc
