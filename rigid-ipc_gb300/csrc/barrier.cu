@@ -737,6 +737,87 @@ __global__ void k_seg_starts(const int32_t* __restrict__ head, const int32_t* __
     if (head[i]) seg_start[segid[i]] = (int32_t)i;
 }
 
+// the segment `seg` of key k, after one of key `before` (seg > 0): its
+// column, and the row pointers between the two rows
+__device__ __forceinline__ void block_segment(uint64_t k, uint64_t before, int32_t seg, int64_t start, int nb,
+                                              int32_t* __restrict__ seg_start, int32_t* __restrict__ col,
+                                              int32_t* __restrict__ row_ptr)
+{
+    seg_start[seg] = (int32_t)start;
+    const int32_t r = (int32_t)(k / (uint64_t)nb);
+    col[seg] = (int32_t)(k - (uint64_t)r * (uint64_t)nb);
+    for (int32_t q = seg ? (int32_t)(before / (uint64_t)nb) + 1 : 0; q <= r; q++) row_ptr[q] = seg;
+}
+
+// the same for the sorted Hessian block keys, with columns and row pointers
+__global__ void k_block_segs(const uint64_t* __restrict__ keys, const int32_t* __restrict__ head,
+                             const int32_t* __restrict__ segid, int64_t m, int nb,
+                             int32_t* __restrict__ seg_start, int32_t* __restrict__ col,
+                             int32_t* __restrict__ row_ptr)
+{
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= m) return;
+    if (head[i]) block_segment(keys[i], i ? keys[i - 1] : 0, segid[i], i, nb, seg_start, col, row_ptr);
+    if (i == m - 1)
+        for (int32_t q = (int32_t)(keys[i] / (uint64_t)nb) + 1; q <= nb; q++) row_ptr[q] = segid[i] + head[i];
+}
+
+// Few blocks: the sort of the keys by rank (the number of smaller keys, or
+// equal ones before; keys from the constraints' bodies as k_block_keys has
+// them), then the segments by one block; *nseg: their number.
+constexpr int kRankBlocks = 4096;
+
+__global__ void __launch_bounds__(128) k_rank_blocks(const int* __restrict__ bodies, int m, int nb,
+                                                     uint64_t* __restrict__ out, uint32_t* __restrict__ slots)
+{
+    __shared__ uint64_t sh[1024];
+    const auto key = [&](int i) {
+        const int c = i >> 2, blk = i & 3;
+        return (uint64_t)bodies[2 * c + (blk >> 1)] * (uint64_t)nb + (uint64_t)bodies[2 * c + (blk & 1)];
+    };
+    const int i = blockIdx.x * 128 + threadIdx.x;
+    const uint64_t k = i < m ? key(i) : 0;
+    int rank = 0;
+    for (int c = 0; c < m; c += 1024) {
+        const int n = min(1024, m - c);
+        for (int j = threadIdx.x; j < n; j += 128) sh[j] = key(c + j);
+        __syncthreads();
+        for (int j = 0; j < n; j++) rank += sh[j] < k || (sh[j] == k && c + j < i);
+        __syncthreads();
+    }
+    if (i >= m) return;
+    out[rank] = k;
+    slots[rank] = (uint32_t)i;
+}
+
+__global__ void __launch_bounds__(1024) k_block_segs_small(const uint64_t* __restrict__ keys, int m, int nb,
+                                                           int32_t* __restrict__ seg_start, int32_t* __restrict__ col,
+                                                           int32_t* __restrict__ row_ptr, int32_t* __restrict__ nseg)
+{
+    __shared__ int32_t warp_sum[32];
+    __shared__ int32_t carry;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (threadIdx.x == 0) carry = 0;
+    __syncthreads();
+    for (int base = 0; base < m; base += 1024) {
+        const int i = base + (int)threadIdx.x;
+        const bool head = i < m && (i == 0 || keys[i] != keys[i - 1]);
+        const unsigned b = __ballot_sync(0xffffffffu, head);
+        if (lane == 0) warp_sum[warp] = __popc(b);
+        __syncthreads();
+        int s = carry;
+        for (int w = 0; w < warp; w++) s += warp_sum[w];
+        s += __popc(b & ((1u << lane) - 1u));
+        if (head) block_segment(keys[i], i ? keys[i - 1] : 0, s, i, nb, seg_start, col, row_ptr);
+        __syncthreads();
+        if (threadIdx.x == 1023) carry = s + (head ? 1 : 0);
+        __syncthreads();
+    }
+    const int total = carry;
+    for (int32_t q = (int32_t)(keys[m - 1] / (uint64_t)nb) + 1 + (int)threadIdx.x; q <= nb; q += 1024) row_ptr[q] = total;
+    if (threadIdx.x == 0) *nseg = total;
+}
+
 // Sum of a segment's items by a block, one thread per (slice, entry): slice s
 // takes items s, s + S, ... in order, then the slices are added in order, so
 // the sum depends on the segment's items alone and one of at most S items is
@@ -749,13 +830,13 @@ __device__ __forceinline__ double segment_sum(int64_t s0, int64_t s1, double* pa
 {
     const int e = threadIdx.x % E, s = threadIdx.x / E;
     double acc = 0;
-    int64_t i = s0 + s;
+    int64_t i = s < S ? s0 + s : s1;
     for (; i + 3 * S < s1; i += 4 * S) {
         const double a = load(i, e), b = load(i + S, e), c = load(i + 2 * S, e), d = load(i + 3 * S, e);
         acc = (((acc + a) + b) + c) + d;
     }
     for (; i < s1; i += S) acc += load(i, e);
-    part[s * E + e] = acc;
+    if (s < S) part[s * E + e] = acc;
     __syncthreads();
     double sum = 0;
     if (s == 0) {
@@ -768,11 +849,14 @@ __device__ __forceinline__ double segment_sum(int64_t s0, int64_t s1, double* pa
 
 constexpr int kBlockSlices = 16, kGradSlices = 64;
 
-// blocks over the unique Hessian blocks
+// Blocks over the unique Hessian blocks.  A diagonal block's segment lists
+// its body's constraints (slot 4 c: its first body, 4 c + 3: its second) in the
+// order of the gradient's own segment, so its block sums the body's gradient
+// too.
 __global__ void __launch_bounds__(36 * kBlockSlices) k_block_sums(
     const uint64_t* __restrict__ keys, const uint32_t* __restrict__ slots, const int32_t* __restrict__ seg_start,
-    const int32_t* __restrict__ nseg_ptr, int64_t m, const double* __restrict__ blocks, int nb,
-    int32_t* __restrict__ col, double* __restrict__ val, int32_t* __restrict__ row_count)
+    const int32_t* __restrict__ nseg_ptr, int64_t m, const double* __restrict__ blocks,
+    const double* __restrict__ cgrad, int nb, double* __restrict__ val, double* __restrict__ grad)
 {
     __shared__ double part[36 * kBlockSlices];
     const int32_t nseg = *nseg_ptr;
@@ -781,11 +865,14 @@ __global__ void __launch_bounds__(36 * kBlockSlices) k_block_sums(
         const double sum = segment_sum<36, kBlockSlices>(
             s0, s1, part, [&](int64_t i, int e) { return blocks[(size_t)slots[i] * 36 + e]; });
         if (threadIdx.x < 36) val[(size_t)sgi * 36 + threadIdx.x] = sum;
-        if (threadIdx.x == 0) {
-            const uint64_t k = keys[s0];
-            col[sgi] = (int32_t)(k % (uint64_t)nb);
-            atomicAdd(&row_count[(int32_t)(k / (uint64_t)nb)], 1);
-        }
+        const uint64_t k = keys[s0];
+        const uint32_t row = (uint32_t)(k / (uint64_t)nb);
+        if (k != (uint64_t)row * (uint64_t)nb + row) continue;  // uniform over the block
+        const double g = segment_sum<6, kGradSlices>(s0, s1, part, [&](int64_t i, int e) {
+            const uint32_t slot = slots[i];
+            return cgrad[(size_t)(slot >> 2) * 12 + 6 * ((slot & 3) == 3) + e];
+        });
+        if (threadIdx.x < 6) grad[(size_t)row * 6 + threadIdx.x] = g;
     }
 }
 
@@ -820,8 +907,8 @@ int assemble_terms(Ctx& c, const int* bodies, int64_t n, const double* cgrad,
     // scratch usage: 0 keys_in, 1 vals_in, 2 keys_out, 3 vals_out, 4/5 sort tmp,
     // 6 hist/scan tmp, 7 head/segid/seg_start
     DevBuf* S = c.scratch;
-    // ---- gradient
-    {
+    if (!with_hess) {
+        // the gradient alone, by body
         int64_t m = 2 * n;
         RIGC_TRY(S[0].reserve(m * 4));
         RIGC_TRY(S[1].reserve(m * 4));
@@ -848,45 +935,47 @@ int assemble_terms(Ctx& c, const int* bodies, int64_t n, const double* cgrad,
         k_grad_sums<<<(unsigned)std::min<int64_t>(m, kNumSMs * 4), 6 * kGradSlices, 0, st>>>(
             S[2].as<uint32_t>(), S[3].as<uint32_t>(), segst, nseg_dev, m, cgrad,
             grad.as<double>());
+        return RIGC_OK;
     }
-    if (!with_hess) return RIGC_OK;
-    // ---- Hessian blocks
-    {
-        int64_t m = 4 * n;
+    const int64_t m = 4 * n;
+    RIGC_TRY(S[2].reserve(m * 8));
+    RIGC_TRY(S[3].reserve(m * 4));
+    RIGC_TRY(S[7].reserve(m * 12 + 16));
+    // capacity for the upper bound m blocks: no host round trip here
+    RIGC_TRY(col.reserve((size_t)m * sizeof(int32_t)));
+    RIGC_TRY(val.reserve((size_t)m * 36 * sizeof(double)));
+    int32_t* head = S[7].as<int32_t>();
+    int32_t* segid = head + m;
+    int32_t* segst = segid + m;
+    int32_t* nseg_dev = nseg_dev_pair + 1;  // read back by the caller
+    if (m <= kRankBlocks) {
+        RIGC_COUNT_LAUNCH();
+        k_rank_blocks<<<grid_for(m, 128), 128, 0, st>>>(bodies, (int)m, nb, S[2].as<uint64_t>(),
+                                                        S[3].as<uint32_t>());
+        RIGC_COUNT_LAUNCH();
+        k_block_segs_small<<<1, 1024, 0, st>>>(S[2].as<uint64_t>(), (int)m, nb, segst, col.as<int32_t>(),
+                                               row_ptr.as<int32_t>(), nseg_dev);
+    } else {
         RIGC_TRY(S[0].reserve(m * 8));
         RIGC_TRY(S[1].reserve(m * 4));
-        RIGC_TRY(S[2].reserve(m * 8));
-        RIGC_TRY(S[3].reserve(m * 4));
-        RIGC_TRY(S[7].reserve(m * 12 + 16));
         RIGC_COUNT_LAUNCH();
         k_block_keys<<<grid_for(m, 256), 256, 0, st>>>(bodies, n, nb,
                                                       S[0].as<uint64_t>(), S[1].as<uint32_t>());
         RIGC_TRY(radix_sort_pairs<uint64_t>(S[0].as<uint64_t>(), S[1].as<uint32_t>(),
                                             S[2].as<uint64_t>(), S[3].as<uint32_t>(), m,
                                             bits_for((uint64_t)nb * nb), S[4], S[5], S[6], st));
-        int32_t* head = S[7].as<int32_t>();
-        int32_t* segid = head + m;
-        int32_t* segst = segid + m;
         RIGC_COUNT_LAUNCH();
         k_heads<uint64_t><<<grid_for(m, 256), 256, 0, st>>>(S[2].as<uint64_t>(), m, head);
-        int32_t* nseg_dev = nseg_dev_pair + 1;  // read back by the caller
         RIGC_TRY(exclusive_scan_i32(head, segid, m, nseg_dev, S[6], st));
         RIGC_COUNT_LAUNCH();
-        k_seg_starts<<<grid_for(m, 256), 256, 0, st>>>(head, segid, m, segst);
-        // capacity for the upper bound m blocks: no host round trip here
-        RIGC_TRY(col.reserve((size_t)m * sizeof(int32_t)));
-        RIGC_TRY(val.reserve((size_t)m * 36 * sizeof(double)));
-        RIGC_COUNT_LAUNCH();
-        k_block_sums<<<(unsigned)std::min<int64_t>(m, kNumSMs * 3), 36 * kBlockSlices, 0, st>>>(
-            S[2].as<uint64_t>(), S[3].as<uint32_t>(), segst, nseg_dev, m, cblocks, nb,
-            col.as<int32_t>(), val.as<double>(), row_ptr.as<int32_t>() + 1);
-        // row counts -> row_ptr (exclusive scan of counts shifted by one)
-        int32_t* rp = row_ptr.as<int32_t>();
-        RIGC_TRY(S[4].reserve((size_t)(nb + 1) * sizeof(int32_t)));
-        RIGC_CUDA(cudaMemcpyAsync(S[4].ptr, rp + 1, (size_t)nb * sizeof(int32_t),
-                                  cudaMemcpyDeviceToDevice, st));
-        RIGC_TRY(exclusive_scan_i32(S[4].as<int32_t>(), rp, nb, rp + nb, S[6], st));
+        k_block_segs<<<grid_for(m, 256), 256, 0, st>>>(S[2].as<uint64_t>(), head, segid, m, nb, segst,
+                                                       col.as<int32_t>(), row_ptr.as<int32_t>());
     }
+    RIGC_COUNT_LAUNCH();
+    k_block_sums<<<(unsigned)std::min<int64_t>(m, kNumSMs * 3), 36 * kBlockSlices, 0, st>>>(
+        S[2].as<uint64_t>(), S[3].as<uint32_t>(), segst, nseg_dev, m, cblocks, cgrad, nb, val.as<double>(),
+        grad.as<double>());
+    RIGC_CUDA(cudaGetLastError());
     return RIGC_OK;
 }
 

@@ -33,6 +33,8 @@
 //       elements of their scene instead of being binned.
 //     The output is the same set, sorted: ee as (edge0 < edge1), fv as
 //     (face, vertex).
+//     Small scenes skip the grid: every pair of elements is tested, tile by
+//     tile (k_all_pairs).
 #include "common.cuh"
 #include "interval.cuh"
 #include "sort.cuh"
@@ -399,7 +401,8 @@ __global__ void k_vertex_boxes_half(const double* __restrict__ rest, const int* 
     vin[v] = ok ? 1 : 0;
 }
 
-__global__ void k_vertex_boxes_disc(const double* __restrict__ rot, const double* __restrict__ rest,
+__global__ void k_vertex_boxes_disc(const double* __restrict__ x, const double* __restrict__ rot,
+                                    const double* __restrict__ rest,
                                     const int* __restrict__ vbody, const int* __restrict__ body_in,
                                     int nv, double infl, double* __restrict__ vbox,
                                     char* __restrict__ vin)
@@ -411,13 +414,18 @@ __global__ void k_vertex_boxes_disc(const double* __restrict__ rot, const double
         vin[v] = 0;
         return;
     }
-    const double* f = rot + 12 * b;
     double R[9], p[3], r[3], w[3];
-    for (int k = 0; k < 9; k++) R[k] = f[k];
-    for (int k = 0; k < 3; k++) {
-        p[k] = f[9 + k];
-        r[k] = rest[3 * (size_t)v + k];
+    if (rot) {
+        const double* f = rot + 12 * b;
+        for (int k = 0; k < 9; k++) R[k] = f[k];
+        for (int k = 0; k < 3; k++) p[k] = f[9 + k];
+    } else {
+        // few vertices: the rotation here instead of in a launch of its own
+        const double t[3] = { x[6 * b + 3], x[6 * b + 4], x[6 * b + 5] };
+        rot_rn(t, R);
+        for (int k = 0; k < 3; k++) p[k] = x[6 * b + k];
     }
+    for (int k = 0; k < 3; k++) r[k] = rest[3 * (size_t)v + k];
     world_vertex_rn(R, p, r, w);
     for (int j = 0; j < 3; j++) {
         vbox[6 * (size_t)v + j] = RSUB(w[j], infl);
@@ -1008,6 +1016,170 @@ __global__ void k_large_pairs(const uint32_t* __restrict__ large, int nl, int ro
     }
 }
 
+// ---------------------------------------------------------------------------
+// Small scenes: all pairs.  The grid only limits which pairs are tested, and
+// below some 10^5 elements its kernels (statistics, set-up, cell filter, items,
+// sort: ten launches, most of them a few threads' latency) and the item
+// count's read-back cost more than testing every pair.  Elements come in tiles
+// of kTile of one kind, with the tile's box; a block takes a pair of tiles and
+// ends at once when their boxes are apart.
+// Measured (one discrete call, with the grid -> all pairs): 27 cubes (491 edges,
+// 16 pairs of tiles) 290 -> 150 us, 10 icospheres (19 k edges, 17 k pairs) 366
+// -> 169, 25 icospheres (48 k, 103 k) 386 -> 253, 40 icospheres (77 k, 262 k) 427
+// -> 376, 8 slabs (61 k, 168 k) 607 -> 617, 80 icospheres (154 k, 1 M) 479 -> 792:
+// the lines cross between 10^5 and 3 10^5 pairs of tiles.
+
+constexpr int kTile = 128;
+constexpr int64_t kAllPairsTiles = 1 << 17;  // tile pairs up to which all pairs are tested
+
+struct ElemBox {
+    float b[6];     // rounded outward; empty (+inf, -inf) for elements not included
+    int gr, scene;  // group rank, scene
+};
+
+__host__ __device__ __forceinline__ int tiles_of(int n) { return (n + kTile - 1) / kTile; }
+
+// A block per tile (vertices, then edges, then faces): the edges' and faces'
+// boxes (as k_edge_face_boxes), every element's ElemBox, the tile's box.
+__global__ void __launch_bounds__(kTile) k_tile_boxes(
+    const int* __restrict__ Ed, const int* __restrict__ Fa, Elems E, const int* __restrict__ bscene,
+    const int* __restrict__ grank, double* __restrict__ ebox, char* __restrict__ ein, double* __restrict__ fbox,
+    char* __restrict__ fin, ElemBox* __restrict__ out, float* __restrict__ tile_box)
+{
+    __shared__ float sh[kTile / 32][6];
+    const int tv = tiles_of(E.nv), te = tiles_of(E.ne);
+    const int t = (int)blockIdx.x < tv ? 0 : (int)blockIdx.x < tv + te ? 1 : 2;
+    const int i = ((int)blockIdx.x - (t == 0 ? 0 : t == 1 ? tv : tv + te)) * kTile + threadIdx.x;
+    const int n = t == 0 ? E.nv : t == 1 ? E.ne : E.nf;
+    float b[6] = { INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY };
+    if (i < n) {
+        const int m = t + 1;  // the element's vertices
+        int v[3] = { i, i, i };
+        if (t == 1) {
+            v[0] = Ed[2 * i];
+            v[1] = Ed[2 * i + 1];
+        } else if (t == 2) {
+            for (int k = 0; k < 3; k++) v[k] = Fa[3 * i + k];
+        }
+        bool in = true;
+        for (int k = 0; k < m; k++) in = in && E.vin[v[k]];
+        if (t == 1) ein[i] = in;
+        if (t == 2) fin[i] = in;
+        if (in)
+            for (int j = 0; j < 3; j++) {
+                double lo = E.vb[6 * (size_t)v[0] + j], hi = E.vb[6 * (size_t)v[0] + 3 + j];
+                for (int k = 1; k < m; k++) {
+                    lo = smin(lo, E.vb[6 * (size_t)v[k] + j]);
+                    hi = smax(hi, E.vb[6 * (size_t)v[k] + 3 + j]);
+                }
+                if (t > 0) {
+                    double* o = (t == 1 ? ebox : fbox) + 6 * (size_t)i;
+                    o[j] = lo;
+                    o[3 + j] = hi;
+                }
+                b[j] = __double2float_rd(lo);
+                b[3 + j] = __double2float_ru(hi);
+            }
+        const int body = E.body(t, i);
+        ElemBox r;
+        for (int j = 0; j < 6; j++) r.b[j] = b[j];
+        r.gr = grank[body];
+        r.scene = bscene[body];
+        out[E.index(t, i)] = r;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int j = 0; j < 3; j++) {
+            b[j] = fminf(b[j], __shfl_xor_sync(0xffffffffu, b[j], o));
+            b[3 + j] = fmaxf(b[3 + j], __shfl_xor_sync(0xffffffffu, b[3 + j], o));
+        }
+    if ((threadIdx.x & 31) == 0)
+        for (int j = 0; j < 6; j++) sh[threadIdx.x >> 5][j] = b[j];
+    __syncthreads();
+    if (threadIdx.x < 6) {
+        const int j = threadIdx.x;
+        float x = sh[0][j];
+        for (int w = 1; w < kTile / 32; w++) x = j < 3 ? fminf(x, sh[w][j]) : fmaxf(x, sh[w][j]);
+        tile_box[6 * blockIdx.x + j] = x;
+    }
+}
+
+// A block per pair of tiles: edges with edges (tiles a <= b), then faces with
+// vertices, or (kPairsEF) faces with edges alone.
+__global__ void __launch_bounds__(kTile) k_all_pairs(Elems E, int kind, const ElemBox* __restrict__ eb,
+                                                     const float* __restrict__ tile_box, PairOut o)
+{
+    __shared__ ElemBox sh[kTile];
+    const int tv = tiles_of(E.nv), te = tiles_of(E.ne);
+    int p = blockIdx.x, ta, tb, a, b;  // kinds and tiles
+    const int nee = kind == kPairsEF ? 0 : te * (te + 1) / 2;
+    if (p < nee) {
+        // row b of the triangle holds tiles a = 0 .. b
+        ta = tb = 1;
+        b = (int)((sqrtf(8.0f * (float)p + 1.0f) - 1.0f) * 0.5f);
+        while ((b + 1) * (b + 2) / 2 <= p) b++;
+        while (b * (b + 1) / 2 > p) b--;
+        a = p - b * (b + 1) / 2;
+    } else {
+        p -= nee;
+        ta = 2;
+        tb = kind == kPairsEF ? 1 : 0;
+        const int cols = tb ? te : tv;
+        a = p / cols;
+        b = p % cols;
+    }
+    const int first[3] = { 0, tv, tv + te };
+    if (fboxes_disjoint(tile_box + 6 * (first[ta] + a), tile_box + 6 * (first[tb] + b))) return;
+    const int ia = a * kTile + threadIdx.x, ib0 = b * kTile;
+    const int na = ta == 1 ? E.ne : E.nf, nb = tb == 0 ? E.nv : E.ne;
+    ElemBox mine;
+    mine.b[0] = INFINITY;
+    if (ia < na) mine = eb[E.index(ta, ia)];
+    ElemBox other;
+    other.b[0] = INFINITY;
+    if (ib0 + (int)threadIdx.x < nb) other = eb[E.index(tb, ib0 + threadIdx.x)];
+    sh[threadIdx.x] = other;
+    __syncthreads();
+    if (mine.b[0] == INFINITY) return;
+    const int end = min(kTile, nb - ib0);
+    for (int j = 0; j < end; j++) {
+        const ElemBox& x = sh[j];
+        if (x.gr == mine.gr || x.scene != mine.scene || fboxes_disjoint(mine.b, x.b)) continue;
+        if (ta == 1 && tb == 1 && ib0 + j <= ia) continue;
+        exact_pair(E, ta, ia, tb, ib0 + j, o);
+    }
+}
+
+// The canonical order of few pairs: each stream's keys are distinct, so a
+// pair's place is the number of smaller keys (4096 pairs: some 10 us in one
+// launch, against five for the buckets).
+constexpr int kRankPairs = 4096;
+
+__global__ void __launch_bounds__(128) k_rank_pairs(const unsigned long long* __restrict__ kee, int nee,
+                                                    const unsigned long long* __restrict__ kfv, int nfv,
+                                                    unsigned long long ee_stride, unsigned long long fv_stride,
+                                                    int2* __restrict__ out_ee, int2* __restrict__ out_fv)
+{
+    __shared__ unsigned long long sh[1024];
+    const int be = (nee + 127) / 128;  // blocks of the first stream
+    const bool ee = (int)blockIdx.x < be;
+    const unsigned long long* keys = ee ? kee : kfv;
+    const int n = ee ? nee : nfv, i = ((int)blockIdx.x - (ee ? 0 : be)) * 128 + threadIdx.x;
+    const unsigned long long k = i < n ? keys[i] : 0;
+    int rank = 0;
+    for (int c = 0; c < n; c += 1024) {
+        const int m = min(1024, n - c);
+        for (int j = threadIdx.x; j < m; j += 128) sh[j] = keys[c + j];
+        __syncthreads();
+        for (int j = 0; j < m; j++) rank += sh[j] < k;
+        __syncthreads();
+    }
+    if (i >= n) return;
+    const unsigned long long stride = ee ? ee_stride : fv_stride;
+    (ee ? out_ee : out_fv)[rank] = make_int2((int)(k / stride), (int)(k % stride));
+}
+
 // the two pair streams as one array of sort keys: EE keys as they are, FV
 // keys with bit tbit set (above every key of either stream), values 0 .. n-1
 __global__ void k_pack_pairs(const unsigned long long* __restrict__ kee, int64_t nee,
@@ -1187,6 +1359,7 @@ __global__ void k_iota(uint32_t* __restrict__ v, int64_t n)
 
 // ---------------------------------------------------------------------------
 
+constexpr int kDirectVertices = 16384;  // as compute_world_vertices_rn has it
 int body_rot_rn(Ctx& c, const double* x, double* out);
 int reserve_rot_table(Ctx& c);
 
@@ -1269,25 +1442,49 @@ int detect_pairs(Ctx& c, const double* x0, const double* x1, bool continuous, do
             x0, x1, s.rest, s.bvs, c.body_in.as<int>(), c.bp_deeper.as<int>(), table, d_domain,
             infl, c.vbox.as<double>(), c.vin.as<char>());
     } else {
-        RIGC_TRY(S[0].reserve((size_t)12 * s.nb * sizeof(double)));
-        RIGC_TRY(body_rot_rn(c, x0, S[0].as<double>()));
+        const double* rot = nullptr;
+        if (s.nv > kDirectVertices) {
+            RIGC_TRY(S[0].reserve((size_t)12 * s.nb * sizeof(double)));
+            RIGC_TRY(body_rot_rn(c, x0, S[0].as<double>()));
+            rot = S[0].as<double>();
+        }
         RIGC_COUNT_LAUNCH();
-        k_vertex_boxes_disc<<<grid_for(s.nv, 256), 256, 0, st>>>(
-            S[0].as<double>(), s.rest, s.vbody, c.body_in.as<int>(), s.nv, infl, c.vbox.as<double>(),
+        k_vertex_boxes_disc<<<grid_for(s.nv, 128), 128, 0, st>>>(
+            x0, rot, s.rest, s.vbody, c.body_in.as<int>(), s.nv, infl, c.vbox.as<double>(),
             c.vin.as<char>());
     }
-    RIGC_COUNT_LAUNCH();
-    k_edge_face_boxes<<<grid_for((int64_t)s.ne + s.nf, 256), 256, 0, st>>>(
-        s.edges, s.ne, s.faces, s.nf, c.vbox.as<double>(), c.vin.as<char>(), c.ebox.as<double>(),
-        c.ein.as<char>(), c.fbox.as<double>(), c.fin.as<char>());
-    RIGC_CUDA(cudaGetLastError());
     const Elems E { c.vbox.as<double>(), c.ebox.as<double>(), c.fbox.as<double>(),
                     c.vin.as<char>(), c.ein.as<char>(), c.fin.as<char>(),
                     s.vbody, s.ebody, s.fbody, s.nv, s.ne, s.nf };
+    const int64_t tv = tiles_of(s.nv), te = tiles_of(s.ne), tf = tiles_of(s.nf);
+    const int64_t tile_pairs = kind == kPairsEF ? tf * te : te * (te + 1) / 2 + tf * tv;
+    const bool all_pairs = tile_pairs <= kAllPairsTiles;
+    if (!all_pairs) {
+        RIGC_COUNT_LAUNCH();
+        k_edge_face_boxes<<<grid_for((int64_t)s.ne + s.nf, 256), 256, 0, st>>>(
+            s.edges, s.ne, s.faces, s.nf, c.vbox.as<double>(), c.vin.as<char>(), c.ebox.as<double>(),
+            c.ein.as<char>(), c.fbox.as<double>(), c.fin.as<char>());
+        RIGC_CUDA(cudaGetLastError());
+    }
+    int64_t nitems = 0;
+    int nlarge = 0;
+    int group_key_bits = 0;
+    const uint64_t nslots = filter_slots(ntot);
+    ElemBox* elem_boxes = nullptr;
+    float* tile_boxes = nullptr;
+    if (all_pairs) {
+        RIGC_TRY(c.bp_f32.reserve((size_t)ntot * sizeof(ElemBox) + (size_t)(tv + te + tf) * 6 * sizeof(float) + 8));
+        elem_boxes = c.bp_f32.as<ElemBox>();
+        tile_boxes = reinterpret_cast<float*>(elem_boxes + ntot);
+        RIGC_COUNT_LAUNCH();
+        k_tile_boxes<<<(unsigned)(tv + te + tf), kTile, 0, st>>>(
+            s.edges, s.faces, E, s.bscene, s.grank, c.ebox.as<double>(), c.ein.as<char>(), c.fbox.as<double>(),
+            c.fin.as<char>(), elem_boxes, tile_boxes);
+        RIGC_CUDA(cudaGetLastError());
+    } else {
     // ---- 3. grid and cell filter
     RIGC_COUNT_LAUNCH();
     k_elem_stats<<<kStatBlocks, kStatThreads, 0, st>>>(E, d_part, d_part_n);
-    const uint64_t nslots = filter_slots(ntot);
     RIGC_COUNT_LAUNCH();
     k_grid_setup<<<1, 32, 0, st>>>(d_part, d_part_n, kStatBlocks, s.avg_edge_len, s.nscenes,
                                    s.group_bits, nslots, d_grid);
@@ -1316,8 +1513,9 @@ int detect_pairs(Ctx& c, const double* x0, const double* x1, bool continuous, do
     RIGC_CUDA(cudaMemcpyAsync(counts, d_count, sizeof(counts), cudaMemcpyDeviceToHost, st));
     RIGC_CUDA(cudaMemcpyAsync(&hg, d_grid, sizeof(Grid), cudaMemcpyDeviceToHost, st));
     RIGC_CUDA(cudaStreamSynchronize(st));
-    const int64_t nitems = counts[0];
-    const int nlarge = counts[1];
+    nitems = counts[0];
+    nlarge = counts[1];
+    group_key_bits = hg.key_bits + s.group_bits + 3;
     c.stats.grid_items = nitems;
     c.stats.large_elements = nlarge;
     // ---- 4. items of the marked cells, sorted
@@ -1333,12 +1531,13 @@ int detect_pairs(Ctx& c, const double* x0, const double* x1, bool continuous, do
             c.items_val.as<uint32_t>());
         RIGC_TRY(radix_sort_pairs<uint64_t>(c.items_key.as<uint64_t>(), c.items_val.as<uint32_t>(),
                                             c.items_key2.as<uint64_t>(), c.items_val2.as<uint32_t>(),
-                                            nitems, hg.key_bits + s.group_bits + 3, S[4], S[5], S[7],
+                                            nitems, group_key_bits, S[4], S[5], S[7],
                                             st));
+    }
     }
     // ---- 5. pairs (retry once with exact capacity on overflow)
     unsigned long long* pn = reinterpret_cast<unsigned long long*>(c.d_scalars.as<char>() + 1024);
-    unsigned long long cap_ee = std::max<unsigned long long>(1 << 16, (unsigned long long)nitems);
+    unsigned long long cap_ee = std::max<unsigned long long>(1 << 16, (unsigned long long)(all_pairs ? 32 * ntot : nitems));
     unsigned long long cap_fv = cap_ee;
     cap_ee = std::max<unsigned long long>(cap_ee, (unsigned long long)c.bp_pair_hint[0]);
     cap_fv = std::max<unsigned long long>(cap_fv, (unsigned long long)c.bp_pair_hint[1]);
@@ -1348,6 +1547,10 @@ int detect_pairs(Ctx& c, const double* x0, const double* x1, bool continuous, do
         PairOut o { c.pair_out.as<unsigned long long>(), c.pair_out.as<unsigned long long>() + cap_ee,
                     cap_ee, cap_fv, pn, pn + 1 };
         RIGC_CUDA(cudaMemsetAsync(pn, 0, 2 * sizeof(unsigned long long), st));
+        if (all_pairs) {
+            RIGC_COUNT_LAUNCH();
+            k_all_pairs<<<(unsigned)tile_pairs, kTile, 0, st>>>(E, kind, elem_boxes, tile_boxes, o);
+        }
         if (nitems > 0) {
             RIGC_COUNT_LAUNCH();
             k_cell_pairs<<<grid_for(nitems, 128), 128, 0, st>>>(
@@ -1396,7 +1599,12 @@ int detect_pairs(Ctx& c, const double* x0, const double* x1, bool continuous, do
                               bits_for((uint64_t)s.nf * fv_stride));
     const int64_t np = nee + nfv;
     const int64_t nbuckets = (int64_t)s.ne + s.nf;
-    if (np > 0 && np < (int64_t)INT32_MAX && nbuckets < (int64_t)INT32_MAX) {
+    if (np > 0 && np <= kRankPairs) {
+        RIGC_COUNT_LAUNCH();
+        k_rank_pairs<<<(unsigned)((nee + 127) / 128 + (nfv + 127) / 128), 128, 0, st>>>(
+            kee, (int)nee, kfv, (int)nfv, (unsigned long long)s.ne, fv_stride, out.ee.as<int2>(),
+            out.fv.as<int2>());
+    } else if (np > 0 && np < (int64_t)INT32_MAX && nbuckets < (int64_t)INT32_MAX) {
         // by buckets of the first element
         RIGC_TRY(S[0].reserve((size_t)2 * nbuckets * sizeof(int32_t)));
         RIGC_TRY(S[1].reserve((size_t)(nbuckets + np) * sizeof(int32_t)));

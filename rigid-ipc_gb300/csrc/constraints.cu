@@ -14,6 +14,9 @@
 
 namespace rigc {
 
+// vertices up to which a thread per vertex computes its body's rotation
+constexpr int kDirectVertices = 16384;
+
 // per-body R (9) and p (3), exact round-to-nearest evaluation
 __global__ void k_body_rot_rn(const double* __restrict__ x, int nb, double* __restrict__ out)
 {
@@ -47,6 +50,23 @@ __global__ void k_world_vertices_rn(const double* __restrict__ rest, const int* 
     V[3 * (size_t)i + 2] = o[2];
 }
 
+// few vertices: one launch, a thread per vertex computing its body's rotation
+// itself (the chain of the rotation is the latency of k_body_rot_rn either
+// way; 16 k vertices' FP64 is some 7 us of the GPU)
+__global__ void k_world_vertices_direct(const double* __restrict__ rest, const int* __restrict__ vbody, int nv,
+                                        const double* __restrict__ x, double* __restrict__ V)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= nv) return;
+    const double* q = x + 6 * (size_t)vbody[i];
+    const double t[3] = { q[3], q[4], q[5] }, p[3] = { q[0], q[1], q[2] };
+    const double v[3] = { rest[3 * (size_t)i], rest[3 * (size_t)i + 1], rest[3 * (size_t)i + 2] };
+    double R[9], o[3];
+    rot_rn(t, R);
+    world_vertex_rn(R, p, v, o);
+    for (int k = 0; k < 3; k++) V[3 * (size_t)i + k] = o[k];
+}
+
 int body_rot_rn(Ctx& c, const double* x, double* out)
 {
     RIGC_COUNT_LAUNCH();
@@ -57,6 +77,12 @@ int body_rot_rn(Ctx& c, const double* x, double* out)
 
 int compute_world_vertices_rn(Ctx& c, const double* x, double* V, DevBuf& rotbuf)
 {
+    if (c.s.nv <= kDirectVertices) {
+        RIGC_COUNT_LAUNCH();
+        k_world_vertices_direct<<<grid_for(c.s.nv, 64), 64, 0, c.stream>>>(c.s.rest, c.s.vbody, c.s.nv, x, V);
+        RIGC_CUDA(cudaGetLastError());
+        return RIGC_OK;
+    }
     RIGC_TRY(rotbuf.reserve((size_t)12 * c.s.nb * sizeof(double)));
     RIGC_COUNT_LAUNCH();
     k_body_rot_rn<<<grid_for(c.s.nb, 128), 128, 0, c.stream>>>(x, c.s.nb, rotbuf.as<double>());
@@ -186,36 +212,55 @@ __device__ __forceinline__ bool classify(int64_t i, int64_t nee, const int2* __r
     return true;
 }
 
-__global__ void k_classify_count(int64_t n, int64_t nee, const int2* __restrict__ ee,
-                                 const int2* __restrict__ fv, const int* __restrict__ E,
-                                 const int* __restrict__ F, const int* __restrict__ F2E,
-                                 const double* __restrict__ V, double off,
-                                 int32_t* __restrict__ flag)
+// One pass: the active candidates' records, appended in any order (the
+// records of a key are the same whatever candidate they come from, and the
+// sort below orders the keys).  key = kind (2 bits) | p0 (30) | p1 (30)
+__global__ void k_classify(int64_t n, int64_t nee, const int2* __restrict__ ee,
+                           const int2* __restrict__ fv, const int* __restrict__ E,
+                           const int* __restrict__ F, const int* __restrict__ F2E,
+                           const double* __restrict__ V, double off, uint64_t* __restrict__ keys,
+                           uint32_t* __restrict__ idx, int4* __restrict__ rverts,
+                           double* __restrict__ reps, int32_t* __restrict__ count)
 {
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     Raw r;
-    flag[i] = classify(i, nee, ee, fv, E, F, F2E, V, off, r) ? 1 : 0;
-}
-
-// key = kind (2 bits) | p0 (30 bits) | p1 (30 bits)
-__global__ void k_classify_write(int64_t n, int64_t nee, const int2* __restrict__ ee,
-                                 const int2* __restrict__ fv, const int* __restrict__ E,
-                                 const int* __restrict__ F, const int* __restrict__ F2E,
-                                 const double* __restrict__ V, double off,
-                                 const int32_t* __restrict__ flag, const int32_t* __restrict__ pos,
-                                 uint64_t* __restrict__ keys, uint32_t* __restrict__ idx,
-                                 int4* __restrict__ rverts, double* __restrict__ reps)
-{
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n || !flag[i]) return;
-    Raw r;
-    classify(i, nee, ee, fv, E, F, F2E, V, off, r);
-    int32_t o = pos[i];
+    const bool active = i < n && classify(i, nee, ee, fv, E, F, F2E, V, off, r);
+    const unsigned m = __ballot_sync(0xffffffffu, active);
+    if (!m) return;
+    const int lane = threadIdx.x & 31;
+    int32_t o = 0;
+    if (lane == 0) o = atomicAdd(count, __popc(m));
+    o = __shfl_sync(0xffffffffu, o, 0) + __popc(m & ((1u << lane) - 1u));
+    if (!active) return;
     keys[o] = ((uint64_t)r.kind << 60) | ((uint64_t)(uint32_t)r.p0 << 30) | (uint64_t)(uint32_t)r.p1;
     idx[o] = (uint32_t)o;
     rverts[o] = make_int4(r.v[0], r.v[1], r.v[2], r.v[3]);
     reps[o] = r.eps;
+}
+
+// Few records: a record's place is the number of smaller keys (equal keys
+// hold equal records, in the order of their slots).
+constexpr int kRankRecords = 4096;
+
+__global__ void __launch_bounds__(128) k_rank_records(const uint64_t* __restrict__ keys,
+                                                      const int32_t* __restrict__ count,
+                                                      uint64_t* __restrict__ out, uint32_t* __restrict__ idx)
+{
+    __shared__ uint64_t sh[1024];
+    const int n = *count, i = blockIdx.x * 128 + threadIdx.x;
+    if ((int)blockIdx.x * 128 >= n) return;
+    const uint64_t k = i < n ? keys[i] : 0;
+    int rank = 0;
+    for (int c = 0; c < n; c += 1024) {
+        const int m = min(1024, n - c);
+        for (int j = threadIdx.x; j < m; j += 128) sh[j] = keys[c + j];
+        __syncthreads();
+        for (int j = 0; j < m; j++) rank += sh[j] < k || (sh[j] == k && c + j < i);
+        __syncthreads();
+    }
+    if (i >= n) return;
+    out[rank] = k;
+    idx[rank] = (uint32_t)i;
 }
 
 __global__ void k_cons_heads(const uint64_t* __restrict__ keys, int64_t m, int32_t* __restrict__ head)
@@ -225,38 +270,81 @@ __global__ void k_cons_heads(const uint64_t* __restrict__ keys, int64_t m, int32
     head[i] = (i == 0 || keys[i] != keys[i - 1]) ? 1 : 0;
 }
 
-__global__ void k_cons_emit(const uint64_t* __restrict__ keys, const uint32_t* __restrict__ idx,
-                            const int4* __restrict__ rverts, const double* __restrict__ reps,
-                            const int32_t* __restrict__ head, const int32_t* __restrict__ segid,
-                            int64_t m, const int* __restrict__ vbody, const int* __restrict__ ebody,
-                            const int* __restrict__ fbody, int* __restrict__ type,
-                            int4* __restrict__ verts, int2* __restrict__ prims,
-                            int2* __restrict__ bodies, double* __restrict__ weight,
-                            double* __restrict__ eps, int32_t* __restrict__ kind_count)
+struct ConsOut {
+    const uint64_t* keys;    // sorted
+    const uint32_t* idx;
+    const int4* rverts;
+    const double* reps;
+    const int *vbody, *ebody, *fbody;
+    int* type;
+    int4* verts;
+    int2 *prims, *bodies;
+    double *weight, *eps;
+    int32_t* kind_count;
+};
+
+// the constraint of the records [i, j) of one key, in slot s
+__device__ __forceinline__ void emit_constraint(const ConsOut& o, int64_t i, int64_t j, int s)
+{
+    const uint64_t k = o.keys[i];
+    const int kind = (int)(k >> 60);
+    const int p0 = (int)((k >> 30) & 0x3fffffffull), p1 = (int)(k & 0x3fffffffull);
+    const int4 rv = o.rverts[o.idx[i]];
+    o.type[s] = kind;
+    o.verts[s] = rv;
+    o.prims[s] = make_int2(p0, p1);
+    int b0, b1;
+    switch (kind) {
+    case 0: b0 = o.vbody[rv.x]; b1 = o.vbody[rv.y]; break;
+    case 1: b0 = o.vbody[p1]; b1 = o.ebody[p0]; break;
+    case 2: b0 = o.ebody[p0]; b1 = o.ebody[p1]; break;
+    default: b0 = o.vbody[p1]; b1 = o.fbody[p0]; break;
+    }
+    o.bodies[s] = make_int2(b0, b1);
+    o.weight[s] = (double)(j - i);
+    o.eps[s] = o.reps[o.idx[i]];
+    atomicAdd(&o.kind_count[kind], 1);
+}
+
+__global__ void k_cons_emit(ConsOut o, const int32_t* __restrict__ head, const int32_t* __restrict__ segid,
+                            int64_t m)
 {
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= m || !head[i]) return;
     int64_t j = i + 1;
     while (j < m && !head[j]) j++;
-    uint64_t k = keys[i];
-    int kind = (int)(k >> 60);
-    int p0 = (int)((k >> 30) & 0x3fffffffull), p1 = (int)(k & 0x3fffffffull);
-    int s = segid[i];
-    int4 rv = rverts[idx[i]];
-    type[s] = kind;
-    verts[s] = rv;
-    prims[s] = make_int2(p0, p1);
-    int b0, b1;
-    switch (kind) {
-    case 0: b0 = vbody[rv.x]; b1 = vbody[rv.y]; break;
-    case 1: b0 = vbody[p1]; b1 = ebody[p0]; break;
-    case 2: b0 = ebody[p0]; b1 = ebody[p1]; break;
-    default: b0 = vbody[p1]; b1 = fbody[p0]; break;
+    emit_constraint(o, i, j, segid[i]);
+}
+
+// Few records: heads, their numbers and the constraints by one block;
+// *total: the constraints
+__global__ void __launch_bounds__(1024) k_cons_small(ConsOut o, const int32_t* __restrict__ count,
+                                                     int32_t* __restrict__ total)
+{
+    __shared__ int32_t warp_sum[32];
+    __shared__ int32_t carry;
+    const int m = *count, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (threadIdx.x == 0) carry = 0;
+    __syncthreads();
+    for (int base = 0; base < m; base += 1024) {
+        const int i = base + (int)threadIdx.x;
+        const bool head = i < m && (i == 0 || o.keys[i] != o.keys[i - 1]);
+        const unsigned b = __ballot_sync(0xffffffffu, head);
+        if (lane == 0) warp_sum[warp] = __popc(b);
+        __syncthreads();
+        int s = carry;
+        for (int w = 0; w < warp; w++) s += warp_sum[w];
+        s += __popc(b & ((1u << lane) - 1u));
+        if (head) {
+            int j = i + 1;
+            while (j < m && o.keys[j] == o.keys[i]) j++;
+            emit_constraint(o, i, j, s);
+        }
+        __syncthreads();
+        if (threadIdx.x == 1023) carry = s + (head ? 1 : 0);
+        __syncthreads();
     }
-    bodies[s] = make_int2(b0, b1);
-    weight[s] = (double)(j - i);
-    eps[s] = reps[idx[i]];
-    atomicAdd(&kind_count[kind], 1);
+    if (threadIdx.x == 0) *total = carry;
 }
 
 int construct_constraints(Ctx& c, const double* x, double dhat, double dmin)
@@ -271,61 +359,72 @@ int construct_constraints(Ctx& c, const double* x, double dhat, double dmin)
     const double off = (dhat + dmin) * (dhat + dmin);
     c.cons.num = c.cons.num_vv = c.cons.num_ev = c.cons.num_ee = c.cons.num_fv = 0;
     if (n == 0) return RIGC_OK;
-    RIGC_TRY(S[6].reserve((size_t)(2 * n + 16) * sizeof(int32_t)));
-    int32_t* flag = S[6].as<int32_t>();
-    int32_t* pos = flag + n;
-    int32_t* cnt_dev = c.d_scalars.as<int32_t>();
-    RIGC_COUNT_LAUNCH();
-    k_classify_count<<<grid_for(n, 128), 128, 0, st>>>(
-        n, nee, c.cand.ee.as<int2>(), c.cand.fv.as<int2>(), c.s.edges, c.s.faces, c.s.f2e, V, off,
-        flag);
-    RIGC_TRY(exclusive_scan_i32(flag, pos, n, cnt_dev, S[7], st));
-    int32_t m;
-    RIGC_CUDA(cudaMemcpyAsync(&m, cnt_dev, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-    RIGC_CUDA(cudaStreamSynchronize(st));
-    if (m == 0) return RIGC_OK;
-    // raw records
-    RIGC_TRY(S[0].reserve((size_t)m * 8));
-    RIGC_TRY(S[1].reserve((size_t)m * 4));
-    RIGC_TRY(S[2].reserve((size_t)m * 8));
-    RIGC_TRY(S[3].reserve((size_t)m * 4));
+    // raw records, at most one per candidate
+    RIGC_TRY(S[0].reserve((size_t)n * 8));
+    RIGC_TRY(S[1].reserve((size_t)n * 4));
     DevBuf& rv = c.items_key2;
     DevBuf& re = c.items_val2;
-    RIGC_TRY(rv.reserve((size_t)m * sizeof(int4)));
-    RIGC_TRY(re.reserve((size_t)m * sizeof(double)));
+    RIGC_TRY(rv.reserve((size_t)n * sizeof(int4)));
+    RIGC_TRY(re.reserve((size_t)n * sizeof(double)));
+    // device counters: [0] records, [1] constraints, [2..5] per kind
+    int32_t* cnt_dev = c.d_scalars.as<int32_t>();
+    RIGC_CUDA(cudaMemsetAsync(cnt_dev, 0, 6 * sizeof(int32_t), st));
     RIGC_COUNT_LAUNCH();
-    k_classify_write<<<grid_for(n, 128), 128, 0, st>>>(
+    k_classify<<<grid_for(n, 128), 128, 0, st>>>(
         n, nee, c.cand.ee.as<int2>(), c.cand.fv.as<int2>(), c.s.edges, c.s.faces, c.s.f2e, V, off,
-        flag, pos, S[0].as<uint64_t>(), S[1].as<uint32_t>(), rv.as<int4>(), re.as<double>());
-    RIGC_TRY(radix_sort_pairs<uint64_t>(S[0].as<uint64_t>(), S[1].as<uint32_t>(),
-                                        S[2].as<uint64_t>(), S[3].as<uint32_t>(), m, 62,
-                                        c.items_key, c.items_val, S[7], st));
-    RIGC_TRY(S[6].reserve((size_t)(2 * m + 16) * sizeof(int32_t)));
-    int32_t* head = S[6].as<int32_t>();
-    int32_t* segid = head + m;
-    RIGC_COUNT_LAUNCH();
-    k_cons_heads<<<grid_for(m, 256), 256, 0, st>>>(S[2].as<uint64_t>(), m, head);
-    RIGC_TRY(exclusive_scan_i32(head, segid, m, cnt_dev, S[7], st));
-    int32_t nc;
-    RIGC_CUDA(cudaMemcpyAsync(&nc, cnt_dev, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-    RIGC_CUDA(cudaStreamSynchronize(st));
+        S[0].as<uint64_t>(), S[1].as<uint32_t>(), rv.as<int4>(), re.as<double>(), cnt_dev);
+    RIGC_CUDA(cudaGetLastError());
+    // few candidates: everything sized by them, one read-back at the end
+    const bool small = n <= kRankRecords;
+    int32_t m = (int32_t)n;
+    if (!small) {
+        RIGC_CUDA(cudaMemcpyAsync(&m, cnt_dev, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+        RIGC_CUDA(cudaStreamSynchronize(st));
+        if (m == 0) return RIGC_OK;
+    }
+    RIGC_TRY(S[2].reserve((size_t)m * 8));
+    RIGC_TRY(S[3].reserve((size_t)m * 4));
     Constraints& C = c.cons;
-    RIGC_TRY(C.type.reserve((size_t)nc * 4));
-    RIGC_TRY(C.verts.reserve((size_t)nc * 16));
-    RIGC_TRY(C.prims.reserve((size_t)nc * 8));
-    RIGC_TRY(C.bodies.reserve((size_t)nc * 8));
-    RIGC_TRY(C.weight.reserve((size_t)nc * 8));
-    RIGC_TRY(C.eps.reserve((size_t)nc * 8));
-    int32_t* kc = cnt_dev + 4;
-    RIGC_CUDA(cudaMemsetAsync(kc, 0, 4 * sizeof(int32_t), st));
-    RIGC_COUNT_LAUNCH();
-    k_cons_emit<<<grid_for(m, 256), 256, 0, st>>>(
-        S[2].as<uint64_t>(), S[3].as<uint32_t>(), rv.as<int4>(), re.as<double>(), head, segid, m,
-        c.s.vbody, c.s.ebody, c.s.fbody, C.type.as<int>(), C.verts.as<int4>(), C.prims.as<int2>(),
-        C.bodies.as<int2>(), C.weight.as<double>(), C.eps.as<double>(), kc);
-    int32_t kinds[4];
-    RIGC_CUDA(cudaMemcpyAsync(kinds, kc, sizeof(kinds), cudaMemcpyDeviceToHost, st));
+    auto out = [&](int64_t nc, ConsOut& o) -> int {
+        RIGC_TRY(C.type.reserve((size_t)nc * 4));
+        RIGC_TRY(C.verts.reserve((size_t)nc * 16));
+        RIGC_TRY(C.prims.reserve((size_t)nc * 8));
+        RIGC_TRY(C.bodies.reserve((size_t)nc * 8));
+        RIGC_TRY(C.weight.reserve((size_t)nc * 8));
+        RIGC_TRY(C.eps.reserve((size_t)nc * 8));
+        o = ConsOut { S[2].as<uint64_t>(), S[3].as<uint32_t>(), rv.as<int4>(), re.as<double>(), c.s.vbody,
+                      c.s.ebody, c.s.fbody, C.type.as<int>(), C.verts.as<int4>(), C.prims.as<int2>(),
+                      C.bodies.as<int2>(), C.weight.as<double>(), C.eps.as<double>(), cnt_dev + 2 };
+        return RIGC_OK;
+    };
+    ConsOut o;
+    if (small) {
+        RIGC_TRY(out(m, o));
+        RIGC_COUNT_LAUNCH();
+        k_rank_records<<<grid_for(m, 128), 128, 0, st>>>(S[0].as<uint64_t>(), cnt_dev, S[2].as<uint64_t>(),
+                                                         S[3].as<uint32_t>());
+        RIGC_COUNT_LAUNCH();
+        k_cons_small<<<1, 1024, 0, st>>>(o, cnt_dev, cnt_dev + 1);
+    } else {
+        RIGC_TRY(radix_sort_pairs<uint64_t>(S[0].as<uint64_t>(), S[1].as<uint32_t>(),
+                                            S[2].as<uint64_t>(), S[3].as<uint32_t>(), m, 62,
+                                            c.items_key, c.items_val, S[7], st));
+        RIGC_TRY(S[6].reserve((size_t)(2 * m + 16) * sizeof(int32_t)));
+        int32_t* head = S[6].as<int32_t>();
+        int32_t* segid = head + m;
+        RIGC_COUNT_LAUNCH();
+        k_cons_heads<<<grid_for(m, 256), 256, 0, st>>>(S[2].as<uint64_t>(), m, head);
+        RIGC_TRY(exclusive_scan_i32(head, segid, m, cnt_dev + 1, S[7], st));
+        RIGC_TRY(out(m, o));
+        RIGC_COUNT_LAUNCH();
+        k_cons_emit<<<grid_for(m, 256), 256, 0, st>>>(o, head, segid, m);
+    }
+    RIGC_CUDA(cudaGetLastError());
+    int32_t h[6];
+    RIGC_CUDA(cudaMemcpyAsync(h, cnt_dev, sizeof(h), cudaMemcpyDeviceToHost, st));
     RIGC_CUDA(cudaStreamSynchronize(st));
+    const int32_t nc = h[1];
+    const int32_t* kinds = h + 2;
     C.num = nc;
     C.num_vv = kinds[0];
     C.num_ev = kinds[1];
