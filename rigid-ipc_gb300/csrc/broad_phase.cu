@@ -64,11 +64,16 @@ __global__ void k_body_boxes(const double* __restrict__ x0, const double* __rest
             lo[j] = INFINITY;
             hi[j] = -INFINITY;
         }
-        for (int s = 0; s < 2; s++) {
+        // one pass when both poses are the same, one rotation when both
+        // rotations are (its chain is the kernel's latency)
+        const bool same = same_rot && p0[0] == p1[0] && p0[1] == p1[1] && p0[2] == p1[2];
+        double R[9];
+        for (int s = 0; s < (same ? 1 : 2); s++) {
             const double* pp = s ? p1 : p0;
-            double t[3] = { pp[3], pp[4], pp[5] };
-            double R[9];
-            rot_rn(t, R);
+            if (s == 0 || !same_rot) {
+                double t[3] = { pp[3], pp[4], pp[5] };
+                rot_rn(t, R);
+            }
             double p[3] = { pp[0], pp[1], pp[2] };
             for (int v = bvs[b] + lane; v < bvs[b + 1]; v += 32) {
                 double r[3] = { rest[3 * (size_t)v], rest[3 * (size_t)v + 1], rest[3 * (size_t)v + 2] };
@@ -1105,14 +1110,19 @@ __global__ void __launch_bounds__(kTile) k_tile_boxes(
     }
 }
 
-// A block per pair of tiles: edges with edges (tiles a <= b), then faces with
-// vertices, or (kPairsEF) faces with edges alone.
+// A block per pair of tiles and part of the second tile (cols elements, so
+// that few pairs of tiles still fill the GPU): edges with edges (tiles a <=
+// b), then faces with vertices, or (kPairsEF) faces with edges alone.  The
+// float tests of 32 elements come first, as a mask; the exact tests of the
+// pairs left then run for all threads together (in the loop over elements,
+// one thread's exact test would hold up its warp 128 times).
 __global__ void __launch_bounds__(kTile) k_all_pairs(Elems E, int kind, const ElemBox* __restrict__ eb,
-                                                     const float* __restrict__ tile_box, PairOut o)
+                                                     const float* __restrict__ tile_box, int cols_log2, PairOut o)
 {
     __shared__ ElemBox sh[kTile];
     const int tv = tiles_of(E.nv), te = tiles_of(E.ne);
-    int p = blockIdx.x, ta, tb, a, b;  // kinds and tiles
+    const int parts_log2 = 7 - cols_log2;
+    int p = blockIdx.x >> parts_log2, ta, tb, a, b;  // kinds and tiles
     const int nee = kind == kPairsEF ? 0 : te * (te + 1) / 2;
     if (p < nee) {
         // row b of the triangle holds tiles a = 0 .. b
@@ -1131,23 +1141,28 @@ __global__ void __launch_bounds__(kTile) k_all_pairs(Elems E, int kind, const El
     }
     const int first[3] = { 0, tv, tv + te };
     if (fboxes_disjoint(tile_box + 6 * (first[ta] + a), tile_box + 6 * (first[tb] + b))) return;
-    const int ia = a * kTile + threadIdx.x, ib0 = b * kTile;
+    const int cols = 1 << cols_log2;
+    const int ia = a * kTile + threadIdx.x, ib0 = b * kTile + ((blockIdx.x & ((1 << parts_log2) - 1)) << cols_log2);
     const int na = ta == 1 ? E.ne : E.nf, nb = tb == 0 ? E.nv : E.ne;
     ElemBox mine;
     mine.b[0] = INFINITY;
     if (ia < na) mine = eb[E.index(ta, ia)];
     ElemBox other;
     other.b[0] = INFINITY;
-    if (ib0 + (int)threadIdx.x < nb) other = eb[E.index(tb, ib0 + threadIdx.x)];
-    sh[threadIdx.x] = other;
+    if ((int)threadIdx.x < cols && ib0 + (int)threadIdx.x < nb) other = eb[E.index(tb, ib0 + threadIdx.x)];
+    if ((int)threadIdx.x < cols) sh[threadIdx.x] = other;
     __syncthreads();
     if (mine.b[0] == INFINITY) return;
-    const int end = min(kTile, nb - ib0);
-    for (int j = 0; j < end; j++) {
-        const ElemBox& x = sh[j];
-        if (x.gr == mine.gr || x.scene != mine.scene || fboxes_disjoint(mine.b, x.b)) continue;
-        if (ta == 1 && tb == 1 && ib0 + j <= ia) continue;
-        exact_pair(E, ta, ia, tb, ib0 + j, o);
+    const bool tri = ta == 1 && tb == 1;
+    for (int c = 0; c < cols; c += 32) {
+        unsigned m = 0;
+        const int end = min(32, cols);
+        for (int j = 0; j < end; j++) {
+            const ElemBox& x = sh[c + j];
+            if (x.gr != mine.gr && x.scene == mine.scene && !fboxes_disjoint(mine.b, x.b) && (!tri || ib0 + c + j > ia))
+                m |= 1u << j;
+        }
+        for (; m; m &= m - 1) exact_pair(E, ta, ia, tb, ib0 + c + __ffs(m) - 1, o);
     }
 }
 
@@ -1549,7 +1564,9 @@ int detect_pairs(Ctx& c, const double* x0, const double* x1, bool continuous, do
         RIGC_CUDA(cudaMemsetAsync(pn, 0, 2 * sizeof(unsigned long long), st));
         if (all_pairs) {
             RIGC_COUNT_LAUNCH();
-            k_all_pairs<<<(unsigned)tile_pairs, kTile, 0, st>>>(E, kind, elem_boxes, tile_boxes, o);
+            const int cols_log2 = tile_pairs <= 256 ? 3 : tile_pairs <= 1024 ? 4 : tile_pairs <= 4096 ? 5 : 7;
+            k_all_pairs<<<(unsigned)(tile_pairs << (7 - cols_log2)), kTile, 0, st>>>(E, kind, elem_boxes, tile_boxes,
+                                                                                    cols_log2, o);
         }
         if (nitems > 0) {
             RIGC_COUNT_LAUNCH();

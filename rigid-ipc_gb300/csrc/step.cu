@@ -446,191 +446,167 @@ __global__ void k_dense_fill(HessView H, const int* __restrict__ free_idx, int n
     row[fi] += H.reg;
 }
 
-// Dense LDL^T (no pivoting) of the free part of the Hessian, blocked: for
-// each panel of kPanel columns, k_ldlt_panel factorises the panel (rows
-// j0..n-1) in shared memory, one column at a time (d_c = a_cc,
-// l_rc = a_rc / d_c, then a_rc' -= l_rc d_c l_c'c within the panel), and
-// k_ldlt_update applies the panel to the trailing lower triangle
-// (A22 -= L21 D L21^T) in 32 x 32 tiles over many CTAs.  k_ldlt_solve then
-// solves L D L^T x = b with blocked forward and backward substitution in one
-// CTA.  flags[0] = 1 on a zero or non-finite pivot or a non-finite solution.
-// A's lower triangle is overwritten by L (unit diagonal implied), D by the
-// pivots.
+// Dense LDL^T (no pivoting) of the free part of the Hessian with the right-hand
+// side as one more row, blocked by panels of kPanel columns: k_ldlt_panel
+// factorises a panel, one column at a time (d_c = a_cc, l_rc = a_rc / d_c, then
+// a_rc' -= l_rc d_c l_c'c within the panel), and k_ldlt_update applies it to
+// the trailing lower triangle (A22 -= L21 D L21^T).  The right-hand side's row
+// ends as y = D^-1 L^-1 b, and k_ldlt_back solves L^T x = y.  flags[0] = 1 on a
+// zero or non-finite pivot or a non-finite solution.  A's lower triangle is
+// overwritten by L (unit diagonal implied; the diagonal blocks' by transposes
+// above the diagonal).
+//
+// All of it is FP64 latency and issue (an FP64 warp instruction takes 64 cycles
+// of its sub-partition): one SM took 66 us for a panel of 162 rows, 28 us for
+// an update in 32 x 32 tiles with separate products, 92 us for both
+// substitutions.  So every block factorises the panel's diagonal block again
+// beside 32 rows of its own (the chain of 32 columns is the panel's latency
+// either way), columns dealt to four warps; updates go by 16 x 16 tiles with
+// one fused multiply-add per term: 17, 5 and 46 us (the back substitution alone).
 constexpr int kPanel = 32;
-constexpr int kPanelStride = kPanel + 1;  // shared-memory row stride (no bank conflicts down a column)
 
-__global__ void __launch_bounds__(512) k_ldlt_panel(double* __restrict__ A, int n, int j0, int rows,
-                                                    double* __restrict__ D, int* __restrict__ flags)
+// 1 / d for normal d: the hardware approximation (about 20 bits) and one
+// third-order step
+__device__ __forceinline__ double reciprocal(double d)
 {
-    extern __shared__ double P[];  // rows x kPanel, row stride kPanelStride
-    const int m = min(rows, n - j0), w = min(kPanel, n - j0);
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+    const double e = fma(-d, y, 1.0);
+    return fma(y, fma(e, e, e), y);
+}
+
+// Warps 0-3: the panel's diagonal block, lane = row, warp q taking columns
+// q, q + 4, ...; warps 4-7: the block's own rows j0 + w + 32 blockIdx.x + lane
+// (row n: the right-hand side) in the same way.
+__global__ void __launch_bounds__(256) k_ldlt_panel(double* __restrict__ A, int n, int j0, double* __restrict__ D,
+                                                    int* __restrict__ flags)
+{
+    __shared__ double col[2][2][kPanel];  // [column parity][half][row]: the column before scaling
+    __shared__ double inv[2];
     if (flags[0]) return;
-    for (int e = threadIdx.x; e < m * w; e += blockDim.x) {
-        const int r = e / w, c = e % w;
-        P[r * kPanelStride + c] = r >= c ? A[(size_t)(j0 + r) * n + j0 + c] : 0.0;
+    const int w = min(kPanel, n - j0);
+    const int lane = threadIdx.x & 31, half = threadIdx.x >> 7, q = (threadIdx.x >> 5) & 3;
+    const int row = half ? j0 + w + 32 * (int)blockIdx.x + lane : j0 + lane;
+    const bool live = half ? row <= n : lane < w;
+    double v[kPanel / 4];
+#pragma unroll
+    for (int k = 0; k < kPanel / 4; k++) {
+        const int c = 4 * k + q;
+        v[k] = live && c < w && (half || c <= lane) ? A[(size_t)row * n + j0 + c] : 0.0;
     }
-    __syncthreads();
     bool bad = false;
-    for (int c = 0; c < w; c++) {
-        const double d = P[c * kPanelStride + c];
+    double pivot = 0;  // half 0, lane c of column c's warp
+#pragma unroll
+    for (int c = 0; c < kPanel; c++) {
+        if (c >= w) break;
+        const int b = c & 1;
+        if ((c & 3) == q) {
+            col[b][half][lane] = v[c >> 2];
+            if (half == 0 && lane == c) {
+                pivot = v[c >> 2];
+                inv[b] = reciprocal(pivot);
+            }
+        }
+        __syncthreads();
+        const double d = col[b][0][c];
         if (!(fabs(d) > 0) || !isfinite(d)) {
-            bad = true;
+            bad = true;  // the same in every thread
             break;
         }
-        for (int r = c + 1 + threadIdx.x; r < m; r += blockDim.x) P[r * kPanelStride + c] /= d;
-        __syncthreads();
-        // a_rc' -= l_rc d l_c'c for c < c' <= r
-        const int cols = w - c - 1;
-        for (int e = threadIdx.x; e < (m - c - 1) * cols; e += blockDim.x) {
-            const int r = c + 1 + e / cols, cc = c + 1 + e % cols;
-            if (cc <= r) P[r * kPanelStride + cc] -= P[r * kPanelStride + c] * d * P[cc * kPanelStride + c];
-        }
-        __syncthreads();
+        const double l = __dmul_rn(col[b][half][lane], inv[b]);
+        if ((c & 3) == q) v[c >> 2] = l;
+#pragma unroll
+        for (int k = 0; k < kPanel / 4; k++)
+            if (4 * k + q > c) v[k] = fma(-l, col[b][0][4 * k + q], v[k]);
     }
     if (bad) {
         if (threadIdx.x == 0) flags[0] = 1;
         return;
     }
-    for (int e = threadIdx.x; e < m * w; e += blockDim.x) {
-        const int r = e / w, c = e % w;
-        if (r > c) A[(size_t)(j0 + r) * n + j0 + c] = P[r * kPanelStride + c];
-        else if (r == c) D[j0 + c] = P[r * kPanelStride + c];
+    // the diagonal block's L and pivots by the first block: L transposed, above
+    // the diagonal, since other blocks may still load the triangle below it
+    if (half == 0 && blockIdx.x > 0) return;
+    if (half == 0 && lane < w && (lane & 3) == q) D[j0 + lane] = pivot;
+#pragma unroll
+    for (int k = 0; k < kPanel / 4; k++) {
+        const int c = 4 * k + q;
+        if (!live || c >= w) continue;
+        if (half) A[(size_t)row * n + j0 + c] = v[k];
+        else if (c < lane) A[(size_t)(j0 + c) * n + row] = v[k];
     }
-}
-
-// Systems too large for a panel in shared memory: after k_ldlt_panel has
-// factorised the panel's w x w diagonal block, each row r below it takes its
-// panel entries through the same column-by-column elimination as
-// k_ldlt_panel's (divide by the pivot, then subtract l_rc d_c l_c'c from the
-// later columns), one thread per row
-__global__ void __launch_bounds__(128) k_ldlt_trsm(double* __restrict__ A, int n, int j0, int w,
-                                                   const double* __restrict__ D,
-                                                   const int* __restrict__ flags)
-{
-    if (flags[0]) return;
-    __shared__ double L[kPanel][kPanel + 1], d[kPanel];
-    for (int e = threadIdx.x; e < kPanel * kPanel; e += blockDim.x) {
-        const int r = e / kPanel, c = e % kPanel;
-        L[r][c] = (r < w && c < r) ? A[(size_t)(j0 + r) * n + j0 + c] : 0.0;
-    }
-    if (threadIdx.x < kPanel) d[threadIdx.x] = threadIdx.x < w ? D[j0 + threadIdx.x] : 1.0;
-    __syncthreads();
-    const int r = j0 + w + blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= n) return;
-    double x[kPanel];
-#pragma unroll
-    for (int c = 0; c < kPanel; c++) x[c] = c < w ? A[(size_t)r * n + j0 + c] : 0.0;
-#pragma unroll
-    for (int c = 0; c < kPanel; c++) {
-        if (c >= w) break;
-        x[c] /= d[c];
-#pragma unroll
-        for (int cc = c + 1; cc < kPanel; cc++)
-            if (cc < w) x[cc] -= x[c] * d[c] * L[cc][c];
-    }
-#pragma unroll
-    for (int c = 0; c < kPanel; c++)
-        if (c < w) A[(size_t)r * n + j0 + c] = x[c];
 }
 
 // A[i][k] -= sum_c L[i][c] D[c] L[k][c] over the panel columns c, for the
-// trailing lower triangle i >= k >= j0 + w; one 32 x 32 tile per CTA
+// trailing rows i <= n (n: the right-hand side) and columns k <= i, k < n;
+// one 16 x 16 tile per block
 __global__ void __launch_bounds__(256) k_ldlt_update(double* __restrict__ A, int n, int j0, int w,
-                                                     const double* __restrict__ D,
-                                                     const int* __restrict__ flags)
+                                                     const double* __restrict__ D, const int* __restrict__ flags)
 {
     if (flags[0]) return;
     // tile (bi, bk), bi >= bk, from the linear block index
     const int t = blockIdx.x;
-    int bi = (int)((sqrt(8.0 * t + 1.0) - 1.0) * 0.5);
+    int bi = (int)((sqrtf(8.0f * (float)t + 1.0f) - 1.0f) * 0.5f);
     while ((bi + 1) * (bi + 2) / 2 <= t) bi++;
     while (bi * (bi + 1) / 2 > t) bi--;
     const int bk = t - bi * (bi + 1) / 2;
     const int base = j0 + w;
-    const int i0 = base + 32 * bi, k0 = base + 32 * bk;
-    __shared__ double Li[32][kPanel + 1], Lk[32][kPanel + 1], d[kPanel];
-    for (int e = threadIdx.x; e < 32 * kPanel; e += blockDim.x) {
+    const int i0 = base + 16 * bi, k0 = base + 16 * bk;
+    __shared__ double Li[16][kPanel + 1], Lk[16][kPanel + 1];
+    for (int e = threadIdx.x; e < 16 * kPanel; e += 256) {
         const int r = e / kPanel, c = e % kPanel;
-        Li[r][c] = (i0 + r < n && c < w) ? A[(size_t)(i0 + r) * n + j0 + c] : 0.0;
+        Li[r][c] = (i0 + r <= n && c < w) ? A[(size_t)(i0 + r) * n + j0 + c] * D[j0 + c] : 0.0;
         Lk[r][c] = (k0 + r < n && c < w) ? A[(size_t)(k0 + r) * n + j0 + c] : 0.0;
     }
-    if (threadIdx.x < kPanel) d[threadIdx.x] = threadIdx.x < w ? D[j0 + threadIdx.x] : 0.0;
     __syncthreads();
-    for (int e = threadIdx.x; e < 32 * 32; e += blockDim.x) {
-        const int r = e / 32, q = e % 32;
-        const int i = i0 + r, k = k0 + q;
-        if (i >= n || k >= n || k > i) continue;
-        double acc = 0;
-        for (int c = 0; c < w; c++) acc += Li[r][c] * d[c] * Lk[q][c];
-        A[(size_t)i * n + k] -= acc;
-    }
+    const int r = threadIdx.x >> 4, q = threadIdx.x & 15, i = i0 + r, k = k0 + q;
+    if (i > n || k >= n || k > i) return;
+    double acc = 0;
+#pragma unroll 8
+    for (int c = 0; c < kPanel; c++) acc = fma(Li[r][c], Lk[q][c], acc);
+    A[(size_t)i * n + k] -= acc;
 }
 
-// L D L^T x = b by blocks of 32: y = L^-1 b, y /= D, x = L^-T y
-__global__ void __launch_bounds__(256) k_ldlt_solve(const double* __restrict__ A, int n,
-                                                    const double* __restrict__ D,
-                                                    const double* __restrict__ b,
-                                                    double* __restrict__ x, int* __restrict__ flags)
+// L^T x = y (y: row n of A) by blocks of 32 from the last: the block's
+// triangle by one warp, then its rows off the earlier entries
+__global__ void __launch_bounds__(256) k_ldlt_back(const double* __restrict__ A, int n, double* __restrict__ x,
+                                                   int* __restrict__ flags)
 {
     if (flags[0]) return;
-    __shared__ double Lb[32][33];  // the diagonal block of the current block row
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) x[i] = b[i];
+    __shared__ double Lb[32][33], xb[32];
+    const int lane = threadIdx.x & 31;
+    for (int i = threadIdx.x; i < n; i += 256) x[i] = A[(size_t)n * n + i];
     __syncthreads();
-    // forward: rows of block [b0, b0 + 32) minus the solved columns [0, b0)
-    for (int b0 = 0; b0 < n; b0 += 32) {
-        const int nb = min(32, n - b0);
-        for (int r = warp; r < nb; r += 8) {
-            double acc = 0;
-            for (int k = lane; k < b0; k += 32) acc += A[(size_t)(b0 + r) * n + k] * x[k];
-            for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-            if (lane == 0) x[b0 + r] -= acc;
-        }
-        for (int e = threadIdx.x; e < nb * 32; e += blockDim.x) {
-            const int r = e / 32, q = e % 32;
-            Lb[r][q] = q < nb ? A[(size_t)(b0 + r) * n + b0 + q] : 0.0;
-        }
-        __syncthreads();
-        if (warp == 0) {
-            double y = lane < nb ? x[b0 + lane] : 0.0;
-            for (int r = 1; r < nb; r++) {
-                const double yr = __shfl_sync(0xffffffffu, y, r - 1);
-                // lanes >= r subtract column r - 1
-                if (lane >= r && lane < nb) y -= Lb[lane][r - 1] * yr;
-            }
-            if (lane < nb) x[b0 + lane] = y;
-        }
-        __syncthreads();
-    }
-    for (int i = threadIdx.x; i < n; i += blockDim.x) x[i] /= D[i];
-    __syncthreads();
-    // backward: block [b0, b0 + 32) minus the solved rows [b0 + 32, n)
+    bool bad = false;
     for (int b0 = ((n - 1) / 32) * 32; b0 >= 0; b0 -= 32) {
         const int nb = min(32, n - b0);
-        for (int r = warp; r < nb; r += 8) {
-            double acc = 0;
-            for (int k = b0 + 32 + lane; k < n; k += 32) acc += A[(size_t)k * n + b0 + r] * x[k];
-            for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-            if (lane == 0) x[b0 + r] -= acc;
-        }
-        for (int e = threadIdx.x; e < nb * 32; e += blockDim.x) {
+        for (int e = threadIdx.x; e < nb * 32; e += 256) {
             const int r = e / 32, q = e % 32;
-            Lb[r][q] = q < nb ? A[(size_t)(b0 + r) * n + b0 + q] : 0.0;
+            // the factor's triangle is stored transposed (k_ldlt_panel)
+            if (q < nb) Lb[q][r] = r < q ? A[(size_t)(b0 + r) * n + b0 + q] : 0.0;
         }
         __syncthreads();
-        if (warp == 0) {
+        if (threadIdx.x < 32) {
             double y = lane < nb ? x[b0 + lane] : 0.0;
             for (int r = nb - 1; r > 0; r--) {
                 const double yr = __shfl_sync(0xffffffffu, y, r);
                 // lanes < r subtract row r's entry in their column
-                if (lane < r) y -= Lb[r][lane] * yr;
+                if (lane < r) y = fma(-Lb[r][lane], yr, y);
             }
-            if (lane < nb) x[b0 + lane] = y;
+            if (lane < nb) {
+                x[b0 + lane] = y;
+                bad = bad || !isfinite(y);
+            }
+            xb[lane] = lane < nb ? y : 0.0;
+        }
+        __syncthreads();
+        for (int k = threadIdx.x; k < b0; k += 256) {
+            double acc = x[k];
+            for (int r = 0; r < nb; r++) acc = fma(-A[(size_t)(b0 + r) * n + k], xb[r], acc);
+            x[k] = acc;
         }
         __syncthreads();
     }
-    for (int i = threadIdx.x; i < n; i += blockDim.x)
-        if (!isfinite(x[i])) flags[0] = 1;
+    if (bad) flags[0] = 1;
 }
 
 // ---------------------------------------------------------------------------
@@ -1142,7 +1118,7 @@ constexpr long long kCGTry = 300;
 struct Sim {
     rigc_sim_params p {};
     int nb = 0, nv = 0, nfree = 0;
-    DevBuf free_idx, dense, dense_b, dense_x, dense_d;  // dense LDL^T path
+    DevBuf free_idx, dense, dense_x, dense_d;  // dense LDL^T path (dense: a row more, the right-hand side)
     DevBuf mass, moment, fixed, x0, vel, Qdot;          // body state
     DevBuf x, xt, dir, g, gE, hE, gtmp;                 // Newton vectors
     DevBuf r, z, pp, Ap, Minv, sol, part, scal;         // CG
@@ -1423,31 +1399,16 @@ int pcg(Ctx& c, Sim& S, const HessView& H, bool& ok, int64_t& iters, long long c
     return RIGC_OK;
 }
 
+// factorisation of the n x n A in place with its row n, the right-hand side
 int dense_ldlt(Ctx& c, double* A, int n, double* D, int* flags)
 {
-    static bool attr = false;
-    const size_t smem = (size_t)kDenseMax * kPanelStride * sizeof(double);
-    if (!attr) {
-        RIGC_CUDA(cudaFuncSetAttribute(k_ldlt_panel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)smem));
-        attr = true;
-    }
-    // up to kDenseMax unknowns the whole panel column is factorised in shared
-    // memory; above, its diagonal block there and the rows below by k_ldlt_trsm
-    const bool big = n > kDenseMax;
     for (int j0 = 0; j0 < n; j0 += kPanel) {
         const int w = std::min(kPanel, n - j0);
-        const int rows = big ? w : n - j0;
+        const int rest = n + 1 - j0 - w;  // rows below the panel, the right-hand side's among them
         RIGC_COUNT_LAUNCH();
-        k_ldlt_panel<<<1, 512, (size_t)rows * kPanelStride * sizeof(double), c.stream>>>(
-            A, n, j0, rows, D, flags);
-        const int rest = n - j0 - w;
-        if (big && rest > 0) {
-            RIGC_COUNT_LAUNCH();
-            k_ldlt_trsm<<<grid_for(rest, 128), 128, 0, c.stream>>>(A, n, j0, w, D, flags);
-        }
-        if (rest > 0) {
-            const int tiles = (rest + 31) / 32;
+        k_ldlt_panel<<<(rest + 31) / 32, 256, 0, c.stream>>>(A, n, j0, D, flags);
+        if (rest > 1) {
+            const int tiles = (rest + 15) / 16;
             RIGC_COUNT_LAUNCH();
             k_ldlt_update<<<tiles * (tiles + 1) / 2, 256, 0, c.stream>>>(A, n, j0, w, D, flags);
         }
@@ -1463,8 +1424,7 @@ int dense_solve(Ctx& c, Sim& S, const HessView& H, bool& ok)
     const int n6 = 6 * S.nb;
     cudaStream_t st = c.stream;
     if (n > kDenseMax) {
-        RIGC_TRY(S.dense.reserve((size_t)n * n * sizeof(double) + 8));
-        RIGC_TRY(S.dense_b.reserve((size_t)n * sizeof(double) + 8));
+        RIGC_TRY(S.dense.reserve((size_t)(n + 1) * n * sizeof(double) + 8));
         RIGC_TRY(S.dense_x.reserve((size_t)n * sizeof(double) + 8));
         RIGC_TRY(S.dense_d.reserve((size_t)n * sizeof(double) + 8));
     }
@@ -1475,11 +1435,10 @@ int dense_solve(Ctx& c, Sim& S, const HessView& H, bool& ok)
     k_dense_fill<<<grid_for(n6, 128), 128, 0, st>>>(H, S.free_idx.as<int>(), n, S.dense.as<double>());
     RIGC_COUNT_LAUNCH();
     k_gather_neg<<<grid_for(n6, 256), 256, 0, st>>>(n6, S.free_idx.as<int>(), S.g.as<double>(),
-                                                    S.dense_b.as<double>());
+                                                    S.dense.as<double>() + (size_t)n * n);
     RIGC_TRY(dense_ldlt(c, S.dense.as<double>(), n, S.dense_d.as<double>(), flags));
     RIGC_COUNT_LAUNCH();
-    k_ldlt_solve<<<1, 256, 0, st>>>(S.dense.as<double>(), n, S.dense_d.as<double>(),
-                                    S.dense_b.as<double>(), S.dense_x.as<double>(), flags);
+    k_ldlt_back<<<1, 256, 0, st>>>(S.dense.as<double>(), n, S.dense_x.as<double>(), flags);
     RIGC_COUNT_LAUNCH();
     k_scatter_free<<<grid_for(n6, 256), 256, 0, st>>>(n6, S.free_idx.as<int>(), S.dense_x.as<double>(),
                                                       S.sol.as<double>());
@@ -1878,8 +1837,7 @@ int set_free_dofs(Ctx& c, Sim& S)
     RIGC_CUDA(cudaMemcpyAsync(S.free_idx.ptr, fidx.data(), fidx.size() * sizeof(int),
                               cudaMemcpyHostToDevice, c.stream));
     if (nf <= kDenseMax) {
-        RIGC_TRY(S.dense.reserve((size_t)nf * nf * sizeof(double) + 8));
-        RIGC_TRY(S.dense_b.reserve((size_t)nf * sizeof(double) + 8));
+        RIGC_TRY(S.dense.reserve((size_t)(nf + 1) * nf * sizeof(double) + 8));
         RIGC_TRY(S.dense_x.reserve((size_t)nf * sizeof(double) + 8));
         RIGC_TRY(S.dense_d.reserve((size_t)nf * sizeof(double) + 8));
     }
@@ -2719,7 +2677,7 @@ void sim_release(Ctx& c)
     DevBuf* bufs[] = { &S.mass, &S.moment, &S.fixed, &S.x0, &S.vel, &S.Qdot, &S.x, &S.xt,
                        &S.dir, &S.g, &S.gE, &S.hE, &S.gtmp, &S.r, &S.z, &S.pp, &S.Ap,
                        &S.Minv, &S.sol, &S.part, &S.scal, &S.V0, &S.V1, &S.free_idx,
-                       &S.dense, &S.dense_b, &S.dense_x, &S.dense_d, &S.ckpt,
+                       &S.dense, &S.dense_x, &S.dense_d, &S.ckpt,
                        &S.final_state, &S.seg_pre, &S.seg_x, &S.adj, &S.adj_out, &S.xbar,
                        &S.u1, &S.u2, &S.sc_dev, &S.sc_red, &S.sc_vstart, &S.al_xpred,
                        &S.al_lam, &S.al_Lam, &S.al_e, &S.hview };
