@@ -101,38 +101,6 @@ __device__ __forceinline__ int local_body_of(int type, int i)
     return i == 0 ? 0 : 1;
 }
 
-// H += J_i^T Hb J_j (+ its transpose when i and j are different vertices),
-// J_i = [I | D_i]
-__device__ __forceinline__ void add_vertex_block(SMat H, const Vtx& Vi, int bi, const Vtx& Vj, int bj,
-                                                 const double (*Hb)[3], bool same_vertex)
-{
-    double HD[3][3], DH[3][3], DHD[3][3];
-    for (int r = 0; r < 3; r++)
-        for (int c = 0; c < 3; c++) {
-            HD[r][c] = Hb[r][0] * Vj.D[0][c] + Hb[r][1] * Vj.D[1][c] + Hb[r][2] * Vj.D[2][c];
-            DH[r][c] = Vi.D[0][r] * Hb[0][c] + Vi.D[1][r] * Hb[1][c] + Vi.D[2][r] * Hb[2][c];
-        }
-    for (int r = 0; r < 3; r++)
-        for (int c = 0; c < 3; c++)
-            DHD[r][c] = Vi.D[0][r] * HD[0][c] + Vi.D[1][r] * HD[1][c] + Vi.D[2][r] * HD[2][c];
-    if (!same_vertex) {
-        double tt[3][3];
-        for (int r = 0; r < 3; r++)
-            for (int c = 0; c < 3; c++) tt[r][c] = Hb[r][c] + Hb[c][r];
-        add_pair_blocks(H, bi, bj, tt, HD, DH, DHD);
-        return;
-    }
-    const int o = red_rot(bi);
-    for (int r = 0; r < 3; r++)
-        for (int c = 0; c < 3; c++) {
-            if (bi == 0) {
-                if (r <= c) H.at(r, c) += Hb[r][c];
-                H.at(r, o + c) += HD[r][c];
-            }
-            if (r <= c) H.at(o + r, o + c) += DHD[r][c];
-        }
-}
-
 // A mollified EE constraint whose closest features are endpoints (kept as EE
 // by the constraint set because the edges are nearly parallel): f = w m(D)
 // b(d - dmin^2) with D = |A x B|^2 of the two edges and d the point-point or
@@ -140,8 +108,13 @@ __device__ __forceinline__ void add_vertex_block(SMat H, const Vtx& Vi, int bi, 
 // gradients and 3x3 Hessian blocks in closed form:
 //   grad D_i = 2 M_i^T n, M_i = alpha_i (-[B]x) + beta_i [A]x,
 //   hess D_ij = 2 M_i^T M_j + 2 (beta_i alpha_j - alpha_i beta_j) [n]x,
-// and the same for N = |a x b|^2 of a point-edge distance d = N / |e|^2;
-// then J^T (.) J and the curvature term into body space.
+// and the same for N = |a x b|^2 of a point-edge distance d = N / |e|^2, so the
+// body Hessian is outer products of the body-space gradients, Gram terms, skew
+// pair blocks and the curvature term, as barrier_build's: bound by FP64 issue,
+// and most constraints of box-like bodies in contact end here (104 k of 163 k
+// between 32 slabs).  J_i^T (.) J_j of the ten 3x3 vertex blocks took 2.20 ms
+// there, with the other kinds, unprojected; this 1.34 ms (338 constraints
+// between 27 cubes, one per lane: 256 -> 212 us).
 static __device__ __noinline__ bool ee_endpoint_build(const BarrierArgs& a, int64_t ci, SMat H,
                                                       const Vtx* V, const double (*vrest)[3],
                                                       const int* lbody, const double* const* fr,
@@ -258,53 +231,61 @@ static __device__ __noinline__ bool ee_endpoint_build(const BarrierArgs& a, int6
     if (!want_h) return false;
 
     H.clear();
-    // M_i = alpha_i (-[B]x) + beta_i [A]x (dn/dX_i), C_i likewise for c = a x b
-    auto skew_of = [](double sa, const double* Bv, double sb, const double* Av, double (*M)[3]) {
-        double v0 = -sa * Bv[0] + sb * Av[0], v1 = -sa * Bv[1] + sb * Av[1],
-               v2 = -sa * Bv[2] + sb * Av[2];
-        M[0][0] = 0; M[0][1] = -v2; M[0][2] = v1;
-        M[1][0] = v2; M[1][1] = 0; M[1][2] = -v0;
-        M[2][0] = -v1; M[2][1] = v0; M[2][2] = 0;
+    const double cd = weight * m * b1, cD = weight * bv * m1;  // on hess d, hess D
+    const double kdd = weight * m * b2, kdD = weight * m1 * b1, kDD = weight * bv * m2;
+    double M[4][9];
+    // M_i = alpha_i (-[B]x) + beta_i [A]x (dn/dX_i, likewise of c = pa x pb)
+    auto skew_of = [](double sa, const double* Bv, double sb, const double* Av, double* Mi) {
+        const double v0 = -sa * Bv[0] + sb * Av[0], v1 = -sa * Bv[1] + sb * Av[1], v2 = -sa * Bv[2] + sb * Av[2];
+        Mi[0] = 0; Mi[1] = -v2; Mi[2] = v1;
+        Mi[3] = v2; Mi[4] = 0; Mi[5] = -v0;
+        Mi[6] = -v1; Mi[7] = v0; Mi[8] = 0;
     };
-    for (int i = 0; i < 4; i++)
-        for (int j = i; j < 4; j++) {
-            double Mi[3][3], Mj[3][3], Hb[3][3];
-            skew_of(alD[i], B, beD[i], A, Mi);
-            skew_of(alD[j], B, beD[j], A, Mj);
-            const double kD = 2 * (beD[i] * alD[j] - alD[i] * beD[j]);
-            const double nx[3][3] = { { 0, -n[2], n[1] }, { n[2], 0, -n[0] }, { -n[1], n[0], 0 } };
-            double Ci[3][3], Cj[3][3], kN = 0;
-            const double cx[3][3] = { { 0, -c[2], c[1] }, { c[2], 0, -c[0] }, { -c[1], c[0], 0 } };
-            if (kind == 1) {
-                skew_of(alE[i], pb, beE[i], pa, Ci);
-                skew_of(alE[j], pb, beE[j], pa, Cj);
-                kN = 2 * (beE[i] * alE[j] - alE[i] * beE[j]);
-            }
-            for (int r = 0; r < 3; r++)
-                for (int q2 = 0; q2 < 3; q2++) {
-                    // hess D block
-                    double hD = kD * nx[r][q2];
-                    for (int k = 0; k < 3; k++) hD += 2 * Mi[k][r] * Mj[k][q2];
-                    // hess d block
-                    double hd;
-                    if (kind == 0) {
-                        double si = i == p ? 1.0 : (i == q ? -1.0 : 0.0);
-                        double sj = j == p ? 1.0 : (j == q ? -1.0 : 0.0);
-                        hd = r == q2 ? 2 * si * sj : 0.0;
-                    } else {
-                        double hN = kN * cx[r][q2];
-                        for (int k = 0; k < 3; k++) hN += 2 * Ci[k][r] * Cj[k][q2];
-                        double hE = r == q2 ? 2 * gaE[i] * gaE[j] : 0.0;
-                        hd = hN / De - (gN[i][r] * gE[j][q2] + gE[i][r] * gN[j][q2]) / (De * De)
-                            + 2 * N / (De * De * De) * gE[i][r] * gE[j][q2] - N / (De * De) * hE;
-                    }
-                    Hb[r][q2] = weight * (m * b2 * gd[i][r] * gd[j][q2] + m * b1 * hd
-                                          + m1 * b1 * (gd[i][r] * gD[j][q2] + gD[i][r] * gd[j][q2])
-                                          + bv * m2 * gD[i][r] * gD[j][q2] + bv * m1 * hD);
-                }
-            add_vertex_block(H, V[i], lbody[i], V[j], lbody[j], Hb, i == j);
+    for (int i = 0; i < 4; i++) skew_of(alD[i], B, beD[i], A, M[i]);
+    add_gram(H, 2 * cD, V, lbody, 4, M);
+    double gr[3][kRed];
+    to_body(V, lbody, 4, gD, G);
+    reduce12(G, gr[2]);
+    if (kind == 0) {
+        // d = |w|^2: hess = 2 (dw)^T (dw)
+        to_body(V, lbody, 4, gd, G);
+        reduce12(G, gr[1]);
+        add_quadratic(H, kdd, kdD, kDD, gr[1], gr[2]);
+        for (int i = 0; i < 4; i++) {
+            for (int k = 0; k < 9; k++) M[i][k] = 0;
+            M[i][0] = M[i][4] = M[i][8] = i == p ? 1.0 : (i == q ? -1.0 : 0.0);
         }
-    for (int i = 0; i < 4; i++) add_curvature(H, fr[lbody[i]], lbody[i], vrest[i], gv[i]);
+        add_gram(H, 2 * cd, V, lbody, 4, M);
+    } else {
+        // grad d = gN / De - N / De^2 gE,
+        // hess d = (1/De) H_N - (1/De^2)(gN gE + gE gN) + (2N/De^3) gE gE - (N/De^2) H_E
+        const double pn = 1 / De, pe = -N / (De * De);
+        to_body(V, lbody, 4, gN, G);
+        reduce12(G, gr[0]);
+        to_body(V, lbody, 4, gE, G);
+        reduce12(G, gr[1]);
+        double gdr[kRed];  // reduced body gradient of d
+        for (int k = 0; k < kRed; k++) gdr[k] = pn * gr[0][k] + pe * gr[1][k];
+        add_quadratic(H, kdd, kdD, kDD, gdr, gr[2]);
+        add_quadratic(H, 0, -cd / (De * De), 2 * cd * N / (De * De * De), gr[0], gr[1]);
+        for (int i = 0; i < 4; i++) skew_of(alE[i], pb, beE[i], pa, M[i]);
+        add_gram(H, 2 * cd / De, V, lbody, 4, M);
+        for (int i = 0; i < 4; i++) {
+            for (int k = 0; k < 9; k++) M[i][k] = 0;
+            M[i][0] = M[i][4] = M[i][8] = gaE[i];
+        }
+        add_gram(H, 2 * cd * pe, V, lbody, 4, M);
+    }
+    for (int i = 0; i < 4; i++)
+        for (int j = i + 1; j < 4; j++) {
+            const double kD = 2 * cD * (beD[i] * alD[j] - alD[i] * beD[j]);
+            const double kN = kind == 1 ? 2 * cd / De * (beE[i] * alE[j] - alE[i] * beE[j]) : 0.0;
+            if (kD == 0 && kN == 0) continue;
+            double sv[3];
+            for (int k = 0; k < 3; k++) sv[k] = kD * n[k] + (kind == 1 ? kN * c[k] : 0.0);
+            add_skew_pair(H, V[i], lbody[i], V[j], lbody[j], sv);
+        }
+    add_curvature(H, fr, lbody, 4, vrest, gv);
     return true;
 }
 
@@ -485,11 +466,11 @@ static __device__ __noinline__ bool barrier_build(const BarrierArgs& a, int64_t 
 
     // ---- Hessian
     H.clear();
-    double G1[kRed], G2[kRed];
+    double G12[2][kRed];
     to_body(V, lbody, nvc, g1v, G);
-    reduce12(G, G1);
+    reduce12(G, G12[0]);
     to_body(V, lbody, nvc, g2v, G);
-    reduce12(G, G2);
+    reduce12(G, G12[1]);
     // second-derivative coefficients of d in terms of (g1, g2) and the
     // Hessians of the basic scalars:
     //  PT/EE: hess d = (2/D) g1g1 + c1 H_u - (2u/D^2)(g1g2 + g2g1) + (2u^2/D^3) g2g2 + c2 H_D
@@ -515,9 +496,7 @@ static __device__ __noinline__ bool barrier_build(const BarrierArgs& a, int64_t 
     const double a11 = P1 * c1 * c1 + P2 * duu;
     const double a12 = P1 * c1 * c2 + P2 * duD + P5 * c1;
     const double a22 = P1 * c2 * c2 + P2 * dDD + P3 + 2 * P5 * c2;
-    add_outer(H, a11, G1);
-    add_sym_outer(H, a12, G1, G2);
-    add_outer(H, a22, G2);
+    add_quadratic(H, a11, a12, a22, G12[0], G12[1]);
 
     // coefficients of the scalar Hessians
     const double bu = P2 * c1;            // on H_u (PT/EE) or H_N (PE)
@@ -584,7 +563,7 @@ static __device__ __noinline__ bool barrier_build(const BarrierArgs& a, int64_t 
         add_gram(H, 2 * P2, V, lbody, 2, M);
     }
     // curvature of the rigid maps
-    for (int i = 0; i < nvc; i++) add_curvature(H, fr[lbody[i]], lbody[i], vrest[i], gv[i]);
+    add_curvature(H, fr, lbody, nvc, vrest, gv);
     return true;
 }
 

@@ -246,20 +246,18 @@ static __device__ __noinline__ bool friction_build(const FrictionArgs& a, int64_
         for (int k = 0; k < 12; k++) a.grad[ci * 12 + k] = G[k];
     if (!want_h) return false;
     H.clear();
-    double A0[4][3], A1[4][3], G0[kRed], G1[kRed];
+    double A0[4][3], A1[4][3], GA[2][kRed];
     for (int i = 0; i < nvc; i++)
         for (int j = 0; j < 3; j++) {
             A0[i][j] = g[i] * t1[j];
             A1[i][j] = g[i] * t2[j];
         }
     to_body(V, lbody, nvc, A0, G);
-    reduce12(G, G0);
+    reduce12(G, GA[0]);
     to_body(V, lbody, nvc, A1, G);
-    reduce12(G, G1);
-    add_outer(H, ml * h00, G0);
-    add_sym_outer(H, ml * h01, G0, G1);
-    add_outer(H, ml * h11, G1);
-    for (int i = 0; i < nvc; i++) add_curvature(H, fr[lbody[i]], lbody[i], vrest[i], gX[i]);
+    reduce12(G, GA[1]);
+    add_quadratic(H, ml * h00, ml * h01, ml * h11, GA[0], GA[1]);
+    add_curvature(H, fr, lbody, nvc, vrest, gX);
     return true;
 }
 

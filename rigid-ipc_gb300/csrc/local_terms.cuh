@@ -69,19 +69,13 @@ __device__ __forceinline__ void reduce12(const double* g, double* r)
     for (int k = 6; k < 9; k++) r[k] = g[k + 3];
 }
 
-// H += coef * (a b^T + b a^T) (a, b reduced)
-__device__ __forceinline__ void add_sym_outer(SMat H, double coef, const double* a, const double* b)
+// H += a00 v0 v0^T + a01 (v0 v1^T + v1 v0^T) + a11 v1 v1^T (v0, v1 reduced)
+__device__ __forceinline__ void add_quadratic(SMat H, double a00, double a01, double a11, const double* v0,
+                                              const double* v1)
 {
     for (int r = 0; r < kRed; r++) {
-        double ar = coef * a[r], br = coef * b[r];
-        for (int c = r; c < kRed; c++) H.at(r, c) += ar * b[c] + br * a[c];
-    }
-}
-__device__ __forceinline__ void add_outer(SMat H, double coef, const double* a)
-{
-    for (int r = 0; r < kRed; r++) {
-        double ar = coef * a[r];
-        for (int c = r; c < kRed; c++) H.at(r, c) += ar * a[c];
+        const double u0 = a00 * v0[r] + a01 * v1[r], u1 = a01 * v0[r] + a11 * v1[r];
+        for (int c = r; c < kRed; c++) H.at(r, c) += u1 * v1[c] + u0 * v0[c];
     }
 }
 
@@ -170,20 +164,28 @@ __device__ __forceinline__ void add_skew_pair(SMat H, const Vtx& Vi, int bi, con
     add_pair_blocks(H, bi, bj, nullptr, KD, DK, DKD);
 }
 
-// curvature term: H(rot lb, rot lb) += sum_j g_j (d2R_kl v)_j
-__device__ __forceinline__ void add_curvature(SMat H, const double* frame, int lb,
-                                              const double* v, const double* g)
+// curvature term: H(rot lb, rot lb) += sum_i g_i . (d2R_kl v_i) over the
+// vertices i of each body, as d2R_kl : (sum_i g_i v_i^T)
+__device__ __forceinline__ void add_curvature(SMat H, const double* const* frames, const int* lbody, int nvc,
+                                              const double (*v)[3], const double (*g)[3])
 {
-    const double* d2 = frame + 36;
-    const int o = red_rot(lb);
-    for (int k = 0; k < 3; k++)
-        for (int l = k; l < 3; l++) {
-            const double* M = d2 + 9 * sym_index(k, l);
-            double acc = 0;
-            for (int j = 0; j < 3; j++)
-                acc += g[j] * (M[3 * j] * v[0] + M[3 * j + 1] * v[1] + M[3 * j + 2] * v[2]);
-            H.at(o + k, o + l) += acc;
-        }
+    for (int b = 0; b < 2; b++) {
+        double S[9];
+        for (int k = 0; k < 9; k++) S[k] = 0;
+        for (int i = 0; i < nvc; i++)
+            if (lbody[i] == b)
+                for (int j = 0; j < 3; j++)
+                    for (int c = 0; c < 3; c++) S[3 * j + c] += g[i][j] * v[i][c];
+        const double* d2 = frames[b] + 36;
+        const int o = red_rot(b);
+        for (int k = 0; k < 3; k++)
+            for (int l = k; l < 3; l++) {
+                const double* M = d2 + 9 * sym_index(k, l);
+                double acc = 0;
+                for (int e = 0; e < 9; e++) acc += M[e] * S[e];
+                H.at(o + k, o + l) += acc;
+            }
+    }
 }
 
 // ---------------------------------------------------------------------------
