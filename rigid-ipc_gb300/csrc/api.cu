@@ -9,6 +9,7 @@
 
 namespace rigc {
 
+int build_patches(Ctx& c);
 int detect_candidates(Ctx& c, const double* x0, const double* x1, bool continuous, double infl);
 int construct_constraints(Ctx& c, const double* x, double dhat, double dmin);
 int launch_barrier_local(Ctx& c, const double* x, double dhat, double dmin, int flags,
@@ -147,6 +148,7 @@ static void release_all(Ctx* c)
                        &c->fric.coef, &c->fric.v0c, &c->fric.V0, &c->fric.c_energy,
                        &c->fric.c_grad, &c->fric.c_blocks, &c->fric.grad, &c->fric.row_ptr,
                        &c->fric.col, &c->fric.val, &c->scene_toi, &c->scene_energy,
+                       &c->bp_patch, &c->s.patches, &c->s.patch_start, &c->s.patch_order,
                        &c->bp_misc, &c->bp_deeper, &c->bp_sig, &c->bp_ec0,
                        &c->bp_eext, &c->bp_f32, &c->bp_cnt, &c->md_V, &c->md_rot,
                        &c->md_out, &c->isect.ee, &c->isect.fv };
@@ -301,6 +303,7 @@ static int ctx_create(const rigc_scene_desc* d, int num_scenes, const int32_t* b
     chk(upload(s.bscene, bscene.data(), (size_t)nb));
     chk(upload(s.scene_bstart, sstart.data(), (size_t)num_scenes + 1));
     chk(c->d_scalars.reserve(4096));
+    if (st == RIGC_OK) chk(build_patches(*c));
     if (st == RIGC_OK) {
         cudaError_t e = cudaMallocHost(&c->h_scalars, 4096);
         if (e != cudaSuccess) st = RIGC_ERR_OOM;

@@ -33,8 +33,9 @@
 //       elements of their scene instead of being binned.
 //     The output is the same set, sorted: ee as (edge0 < edge1), fv as
 //     (face, vertex).
-//     Small scenes skip the grid: every pair of elements is tested, tile by
-//     tile (k_all_pairs).
+//     The smallest scenes test every pair of elements, tile by tile
+//     (k_all_pairs); the others pair patches of neighbouring elements
+//     (patch_pairs.cuh) unless those meet too many others.
 #include "common.cuh"
 #include "interval.cuh"
 #include "sort.cuh"
@@ -885,22 +886,21 @@ __device__ __forceinline__ bool pair_types(int kind, int ta, int tb)
 
 // an EE (edges) or FV (face, vertex in either order) pair of elements whose
 // groups differ, or an EF pair (edge, face in either order; output in the FV
-// stream, key face * ne + edge): the overlap tests and the output key
-// (after the float boxes overlap) the double boxes and the output key
+// stream, key face * ne + edge): the output key
+__device__ __forceinline__ unsigned long long element_pair_key(const Elems& E, int ta, int ia, int tb, int ib)
+{
+    const int lo = min(ia, ib), hi = max(ia, ib);
+    if (ta == 1 && tb == 1) return (unsigned long long)lo * (unsigned long long)E.ne + (unsigned long long)hi;
+    const int f = ta == 2 ? ia : ib, x = ta == 2 ? ib : ia;
+    return (unsigned long long)f * (unsigned long long)(ta + tb == 3 ? E.ne : E.nv) + (unsigned long long)x;
+}
+
+// after the float boxes overlap: the double boxes and the output key
 __device__ __forceinline__ void exact_pair(const Elems& E, int ta, int ia, int tb, int ib,
                                            const PairOut& o)
 {
-    if (!boxes_overlap(E.box(ta, ia), E.box(tb, ib))) return;
-    if (ta + tb == 3) {
-        const int f = ta == 2 ? ia : ib, e = ta == 2 ? ib : ia;
-        push_pair(o, false, (unsigned long long)f * (unsigned long long)E.ne + (unsigned long long)e);
-    } else if (ta == 1) {
-        const int lo = min(ia, ib), hi = max(ia, ib);
-        push_pair(o, true, (unsigned long long)lo * (unsigned long long)E.ne + (unsigned long long)hi);
-    } else {
-        const int f = ta == 2 ? ia : ib, v = ta == 2 ? ib : ia;
-        push_pair(o, false, (unsigned long long)f * (unsigned long long)E.nv + (unsigned long long)v);
-    }
+    if (boxes_overlap(E.box(ta, ia), E.box(tb, ib)))
+        push_pair(o, ta == 1 && tb == 1, element_pair_key(E, ta, ia, tb, ib));
 }
 
 __device__ __forceinline__ void test_pair(const Elems& E, const float* __restrict__ f32, int ta, int ia,
@@ -1022,20 +1022,17 @@ __global__ void k_large_pairs(const uint32_t* __restrict__ large, int nl, int ro
 }
 
 // ---------------------------------------------------------------------------
-// Small scenes: all pairs.  The grid only limits which pairs are tested, and
-// below some 10^5 elements its kernels (statistics, set-up, cell filter, items,
-// sort: ten launches, most of them a few threads' latency) and the item
-// count's read-back cost more than testing every pair.  Elements come in tiles
-// of kTile of one kind, with the tile's box; a block takes a pair of tiles and
-// ends at once when their boxes are apart.
-// Measured (one discrete call, with the grid -> all pairs): 27 cubes (491 edges,
-// 16 pairs of tiles) 290 -> 150 us, 10 icospheres (19 k edges, 17 k pairs) 366
-// -> 169, 25 icospheres (48 k, 103 k) 386 -> 253, 40 icospheres (77 k, 262 k) 427
-// -> 376, 8 slabs (61 k, 168 k) 607 -> 617, 80 icospheres (154 k, 1 M) 479 -> 792:
-// the lines cross between 10^5 and 3 10^5 pairs of tiles.
+// Small scenes: all pairs, two launches of a few microseconds.  Elements come in
+// tiles of kTile of one kind, with the tile's box; a block takes a pair of tiles
+// and ends at once when their boxes are apart.
+// Measured (a discrete and a continuous call, all pairs against patches): 27
+// cubes (491 edges, 16 pairs of tiles) 328 and 338 us, 216 cubes (480 pairs) 421
+// and 428, 54 hulls (800) 463 and 366, 28 icospheres (1.3 10^5) 838 and 611.
 
 constexpr int kTile = 128;
-constexpr int64_t kAllPairsTiles = 1 << 17;  // tile pairs up to which all pairs are tested
+constexpr int64_t kAllPairsTiles = 256;  // tile pairs up to which all pairs are tested
+
+constexpr int kTileCols = 8, kTileParts = kTile / kTileCols;
 
 struct ElemBox {
     float b[6];     // rounded outward; empty (+inf, -inf) for elements not included
@@ -1110,19 +1107,18 @@ __global__ void __launch_bounds__(kTile) k_tile_boxes(
     }
 }
 
-// A block per pair of tiles and part of the second tile (cols elements, so
+// A block per pair of tiles and part of the second tile (kTileCols elements, so
 // that few pairs of tiles still fill the GPU): edges with edges (tiles a <=
 // b), then faces with vertices, or (kPairsEF) faces with edges alone.  The
-// float tests of 32 elements come first, as a mask; the exact tests of the
-// pairs left then run for all threads together (in the loop over elements,
-// one thread's exact test would hold up its warp 128 times).
+// float tests come first, as a mask; the exact tests of the pairs left then run
+// for all threads together (in the loop over elements, one thread's exact test
+// would hold up its warp).
 __global__ void __launch_bounds__(kTile) k_all_pairs(Elems E, int kind, const ElemBox* __restrict__ eb,
-                                                     const float* __restrict__ tile_box, int cols_log2, PairOut o)
+                                                     const float* __restrict__ tile_box, PairOut o)
 {
-    __shared__ ElemBox sh[kTile];
+    __shared__ ElemBox sh[kTileCols];
     const int tv = tiles_of(E.nv), te = tiles_of(E.ne);
-    const int parts_log2 = 7 - cols_log2;
-    int p = blockIdx.x >> parts_log2, ta, tb, a, b;  // kinds and tiles
+    int p = blockIdx.x / kTileParts, ta, tb, a, b;  // kinds and tiles
     const int nee = kind == kPairsEF ? 0 : te * (te + 1) / 2;
     if (p < nee) {
         // row b of the triangle holds tiles a = 0 .. b
@@ -1141,30 +1137,28 @@ __global__ void __launch_bounds__(kTile) k_all_pairs(Elems E, int kind, const El
     }
     const int first[3] = { 0, tv, tv + te };
     if (fboxes_disjoint(tile_box + 6 * (first[ta] + a), tile_box + 6 * (first[tb] + b))) return;
-    const int cols = 1 << cols_log2;
-    const int ia = a * kTile + threadIdx.x, ib0 = b * kTile + ((blockIdx.x & ((1 << parts_log2) - 1)) << cols_log2);
+    const int ia = a * kTile + threadIdx.x, ib0 = b * kTile + (int)(blockIdx.x % kTileParts) * kTileCols;
     const int na = ta == 1 ? E.ne : E.nf, nb = tb == 0 ? E.nv : E.ne;
     ElemBox mine;
     mine.b[0] = INFINITY;
     if (ia < na) mine = eb[E.index(ta, ia)];
     ElemBox other;
     other.b[0] = INFINITY;
-    if ((int)threadIdx.x < cols && ib0 + (int)threadIdx.x < nb) other = eb[E.index(tb, ib0 + threadIdx.x)];
-    if ((int)threadIdx.x < cols) sh[threadIdx.x] = other;
+    if ((int)threadIdx.x < kTileCols && ib0 + (int)threadIdx.x < nb) other = eb[E.index(tb, ib0 + threadIdx.x)];
+    if ((int)threadIdx.x < kTileCols) sh[threadIdx.x] = other;
     __syncthreads();
     if (mine.b[0] == INFINITY) return;
     const bool tri = ta == 1 && tb == 1;
-    for (int c = 0; c < cols; c += 32) {
-        unsigned m = 0;
-        const int end = min(32, cols);
-        for (int j = 0; j < end; j++) {
-            const ElemBox& x = sh[c + j];
-            if (x.gr != mine.gr && x.scene == mine.scene && !fboxes_disjoint(mine.b, x.b) && (!tri || ib0 + c + j > ia))
-                m |= 1u << j;
-        }
-        for (; m; m &= m - 1) exact_pair(E, ta, ia, tb, ib0 + c + __ffs(m) - 1, o);
+    unsigned m = 0;
+    for (int j = 0; j < kTileCols; j++) {
+        const ElemBox& x = sh[j];
+        if (x.gr != mine.gr && x.scene == mine.scene && !fboxes_disjoint(mine.b, x.b) && (!tri || ib0 + j > ia))
+            m |= 1u << j;
     }
+    for (; m; m &= m - 1) exact_pair(E, ta, ia, tb, ib0 + __ffs(m) - 1, o);
 }
+
+#include "patch_pairs.cuh"
 
 // The canonical order of few pairs: each stream's keys are distinct, so a
 // pair's place is the number of smaller keys (4096 pairs: some 10 us in one
@@ -1387,6 +1381,65 @@ static uint64_t filter_slots(int64_t ntot)
     return t;
 }
 
+// pairs of element tiles of a call, and whether they are few enough to test all
+static int64_t tile_pairs_of(const Scene& s, int kind)
+{
+    const int64_t tv = tiles_of(s.nv), te = tiles_of(s.ne), tf = tiles_of(s.nf);
+    return kind == kPairsEF ? tf * te : te * (te + 1) / 2 + tf * tv;
+}
+
+// Set-up of a scene's patches, for scenes where all pairs are not tested.
+int build_patches(Ctx& c)
+{
+    Scene& s = c.s;
+    const int64_t ntot = (int64_t)s.nv + s.ne + s.nf;
+    int64_t body_tests = 0;
+    for (int k = 0; k < s.nscenes; k++) {
+        const int64_t n = s.h_scene_bstart[k + 1] - s.h_scene_bstart[k];
+        body_tests += n * n / 2;
+    }
+    s.num_patches = 0;
+    if (std::max(tile_pairs_of(s, kPairsEEFV), tile_pairs_of(s, kPairsEF)) <= kAllPairsTiles
+        || body_tests > kMaxBodyTests || ntot > INT32_MAX)
+        return RIGC_OK;
+    const int* starts[3] = { s.h_bvs.data(), s.h_bes.data(), s.h_bfs.data() };
+    const int base[3] = { 0, s.nv, s.nv + s.ne };
+    std::vector<Patch> patches;
+    std::vector<int> start((size_t)3 * (s.nb + 1));
+    for (int t = 0; t < 3; t++)
+        for (int b = 0; b <= s.nb; b++) {
+            start[(size_t)t * (s.nb + 1) + b] = (int)patches.size();
+            if (b == s.nb) break;
+            for (int i = starts[t][b]; i < starts[t][b + 1]; i += kPatch)
+                patches.push_back(Patch { base[t] + i, std::min(kPatch, starts[t][b + 1] - i), b, t });
+        }
+    RIGC_TRY(s.patches.reserve(patches.size() * sizeof(Patch)));
+    RIGC_TRY(s.patch_start.reserve(start.size() * sizeof(int)));
+    RIGC_TRY(s.patch_order.reserve((size_t)ntot * sizeof(uint32_t)));
+    RIGC_CUDA(cudaMemcpy(s.patches.ptr, patches.data(), patches.size() * sizeof(Patch), cudaMemcpyHostToDevice));
+    RIGC_CUDA(cudaMemcpy(s.patch_start.ptr, start.data(), start.size() * sizeof(int), cudaMemcpyHostToDevice));
+    DevBuf keys, keys_out, vals, tmp[3];
+    auto sorted = [&]() -> int {
+        RIGC_TRY(keys.reserve((size_t)ntot * 8));
+        RIGC_TRY(keys_out.reserve((size_t)ntot * 8));
+        RIGC_TRY(vals.reserve((size_t)ntot * 4));
+        RIGC_COUNT_LAUNCH();
+        k_patch_keys<<<grid_for(ntot, 256), 256, 0, c.stream>>>(
+            s.rest, s.edges, s.faces, s.vbody, s.ebody, s.fbody, s.rmax, s.nv, s.ne, s.nf, s.nb,
+            keys.as<uint64_t>(), vals.as<uint32_t>());
+        RIGC_TRY(radix_sort_pairs<uint64_t>(keys.as<uint64_t>(), vals.as<uint32_t>(), keys_out.as<uint64_t>(),
+                                            s.patch_order.as<uint32_t>(), ntot,
+                                            30 + bits_for((uint64_t)3 * s.nb), tmp[0], tmp[1], tmp[2], c.stream));
+        RIGC_CUDA(cudaStreamSynchronize(c.stream));
+        return RIGC_OK;
+    };
+    const int st = sorted();
+    for (DevBuf* b : { &keys, &keys_out, &vals, &tmp[0], &tmp[1], &tmp[2] }) b->release();
+    RIGC_TRY(st);
+    s.num_patches = (int)patches.size();
+    return RIGC_OK;
+}
+
 // Candidate pairs of the kind (kPairsEEFV: out.ee, out.fv; kPairsEF: (face,
 // edge) pairs in out.fv) between x0 and x1 (continuous) or at x0.
 int detect_pairs(Ctx& c, const double* x0, const double* x1, bool continuous, double infl, int kind,
@@ -1471,16 +1524,16 @@ int detect_pairs(Ctx& c, const double* x0, const double* x1, bool continuous, do
     const Elems E { c.vbox.as<double>(), c.ebox.as<double>(), c.fbox.as<double>(),
                     c.vin.as<char>(), c.ein.as<char>(), c.fin.as<char>(),
                     s.vbody, s.ebody, s.fbody, s.nv, s.ne, s.nf };
-    const int64_t tv = tiles_of(s.nv), te = tiles_of(s.ne), tf = tiles_of(s.nf);
-    const int64_t tile_pairs = kind == kPairsEF ? tf * te : te * (te + 1) / 2 + tf * tv;
+    const int64_t tiles = tiles_of(s.nv) + tiles_of(s.ne) + tiles_of(s.nf);
+    const int64_t tile_pairs = tile_pairs_of(s, kind);
     const bool all_pairs = tile_pairs <= kAllPairsTiles;
-    if (!all_pairs) {
-        RIGC_COUNT_LAUNCH();
-        k_edge_face_boxes<<<grid_for((int64_t)s.ne + s.nf, 256), 256, 0, st>>>(
-            s.edges, s.ne, s.faces, s.nf, c.vbox.as<double>(), c.vin.as<char>(), c.ebox.as<double>(),
-            c.ein.as<char>(), c.fbox.as<double>(), c.fin.as<char>());
-        RIGC_CUDA(cudaGetLastError());
-    }
+    // patches wherever they are built, until their lists run over: a discrete and
+    // a continuous call by the grid and by patches, 54 hulls 1025 and 366 us, 28
+    // icospheres 1169 and 611, 1000 icospheres 4603 and 2413; beyond some 32
+    // overlapping others a patch, its element tests cost what the grid's items do
+    bool by_patches = !all_pairs && s.num_patches > 0;
+    // counters: EE pairs, second stream's pairs, patch work items, patch pairs
+    unsigned long long* pn = reinterpret_cast<unsigned long long*>(c.d_scalars.as<char>() + 1024);
     int64_t nitems = 0;
     int nlarge = 0;
     int group_key_bits = 0;
@@ -1488,16 +1541,22 @@ int detect_pairs(Ctx& c, const double* x0, const double* x1, bool continuous, do
     ElemBox* elem_boxes = nullptr;
     float* tile_boxes = nullptr;
     if (all_pairs) {
-        RIGC_TRY(c.bp_f32.reserve((size_t)ntot * sizeof(ElemBox) + (size_t)(tv + te + tf) * 6 * sizeof(float) + 8));
+        RIGC_TRY(c.bp_f32.reserve((size_t)ntot * sizeof(ElemBox) + (size_t)tiles * 6 * sizeof(float) + 8));
         elem_boxes = c.bp_f32.as<ElemBox>();
         tile_boxes = reinterpret_cast<float*>(elem_boxes + ntot);
         RIGC_COUNT_LAUNCH();
-        k_tile_boxes<<<(unsigned)(tv + te + tf), kTile, 0, st>>>(
+        k_tile_boxes<<<(unsigned)tiles, kTile, 0, st>>>(
             s.edges, s.faces, E, s.bscene, s.grank, c.ebox.as<double>(), c.ein.as<char>(), c.fbox.as<double>(),
             c.fin.as<char>(), elem_boxes, tile_boxes);
         RIGC_CUDA(cudaGetLastError());
-    } else {
+    }
     // ---- 3. grid and cell filter
+    auto grid_items = [&]() -> int {
+    RIGC_COUNT_LAUNCH();
+    k_edge_face_boxes<<<grid_for((int64_t)s.ne + s.nf, 256), 256, 0, st>>>(
+        s.edges, s.ne, s.faces, s.nf, c.vbox.as<double>(), c.vin.as<char>(), c.ebox.as<double>(),
+        c.ein.as<char>(), c.fbox.as<double>(), c.fin.as<char>());
+    RIGC_CUDA(cudaGetLastError());
     RIGC_COUNT_LAUNCH();
     k_elem_stats<<<kStatBlocks, kStatThreads, 0, st>>>(E, d_part, d_part_n);
     RIGC_COUNT_LAUNCH();
@@ -1549,14 +1608,45 @@ int detect_pairs(Ctx& c, const double* x0, const double* x1, bool continuous, do
                                             nitems, group_key_bits, S[4], S[5], S[7],
                                             st));
     }
+    return RIGC_OK;
+    };
+    if (!all_pairs && !by_patches) RIGC_TRY(grid_items());
+    // ---- 3'. patches of the included bodies
+    float* patch_boxes = nullptr;
+    PatchLists pl {};
+    if (by_patches) {
+        const size_t np = (size_t)s.num_patches;
+        pl.cap_items = std::max<size_t>(1 << 14, 4 * np);
+        pl.cap_pairs = std::max<size_t>(1 << 16, kPatchPairsPerPatch * np);
+        RIGC_TRY(c.bp_f32.reserve(np * (kPatch + 1) * 6 * sizeof(float)));
+        RIGC_TRY(c.bp_patch.reserve(pl.cap_items * sizeof(int4) + pl.cap_pairs * sizeof(int2)
+                                    + (size_t)6 * s.nb * sizeof(int)));
+        patch_boxes = c.bp_f32.as<float>() + np * kPatch * 6;
+        pl.items = c.bp_patch.as<int4>();
+        pl.pairs = reinterpret_cast<int2*>(pl.items + pl.cap_items);
+        pl.n_items = pn + 2;
+        pl.n_pairs = pn + 3;
+        int* bounds = reinterpret_cast<int*>(pl.pairs + pl.cap_pairs);
+        RIGC_CUDA(cudaMemsetAsync(bounds, 0x7f, (size_t)6 * s.nb * sizeof(int), st));
+        RIGC_CUDA(cudaMemsetAsync(pn + 2, 0, 2 * sizeof(unsigned long long), st));
+        RIGC_COUNT_LAUNCH();
+        k_patch_boxes<<<grid_for((int64_t)np * 32, 128), 128, 0, st>>>(
+            s.patches.as<Patch>(), (int)np, s.patch_order.as<uint32_t>(), s.edges, s.faces, E, c.body_in.as<int>(),
+            c.bp_f32.as<float>(), patch_boxes, bounds);
+        RIGC_COUNT_LAUNCH();
+        k_body_pairs<<<grid_for((int64_t)s.nb * 32, 128), 128, 0, st>>>(
+            bounds, c.body_in.as<int>(), s.grank, s.bscene, s.scene_bstart, s.nb, s.patch_start.as<int>(), kind, pl);
+        RIGC_COUNT_LAUNCH();
+        k_patch_pairs<<<kPatchBlocks, 128, 0, st>>>(s.patch_start.as<int>(), s.nb, kind, patch_boxes, pl);
+        RIGC_CUDA(cudaGetLastError());
     }
     // ---- 5. pairs (retry once with exact capacity on overflow)
-    unsigned long long* pn = reinterpret_cast<unsigned long long*>(c.d_scalars.as<char>() + 1024);
-    unsigned long long cap_ee = std::max<unsigned long long>(1 << 16, (unsigned long long)(all_pairs ? 32 * ntot : nitems));
+    unsigned long long cap_ee = std::max<unsigned long long>(
+        1 << 16, (unsigned long long)(all_pairs ? 32 * ntot : by_patches ? 4 * ntot : nitems));
     unsigned long long cap_fv = cap_ee;
     cap_ee = std::max<unsigned long long>(cap_ee, (unsigned long long)c.bp_pair_hint[0]);
     cap_fv = std::max<unsigned long long>(cap_fv, (unsigned long long)c.bp_pair_hint[1]);
-    const float* f32 = c.bp_f32.as<float>();
+    const float* f32 = c.bp_f32.as<float>();  // (reserved again by the grid)
     for (int attempt = 0; attempt < 3; attempt++) {
         RIGC_TRY(c.pair_out.reserve((size_t)(cap_ee + cap_fv) * 8));
         PairOut o { c.pair_out.as<unsigned long long>(), c.pair_out.as<unsigned long long>() + cap_ee,
@@ -1564,9 +1654,12 @@ int detect_pairs(Ctx& c, const double* x0, const double* x1, bool continuous, do
         RIGC_CUDA(cudaMemsetAsync(pn, 0, 2 * sizeof(unsigned long long), st));
         if (all_pairs) {
             RIGC_COUNT_LAUNCH();
-            const int cols_log2 = tile_pairs <= 256 ? 3 : tile_pairs <= 1024 ? 4 : tile_pairs <= 4096 ? 5 : 7;
-            k_all_pairs<<<(unsigned)(tile_pairs << (7 - cols_log2)), kTile, 0, st>>>(E, kind, elem_boxes, tile_boxes,
-                                                                                    cols_log2, o);
+            k_all_pairs<<<(unsigned)(tile_pairs * kTileParts), kTile, 0, st>>>(E, kind, elem_boxes, tile_boxes, o);
+        }
+        if (by_patches) {
+            RIGC_COUNT_LAUNCH();
+            k_patch_elements<<<kPatchBlocks, 128, 0, st>>>(s.patches.as<Patch>(), s.patch_order.as<uint32_t>(),
+                                                           s.edges, s.faces, E, c.bp_f32.as<float>(), pl, o);
         }
         if (nitems > 0) {
             RIGC_COUNT_LAUNCH();
@@ -1587,9 +1680,19 @@ int detect_pairs(Ctx& c, const double* x0, const double* x1, bool continuous, do
             }
         }
         RIGC_CUDA(cudaGetLastError());
-        unsigned long long hn[2];
+        unsigned long long hn[4];
         RIGC_CUDA(cudaMemcpyAsync(hn, pn, sizeof(hn), cudaMemcpyDeviceToHost, st));
         RIGC_CUDA(cudaStreamSynchronize(st));
+        if (by_patches && (hn[2] > pl.cap_items || hn[3] > pl.cap_pairs)) {
+            // patches that meet too many others: the grid, from the boxes that are there
+            by_patches = false;
+            RIGC_TRY(grid_items());
+            f32 = c.bp_f32.as<float>();
+            cap_ee = std::max<unsigned long long>(cap_ee, (unsigned long long)nitems);
+            cap_fv = std::max<unsigned long long>(cap_fv, (unsigned long long)nitems);
+            attempt--;
+            continue;
+        }
         if (hn[0] <= cap_ee && hn[1] <= cap_fv) {
             out.num_ee = (int64_t)hn[0];
             out.num_fv = (int64_t)hn[1];

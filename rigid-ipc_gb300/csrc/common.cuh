@@ -118,6 +118,10 @@ struct Scene {
     int* bscene = nullptr;         // nb, scene of each body
     int* scene_bstart = nullptr;   // nscenes + 1, first body of each scene
     std::vector<int> h_scene_bstart, h_bes, h_bfs;
+    // patches of neighbouring elements (patch_pairs.cuh): the elements by type, body and Morton
+    // code, the patches, the first patch of each type's bodies; 0 patches: not built
+    int num_patches = 0;
+    DevBuf patch_order, patches, patch_start;
 };
 
 struct Candidates {
@@ -166,6 +170,7 @@ struct Ctx {
     DevBuf large_list;
     // hash grid: call state, deeper-bisection flags,
     // cell filter, per-element cell ranges, float boxes, item counts
+    DevBuf bp_patch;  // patch work items, patch pairs, body bounds
     DevBuf bp_misc, bp_deeper, bp_sig, bp_ec0, bp_eext, bp_f32, bp_cnt;
     int64_t bp_pair_hint[2] = { 0, 0 };  // largest EE / FV pair counts seen
     // The continuous broad phase leaves the interval frames of the included
