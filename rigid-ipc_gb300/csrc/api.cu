@@ -148,7 +148,7 @@ static void release_all(Ctx* c)
                        &c->fric.coef, &c->fric.v0c, &c->fric.V0, &c->fric.c_energy,
                        &c->fric.c_grad, &c->fric.c_blocks, &c->fric.grad, &c->fric.row_ptr,
                        &c->fric.col, &c->fric.val, &c->scene_toi, &c->scene_energy,
-                       &c->bp_patch, &c->s.patches, &c->s.patch_start, &c->s.patch_order,
+                       &c->bp_patch, &c->bp_hulls, &c->s.patches, &c->s.patch_start, &c->s.patch_order,
                        &c->bp_misc, &c->bp_deeper, &c->bp_sig, &c->bp_ec0,
                        &c->bp_eext, &c->bp_f32, &c->bp_cnt, &c->md_V, &c->md_rot,
                        &c->md_out, &c->isect.ee, &c->isect.fv };

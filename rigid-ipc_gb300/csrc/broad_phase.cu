@@ -215,8 +215,54 @@ __device__ __forceinline__ void vertex_at_frame(const double* f, const double rv
     iworld_vertex(R, p, rv, w);
 }
 
-// The whole bisection of RigidBodyHashGrid::compute_vertices_intervals for
-// one body per block: block b handles body b when it is included and
+// Accepted time nodes whose vertices are yet to be hulled (k_vertex_hulls)
+constexpr int kHullNodes = 1 << 14;
+struct HullNode {
+    int body, pad;
+    double frame[kHalfFrame];
+};
+struct HullList {
+    HullNode* nodes;  // kHullNodes
+    int* n;           // nodes appended (above kHullNodes: none written)
+    int* pending;     // per body: its nodes in the list
+};
+
+// hulls in the output array while nodes are pending: doubles as integers of
+// the same order (order_key), minima of lo and maxima of hi
+__device__ __forceinline__ double key_double(long long k)
+{
+    return __longlong_as_double(k ^ ((k >> 63) & 0x7fffffffffffffffll));
+}
+
+__device__ __forceinline__ void hull_vertex(const double* frame, const double* __restrict__ rest, int v,
+                                            long long* __restrict__ hull)
+{
+    const double rv[3] = { rest[3 * (size_t)v], rest[3 * (size_t)v + 1], rest[3 * (size_t)v + 2] };
+    Itv w[3];
+    vertex_at_frame(frame, rv, w);
+    for (int j = 0; j < 3; j++) {
+        atomicMin(hull + 6 * (size_t)v + j, order_key(w[j].lo));
+        atomicMax(hull + 6 * (size_t)v + 3 + j, order_key(w[j].hi));
+    }
+}
+
+// inflate; a vertex with an empty coordinate stays excluded
+__device__ __forceinline__ void finish_vertex(double* __restrict__ vbox, int v, double infl, char* __restrict__ vin)
+{
+    const long long* hull = reinterpret_cast<const long long*>(vbox);
+    bool ok = true;
+    for (int j = 0; j < 3; j++) {
+        const double lo = key_double(__ldcg(hull + 6 * (size_t)v + j));
+        const double hi = key_double(__ldcg(hull + 6 * (size_t)v + 3 + j));
+        if (!(lo <= hi)) ok = false;
+        vbox[6 * (size_t)v + j] = RSUB(lo, infl);
+        vbox[6 * (size_t)v + 3 + j] = RADD(hi, infl);
+    }
+    vin[v] = ok ? 1 : 0;
+}
+
+// The bisection of RigidBodyHashGrid::compute_vertices_intervals for one body
+// per block: block b handles body b when it is included and
 // k_vertex_boxes_half flagged it (a vertex of one of the forced halves left
 // the padded scene box).  A time node is accepted when every vertex fits
 // the padded scene box (or at depth 16), else both halves are visited; the
@@ -224,36 +270,52 @@ __device__ __forceinline__ void vertex_at_frame(const double* f, const double rv
 // depend on the order nodes are visited.  So nodes are taken from the stack
 // kVBBatch at a time: warp 0 computes their frames in parallel (one interval
 // rotation is a long chain of dependent FP64 operations), then the block
-// checks and hulls every (node, vertex) pair.  Each round pops up to
-// kVBBatch nodes and pushes at most twice as many one level deeper, so the
-// stack never holds more than 2 kVBBatch nodes per depth.
-// vbox holds lo[3], hi[3] per vertex.
+// checks every (node, vertex) pair.  Each round pops up to kVBBatch nodes and
+// pushes at most twice as many one level deeper, so the stack never holds
+// more than 2 kVBBatch nodes per depth.
+//
+// Few bodies are flagged (those at the scene's rim), so one block's FP64 unit
+// was the bound: 72 FP64 instructions per node and vertex, 12 us a node of a
+// 642-vertex icosphere.  The check runs in single precision with an error
+// bound, in double where that cannot decide (|w| of the exact bounds from the
+// same sums, each rounding 2^-24 of the terms' sum; 2^-20 is asked), and the
+// accepted nodes are hulled by k_vertex_hulls over the whole GPU.  A pile of
+// 131 icospheres: 847 -> 116 us; of 417 and of 1000: 192 -> 40 with the hulls.
+// vbox holds the hulls' lo[3], hi[3] per vertex.
 __global__ void __launch_bounds__(kVBThreads)
 k_vertex_boxes_cont(const double* __restrict__ x0, const double* __restrict__ x1,
                     const double* __restrict__ rest, const int* __restrict__ bvs,
                     const int* __restrict__ body_in, const int* __restrict__ deeper,
                     const double* __restrict__ table, const double* __restrict__ domain,
-                    double infl, double* __restrict__ vbox, char* __restrict__ vin)
+                    double infl, double* __restrict__ vbox, char* __restrict__ vin, HullList list)
 {
     __shared__ double st_lo[kMaxTNodes], st_hi[kMaxTNodes];
     __shared__ int st_depth[kMaxTNodes];
-    __shared__ int sp, nbat;
+    __shared__ int sp, nbat, slot[kVBBatch], listed;
     __shared__ double b_lo[kVBBatch], b_hi[kVBBatch];
     __shared__ int b_depth[kVBBatch], b_fail[kVBBatch];
     __shared__ double sF[kVBBatch][kHalfFrame];
+    __shared__ float sf[kVBBatch][kHalfFrame];
     const int b = blockIdx.x;
     if (!body_in[b] || !deeper[b]) return;  // uniform over the block
-    const int v0 = bvs[b], v1 = bvs[b + 1], nvb = v1 - v0;
-    double dlo[3] = { domain[0], domain[1], domain[2] }, dhi[3] = { domain[3], domain[4], domain[5] };
-    // hull accumulators in the output array
+    const int v0 = bvs[b], v1 = bvs[b + 1];
+    const double dlo[3] = { domain[0], domain[1], domain[2] }, dhi[3] = { domain[3], domain[4], domain[5] };
+    float lim[6], size[3];  // bounds of the vertices' intervals, magnitudes
+    for (int j = 0; j < 3; j++) {
+        lim[j] = (float)(dlo[j] + infl);
+        lim[3 + j] = (float)(dhi[j] - infl);
+        size[j] = fabsf((float)infl) + fmaxf(fabsf((float)dlo[j]), fabsf((float)dhi[j]));
+    }
+    long long* hull = reinterpret_cast<long long*>(vbox);
     for (int v = v0 + threadIdx.x; v < v1; v += blockDim.x)
         for (int j = 0; j < 3; j++) {
-            vbox[6 * (size_t)v + j] = INFINITY;
-            vbox[6 * (size_t)v + 3 + j] = -INFINITY;
+            hull[6 * (size_t)v + j] = order_key(INFINITY);
+            hull[6 * (size_t)v + 3 + j] = order_key(-INFINITY);
         }
     if (threadIdx.x == 0) {
         // forced first bisection: [0, 0.5] and [0.5, 1], depth 1
         sp = 0;
+        listed = 0;
         double m = RMUL(0.5, RADD(0.0, 1.0));
         st_lo[sp] = m; st_hi[sp] = 1.0; st_depth[sp] = 1; sp++;
         st_lo[sp] = 0.0; st_hi[sp] = m; st_depth[sp] = 1; sp++;
@@ -262,81 +324,123 @@ k_vertex_boxes_cont(const double* __restrict__ x0, const double* __restrict__ x1
         __syncthreads();
         if (sp == 0) break;
         // pop up to kVBBatch nodes
-        if (threadIdx.x < kVBBatch) {
-            const int nb_ = min(sp, kVBBatch);
-            if ((int)threadIdx.x < nb_) {
-                const int q = sp - nb_ + threadIdx.x;
-                b_lo[threadIdx.x] = st_lo[q];
-                b_hi[threadIdx.x] = st_hi[q];
-                b_depth[threadIdx.x] = st_depth[q];
-                b_fail[threadIdx.x] = 0;
+        const int nq = min(sp, kVBBatch);
+        if ((int)threadIdx.x < nq) {
+            const int q = sp - nq + threadIdx.x;
+            b_lo[threadIdx.x] = st_lo[q];
+            b_hi[threadIdx.x] = st_hi[q];
+            b_depth[threadIdx.x] = st_depth[q];
+            b_fail[threadIdx.x] = 0;
+            // nodes of depth <= 6 from the table (their intervals are the
+            // dyadic [k 2^-d, (k + 1) 2^-d], midpoints being exact), deeper
+            // ones computed here
+            const int d = st_depth[q];
+            if (d < 7) {
+                const int k = (int)ldexp(st_lo[q], d);
+                const double* f = table + ((size_t)b * kRotTableSlots + (1 << d) - 1 + k) * kRotTableEntry;
+                for (int j = 0; j < kHalfFrame; j++) sF[threadIdx.x][j] = f[j];
+            } else {
+                body_time_frame(x0, x1, b, st_lo[q], st_hi[q], sF[threadIdx.x]);
+            }
+        }
+        __syncthreads();
+        for (int k = threadIdx.x; k < nq * kHalfFrame; k += blockDim.x)
+            sf[k / kHalfFrame][k % kHalfFrame] = (float)sF[k / kHalfFrame][k % kHalfFrame];
+        __syncthreads();
+        for (int v = v0 + threadIdx.x; v < v1; v += blockDim.x) {
+            const double rv[3] = { rest[3 * (size_t)v], rest[3 * (size_t)v + 1], rest[3 * (size_t)v + 2] };
+            const float r[3] = { (float)rv[0], (float)rv[1], (float)rv[2] };
+            for (int k = 0; k < nq; k++) {
+                if (b_fail[k]) continue;
+                int out = -1;  // inside, 0 unknown, 1 outside
+                for (int j = 0; j < 3; j++) {
+                    float lo = sf[k][18 + 2 * j], hi = sf[k][19 + 2 * j], mag = size[j] + fabsf(lo) + fabsf(hi);
+                    for (int i = 0; i < 3; i++) {
+                        const float p = r[i] * sf[k][6 * j + 2 * i], q = r[i] * sf[k][6 * j + 2 * i + 1];
+                        lo += fminf(p, q);
+                        hi += fmaxf(p, q);
+                        mag += fabsf(p) + fabsf(q);  // (not finite: unknown)
+                    }
+                    const float e = 9.5367431640625e-07f * mag, g = fminf(lo - lim[j], lim[3 + j] - hi);
+                    out = max(out, g > e ? -1 : (g < -e ? 1 : 0));
+                }
+                if (out == 0) {
+                    Itv w[3];
+                    vertex_at_frame(sF[k], rv, w);
+                    for (int j = 0; j < 3; j++)
+                        if (RSUB(w[j].lo, infl) < dlo[j] || RADD(w[j].hi, infl) > dhi[j]) out = 1;
+                }
+                if (out == 1) b_fail[k] = 1;
             }
         }
         __syncthreads();
         if (threadIdx.x == 0) {
-            nbat = min(sp, kVBBatch);
-            sp -= nbat;
-        }
-        __syncthreads();
-        const int nq = nbat;
-        if ((int)threadIdx.x < nq) {
-            // nodes of depth <= 6 from the table (their intervals are the
-            // dyadic [k 2^-d, (k + 1) 2^-d], midpoints being exact), deeper
-            // ones computed here
-            const int d = b_depth[threadIdx.x];
-            if (d < 7) {
-                const int k = (int)ldexp(b_lo[threadIdx.x], d);
-                const double* f = table + ((size_t)b * kRotTableSlots + (1 << d) - 1 + k) * kRotTableEntry;
-                for (int j = 0; j < kHalfFrame; j++) sF[threadIdx.x][j] = f[j];
-            } else {
-                body_time_frame(x0, x1, b, b_lo[threadIdx.x], b_hi[threadIdx.x], sF[threadIdx.x]);
-            }
-        }
-        __syncthreads();
-        for (int idx = threadIdx.x; idx < nq * nvb; idx += blockDim.x) {
-            const int k = idx / nvb, v = v0 + idx % nvb;
-            const double rv[3] = { rest[3 * (size_t)v], rest[3 * (size_t)v + 1], rest[3 * (size_t)v + 2] };
-            Itv w[3];
-            vertex_at_frame(sF[k], rv, w);
-            for (int j = 0; j < 3; j++)
-                if (RSUB(w[j].lo, infl) < dlo[j] || RADD(w[j].hi, infl) > dhi[j]) b_fail[k] = 1;
-        }
-        __syncthreads();
-        // accepted nodes: hull into the vertex boxes (each thread owns its vertices)
-        for (int v = v0 + threadIdx.x; v < v1; v += blockDim.x) {
-            const double rv[3] = { rest[3 * (size_t)v], rest[3 * (size_t)v + 1], rest[3 * (size_t)v + 2] };
+            nbat = 0;
+            sp -= nq;
             for (int k = 0; k < nq; k++) {
-                if (b_fail[k] && b_depth[k] < kMaxTDepth) continue;
-                Itv w[3];
-                vertex_at_frame(sF[k], rv, w);
-                for (int j = 0; j < 3; j++) {
-                    vbox[6 * (size_t)v + j] = smin(vbox[6 * (size_t)v + j], w[j].lo);
-                    vbox[6 * (size_t)v + 3 + j] = smax(vbox[6 * (size_t)v + 3 + j], w[j].hi);
+                if (b_fail[k] && b_depth[k] < kMaxTDepth) {
+                    // rejected: both halves, one level deeper
+                    const double tl = b_lo[k], th = b_hi[k];
+                    const double m = RMUL(0.5, RADD(tl, th));
+                    if (sp + 2 <= kMaxTNodes) {
+                        st_lo[sp] = m; st_hi[sp] = th; st_depth[sp] = b_depth[k] + 1; sp++;
+                        st_lo[sp] = tl; st_hi[sp] = m; st_depth[sp] = b_depth[k] + 1; sp++;
+                    }
+                } else {
+                    slot[nbat++] = k;
                 }
             }
         }
-        // rejected nodes: both halves, one level deeper
-        if (threadIdx.x == 0)
-            for (int k = 0; k < nq; k++) {
-                if (!b_fail[k] || b_depth[k] >= kMaxTDepth) continue;
-                const double tl = b_lo[k], th = b_hi[k];
-                const double m = RMUL(0.5, RADD(tl, th));
-                if (sp + 2 <= kMaxTNodes) {
-                    st_lo[sp] = m; st_hi[sp] = th; st_depth[sp] = b_depth[k] + 1; sp++;
-                    st_lo[sp] = tl; st_hi[sp] = m; st_depth[sp] = b_depth[k] + 1; sp++;
-                }
+        __syncthreads();
+        // accepted nodes: listed, or hulled here when the list is full
+        const int na = nbat;
+        __syncthreads();
+        if (threadIdx.x == 0 && na > 0) {
+            nbat = atomicAdd(list.n, na);
+            if (nbat + na <= kHullNodes) listed += na;
+        }
+        __syncthreads();
+        const int at = nbat;
+        if (na == 0) continue;
+        if (at + na <= kHullNodes) {
+            for (int k = threadIdx.x; k < na * kHalfFrame; k += blockDim.x) {
+                HullNode& h = list.nodes[at + k / kHalfFrame];
+                h.frame[k % kHalfFrame] = sF[slot[k / kHalfFrame]][k % kHalfFrame];
+                if (k % kHalfFrame == 0) h.body = b;
             }
+        } else {
+            for (int k = threadIdx.x; k < na && at + k < kHullNodes; k += blockDim.x) list.nodes[at + k].body = -1;
+            for (int v = v0 + threadIdx.x; v < v1; v += blockDim.x)
+                for (int k = 0; k < na; k++) hull_vertex(sF[slot[k]], rest, v, hull);
+        }
     }
-    // inflate; a vertex with an empty coordinate stays excluded
-    for (int v = v0 + threadIdx.x; v < v1; v += blockDim.x) {
-        bool ok = true;
-        for (int j = 0; j < 3; j++) {
-            double lo = vbox[6 * (size_t)v + j], hi = vbox[6 * (size_t)v + 3 + j];
-            if (!(lo <= hi)) ok = false;
-            vbox[6 * (size_t)v + j] = RSUB(lo, infl);
-            vbox[6 * (size_t)v + 3 + j] = RADD(hi, infl);
-        }
-        vin[v] = ok ? 1 : 0;
+    if (threadIdx.x == 0) list.pending[b] = listed;
+    if (listed == 0)
+        for (int v = v0 + threadIdx.x; v < v1; v += blockDim.x) finish_vertex(vbox, v, infl, vin);
+}
+
+// A block per listed node: its body's vertices; the block that ends a body's
+// last node makes its boxes.
+__global__ void __launch_bounds__(kVBThreads) k_vertex_hulls(HullList list, const double* __restrict__ rest,
+                                                             const int* __restrict__ bvs, double infl,
+                                                             double* __restrict__ vbox, char* __restrict__ vin)
+{
+    __shared__ int last;
+    const int n = min(*list.n, kHullNodes);
+    for (int k = blockIdx.x; k < n; k += gridDim.x) {
+        const HullNode& h = list.nodes[k];
+        const int b = h.body;
+        if (b < 0) continue;
+        const int v0 = bvs[b], v1 = bvs[b + 1];
+        for (int v = v0 + threadIdx.x; v < v1; v += blockDim.x)
+            hull_vertex(h.frame, rest, v, reinterpret_cast<long long*>(vbox));
+        __threadfence();
+        __syncthreads();
+        if (threadIdx.x == 0) last = atomicSub(list.pending + b, 1) == 1;
+        __syncthreads();
+        if (!last) continue;
+        __threadfence();
+        for (int v = v0 + threadIdx.x; v < v1; v += blockDim.x) finish_vertex(vbox, v, infl, vin);
     }
 }
 
@@ -1493,14 +1597,18 @@ int detect_pairs(Ctx& c, const double* x0, const double* x1, bool continuous, do
     RIGC_TRY(c.fin.reserve((size_t)s.nf + 8));
     if (continuous) {
         RIGC_TRY(reserve_rot_table(c));
-        RIGC_TRY(c.bp_deeper.reserve((size_t)s.nb * sizeof(int)));
+        // flags, hull list: its length and the bodies' pending nodes
+        const size_t deeper_bytes = ((size_t)2 * s.nb + 1) * sizeof(int);
+        RIGC_TRY(c.bp_deeper.reserve(deeper_bytes));
+        RIGC_TRY(c.bp_hulls.reserve(kHullNodes * sizeof(HullNode)));
+        const HullList hulls { c.bp_hulls.as<HullNode>(), c.bp_deeper.as<int>() + s.nb, c.bp_deeper.as<int>() + s.nb + 1 };
         double* table = c.rot_table.as<double>();
         RIGC_COUNT_LAUNCH();
         k_scene_box<<<1, 256, 0, st>>>(c.body_box.as<double>(), c.body_in.as<int>(), s.nb, d_domain);
         RIGC_COUNT_LAUNCH();
         k_bp_frames<<<grid_for((int64_t)s.nb * kRotTableSlots, 128), 128, 0, st>>>(
             x0, x1, c.body_in.as<int>(), s.nb, kDefaultToiTol, table);
-        RIGC_CUDA(cudaMemsetAsync(c.bp_deeper.ptr, 0, (size_t)s.nb * sizeof(int), st));
+        RIGC_CUDA(cudaMemsetAsync(c.bp_deeper.ptr, 0, deeper_bytes, st));
         RIGC_COUNT_LAUNCH();
         k_vertex_boxes_half<<<grid_for(s.nv, 128), 128, 0, st>>>(
             s.rest, s.vbody, c.body_in.as<int>(), s.nv, table, d_domain, infl,
@@ -1508,7 +1616,10 @@ int detect_pairs(Ctx& c, const double* x0, const double* x1, bool continuous, do
         RIGC_COUNT_LAUNCH();
         k_vertex_boxes_cont<<<(unsigned)s.nb, kVBThreads, 0, st>>>(
             x0, x1, s.rest, s.bvs, c.body_in.as<int>(), c.bp_deeper.as<int>(), table, d_domain,
-            infl, c.vbox.as<double>(), c.vin.as<char>());
+            infl, c.vbox.as<double>(), c.vin.as<char>(), hulls);
+        RIGC_COUNT_LAUNCH();
+        k_vertex_hulls<<<152 * 2, kVBThreads, 0, st>>>(hulls, s.rest, s.bvs, infl, c.vbox.as<double>(),
+                                                       c.vin.as<char>());
     } else {
         const double* rot = nullptr;
         if (s.nv > kDirectVertices) {

@@ -171,6 +171,7 @@ struct Ctx {
     // hash grid: call state, deeper-bisection flags,
     // cell filter, per-element cell ranges, float boxes, item counts
     DevBuf bp_patch;  // patch work items, patch pairs, body bounds
+    DevBuf bp_hulls;  // time nodes whose vertices are yet to be hulled
     DevBuf bp_misc, bp_deeper, bp_sig, bp_ec0, bp_eext, bp_f32, bp_cnt;
     int64_t bp_pair_hint[2] = { 0, 0 };  // largest EE / FV pair counts seen
     // The continuous broad phase leaves the interval frames of the included

@@ -57,6 +57,9 @@ def _make(kind):
         P = rng.normal(size=(50, 3))
         P = 2.1 * P / np.linalg.norm(P, axis=1, keepdims=True)
         return _scene(M, np.concatenate([[[0, 0, 0]], P])), None, False
+    if kind == "rim":  # bodies that turn at the scene's rim, more time nodes than the list takes
+        P = np.stack([0.7 * (np.arange(1600) // 40), np.zeros(1600), 0.7 * (np.arange(1600) % 40)], 1)
+        return _scene([_hull(rng, 16 + i % 9) for i in range(1600)], P), None, False
     # boxes in one another: their patches all overlap, their elements do not
     M = [meshes.cube(1.0 + 0.01 * i) for i in range(400)] + [_hull(rng, 40) for _ in range(6)]
     P = np.concatenate([np.zeros((400, 3)), rng.uniform(-0.5, 0.5, (6, 3)) + [9, 0, 0]])
@@ -64,7 +67,7 @@ def _make(kind):
 
 
 @pytest.mark.parametrize("continuous", [False, True])
-@pytest.mark.parametrize("kind", ["tiles", "patches", "scenes", "one_large", "nested"])
+@pytest.mark.parametrize("kind", ["tiles", "patches", "scenes", "one_large", "nested", "rim"])
 def test_candidates(oracle, kind, continuous):
     import rigc
 
@@ -72,6 +75,8 @@ def test_candidates(oracle, kind, continuous):
     rng = np.random.default_rng(3)
     x0 = sc.poses()
     x1 = x0 + rng.normal(0, 0.02, x0.shape) if continuous else x0
+    if continuous and kind == "rim":
+        x1.reshape(-1, 6)[:, 3:] = x0.reshape(-1, 6)[:, 3:] + rng.normal(0, 2.0, (sc.num_bodies, 3))
     infl = 0.0 if continuous else 1e-3
     ctx = rigc.Context(sc, scene_of_body=sob)
     ee, fv = ctx.detect_collision_candidates_rigid(x0, x1, continuous, infl)
