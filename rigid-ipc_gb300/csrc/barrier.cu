@@ -10,21 +10,19 @@
 // local_hessian_to_global_triplets (:1157-1179) and merge_derivative_storage
 // (:1260-1297).
 //
-// Derivation used by k_barrier_local.  With X the constraint's vertex
-// positions and x the two bodies' 6-dof poses, X_i = R_b v_i + p_b and
-// J_i = dX_i/dx_b = [I | D_i], D_i[:, k] = (dR/dtheta_k) v_i.
-//  * PT / EE: d = u^2 / D with u = (A x B).w and D = |A x B|^2, where
-//    A, B, w are signed sums of the vertices (coefficients alpha, beta,
-//    gamma).  grad u = {alpha_i (B x w) + beta_i (w x A) + gamma_i n},
-//    grad D = {2 alpha_i (B x n) + 2 beta_i (n x A)}; the Hessians are
-//    Gram(dn) terms and skew bilinear blocks [s_ij]x between vertices i != j.
-//  * PE: d = |a x b|^2 / |e|^2, the same pieces with a Gram(de) term.
-//  * PP: d = |w|^2.
-// f = weight * m(D) * b(d - dmin^2) (m = 1 except mollified EE), so the body
-// Hessian is  sum of outer products of the body-space gradients of the basic
-// scalars + Gram terms + skew pair blocks + the curvature term
-// sum_i grad_Xi f . d2X_i/dtheta2.  It is then projected to the PSD cone,
-// V max(L, 0) V^T (local_terms.cuh).
+// Derivation used by k_barrier_local.  The distances are functions of a few
+// signed sums of the vertices:
+//  * PT / EE: d = u^2 / D with u = n.W, n = A x B and D = |n|^2;
+//  * PE: d = |n|^2 / |W|^2, W the edge;
+//  * PP: d = |W|^2;
+//  * a mollified EE whose closest feature is an endpoint has its edges' n and a
+//    PE or PP distance of its own (P x Q and W).
+// f = weight * m(D) * b(d - dmin^2) (m = 1 except mollified EE).  Along a pose
+// coordinate the vectors move by dA .. dW (a body's part of A moves by dR/dtheta_k
+// times that part's rest vector), which gives the scalars' derivatives; the body
+// Hessian is a quadratic form of those, products of the moved vectors, and the
+// curvature term sum_i grad_Xi f . d2X_i/dtheta2 (BarrierBase).  It is then
+// projected to the PSD cone, V max(L, 0) V^T (local_terms.cuh).
 #include <algorithm>
 
 #include "common.cuh"
@@ -101,279 +99,128 @@ __device__ __forceinline__ int local_body_of(int type, int i)
     return i == 0 ? 0 : 1;
 }
 
-// A mollified EE constraint whose closest features are endpoints (kept as EE
-// by the constraint set because the edges are nearly parallel): f = w m(D)
-// b(d - dmin^2) with D = |A x B|^2 of the two edges and d the point-point or
-// point-edge squared distance of the closest features.  Vertex-space
-// gradients and 3x3 Hessian blocks in closed form:
-//   grad D_i = 2 M_i^T n, M_i = alpha_i (-[B]x) + beta_i [A]x,
-//   hess D_ij = 2 M_i^T M_j + 2 (beta_i alpha_j - alpha_i beta_j) [n]x,
-// and the same for N = |a x b|^2 of a point-edge distance d = N / |e|^2, so the
-// body Hessian is outer products of the body-space gradients, Gram terms, skew
-// pair blocks and the curvature term, as barrier_build's: bound by FP64 issue,
-// and most constraints of box-like bodies in contact end here (104 k of 163 k
-// between 32 slabs).  J_i^T (.) J_j of the ten 3x3 vertex blocks took 2.20 ms
-// there, with the other kinds, unprojected; this 1.34 ms (338 constraints
-// between 27 cubes, one per lane: 256 -> 212 us).
-static __device__ __noinline__ bool ee_endpoint_build(const BarrierArgs& a, int64_t ci, SMat H,
-                                                      const Vtx* V, const double (*vrest)[3],
-                                                      const int* lbody, const double* const* fr,
-                                                      int dtype)
-{
-    const double weight = a.cweight[ci];
-    int kind = 1, p = 0, q = 0, e0 = 0, e1 = 0;
-    switch (dtype) {
-    case EE_EA0_EB0: kind = 0; p = 0; q = 2; break;
-    case EE_EA0_EB1: kind = 0; p = 0; q = 3; break;
-    case EE_EA1_EB0: kind = 0; p = 1; q = 2; break;
-    case EE_EA1_EB1: kind = 0; p = 1; q = 3; break;
-    case EE_EA_EB0: p = 2; e0 = 0; e1 = 1; break;
-    case EE_EA_EB1: p = 3; e0 = 0; e1 = 1; break;
-    case EE_EA0_EB: p = 0; e0 = 2; e1 = 3; break;
-    default: p = 1; e0 = 2; e1 = 3; break;
-    }
-    const double alD[4] = { -1, 1, 0, 0 }, beD[4] = { 0, 0, -1, 1 };
-    double A[3], B[3], n[3];
-    for (int j = 0; j < 3; j++) {
-        A[j] = V[1].X[j] - V[0].X[j];
-        B[j] = V[3].X[j] - V[2].X[j];
-    }
-    cross(A, B, n);
-    const double Dm = dot(n, n);
-    double gD[4][3], gd[4][3];
-    {
-        double Bn[3], nA[3];
-        cross(B, n, Bn);
-        cross(n, A, nA);
-        for (int i = 0; i < 4; i++)
-            for (int j = 0; j < 3; j++) {
-                gD[i][j] = 2 * (alD[i] * Bn[j] + beD[i] * nA[j]);
-                gd[i][j] = 0;
-            }
-    }
-    double d, N = 0, De = 1;
-    double pa[3], pb[3], c[3], e[3];
-    double alE[4] = { 0, 0, 0, 0 }, beE[4] = { 0, 0, 0, 0 }, gaE[4] = { 0, 0, 0, 0 };
-    double gN[4][3], gE[4][3];
-    if (kind == 0) {
-        double w[3];
-        for (int j = 0; j < 3; j++) w[j] = V[p].X[j] - V[q].X[j];
-        d = dot(w, w);
-        for (int j = 0; j < 3; j++) {
-            gd[p][j] = 2 * w[j];
-            gd[q][j] = -2 * w[j];
-        }
-    } else {
-        alE[p] = -1; alE[e0] = 1; beE[p] = -1; beE[e1] = 1; gaE[e0] = -1; gaE[e1] = 1;
-        for (int j = 0; j < 3; j++) {
-            pa[j] = V[e0].X[j] - V[p].X[j];
-            pb[j] = V[e1].X[j] - V[p].X[j];
-            e[j] = V[e1].X[j] - V[e0].X[j];
-        }
-        cross(pa, pb, c);
-        N = dot(c, c);
-        De = dot(e, e);
-        d = N / De;
-        double bc[3], ca[3];
-        cross(pb, c, bc);
-        cross(c, pa, ca);
-        for (int i = 0; i < 4; i++)
-            for (int j = 0; j < 3; j++) {
-                gN[i][j] = 2 * (alE[i] * bc[j] + beE[i] * ca[j]);
-                gE[i][j] = 2 * gaE[i] * e[j];
-                gd[i][j] = gN[i][j] / De - N / (De * De) * gE[i][j];
-            }
-    }
-    // barrier of the shifted squared distance and the mollifier
-    const double s = 2 * a.dmin * a.dhat + a.dhat * a.dhat;
-    const double dd = d - a.dmin * a.dmin;
-    double bv = 0, b1 = 0, b2 = 0;
-    bool active = dd < s;
-    if (dd <= 0.0) {
-        bv = INFINITY;
-        active = false;
-    } else if (active) {
-        double lg = log(dd / s);
-        double dm = dd - s;
-        bv = -dm * dm * lg;
-        b1 = (s - dd) * (2 * lg - s / dd + 1);
-        double sd = s / dd;
-        b2 = (sd + 2) * sd - 2 * lg - 3;
-    }
-    double m = 1, m1 = 0, m2 = 0;
-    if (Dm < a.ceps[ci]) {
-        double ie = 1.0 / a.ceps[ci];
-        double xe = Dm * ie;
-        m = (2 - xe) * xe;
-        m1 = (2 - 2 * xe) * ie;
-        m2 = -2 * ie * ie;
-    }
-    if (a.energy) a.energy[ci] = weight * m * bv;
-    const bool want_g = (a.flags & (RIGC_GRAD | RIGC_HESS)) != 0;
-    const bool want_h = (a.flags & RIGC_HESS) != 0;
-    if (!active) {
-        if (a.grad)
-            for (int k = 0; k < 12; k++) a.grad[ci * 12 + k] = 0;
-        if (a.blocks && want_h)
-            for (int k = 0; k < 144; k++) a.blocks[ci * 144 + k] = 0;
-        if (a.hess && want_h)
-            for (int k = 0; k < 144; k++) a.hess[ci * 144 + k] = 0;
-        return false;
-    }
-    if (!want_g) return false;
-    double gv[4][3];
-    for (int i = 0; i < 4; i++)
-        for (int j = 0; j < 3; j++) gv[i][j] = weight * (m * b1 * gd[i][j] + bv * m1 * gD[i][j]);
-    double G[12];
-    to_body(V, lbody, 4, gv, G);
-    if (a.grad)
-        for (int k = 0; k < 12; k++) a.grad[ci * 12 + k] = G[k];
-    if (!want_h) return false;
+// What a constraint's terms are made of: cross products n = A x B and c = P x Q
+// (c: the point-edge distance of a mollified EE whose closest feature is an
+// endpoint) and a vector W, each of A, B, P, Q, W a signed sum of the vertices.
+// Along coordinate r of the bodies' poses they move by dA .. dW, and with
+//   N' = tn.dn + tw.dW + tc.dc,  E' = 2 W.dW,  D' = 2 n.dn
+// the gradient is g.(N', E', D') and the Hessian entry
+//   (N', E', D') C (N', E', D')^T + k1 dn.dn + kx (dn.dW + dW.dn) + kw dW.dW
+//   + k2 dc.dc + y1 (dA x dB + dA x dB) n + y2 (dP x dQ + dP x dQ) c (W's part
+//   of the vector in Y1), the products of coordinate r's and column's vectors,
+// plus the curvature of the rotations, the second derivatives of the vertices.
+struct BarrierBase {
+    double A[3], B[3], P[3], Q[3], W[3];
+    double n[3], c[3];
+    double tn[3], tw[3], tc[3];
+    double Y1[3], Y2[3];
+    double k1, kx, kw, k2;
+    double C[6];              // NN, NE, ND, EE, ED, DD
+    double g[3];
+    double f[5][3];           // derivatives of f in A .. W
+    double s[5];              // sums of A, B, P, Q, W's coefficients on body a's vertices
+    double v[2][5][3];        // the bodies' parts of A .. W in rest positions
+    double S[2][9];           // sum of (df/dX_i) v_i^T over the bodies' vertices
+    int cross2;               // P, Q, c are there
+};
+constexpr int kCoord = 24;    // stored per coordinate: Y1 x dA, dB, dn, dW, N', E', D', Y2 x dP, dQ, dc
+enum BarrierState { kNothing, kGradient, kHessian };
 
-    H.clear();
-    const double cd = weight * m * b1, cD = weight * bv * m1;  // on hess d, hess D
-    const double kdd = weight * m * b2, kdD = weight * m1 * b1, kDD = weight * bv * m2;
-    double M[4][9];
-    // M_i = alpha_i (-[B]x) + beta_i [A]x (dn/dX_i, likewise of c = pa x pb)
-    auto skew_of = [](double sa, const double* Bv, double sb, const double* Av, double* Mi) {
-        const double v0 = -sa * Bv[0] + sb * Av[0], v1 = -sa * Bv[1] + sb * Av[1], v2 = -sa * Bv[2] + sb * Av[2];
-        Mi[0] = 0; Mi[1] = -v2; Mi[2] = v1;
-        Mi[3] = v2; Mi[4] = 0; Mi[5] = -v0;
-        Mi[6] = -v1; Mi[7] = v0; Mi[8] = 0;
-    };
-    for (int i = 0; i < 4; i++) skew_of(alD[i], B, beD[i], A, M[i]);
-    add_gram(H, 2 * cD, V, lbody, 4, M);
-    double gr[3][kRed];
-    to_body(V, lbody, 4, gD, G);
-    reduce12(G, gr[2]);
-    if (kind == 0) {
-        // d = |w|^2: hess = 2 (dw)^T (dw)
-        to_body(V, lbody, 4, gd, G);
-        reduce12(G, gr[1]);
-        add_quadratic(H, kdd, kdD, kDD, gr[1], gr[2]);
-        for (int i = 0; i < 4; i++) {
-            for (int k = 0; k < 9; k++) M[i][k] = 0;
-            M[i][0] = M[i][4] = M[i][8] = i == p ? 1.0 : (i == q ? -1.0 : 0.0);
-        }
-        add_gram(H, 2 * cd, V, lbody, 4, M);
-    } else {
-        // grad d = gN / De - N / De^2 gE,
-        // hess d = (1/De) H_N - (1/De^2)(gN gE + gE gN) + (2N/De^3) gE gE - (N/De^2) H_E
-        const double pn = 1 / De, pe = -N / (De * De);
-        to_body(V, lbody, 4, gN, G);
-        reduce12(G, gr[0]);
-        to_body(V, lbody, 4, gE, G);
-        reduce12(G, gr[1]);
-        double gdr[kRed];  // reduced body gradient of d
-        for (int k = 0; k < kRed; k++) gdr[k] = pn * gr[0][k] + pe * gr[1][k];
-        add_quadratic(H, kdd, kdD, kDD, gdr, gr[2]);
-        add_quadratic(H, 0, -cd / (De * De), 2 * cd * N / (De * De * De), gr[0], gr[1]);
-        for (int i = 0; i < 4; i++) skew_of(alE[i], pb, beE[i], pa, M[i]);
-        add_gram(H, 2 * cd / De, V, lbody, 4, M);
-        for (int i = 0; i < 4; i++) {
-            for (int k = 0; k < 9; k++) M[i][k] = 0;
-            M[i][0] = M[i][4] = M[i][8] = gaE[i];
-        }
-        add_gram(H, 2 * cd * pe, V, lbody, 4, M);
-    }
-    for (int i = 0; i < 4; i++)
-        for (int j = i + 1; j < 4; j++) {
-            const double kD = 2 * cD * (beD[i] * alD[j] - alD[i] * beD[j]);
-            const double kN = kind == 1 ? 2 * cd / De * (beE[i] * alE[j] - alE[i] * beE[j]) : 0.0;
-            if (kD == 0 && kN == 0) continue;
-            double sv[3];
-            for (int k = 0; k < 3; k++) sv[k] = kD * n[k] + (kind == 1 ? kN * c[k] : 0.0);
-            add_skew_pair(H, V[i], lbody[i], V[j], lbody[j], sv);
-        }
-    add_curvature(H, fr, lbody, 4, vrest, gv);
-    return true;
+__device__ __forceinline__ void add_outer3(double* S, const double* g, const double* v)
+{
+    for (int j = 0; j < 3; j++)
+        for (int k = 0; k < 3; k++) S[3 * j + k] = fma(g[j], v[k], S[3 * j + k]);
 }
 
-// Energy, gradient and (reduced) unprojected body Hessian of constraint ci
-// into H; returns true when H holds a Hessian to project and
-// write, false when every output of the constraint is already written.
-static __device__ __noinline__ bool barrier_build(const BarrierArgs& a, int64_t ci, SMat H)
+// The vectors, scalars and coefficients of a constraint; its energy.  Run by
+// every lane of the constraint's group, written by the first.
+static __device__ __noinline__ int barrier_base(const BarrierArgs& a, int64_t ci, bool first, BarrierBase& o)
 {
-    if (a.check_nv >= 0 && !constraint_in_range(a, ci)) {
-        const double nan = __longlong_as_double(0x7ff8000000000000ll);
-        if (a.energy) a.energy[ci] = nan;
+    auto fill = [&](double v) {
+        if (!first) return;
         if (a.grad)
-            for (int k = 0; k < 12; k++) a.grad[ci * 12 + k] = nan;
+            for (int k = 0; k < 12; k++) a.grad[ci * 12 + k] = v;
         if (a.flags & RIGC_HESS) {
             if (a.blocks)
-                for (int k = 0; k < 144; k++) a.blocks[ci * 144 + k] = nan;
+                for (int k = 0; k < 144; k++) a.blocks[ci * 144 + k] = v;
             if (a.hess)
-                for (int k = 0; k < 144; k++) a.hess[ci * 144 + k] = nan;
+                for (int k = 0; k < 144; k++) a.hess[ci * 144 + k] = v;
         }
-        return false;
+    };
+    if (a.check_nv >= 0 && !constraint_in_range(a, ci)) {
+        const double nan = __longlong_as_double(0x7ff8000000000000ll);
+        if (a.energy && first) a.energy[ci] = nan;
+        fill(nan);
+        return kNothing;
     }
     const int type = a.ctype[ci];
     const int nvc = type == 0 ? 2 : (type == 1 ? 3 : 4);
     const double weight = a.cweight[ci];
-    int lbody[4];
-    const double* fr[2];
-    int bod[2] = { a.cbodies[2 * ci], a.cbodies[2 * ci + 1] };
-    fr[0] = a.frames + (size_t)bod[0] * 96;
-    fr[1] = a.frames + (size_t)bod[1] * 96;
-    Vtx V[4];
-    double vrest[4][3];
+    double X[4][3], vr[4][3];
     for (int i = 0; i < nvc; i++) {
-        lbody[i] = local_body_of(type, i);
-        int vi = a.cverts[4 * ci + i];
-        const double* f = fr[lbody[i]];
-        for (int j = 0; j < 3; j++) vrest[i][j] = a.rest[3 * (size_t)vi + j];
-        const double* v = vrest[i];
-        for (int j = 0; j < 3; j++) {
-            V[i].X[j] = f[3 * j] * v[0] + f[3 * j + 1] * v[1] + f[3 * j + 2] * v[2] + f[90 + j];
-            for (int k = 0; k < 3; k++) {
-                const double* dR = f + 9 + 9 * k;
-                V[i].D[j][k] = dR[3 * j] * v[0] + dR[3 * j + 1] * v[1] + dR[3 * j + 2] * v[2];
-            }
-        }
+        const double* f = a.frames + (size_t)a.cbodies[2 * ci + local_body_of(type, i)] * 96;
+        const int vi = a.cverts[4 * ci + i];
+        for (int j = 0; j < 3; j++) vr[i][j] = a.rest[3 * (size_t)vi + j];
+        for (int j = 0; j < 3; j++)
+            X[i][j] = f[3 * j] * vr[i][0] + f[3 * j + 1] * vr[i][1] + f[3 * j + 2] * vr[i][2] + f[90 + j];
     }
-
+    // end: an EE's closest feature is an endpoint: 1 two points, 2 a point and an edge
+    int end = 0, p = 0, e0 = 0, e1 = 0;
     if (type == 2) {
-        const int dt = ee_type_rn(V[0].X, V[1].X, V[2].X, V[3].X);
-        if (dt != EE_EA_EB) return ee_endpoint_build(a, ci, H, V, vrest, lbody, fr, dt);
-    }
-
-    // coefficient patterns: A = sum alpha_i X_i, B = sum beta_i X_i, w = sum gamma_i X_i
-    double al[4] = { 0, 0, 0, 0 }, be[4] = { 0, 0, 0, 0 }, ga[4] = { 0, 0, 0, 0 };
-    double A[3], B[3], W[3], n[3];
-    double d, u = 0, Dn = 0;
-    if (type == 2) {        // EE: A = X1 - X0, B = X3 - X2, w = X2 - X0
-        al[0] = -1; al[1] = 1; be[2] = -1; be[3] = 1; ga[0] = -1; ga[2] = 1;
-    } else if (type == 3) { // FV: A = X2 - X1, B = X3 - X1, w = X0 - X1
-        al[1] = -1; al[2] = 1; be[1] = -1; be[3] = 1; ga[0] = 1; ga[1] = -1;
-    } else if (type == 1) { // EV: a = X1 - X0, b = X2 - X0 ; e = X2 - X1 (gamma)
-        al[0] = -1; al[1] = 1; be[0] = -1; be[2] = 1; ga[1] = -1; ga[2] = 1;
-    } else {                // VV: w = X0 - X1
-        ga[0] = 1; ga[1] = -1;
-    }
-    for (int j = 0; j < 3; j++) {
-        A[j] = 0; B[j] = 0; W[j] = 0;
-        for (int i = 0; i < nvc; i++) {
-            A[j] += al[i] * V[i].X[j];
-            B[j] += be[i] * V[i].X[j];
-            W[j] += ga[i] * V[i].X[j];
+        switch (ee_type_rn(X[0], X[1], X[2], X[3])) {
+        case EE_EA_EB: break;
+        case EE_EA0_EB0: end = 1; p = 0; e0 = 2; break;
+        case EE_EA0_EB1: end = 1; p = 0; e0 = 3; break;
+        case EE_EA1_EB0: end = 1; p = 1; e0 = 2; break;
+        case EE_EA1_EB1: end = 1; p = 1; e0 = 3; break;
+        case EE_EA_EB0: end = 2; p = 2; e0 = 0; e1 = 1; break;
+        case EE_EA_EB1: end = 2; p = 3; e0 = 0; e1 = 1; break;
+        case EE_EA0_EB: end = 2; p = 0; e0 = 2; e1 = 3; break;
+        default: end = 2; p = 1; e0 = 2; e1 = 3; break;
         }
     }
-    double De = 0;
-    if (type >= 2) {
-        cross(A, B, n);
-        u = dot(n, W);
-        Dn = dot(n, n);
-        d = u * u / Dn;
-    } else if (type == 1) {
-        cross(A, B, n);  // c = a x b
-        Dn = dot(n, n);  // N = |c|^2
-        De = dot(W, W);  // |e|^2
-        d = Dn / De;
-    } else {
-        d = dot(W, W);
-        n[0] = n[1] = n[2] = 0;
+    // the vectors as differences of vertices (to, from)
+    int to[5] = { 0, 0, 0, 0, 0 }, from[5] = { 0, 0, 0, 0, 0 };
+    if (type == 2) {        // A = X1 - X0, B = X3 - X2, W = X2 - X0
+        to[0] = 1; to[1] = 3; from[1] = 2; to[4] = 2;
+        if (end == 1) {     // W between the two points
+            to[4] = p; from[4] = e0;
+        } else if (end == 2) {  // P, Q from the point to the edge's ends, W the edge
+            to[2] = e0; from[2] = p; to[3] = e1; from[3] = p; to[4] = e1; from[4] = e0;
+        }
+    } else if (type == 3) { // A = X2 - X1, B = X3 - X1, W = X0 - X1
+        to[0] = 2; from[0] = 1; to[1] = 3; from[1] = 1; from[4] = 1;
+    } else if (type == 1) { // A = X1 - X0, B = X2 - X0, W the edge X2 - X1
+        to[0] = 1; to[1] = 2; to[4] = 2; from[4] = 1;
+    } else {                // W = X0 - X1
+        from[4] = 1;
     }
-
+    o.cross2 = end == 2;
+    double* vec[5] = { o.A, o.B, o.P, o.Q, o.W };
+    for (int q = 0; q < 5; q++) {
+        const int t = to[q], f = from[q], bt = local_body_of(type, t), bf = local_body_of(type, f);
+        for (int j = 0; j < 3; j++) {
+            vec[q][j] = X[t][j] - X[f][j];
+            const double vt = vr[t][j], vf = vr[f][j];
+            o.v[0][q][j] = (bt == 0 ? vt : 0.0) - (bf == 0 ? vf : 0.0);
+            o.v[1][q][j] = (bt == 1 ? vt : 0.0) - (bf == 1 ? vf : 0.0);
+        }
+        o.s[q] = (double)((bt == 0) - (bf == 0));
+    }
+    cross(o.A, o.B, o.n);
+    cross(o.P, o.Q, o.c);
+    const double nn = dot(o.n, o.n), ww = dot(o.W, o.W), cc = dot(o.c, o.c);
+    double u = 0, d;
+    if (type == 0 || end == 1) {
+        d = ww;
+    } else if (type == 1) {
+        d = nn / ww;
+    } else if (end == 2) {
+        d = cc / ww;
+    } else {
+        u = dot(o.n, o.W);
+        d = u * u / nn;
+    }
     // barrier of the shifted squared distance
     const double s = 2 * a.dmin * a.dhat + a.dhat * a.dhat;
     const double dd = d - a.dmin * a.dmin;
@@ -392,188 +239,266 @@ static __device__ __noinline__ bool barrier_build(const BarrierArgs& a, int64_t 
     }
     // EE mollifier m(D), D = |A x B|^2
     double m = 1, m1 = 0, m2 = 0;
-    if (type == 2 && Dn < a.ceps[ci]) {
+    if (type == 2 && nn < a.ceps[ci]) {
         double ie = 1.0 / a.ceps[ci];
-        double xe = Dn * ie;
+        double xe = nn * ie;
         m = (2 - xe) * xe;
         m1 = (2 - 2 * xe) * ie;
         m2 = -2 * ie * ie;
     }
-    if (a.energy) a.energy[ci] = weight * m * bv;
-    const bool want_g = (a.flags & (RIGC_GRAD | RIGC_HESS)) != 0;
-    const bool want_h = (a.flags & RIGC_HESS) != 0;
+    if (a.energy && first) a.energy[ci] = weight * m * bv;
     if (!active) {
-        if (a.grad)
-            for (int k = 0; k < 12; k++) a.grad[ci * 12 + k] = 0;
-        if (a.blocks && want_h)
-            for (int k = 0; k < 144; k++) a.blocks[ci * 144 + k] = 0;
-        if (a.hess && want_h)
-            for (int k = 0; k < 144; k++) a.hess[ci * 144 + k] = 0;
-        return false;
+        fill(0.0);
+        return kNothing;
     }
-    if (!want_g) return false;
+    if (!(a.flags & (RIGC_GRAD | RIGC_HESS))) return kNothing;
 
-    // ---- basic scalars and their vertex-space gradients
-    // g1: gradient of the first scalar (u, N or d), g2: of the second (D, |e|^2)
-    double g1v[4][3], g2v[4][3];
-    double c1, c2;  // grad d = c1 g1 + c2 g2
-    if (type >= 2) {
-        double Bw[3], wA[3], Bn[3], nA[3];
-        cross(B, W, Bw);
-        cross(W, A, wA);
-        cross(B, n, Bn);
-        cross(n, A, nA);
-        for (int i = 0; i < 4; i++)
-            for (int j = 0; j < 3; j++) {
-                g1v[i][j] = al[i] * Bw[j] + be[i] * wA[j] + ga[i] * n[j];
-                g2v[i][j] = 2 * (al[i] * Bn[j] + be[i] * nA[j]);
-            }
-        c1 = 2 * u / Dn;
-        c2 = -u * u / (Dn * Dn);
-    } else if (type == 1) {
-        double bc[3], ca[3];
-        cross(B, n, bc);
-        cross(n, A, ca);
-        for (int i = 0; i < 3; i++)
-            for (int j = 0; j < 3; j++) {
-                g1v[i][j] = 2 * (al[i] * bc[j] + be[i] * ca[j]);
-                g2v[i][j] = 2 * ga[i] * W[j];
-            }
-        c1 = 1 / De;
-        c2 = -Dn / (De * De);
-    } else {
-        for (int j = 0; j < 3; j++) {
-            g1v[0][j] = 2 * W[j];
-            g1v[1][j] = -2 * W[j];
-            g2v[0][j] = g2v[1][j] = 0;
-        }
-        c1 = 1;
-        c2 = 0;
-    }
-    // f = weight * m * b(d):  grad f = P_g1 g1 + P_g2 g2
+    // f = weight m(D) b(d).  Hessian of d in the scalars:
+    //  PT/EE: (2/D) u'u' - (2u/D^2)(u'D' + D'u') + (2u^2/D^3) D'D' + (2u/D) u'' - (u^2/D^2) D''
+    //  PE:    -(1/E^2)(N'E' + E'N') + (2N/E^3) E'E' + (1/E) N'' - (N/E^2) E'',  E = |W|^2
+    //  PP:    W''
     const double wm = weight * m;
-    // (the mollifier's gradient lies along grad D = g2, EE only)
-    const double Pg1 = wm * b1 * c1;
-    const double Pg2 = wm * b1 * c2 + (type == 2 ? weight * bv * m1 : 0.0);
-    double gv[4][3];
-    for (int i = 0; i < nvc; i++)
-        for (int j = 0; j < 3; j++) gv[i][j] = Pg1 * g1v[i][j] + Pg2 * g2v[i][j];
-    double G[12];
-    to_body(V, lbody, nvc, gv, G);
-    if (a.grad)
-        for (int k = 0; k < 12; k++) a.grad[ci * 12 + k] = G[k];
-    if (!want_h) return false;
-
-    // ---- Hessian
-    H.clear();
-    double G12[2][kRed];
-    to_body(V, lbody, nvc, g1v, G);
-    reduce12(G, G12[0]);
-    to_body(V, lbody, nvc, g2v, G);
-    reduce12(G, G12[1]);
-    // second-derivative coefficients of d in terms of (g1, g2) and the
-    // Hessians of the basic scalars:
-    //  PT/EE: hess d = (2/D) g1g1 + c1 H_u - (2u/D^2)(g1g2 + g2g1) + (2u^2/D^3) g2g2 + c2 H_D
-    //  PE:    hess d = (1/De) H_N - (1/De^2)(g1g2 + g2g1) + (2N/De^3) g2g2 + c2 H_e
-    //  PP:    hess d = H_w (Gram of dw)
-    double duu, duD, dDD;
-    if (type >= 2) {
-        duu = 2 / Dn;
-        duD = -2 * u / (Dn * Dn);
-        dDD = 2 * u * u / (Dn * Dn * Dn);
-    } else if (type == 1) {
-        duu = 0;
-        duD = -1 / (De * De);
-        dDD = 2 * Dn / (De * De * De);
+    const double P1 = wm * b2, P2 = wm * b1;               // on d'd' and d''
+    const double P3 = weight * bv * m2, P4 = weight * bv * m1, P5 = weight * m1 * b1;  // D'D', D'', d'D' (EE)
+    for (int q = 0; q < 6; q++) o.C[q] = 0;
+    for (int j = 0; j < 3; j++) o.tn[j] = o.tw[j] = o.tc[j] = o.Y1[j] = o.Y2[j] = 0;
+    o.k1 = o.kx = o.kw = o.k2 = 0;
+    o.g[0] = o.g[1] = o.g[2] = 0;
+    if (type == 0 || end == 1) {
+        o.C[0] = P1;
+        o.C[2] = P5;
+        o.C[5] = P3;
+        o.g[0] = P2;
+        o.g[2] = P4;
+        o.kw = 2 * P2;
+        o.k1 = 2 * P4;
+        for (int j = 0; j < 3; j++) {
+            o.tw[j] = 2 * o.W[j];
+            o.Y1[j] = 2 * P4 * o.n[j];
+        }
+    } else if (type == 1 || end == 2) {
+        const double N = type == 1 ? nn : cc, c1 = 1 / ww, c2 = -N / (ww * ww);
+        o.C[0] = P1 * c1 * c1;
+        o.C[1] = P1 * c1 * c2 - P2 / (ww * ww);
+        o.C[3] = P1 * c2 * c2 + P2 * (2 * N / (ww * ww * ww));
+        o.C[2] = P5 * c1;
+        o.C[4] = P5 * c2;
+        o.C[5] = P3;
+        o.g[0] = P2 * c1;
+        o.g[1] = P2 * c2;
+        o.g[2] = P4;
+        o.kw = 2 * P2 * c2;
+        const double kN = 2 * P2 * c1;
+        if (type == 1) o.k1 = kN;
+        else {
+            o.k1 = 2 * P4;
+            o.k2 = kN;
+        }
+        for (int j = 0; j < 3; j++) {
+            (type == 1 ? o.tn : o.tc)[j] = 2 * (type == 1 ? o.n : o.c)[j];
+            o.Y1[j] = o.k1 * o.n[j];
+            o.Y2[j] = o.k2 * o.c[j];
+        }
     } else {
-        duu = duD = dDD = 0;
+        const double c1 = 2 * u / nn, c2 = -u * u / (nn * nn);
+        o.C[0] = P1 * c1 * c1 + P2 * (2 / nn);
+        o.C[2] = P1 * c1 * c2 - P2 * (2 * u / (nn * nn)) + P5 * c1;
+        o.C[5] = P1 * c2 * c2 + P2 * (2 * u * u / (nn * nn * nn)) + P3 + 2 * P5 * c2;
+        o.g[0] = P2 * c1;
+        o.g[2] = P2 * c2 + P4;
+        o.kx = P2 * c1;
+        o.k1 = 2 * (P2 * c2 + P4);
+        for (int j = 0; j < 3; j++) {
+            o.tn[j] = o.W[j];
+            o.tw[j] = o.n[j];
+            o.Y1[j] = o.kx * o.W[j] + o.k1 * o.n[j];
+        }
     }
-    // f Hessian = P1 gd gd^T + P2 hess d + [EE] P3 g2g2 + P4 H_D + P5 (g2 gd^T + gd g2^T)
-    const double P1 = wm * b2, P2 = wm * b1;
-    const double P3 = type == 2 ? weight * bv * m2 : 0.0;
-    const double P4 = type == 2 ? weight * bv * m1 : 0.0;
-    const double P5 = type == 2 ? weight * m1 * b1 : 0.0;
-    const double a11 = P1 * c1 * c1 + P2 * duu;
-    const double a12 = P1 * c1 * c2 + P2 * duD + P5 * c1;
-    const double a22 = P1 * c2 * c2 + P2 * dDD + P3 + 2 * P5 * c2;
-    add_quadratic(H, a11, a12, a22, G12[0], G12[1]);
-
-    // coefficients of the scalar Hessians
-    const double bu = P2 * c1;            // on H_u (PT/EE) or H_N (PE)
-    const double bD = P2 * c2 + P4;       // on H_D (PT/EE) or H_e (PE)
-    double M[4][9];
-    if (type >= 2) {
-        // H_D Gram part: 2 (dn)^T(dn), dn/dX_i = alpha_i(-[B]x) + beta_i [A]x
-        for (int i = 0; i < 4; i++) {
-            double* Mi = M[i];
-            double sa = al[i], sb = be[i];
-            // -[B]x * sa + [A]x * sb
-            double v0 = -sa * B[0] + sb * A[0], v1 = -sa * B[1] + sb * A[1], v2 = -sa * B[2] + sb * A[2];
-            Mi[0] = 0; Mi[1] = -v2; Mi[2] = v1;
-            Mi[3] = v2; Mi[4] = 0; Mi[5] = -v0;
-            Mi[6] = -v1; Mi[7] = v0; Mi[8] = 0;
-        }
-        add_gram(H, 2 * bD, V, lbody, 4, M);
-        // skew pair blocks: s_ij = bu * s_ij(u) + bD * s_ij(D)
-        for (int i = 0; i < 4; i++)
-            for (int j = i + 1; j < 4; j++) {
-                double sv[3];
-                for (int k = 0; k < 3; k++) {
-                    double su = -al[i] * be[j] * W[k] + al[j] * be[i] * W[k]
-                        + al[i] * ga[j] * B[k] - al[j] * ga[i] * B[k]
-                        - be[i] * ga[j] * A[k] + be[j] * ga[i] * A[k];
-                    double sD = 2 * (-al[i] * be[j] * n[k] + al[j] * be[i] * n[k]);
-                    sv[k] = bu * su + bD * sD;
-                }
-                if (sv[0] == 0 && sv[1] == 0 && sv[2] == 0) continue;
-                add_skew_pair(H, V[i], lbody[i], V[j], lbody[j], sv);
-            }
-    } else if (type == 1) {
-        // H_N = 2 (dc)^T(dc) + skew(c); H_e = 2 (de)^T(de)
-        for (int i = 0; i < 3; i++) {
-            double* Mi = M[i];
-            double sa = al[i], sb = be[i];
-            double v0 = -sa * B[0] + sb * A[0], v1 = -sa * B[1] + sb * A[1], v2 = -sa * B[2] + sb * A[2];
-            Mi[0] = 0; Mi[1] = -v2; Mi[2] = v1;
-            Mi[3] = v2; Mi[4] = 0; Mi[5] = -v0;
-            Mi[6] = -v1; Mi[7] = v0; Mi[8] = 0;
-        }
-        add_gram(H, 2 * bu, V, lbody, 3, M);
-        for (int i = 0; i < 3; i++) {
-            double* Mi = M[i];
-            for (int k = 0; k < 9; k++) Mi[k] = 0;
-            Mi[0] = Mi[4] = Mi[8] = ga[i];
-        }
-        add_gram(H, 2 * bD, V, lbody, 3, M);
-        for (int i = 0; i < 3; i++)
-            for (int j = i + 1; j < 3; j++) {
-                double sv[3];
-                for (int k = 0; k < 3; k++)
-                    sv[k] = bu * 2 * (-al[i] * be[j] * n[k] + al[j] * be[i] * n[k]);
-                if (sv[0] == 0 && sv[1] == 0 && sv[2] == 0) continue;
-                add_skew_pair(H, V[i], lbody[i], V[j], lbody[j], sv);
-            }
-    } else {
-        // d = |w|^2: hess = 2 (dw)^T (dw), coefficient P2 (c1 = 1)
-        for (int i = 0; i < 2; i++) {
-            double* Mi = M[i];
-            for (int k = 0; k < 9; k++) Mi[k] = 0;
-            Mi[0] = Mi[4] = Mi[8] = ga[i];
-        }
-        add_gram(H, 2 * P2, V, lbody, 2, M);
+    // derivatives of f in A .. W, then S
+    double q1[3], q2[3], (*gr)[3] = o.f;
+    for (int j = 0; j < 3; j++) {
+        q1[j] = o.g[0] * o.tn[j] + 2 * o.g[2] * o.n[j];
+        q2[j] = o.g[0] * o.tc[j];
+        gr[4][j] = o.g[0] * o.tw[j] + 2 * o.g[1] * o.W[j];
     }
-    // curvature of the rigid maps
-    add_curvature(H, fr, lbody, nvc, vrest, gv);
-    return true;
+    cross(o.B, q1, gr[0]);
+    cross(q1, o.A, gr[1]);
+    cross(o.Q, q2, gr[2]);
+    cross(q2, o.P, gr[3]);
+    if (!(a.flags & RIGC_HESS)) return kGradient;
+    for (int b = 0; b < 2; b++) {
+        for (int k = 0; k < 9; k++) o.S[b][k] = 0;
+        for (int q = 0; q < 5; q++)
+            if (o.cross2 || q < 2 || q == 4) add_outer3(o.S[b], gr[q], o.v[b][q]);
+    }
+    return kHessian;
 }
 
+__device__ __forceinline__ void fcross(const double* x, const double* y, double* r)
+{
+    for (int j = 0; j < 3; j++) {
+        const int k = (j + 1) % 3, l = (j + 2) % 3;
+        r[j] = fma(x[k], y[l], -__dmul_rn(x[l], y[k]));
+    }
+}
+__device__ __forceinline__ double fdot(const double* x, const double* y, double s)
+{
+    return fma(x[2], y[2], fma(x[1], y[1], fma(x[0], y[0], s)));
+}
+
+// Coordinate r: its vectors and scalars into st, its gradient
+static __device__ __noinline__ double barrier_coord(const BarrierBase& o, const double* fa, const double* fb, int r,
+                                                    double* st, int stride)
+{
+    double d[5][3];
+    if (r < 3) {
+        for (int q = 0; q < 5; q++)
+            for (int j = 0; j < 3; j++) d[q][j] = j == r ? o.s[q] : 0.0;
+    } else {
+        const int b = r >= 6;
+        const double* M = (b ? fb : fa) + 9 + 9 * (r - (b ? 6 : 3));
+        for (int q = 0; q < 5; q++) {
+            if ((q == 2 || q == 3) && !o.cross2) continue;
+            for (int j = 0; j < 3; j++) d[q][j] = fdot(M + 3 * j, o.v[b][q], 0.0);
+        }
+    }
+    double x[3], y[3], dn[3];
+    fcross(d[0], o.B, x);
+    fcross(o.A, d[1], y);
+    for (int j = 0; j < 3; j++) dn[j] = __dadd_rn(x[j], y[j]);
+    fcross(o.Y1, d[0], x);
+    double N = fdot(o.tn, dn, fdot(o.tw, d[4], 0.0));
+    for (int j = 0; j < 3; j++) {
+        st[j * stride] = x[j];
+        st[(3 + j) * stride] = d[1][j];
+        st[(6 + j) * stride] = dn[j];
+        st[(9 + j) * stride] = d[4][j];
+    }
+    if (o.cross2) {
+        double dc[3];
+        fcross(d[2], o.Q, x);
+        fcross(o.P, d[3], y);
+        for (int j = 0; j < 3; j++) dc[j] = __dadd_rn(x[j], y[j]);
+        fcross(o.Y2, d[2], x);
+        N = fdot(o.tc, dc, N);
+        for (int j = 0; j < 3; j++) {
+            st[(15 + j) * stride] = x[j];
+            st[(18 + j) * stride] = d[3][j];
+            st[(21 + j) * stride] = dc[j];
+        }
+    }
+    const double E = __dmul_rn(2.0, fdot(o.W, d[4], 0.0)), D = __dmul_rn(2.0, fdot(o.n, dn, 0.0));
+    st[12 * stride] = N;
+    st[13 * stride] = E;
+    st[14 * stride] = D;
+    // by the forces on A .. W (the scalars' parts, N' and D' of a shallow angle
+    // above all, cancel in them before they are rounded)
+    double G = fdot(o.f[1], d[1], fdot(o.f[0], d[0], 0.0));
+    if (o.cross2) G = fdot(o.f[3], d[3], fdot(o.f[2], d[2], G));
+    return fdot(o.f[4], d[4], G);
+}
+
+// Entries (r, col), r <= col, from the coordinates' values
+static __device__ __noinline__ void barrier_column(const BarrierBase& o, const double* fa, const double* fb, int col,
+                                                   const double* st, int stride, SMat H)
+{
+    const double* sc = st + col * kCoord * stride;
+    double ya[3], db[3], z[3], t[3], q[3];
+    const double N = sc[12 * stride], E = sc[13 * stride], D = sc[14 * stride];
+    q[0] = fma(o.C[2], D, fma(o.C[1], E, __dmul_rn(o.C[0], N)));
+    q[1] = fma(o.C[4], D, fma(o.C[3], E, __dmul_rn(o.C[1], N)));
+    q[2] = fma(o.C[5], D, fma(o.C[4], E, __dmul_rn(o.C[2], N)));
+    for (int j = 0; j < 3; j++) {
+        ya[j] = sc[j * stride];
+        db[j] = sc[(3 + j) * stride];
+        const double dn = sc[(6 + j) * stride], dw = sc[(9 + j) * stride];
+        z[j] = fma(o.kx, dw, __dmul_rn(o.k1, dn));
+        t[j] = fma(o.kw, dw, __dmul_rn(o.kx, dn));
+    }
+    for (int r = 0; r <= col; r++) {
+        const double* sr = st + r * kCoord * stride;
+        double h = fma(q[2], sr[14 * stride], fma(q[1], sr[13 * stride], __dmul_rn(q[0], sr[12 * stride])));
+        double k = 0.0;
+        for (int j = 0; j < 3; j++) {
+            h = fma(sr[j * stride], db[j], h);
+            k = fma(sr[(3 + j) * stride], ya[j], k);
+            h = fma(sr[(6 + j) * stride], z[j], h);
+            k = fma(sr[(9 + j) * stride], t[j], k);
+        }
+        H.at(r, col) = __dadd_rn(h, k);
+    }
+    if (o.cross2) {
+        for (int j = 0; j < 3; j++) {
+            ya[j] = sc[(15 + j) * stride];
+            db[j] = sc[(18 + j) * stride];
+            z[j] = __dmul_rn(o.k2, sc[(21 + j) * stride]);
+        }
+        for (int r = 0; r <= col; r++) {
+            const double* sr = st + r * kCoord * stride;
+            double h = H.at(r, col);
+            for (int j = 0; j < 3; j++) {
+                h = fma(sr[(15 + j) * stride], db[j], h);
+                h = fma(sr[(18 + j) * stride], ya[j], h);
+                h = fma(sr[(21 + j) * stride], z[j], h);
+            }
+            H.at(r, col) = h;
+        }
+    }
+    if (col < 3) return;
+    // curvature: the second derivatives of the column's body's rotation
+    const int b = col >= 6, l = col - (b ? 6 : 3);
+    const double* d2 = (b ? fb : fa) + 36;
+    for (int k = 0; k <= l; k++) {
+        const double* M = d2 + 9 * sym_index(k, l);
+        double h = H.at(col - l + k, col);
+        for (int e = 0; e < 9; e++) h = fma(M[e], o.S[b][e], h);
+        H.at(col - l + k, col) = h;
+    }
+}
+
+// The terms of a constraint by its group of W lanes, coordinates and columns
+// dealt out to them.  Bound by FP64 issue: a warp instruction costs the same for
+// 1 lane and for 32, so what the lanes share is worth its rate.  Every
+// coordinate's values are few (Y1 x dA in place of dA: a pair's part of the
+// second derivative is then two dot products), 15 to 24 multiply-adds an entry;
+// by vertices (skew blocks J_i^T [s]x J_j, Gram terms of 3 x 9 Jacobians) one
+// lane took some 2800 instructions.  Unprojected, with the frames: 338
+// constraints of 27 cubes (16 lanes each) 210 -> 88 us, 163 k of 32 slabs (a lane
+// each) 1.33 -> 0.85 ms.
+template <int W>
+__device__ __forceinline__ bool barrier_build(const BarrierArgs& a, int64_t ci, SMat H, int g, unsigned mask,
+                                              double* scratch, int stride)
+{
+    BarrierBase o;
+    const int state = barrier_base(a, ci, g == 0, o);
+    if (state == kNothing) return false;
+    double own[W == 1 ? kRed * kCoord : 1];
+    double* st = W == 1 ? own : scratch;
+    const int ss = W == 1 ? 1 : stride;
+    const double* fa = a.frames + (size_t)a.cbodies[2 * ci] * 96;
+    const double* fb = a.frames + (size_t)a.cbodies[2 * ci + 1] * 96;
+    for (int r = g; r < kRed; r += W) {
+        const double G = barrier_coord(o, fa, fb, r, st + r * kCoord * ss, ss);
+        if (a.grad) {
+            a.grad[ci * 12 + (r < 6 ? r : r + 3)] = G;
+            if (r < 3) a.grad[ci * 12 + 6 + r] = -G;
+        }
+    }
+    if (state != kHessian) return false;
+    group_sync<W>(mask);
+    // (from the last: the longest columns first)
+    for (int c = kRed - 1 - g; c >= 0; c -= W) barrier_column(o, fa, fb, c, st, ss, H);
+    return true;
+}
 
 template <int W>
 __global__ void __launch_bounds__(kBarrierTPB) k_barrier_local(BarrierArgs a, int per_warp)
 {
     extern __shared__ double smem[];
-    local_terms<W>(a.n, per_warp, a.flags, a.hess, a.blocks, smem,
-                   [&](int64_t ci, SMat H) { return barrier_build(a, ci, H); });
+    const int stride = per_warp | 1;
+    local_terms<W>(a.n, per_warp, a.flags, a.hess, a.blocks, smem, [&](int64_t ci, SMat H, int g, unsigned mask) {
+        return barrier_build<W>(a, ci, H, g, mask, H.base + kRed * kRed * stride, stride);
+    });
 }
 
 size_t local_terms_smem_bytes(int per_warp)
@@ -595,7 +520,9 @@ int local_terms_per_warp(int64_t n, int tuned)
 static int launch_barrier(const BarrierArgs& a, int per_warp, cudaStream_t st)
 {
     const unsigned grid = grid_for(a.n, per_warp);
-    const size_t smem = local_terms_smem_bytes(per_warp);
+    // the coordinates' values of a constraint with several lanes are shared
+    const size_t smem = local_terms_smem_bytes(per_warp)
+        + (per_warp == kBarrierTPB ? 0 : (size_t)(kRed * kCoord) * (per_warp | 1) * sizeof(double));
     RIGC_COUNT_LAUNCH();
     switch (per_warp) {
     case 2: k_barrier_local<16><<<grid, kBarrierTPB, smem, st>>>(a, per_warp); break;

@@ -266,7 +266,7 @@ __global__ void __launch_bounds__(kBarrierTPB) k_friction_local(FrictionArgs a, 
 {
     extern __shared__ double smem[];
     local_terms<W>(a.n, per_warp, a.flags, a.hess, a.blocks, smem,
-                   [&](int64_t ci, SMat H) { return friction_build(a, ci, H); });
+                   [&](int64_t ci, SMat H, int g, unsigned) { return g == 0 && friction_build(a, ci, H); });
 }
 
 // ---------------------------------------------------------------------------

@@ -93,77 +93,6 @@ __device__ __forceinline__ void to_body(const Vtx* V, const int* lbody, int nvc,
     }
 }
 
-// Gram term H += coef * JM^T JM where JM (3 x 9) = sum_i M_i J_i and
-// M_i = m_i * I + (skew parts): here M_i given as full 3x3 per vertex.
-__device__ __forceinline__ void add_gram(SMat H, double coef, const Vtx* V, const int* lbody,
-                                         int nvc, const double (*M)[9])
-{
-    double JM[3][kRed];
-    for (int r = 0; r < 3; r++)
-        for (int c = 0; c < kRed; c++) JM[r][c] = 0;
-    for (int i = 0; i < nvc; i++) {
-        const int o = red_rot(lbody[i]);
-        for (int r = 0; r < 3; r++) {
-            if (lbody[i] == 0)
-                for (int j = 0; j < 3; j++) JM[r][j] += M[i][3 * r + j];
-            for (int k = 0; k < 3; k++)
-                JM[r][o + k] += M[i][3 * r] * V[i].D[0][k] + M[i][3 * r + 1] * V[i].D[1][k]
-                    + M[i][3 * r + 2] * V[i].D[2][k];
-        }
-    }
-    for (int r = 0; r < kRed; r++) {
-        double a0 = coef * JM[0][r], a1 = coef * JM[1][r], a2 = coef * JM[2][r];
-        for (int c = r; c < kRed; c++) H.at(r, c) += a0 * JM[0][c] + a1 * JM[1][c] + a2 * JM[2][c];
-    }
-}
-
-// J_i^T B J_j for different vertices i, j (bodies bi <= bj) and its
-// transpose: KD = B D_j, DK = D_i^T B (rows), DKD = D_i^T B D_j; tt = B + B^T
-// (null: zero)
-__device__ __forceinline__ void add_pair_blocks(SMat H, int bi, int bj, const double (*tt)[3],
-                                                const double (*KD)[3], const double (*DK)[3],
-                                                const double (*DKD)[3])
-{
-    const int oi = red_rot(bi), oj = red_rot(bj);
-    if (bi == 0 && bj == 0 && tt)
-        for (int r = 0; r < 3; r++)
-            for (int c = r; c < 3; c++) H.at(r, c) += tt[r][c];
-    // rows t_a: B D_j where vertex i is body a's, (D_i^T B)^T where j is
-    if (bi == 0)
-        for (int r = 0; r < 3; r++)
-            for (int c = 0; c < 3; c++) H.at(r, oj + c) += KD[r][c];
-    if (bj == 0)
-        for (int r = 0; r < 3; r++)
-            for (int c = 0; c < 3; c++) H.at(r, oi + c) += DK[c][r];
-    if (bi == bj) {
-        for (int r = 0; r < 3; r++)
-            for (int c = r; c < 3; c++) H.at(oi + r, oi + c) += DKD[r][c] + DKD[c][r];
-    } else {
-        for (int r = 0; r < 3; r++)
-            for (int c = 0; c < 3; c++) H.at(oi + r, oj + c) += DKD[r][c];
-    }
-}
-
-// skew pair block: J_i^T [s]x J_j and its transpose ([s]x + [s]x^T = 0)
-__device__ __forceinline__ void add_skew_pair(SMat H, const Vtx& Vi, int bi, const Vtx& Vj, int bj,
-                                              const double* s)
-{
-    double KD[3][3], DK[3][3], DKD[3][3];
-    for (int c = 0; c < 3; c++) {
-        // columns s x D_j[:, c]; rows (D_i^T [s]x)[c, :] = D_i[:, c] x s
-        KD[0][c] = s[1] * Vj.D[2][c] - s[2] * Vj.D[1][c];
-        KD[1][c] = s[2] * Vj.D[0][c] - s[0] * Vj.D[2][c];
-        KD[2][c] = s[0] * Vj.D[1][c] - s[1] * Vj.D[0][c];
-        DK[c][0] = Vi.D[1][c] * s[2] - Vi.D[2][c] * s[1];
-        DK[c][1] = Vi.D[2][c] * s[0] - Vi.D[0][c] * s[2];
-        DK[c][2] = Vi.D[0][c] * s[1] - Vi.D[1][c] * s[0];
-    }
-    for (int r = 0; r < 3; r++)
-        for (int c = 0; c < 3; c++)
-            DKD[r][c] = Vi.D[0][r] * KD[0][c] + Vi.D[1][r] * KD[1][c] + Vi.D[2][r] * KD[2][c];
-    add_pair_blocks(H, bi, bj, nullptr, KD, DK, DKD);
-}
-
 // curvature term: H(rot lb, rot lb) += sum_i g_i . (d2R_kl v_i) over the
 // vertices i of each body, as d2R_kl : (sum_i g_i v_i^T)
 __device__ __forceinline__ void add_curvature(SMat H, const double* const* frames, const int* lbody, int nvc,
@@ -206,8 +135,8 @@ __device__ __forceinline__ void add_curvature(SMat H, const double* const* frame
 // for itself; V stays in the matrix's shared memory.
 // Measured against a parallel Jacobi of the 12x12 by a warp (single-precision
 // seed, double refinement), building included: 172 k barrier constraints 41.8
-// -> 4.1 ms (FP64 issue), 98 k friction constraints 25.9 -> 1.4 ms, 180 barrier
-// constraints (16 lanes each) 0.50 -> 0.34 ms (the chain of one matrix).
+// -> 3.1 ms (FP64 issue), 98 k friction constraints 25.9 -> 1.4 ms, 338 barrier
+// constraints (16 lanes each) 0.50 -> 0.17 ms (the chain of one matrix).
 
 // 1 / sqrt(h) for normal h: the hardware approximation (about 20 bits) and one
 // third-order step
@@ -458,9 +387,9 @@ __device__ __forceinline__ void write_local_hessians(const double* base, int str
 }
 
 // One warp per block and per_warp constraints (a power of two) per warp: W =
-// min(16, 32 / per_warp) lanes to each.  The first lane of a group builds its
-// constraint's terms (build(ci, H): true when H holds a Hessian to project
-// and write), the group projects it, the warp writes it.
+// min(16, 32 / per_warp) lanes to each.  The lanes of a group build their
+// constraint's terms (build(ci, H, g, group): true in the first when H holds a
+// Hessian to project and write), the group projects it, the warp writes it.
 template <int W, class Build>
 __device__ __forceinline__ void local_terms(int64_t n, int per_warp, int flags, double* hess, double* blocks,
                                             double* smem, Build build)
@@ -469,11 +398,10 @@ __device__ __forceinline__ void local_terms(int64_t n, int per_warp, int flags, 
     const int64_t ci0 = (int64_t)blockIdx.x * per_warp, ci = ci0 + slot;
     const int stride = per_warp | 1;
     SMat H { smem + slot, stride };
-    const bool mine = g == 0 && slot < per_warp && ci < n;
-    const bool built = mine && build(ci, H);
-    if (!(flags & RIGC_HESS)) return;  // uniform over the block
-    const unsigned leaders = __ballot_sync(0xffffffffu, built);
     const unsigned group = W == 32 ? 0xffffffffu : ((1u << (W & 31)) - 1u) << (slot * W);
+    const bool built = slot < per_warp && ci < n && build(ci, H, g, group);
+    if (!(flags & RIGC_HESS)) return;  // uniform over the block
+    const unsigned leaders = __ballot_sync(0xffffffffu, built && g == 0);
     __syncwarp();
     if ((flags & RIGC_PROJECT_PSD) && ((leaders >> (slot * W)) & 1u)) psd_project<W>(H, g, group);
     __syncwarp();
