@@ -36,19 +36,26 @@ namespace rigc {
 // ---------------------------------------------------------------------------
 // per-body frames (R, dR, d2R) and positions
 
+// a warp per body, or (many bodies) a thread
+template <bool kWarp>
 __global__ void k_body_frames(const double* __restrict__ x, int nb, double* __restrict__ frames)
 {
-    int b = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int b = kWarp ? i >> 5 : i;
     if (b >= nb) return;
-    double t[3] = { x[6 * b + 3], x[6 * b + 4], x[6 * b + 5] };
+    const double t[3] = { x[6 * b + 3], x[6 * b + 4], x[6 * b + 5] };
+    double* out = frames + (size_t)b * 96;
+    if (kWarp) {
+        const int lane = threadIdx.x & 31;
+        warp_body_frame(t, lane, out);
+        if (lane < 3) out[90 + lane] = x[6 * b + lane];
+        return;
+    }
     double F[kFrameDoubles];
     body_frame(t, F);
-    double* out = frames + (size_t)b * 96;
 #pragma unroll
-    for (int i = 0; i < kFrameDoubles; i++) out[i] = F[i];
-    out[90] = x[6 * b];
-    out[91] = x[6 * b + 1];
-    out[92] = x[6 * b + 2];
+    for (int k = 0; k < kFrameDoubles; k++) out[k] = F[k];
+    for (int k = 0; k < 3; k++) out[90 + k] = x[6 * b + k];
 }
 
 // ---------------------------------------------------------------------------
@@ -535,13 +542,19 @@ static int launch_barrier(const BarrierArgs& a, int per_warp, cudaStream_t st)
     return RIGC_OK;
 }
 
+static int body_frames(const double* x, int nb, double* frames, cudaStream_t st)
+{
+    RIGC_COUNT_LAUNCH();
+    if (nb <= kWarpFrames) k_body_frames<true><<<grid_for((int64_t)nb * 32, 32), 32, 0, st>>>(x, nb, frames);
+    else k_body_frames<false><<<grid_for(nb, 128), 128, 0, st>>>(x, nb, frames);
+    RIGC_CUDA(cudaGetLastError());
+    return RIGC_OK;
+}
+
 int launch_body_frames(Ctx& c, const double* x)
 {
     RIGC_TRY(c.frames.reserve((size_t)c.s.nb * 96 * sizeof(double)));
-    RIGC_COUNT_LAUNCH();
-    k_body_frames<<<grid_for(c.s.nb, 128), 128, 0, c.stream>>>(x, c.s.nb, c.frames.as<double>());
-    RIGC_CUDA(cudaGetLastError());
-    return RIGC_OK;
+    return body_frames(x, c.s.nb, c.frames.as<double>(), c.stream);
 }
 
 int launch_barrier_local(Ctx& c, const double* x, double dhat, double dmin, int flags,
@@ -577,9 +590,7 @@ int launch_barrier_local_raw(const double* rest, int64_t nv, int nb, const doubl
                              int flags, double* frames, double* energy, double* grad,
                              double* hess, cudaStream_t stream)
 {
-    RIGC_COUNT_LAUNCH();
-    k_body_frames<<<grid_for(nb, 128), 128, 0, stream>>>(x, nb, frames);
-    RIGC_CUDA(cudaGetLastError());
+    RIGC_TRY(body_frames(x, nb, frames, stream));
     if (n == 0) return RIGC_OK;
     BarrierArgs a;
     a.rest = rest;

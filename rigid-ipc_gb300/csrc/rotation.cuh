@@ -9,8 +9,8 @@
 //    positions: constraint sets, broad-phase boxes);
 //  * body_frame: R with its first and second derivatives in theta, from the
 //    closed-form gradient/Hessian of sinc(|x|) (sinc.cpp:103-141) and the
-//    product rule on I + a K + b K^2 (contraction allowed; used by the
-//    barrier derivatives).
+//    product rule on I + a K + b K^2 (R as rot_rn has it, contraction allowed
+//    in the derivatives; used by the barrier and the inertial energy).
 // sin/cos are evaluated by a Cody-Waite reduction by pi/2 (three-part split,
 // 33-bit leading parts) and the Taylor series of sin and cos to degree 19/20
 // (coefficients 1/n!) by Horner's rule; the error is below 2^-50|y| + 2^-60
@@ -157,11 +157,10 @@ __device__ __forceinline__ double norm3_rn(double a, double b, double c)
     return __dsqrt_rn(RADD(RADD(RMUL(a, a), RMUL(b, b)), RMUL(c, c)));
 }
 
-// R row-major, exact operation order shared with the host restatement
-__device__ __forceinline__ void rot_rn(const double t[3], double R[9])
+// R row-major, exact operation order shared with the host restatement, from
+// a = sinc(|t|) and s = sinc(|t / 2|)
+__device__ __forceinline__ void rot_from_sinc(const double t[3], double a, double s, double R[9])
 {
-    double a = sinc_rn(norm3_rn(t[0], t[1], t[2]));
-    double s = sinc_rn(norm3_rn(RDIV(t[0], 2.0), RDIV(t[1], 2.0), RDIV(t[2], 2.0)));
     double b = RMUL(RMUL(0.5, s), s);
     double K[9] = { 0.0, -t[2], t[1], t[2], 0.0, -t[0], -t[1], t[0], 0.0 };
 #pragma unroll
@@ -173,6 +172,13 @@ __device__ __forceinline__ void rot_rn(const double t[3], double R[9])
             double r = RADD(RMUL(a, K[3 * i + j]), RMUL(b, k2));
             R[3 * i + j] = i == j ? RADD(r, 1.0) : r;
         }
+}
+
+__device__ __forceinline__ void rot_rn(const double t[3], double R[9])
+{
+    const double a = sinc_rn(norm3_rn(t[0], t[1], t[2]));
+    const double s = sinc_rn(norm3_rn(RMUL(t[0], 0.5), RMUL(t[1], 0.5), RMUL(t[2], 0.5)));
+    rot_from_sinc(t, a, s, R);
 }
 
 // V_j = ((v0 R_j0 + v1 R_j1) + v2 R_j2) + p_j
@@ -214,100 +220,109 @@ __device__ __forceinline__ int sym_index(int k, int l)
     return k == 0 ? l : (k == 1 ? 2 + l : 5);
 }
 
+// sinc and its derivatives' factors at x = |t| or |t / 2|
+struct SincTerms {
+    double s, g1, g2;
+};
+__device__ __forceinline__ SincTerms sinc_terms(double x)
+{
+    double sn, cn;
+    det_sincos(x, sn, cn);
+    return SincTerms { x >= 1.220703125e-04 ? RDIV(sn, x) : sinc_rn(x), dsinc_over_x(x, sn, cn), ddsinc_term(x, sn, cn) };
+}
+
+// a(t) = sinc(|t|): gradient a1 t, Hessian a2 t t^T + a1 I; b = 1/2 s^2 with
+// s(t) = sinc(|t / 2|): ds = 1/2 g(t/2), d2s = 1/4 H(t/2), so that gb = s ds,
+// Hb = ds ds^T + s d2s
+struct FrameBase {
+    double t[3], gs[3];
+    double a, a1, a2, b, sh, h1, h2;
+};
+__device__ __forceinline__ FrameBase frame_base(const double t[3], const SincTerms& full, const SincTerms& half)
+{
+    FrameBase f;
+    for (int i = 0; i < 3; i++) {
+        f.t[i] = t[i];
+        f.gs[i] = 0.25 * half.g1 * t[i];
+    }
+    f.a = full.s;
+    f.a1 = full.g1;
+    f.a2 = full.g2;
+    f.sh = half.s;
+    f.b = RMUL(RMUL(0.5, half.s), half.s);
+    f.h1 = 0.25 * half.g1;
+    f.h2 = 0.0625 * half.g2;
+    return f;
+}
+
+// [e_k]x's entry (i, j)
+__device__ __forceinline__ double unit_cross(int k, int i, int j)
+{
+    return i == j || i == k || j == k ? 0.0 : (i - k + 3) % 3 == 1 ? -1.0 : 1.0;
+}
+
+// entry e of the frame: with K = [t]x, E_k = [e_k]x and
+//   (K K)_ij = t_i t_j - |t|^2 d_ij, (E_k K + K E_k)_ij = t_i d_jk + t_j d_ik - 2 t_k d_ij,
+//   (E_k E_l + E_l E_k)_ij = d_il d_jk + d_ik d_jl - 2 d_kl d_ij
+// R = I + a K + b K K and its derivatives by the product rule
+__device__ __forceinline__ double frame_entry(const FrameBase& f, int e)
+{
+    const int i = (e % 9) / 3, j = e % 3;
+    const int m = (3 - i - j + 3) % 3;  // the third index when i != j
+    const double ti = f.t[i], tj = f.t[j];
+    const int u = (i + 1) % 3, v = (i + 2) % 3;
+    const double K = i == j ? 0.0 : unit_cross(m, i, j) * f.t[m];
+    const double K2 = i == j ? -RADD(RMUL(f.t[u], f.t[u]), RMUL(f.t[v], f.t[v])) : RMUL(ti, tj);
+    if (e < 9) {  // as rot_rn
+        const double r = RADD(RMUL(f.a, K), RMUL(f.b, K2));
+        return i == j ? RADD(r, 1.0) : r;
+    }
+    auto pair = [&](int k) { return (j == k ? ti : 0.0) + (i == k ? tj : 0.0) - (i == j ? 2 * f.t[k] : 0.0); };
+    if (e < 36) {
+        const int k = (e - 9) / 9;
+        const double gb = f.sh * f.gs[k];
+        return fma(f.a1 * f.t[k], K, fma(f.a, unit_cross(k, i, j), fma(gb, K2, f.b * pair(k))));
+    }
+    const int q = (e - 36) / 9, k = q < 3 ? 0 : q < 5 ? 1 : 2, l = q < 3 ? q : q < 5 ? q - 2 : 2;
+    const double kl = k == l ? 1.0 : 0.0;
+    const double Ha = fma(f.a2, f.t[k] * f.t[l], kl * f.a1);
+    const double Hb = fma(f.gs[k], f.gs[l], f.sh * fma(f.h2, f.t[k] * f.t[l], kl * f.h1));
+    const double ee = (double)((i == l) * (j == k) + (i == k) * (j == l)) - (i == j ? 2 * kl : 0.0);
+    double r = f.b * ee;
+    r = fma(f.sh * f.gs[l], pair(k), r);
+    r = fma(f.sh * f.gs[k], pair(l), r);
+    r = fma(Hb, K2, r);
+    r = fma(f.a1 * f.t[l], unit_cross(k, i, j), r);
+    r = fma(f.a1 * f.t[k], unit_cross(l, i, j), r);
+    return fma(Ha, K, r);
+}
+
 __device__ inline void body_frame(const double t[3], double* F)
 {
-    // a(t) = sinc(|t|), g_a = dsinc_over_x(|t|) t, H_a = dd(|t|) t t^T + g1 I
-    double n = sqrt(t[0] * t[0] + t[1] * t[1] + t[2] * t[2]);
-    double sn, cn;
-    det_sincos(n, sn, cn);
-    double a = n >= 1.220703125e-04 ? sn / n : sinc_rn(n);
-    double g1 = dsinc_over_x(n, sn, cn), g2 = ddsinc_term(n, sn, cn);
-    // half angle: s(t) = sinc(|t/2|), ds = 1/2 g(t/2), d2s = 1/4 H(t/2)
-    double h[3] = { 0.5 * t[0], 0.5 * t[1], 0.5 * t[2] };
-    double nh = 0.5 * n;
-    double shn, chn;
-    det_sincos(nh, shn, chn);
-    double sh = nh >= 1.220703125e-04 ? shn / nh : sinc_rn(nh);
-    double h1 = dsinc_over_x(nh, shn, chn), h2 = ddsinc_term(nh, shn, chn);
-    double ga[3], gs[3], Ha[3][3], Hs[3][3];
+    const double n = norm3_rn(t[0], t[1], t[2]);
+    const FrameBase f = frame_base(t, sinc_terms(n), sinc_terms(0.5 * n));
 #pragma unroll
-    for (int i = 0; i < 3; i++) {
-        ga[i] = g1 * t[i];
-        gs[i] = 0.5 * h1 * h[i];
-#pragma unroll
-        for (int j = 0; j < 3; j++) {
-            Ha[i][j] = g2 * t[i] * t[j] + (i == j ? g1 : 0.0);
-            Hs[i][j] = 0.25 * (h2 * h[i] * h[j] + (i == j ? h1 : 0.0));
-        }
-    }
-    // b = 1/2 s^2: gb = s gs, Hb = gs gs^T + s Hs
-    double b = 0.5 * sh * sh, gb[3], Hb[3][3];
-#pragma unroll
-    for (int i = 0; i < 3; i++) {
-        gb[i] = sh * gs[i];
-#pragma unroll
-        for (int j = 0; j < 3; j++) Hb[i][j] = gs[i] * gs[j] + sh * Hs[i][j];
-    }
-    // K = [t]x, E_k = [e_k]x, K2 = K K
-    double K[9] = { 0, -t[2], t[1], t[2], 0, -t[0], -t[1], t[0], 0 };
-    double K2[9];
-#pragma unroll
-    for (int i = 0; i < 3; i++)
-#pragma unroll
-        for (int j = 0; j < 3; j++)
-            K2[3 * i + j] = K[3 * i] * K[j] + K[3 * i + 1] * K[3 + j] + K[3 * i + 2] * K[6 + j];
-    auto E = [](int k, int i, int j) -> double {
-        // [e_k]x entries
-        if (k == 0) return (i == 1 && j == 2) ? -1.0 : ((i == 2 && j == 1) ? 1.0 : 0.0);
-        if (k == 1) return (i == 0 && j == 2) ? 1.0 : ((i == 2 && j == 0) ? -1.0 : 0.0);
-        return (i == 0 && j == 1) ? -1.0 : ((i == 1 && j == 0) ? 1.0 : 0.0);
-    };
-    // (E_k K + K E_k) and (E_k E_l + E_l E_k)
-#pragma unroll
-    for (int i = 0; i < 3; i++)
-#pragma unroll
-        for (int j = 0; j < 3; j++)
-            F[3 * i + j] = a * K[3 * i + j] + b * K2[3 * i + j] + (i == j ? 1.0 : 0.0);
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-#pragma unroll
-        for (int i = 0; i < 3; i++)
-#pragma unroll
-            for (int j = 0; j < 3; j++) {
-                double EK = 0, KE = 0;
-#pragma unroll
-                for (int m = 0; m < 3; m++) {
-                    EK += E(k, i, m) * K[3 * m + j];
-                    KE += K[3 * i + m] * E(k, m, j);
-                }
-                F[9 + 9 * k + 3 * i + j] = ga[k] * K[3 * i + j] + a * E(k, i, j)
-                    + gb[k] * K2[3 * i + j] + b * (EK + KE);
-            }
-    }
-#pragma unroll
-    for (int k = 0; k < 3; k++)
-#pragma unroll
-        for (int l = k; l < 3; l++) {
-            int idx = sym_index(k, l);
-#pragma unroll
-            for (int i = 0; i < 3; i++)
-#pragma unroll
-                for (int j = 0; j < 3; j++) {
-                    double EkK = 0, KEk = 0, ElK = 0, KEl = 0, EkEl = 0, ElEk = 0;
-#pragma unroll
-                    for (int m = 0; m < 3; m++) {
-                        EkK += E(k, i, m) * K[3 * m + j];
-                        KEk += K[3 * i + m] * E(k, m, j);
-                        ElK += E(l, i, m) * K[3 * m + j];
-                        KEl += K[3 * i + m] * E(l, m, j);
-                        EkEl += E(k, i, m) * E(l, m, j);
-                        ElEk += E(l, i, m) * E(k, m, j);
-                    }
-                    F[36 + 9 * idx + 3 * i + j] = Ha[k][l] * K[3 * i + j] + ga[k] * E(l, i, j)
-                        + ga[l] * E(k, i, j) + Hb[k][l] * K2[3 * i + j]
-                        + gb[k] * (ElK + KEl) + gb[l] * (EkK + KEk) + b * (EkEl + ElEk);
-                }
-        }
+    for (int e = 0; e < kFrameDoubles; e++) F[e] = frame_entry(f, e);
 }
+
+// The frame by a warp: half the lanes take the whole angle and half the half
+// angle, then three entries each.  A thread's chain of some 1500 FP64
+// instructions took 32 us however few the bodies, this 11.
+__device__ __forceinline__ void warp_body_frame(const double t[3], int lane, double* F)
+{
+    const double n = norm3_rn(t[0], t[1], t[2]);
+    const SincTerms mine = sinc_terms(lane < 16 ? n : 0.5 * n);
+    SincTerms q[2];
+    for (int k = 0; k < 2; k++)
+        q[k] = SincTerms { __shfl_sync(0xffffffffu, mine.s, 16 * k), __shfl_sync(0xffffffffu, mine.g1, 16 * k),
+                           __shfl_sync(0xffffffffu, mine.g2, 16 * k) };
+    const FrameBase f = frame_base(t, q[0], q[1]);
+    for (int e = lane; e < kFrameDoubles; e += 32) F[e] = frame_entry(f, e);
+}
+
+// Bodies up to which a warp takes one, then a thread: a warp's 250 instructions
+// fill the FP64 units (608 sub-partitions, 64 cycles an instruction) longer than
+// one thread's chain lasts from some 2000 bodies on.
+constexpr int kWarpFrames = 2048;
 
 } // namespace rigc
