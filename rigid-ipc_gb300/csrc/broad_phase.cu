@@ -1421,10 +1421,15 @@ __global__ void k_bucket_pairs(const int32_t* __restrict__ count, const int32_t*
     for (int k = 0; k < n; k++) write_pair(b, ne, nee, o + k, v[k], out_ee, out_fv);
 }
 
-// One block per listed bucket (grid-stride over the list): its second
+// One block per listed bucket (grid-stride over the list).  Up to kRankBucket
+// elements: each one's place is the number of smaller ones.  More: the second
 // elements (distinct: each pair is found once) as bits of a bitmap over
 // their range (EE: edges; FV: vertices; EF: edges), then written in the
-// order of the bits.  bitmap: words_per_block words per block.
+// order of the bits.  bitmap: words_per_block words per block.  The bitmap's words
+// are all scanned however few its bits, 82 us over the vertices of 1000
+// icospheres; by places a launch is 10.
+constexpr int kRankBucket = 4096;
+
 __global__ void __launch_bounds__(1024) k_bucket_large(
     const int32_t* __restrict__ large, const int32_t* __restrict__ nlarge,
     const int32_t* __restrict__ count, const int32_t* __restrict__ offset,
@@ -1432,7 +1437,7 @@ __global__ void __launch_bounds__(1024) k_bucket_large(
     unsigned* __restrict__ bitmap_all, int64_t words_per_block,
     int2* __restrict__ out_ee, int2* __restrict__ out_fv)
 {
-    __shared__ int32_t warp_sum[32];
+    __shared__ int32_t warp_sum[32], sec[kRankBucket];
     __shared__ int32_t carry;
     unsigned* bitmap = bitmap_all + (int64_t)blockIdx.x * words_per_block;
     const int nl = *nlarge;
@@ -1441,6 +1446,18 @@ __global__ void __launch_bounds__(1024) k_bucket_large(
         const int b = large[li];
         const int n = count[b];
         const int64_t o = offset[b];
+        if (n <= kRankBucket) {
+            __syncthreads();
+            for (int k = threadIdx.x; k < n; k += blockDim.x) sec[k] = second[o + k];
+            __syncthreads();
+            for (int k = threadIdx.x; k < n; k += blockDim.x) {
+                const int x = sec[k];
+                int rank = 0;
+                for (int j = 0; j < n; j++) rank += sec[j] < x;
+                write_pair(b, ne, nee, o + rank, x, out_ee, out_fv);
+            }
+            continue;
+        }
         const int range = b < ne ? ne : fv_range;
         const int64_t words = ((int64_t)range + 31) / 32;
         for (int64_t w = threadIdx.x; w < words; w += blockDim.x) bitmap[w] = 0u;

@@ -57,6 +57,10 @@ def _make(kind):
         P = rng.normal(size=(50, 3))
         P = 2.1 * P / np.linalg.norm(P, axis=1, keepdims=True)
         return _scene(M, np.concatenate([[[0, 0, 0]], P])), None, False
+    if kind == "floor":  # a face with more pairs than are placed by counting, one with fewer
+        M = [meshes.plane(20.0), meshes.tessellated_box((2, 0.2, 2), (70, 1, 70)),
+             meshes.tessellated_box((2, 0.2, 2), (20, 1, 20))]
+        return _scene(M, [(0, 0, 0), (3, 0.1004, -3), (-3, 0.1004, 3)]), None, False
     if kind == "rim":  # bodies that turn at the scene's rim, more time nodes than the list takes
         P = np.stack([0.7 * (np.arange(1600) // 40), np.zeros(1600), 0.7 * (np.arange(1600) % 40)], 1)
         return _scene([_hull(rng, 16 + i % 9) for i in range(1600)], P), None, False
@@ -67,7 +71,7 @@ def _make(kind):
 
 
 @pytest.mark.parametrize("continuous", [False, True])
-@pytest.mark.parametrize("kind", ["tiles", "patches", "scenes", "one_large", "nested", "rim"])
+@pytest.mark.parametrize("kind", ["tiles", "patches", "scenes", "one_large", "nested", "rim", "floor"])
 def test_candidates(oracle, kind, continuous):
     import rigc
 
