@@ -282,9 +282,9 @@ __device__ __forceinline__ float split_pair(double x, unsigned short& rest)
 }
 __device__ __forceinline__ float pair_rest(unsigned short b) { return __uint_as_float((unsigned)b << 16); }
 
-// the record of a candidate (rest vertices and bodies in q, tolerances in tol)
-__device__ __forceinline__ void filter_record(const Query& q, const double tol[3],
-                                              const double* __restrict__ ref,
+// the record of a candidate (rest vertices and bodies in q) without its
+// tolerances' part
+__device__ __forceinline__ void filter_record(const Query& q, const double* __restrict__ ref,
                                               const float* __restrict__ frames,
                                               const float* __restrict__ bodies, FilterRec& r)
 {
@@ -330,11 +330,18 @@ __device__ __forceinline__ void filter_record(const Query& q, const double tol[3
     r.E = 1.01f * (96.0f * u * D + 120.0f * u * Tv + 9.313225746154785e-10f * m + 1.1368683772161603e-13f * (W + D));
     r.body_a = q.body_a;
     r.body_b = q.body_b;
-    const TolKeys K = tol_keys(tol);
-    unsigned lev = (q.fv ? kRecFV : 0u) | (deep ? 0u : kRecShallow);
+    r.lev = (q.fv ? kRecFV : 0u) | (deep ? 0u : kRecShallow);
     // finite bounds and tolerances whose keys order the splits; anything
     // else is left to the double-precision search from its root
-    if (!K.ok || !(r.E < 1e18f) || !(m < 1e18f)) lev |= kRecDouble;
+    if (!(r.E < 1e18f) || !(m < 1e18f)) r.lev |= kRecDouble;
+}
+
+// the tolerances' part
+__device__ __forceinline__ void filter_levels(const double tol[3], FilterRec& r)
+{
+    const TolKeys K = tol_keys(tol);
+    unsigned lev = r.lev;
+    if (!K.ok) lev |= kRecDouble;
     // K[d] + lv[d] 2^52 (split_dim_keys) in the order of its exponent plus
     // level, then its mantissa: 4 exponent + the mantissa's rank
     unsigned key[3];
@@ -366,6 +373,33 @@ __device__ __forceinline__ void filter_vertex(const float* f, const float v[3], 
         lo[c] = m - r;
         hi[c] = m + r;
     }
+}
+
+// The bounds of y over [0, toi_tol] and the tolerances' boxes of alpha and beta
+// exclude zero on an axis, in double too: |y - Z| is at most the displacements
+// over [0, toi_tol] (the table's last slot), A and B and twice the displacements
+// times the widths, and E covers the rest as for any box.
+__device__ __forceinline__ bool filter_starts_apart(const FilterRec& r, const float* __restrict__ frames,
+                                                    float w1, float w2)
+{
+    if (r.lev & kRecDouble) return false;
+    float d[3] = { 0.0f, 0.0f, 0.0f };
+    const int na = r.lev & kRecFV ? 1 : 2;
+#pragma unroll
+    for (int v = 0; v < 4; v++) {
+        const float* f = frames + ((size_t)(v < na ? r.body_a : r.body_b) * kTableSlots + kTableNodes) * kFrame32;
+        float lo[3], hi[3];
+        filter_vertex(f, r.v[v], lo, hi);
+#pragma unroll
+        for (int c = 0; c < 3; c++) d[c] = fmaxf(d[c], fmaxf(fabsf(lo[c]), fabsf(hi[c])));
+    }
+    bool apart = false;
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+        const float w = 2.0f * d[c] + w1 * (fabsf(r.A[c]) + 2.0f * d[c]) + w2 * (fabsf(r.B[c]) + 2.0f * d[c]);
+        apart = apart || fabsf(r.Z[c]) > 1.001f * (w + r.E);
+    }
+    return apart;
 }
 
 __device__ __forceinline__ void filter_frame(const float* __restrict__ g, float f[kFrame32])

@@ -110,3 +110,15 @@ def test_batched_scenes():
         cb.set_ccd_window(w)
         cb.compute_earliest_toi(X0, X1)
         assert np.array_equal(cb.scene_tois(), np.array(alone)), w
+
+
+@pytest.mark.parametrize("gap", [0.0, 1e-6, 9e-5, 1.1e-4, 2.1e-4, 3e-4])
+def test_starts(gap):
+    """Starts around the length tolerance (1e-4): whether f over the first
+    tolerance's box contains zero sets the candidate's time tolerance."""
+    import rigc
+
+    sc = _cubes(2, 1, 0.0, 0.0, gap)
+    for v in (0.0, -1e-3, -0.5):
+        sc.bodies[0].velocity[1] = v
+        _check(rigc.Context(sc), sc.poses(), sc.predictor_poses())
