@@ -114,6 +114,7 @@ k_body_energy(const double* __restrict__ x, const int* __restrict__ type, int nb
         }
 }
 
+// energy_host null: the energy is in c.h_scalars[8] after the stream's next wait
 int body_energy(Ctx& c, const rigc_body_state& s, const double* x, const double gravity[3],
                 double h, double* energy_host, double* grad, double* hess)
 {
@@ -132,6 +133,7 @@ int body_energy(Ctx& c, const rigc_body_state& s, const double* x, const double 
     double* e_dev = reinterpret_cast<double*>(c.d_scalars.as<char>() + 2560);
     RIGC_TRY(sum_f64(e, nb, e_dev, c.scratch[1], st));
     RIGC_CUDA(cudaMemcpyAsync(c.h_scalars + 8, e_dev, sizeof(double), cudaMemcpyDeviceToHost, st));
+    if (!energy_host) return RIGC_OK;
     RIGC_CUDA(cudaStreamSynchronize(st));
     *energy_host = c.h_scalars[8];
     return RIGC_OK;

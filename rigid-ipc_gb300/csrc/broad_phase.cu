@@ -1831,8 +1831,7 @@ int detect_pairs(Ctx& c, const double* x0, const double* x1, bool continuous, do
         }
         RIGC_CUDA(cudaGetLastError());
         unsigned long long hn[4];
-        RIGC_CUDA(cudaMemcpyAsync(hn, pn, sizeof(hn), cudaMemcpyDeviceToHost, st));
-        RIGC_CUDA(cudaStreamSynchronize(st));
+        RIGC_TRY(read_back(c, hn, pn, sizeof(hn)));
         if (by_patches && (hn[2] > pl.cap_items || hn[3] > pl.cap_pairs)) {
             // patches that meet too many others: the grid, from the boxes that are there
             by_patches = false;

@@ -1893,8 +1893,7 @@ static int run_search(Ctx& c, const double* x0, const double* x1, double toi_tol
                     c.ccd_pieces[other].as<Piece>(), n_now_dev, n_later_dev + other);
                 RIGC_CUDA(cudaGetLastError());
                 unsigned long long h[kCCDCounters];
-                RIGC_CUDA(cudaMemcpyAsync(h, cnt, sizeof(h), cudaMemcpyDeviceToHost, st));
-                RIGC_CUDA(cudaStreamSynchronize(st));
+                RIGC_TRY(read_back(c, h, cnt, sizeof(h)));
                 if (front && from_out) {
                     if (h[10] > a.out_cap) {
                         *redo = true;
@@ -1922,8 +1921,7 @@ static int run_search(Ctx& c, const double* x0, const double* x1, double toi_tol
     }
     c.bp_table.valid = false;
     unsigned long long out[4];
-    RIGC_CUDA(cudaMemcpyAsync(out, cnt, sizeof(out), cudaMemcpyDeviceToHost, st));
-    RIGC_CUDA(cudaStreamSynchronize(st));
+    RIGC_TRY(read_back(c, out, cnt, sizeof(out)));
     double g;
     std::memcpy(&g, &out[0], sizeof(g));
     *toi_host = g;  // +inf bits when no candidate found an impact

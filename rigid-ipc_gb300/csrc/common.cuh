@@ -4,6 +4,8 @@
 
 #include <cuda_runtime.h>
 
+#include <cstring>
+
 #include <cstdint>
 #include <cstdio>
 #include <string>
@@ -222,6 +224,19 @@ struct Ctx {
 };
 
 Ctx* ctx_of(rigc_ctx* c);
+
+// a few bytes to the host, through pinned memory (a copy to pageable memory is
+// staged by the driver), and wait for them
+constexpr size_t kReadBack = 2048;  // bytes from 1024 on in h_scalars
+inline int read_back(Ctx& c, void* host, const void* dev, size_t bytes)
+{
+    char* pinned = reinterpret_cast<char*>(c.h_scalars) + 1024;
+    const bool fits = bytes <= kReadBack;
+    RIGC_CUDA(cudaMemcpyAsync(fits ? pinned : host, dev, bytes, cudaMemcpyDeviceToHost, c.stream));
+    RIGC_CUDA(cudaStreamSynchronize(c.stream));
+    if (fits) std::memcpy(host, pinned, bytes);
+    return RIGC_OK;
+}
 
 // ---------------------------------------------------------------------------
 // launch helpers

@@ -378,8 +378,7 @@ int construct_constraints(Ctx& c, const double* x, double dhat, double dmin)
     const bool small = n <= kRankRecords;
     int32_t m = (int32_t)n;
     if (!small) {
-        RIGC_CUDA(cudaMemcpyAsync(&m, cnt_dev, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-        RIGC_CUDA(cudaStreamSynchronize(st));
+        RIGC_TRY(read_back(c, &m, cnt_dev, sizeof(int32_t)));
         if (m == 0) return RIGC_OK;
     }
     RIGC_TRY(S[2].reserve((size_t)m * 8));
@@ -421,8 +420,7 @@ int construct_constraints(Ctx& c, const double* x, double dhat, double dmin)
     }
     RIGC_CUDA(cudaGetLastError());
     int32_t h[6];
-    RIGC_CUDA(cudaMemcpyAsync(h, cnt_dev, sizeof(h), cudaMemcpyDeviceToHost, st));
-    RIGC_CUDA(cudaStreamSynchronize(st));
+    RIGC_TRY(read_back(c, h, cnt_dev, sizeof(h)));
     const int32_t nc = h[1];
     const int32_t* kinds = h + 2;
     C.num = nc;

@@ -1203,9 +1203,7 @@ int dot_dev(Ctx& c, Sim& S, int64_t n, const double* a, const double* b, double*
 
 int read_scalars(Ctx& c, const double* dev, double* host, int n)
 {
-    RIGC_CUDA(cudaMemcpyAsync(host, dev, n * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
-    RIGC_CUDA(cudaStreamSynchronize(c.stream));
-    return RIGC_OK;
+    return read_back(c, host, dev, n * sizeof(double));
 }
 
 std::vector<unsigned long long> graph_key(std::initializer_list<const void*> ptrs,
@@ -1262,8 +1260,9 @@ int objective(Ctx& c, Sim& S, const double* x, bool grad_hess, Objective& O, boo
     const rigc_sim_params& p = S.p;
     const double m = p.average_mass;
     rigc_body_state bs = state_of(S);
-    double E;
-    RIGC_TRY(body_energy(c, bs, x, p.gravity, p.timestep, &E, grad_hess ? S.gE.as<double>() : nullptr,
+    double al = 0;
+    // (the energy is read with the barrier's, after its wait)
+    RIGC_TRY(body_energy(c, bs, x, p.gravity, p.timestep, nullptr, grad_hess ? S.gE.as<double>() : nullptr,
                          grad_hess ? S.hE.as<double>() : nullptr));
     if (S.has_kinematic && !(S.al_sat_q && S.al_sat_Q)) {
         RIGC_COUNT_LAUNCH();
@@ -1273,13 +1272,12 @@ int objective(Ctx& c, Sim& S, const double* x, bool grad_hess, Objective& O, boo
             grad_hess ? S.gE.as<double>() : nullptr, grad_hess ? S.hE.as<double>() : nullptr);
         double* e_dev = reinterpret_cast<double*>(c.d_scalars.as<char>() + 2568);
         RIGC_TRY(sum_f64(S.al_e.as<double>(), S.nb, e_dev, c.scratch[1], c.stream));
-        double al;
         RIGC_TRY(read_scalars(c, e_dev, &al, 1));
-        E += al;
     }
     RIGC_TRY(build_constraints(c, x, p.dhat, p.dmin));
     const int flags = grad_hess ? (RIGC_GRAD | RIGC_HESS | (project ? RIGC_PROJECT_PSD : 0)) : 0;
     RIGC_TRY(barrier_term_impl(c, x, p.dhat, p.dmin, flags, &O.bo));
+    const double E = c.h_scalars[8] + al;
     double D = 0;
     O.fo = rigc_barrier_out {};
     if (p.coefficient_friction > 0 && c.fric.num > 0) {
@@ -1444,8 +1442,7 @@ int dense_solve(Ctx& c, Sim& S, const HessView& H, bool& ok)
                                                       S.sol.as<double>());
     RIGC_CUDA(cudaGetLastError());
     int fl = 0;
-    RIGC_CUDA(cudaMemcpyAsync(&fl, flags, sizeof(int), cudaMemcpyDeviceToHost, st));
-    RIGC_CUDA(cudaStreamSynchronize(st));
+    RIGC_TRY(read_back(c, &fl, flags, sizeof(int)));
     ok = fl == 0;
     return RIGC_OK;
 }
@@ -1636,8 +1633,7 @@ int objective_scenes(Ctx& c, Sim& S, const double* x, bool grad_hess, const std:
     const rigc_sim_params& p = S.p;
     const int ns = c.s.nscenes;
     rigc_body_state bs = state_of(S);
-    double E;
-    RIGC_TRY(body_energy(c, bs, x, p.gravity, p.timestep, &E, grad_hess ? S.gE.as<double>() : nullptr,
+    RIGC_TRY(body_energy(c, bs, x, p.gravity, p.timestep, nullptr, grad_hess ? S.gE.as<double>() : nullptr,
                          grad_hess ? S.hE.as<double>() : nullptr));
     std::vector<double> Es;
     RIGC_COUNT_LAUNCH();
@@ -1951,8 +1947,7 @@ int sim_step_scenes(Ctx& c, rigc_step_stats* stats)
     // IPCSolver::init_solve per scene
     {
         rigc_body_state bs = state_of(S);
-        double E;
-        RIGC_TRY(body_energy(c, bs, x0, p.gravity, p.timestep, &E, S.gE.as<double>(), nullptr));
+        RIGC_TRY(body_energy(c, bs, x0, p.gravity, p.timestep, nullptr, S.gE.as<double>(), nullptr));
         RIGC_TRY(build_constraints(c, x0, p.dhat, p.dmin));
         rigc_barrier_out bo;
         RIGC_TRY(barrier_term_impl(c, x0, p.dhat, p.dmin, RIGC_GRAD, &bo));
@@ -2258,8 +2253,7 @@ int sim_step(Ctx& c, rigc_step_stats* stats)
     // IPCSolver::init_solve
     {
         rigc_body_state bs = state_of(S);
-        double E;
-        RIGC_TRY(body_energy(c, bs, x0, p.gravity, p.timestep, &E, S.gE.as<double>(), nullptr));
+        RIGC_TRY(body_energy(c, bs, x0, p.gravity, p.timestep, nullptr, S.gE.as<double>(), nullptr));
         RIGC_TRY(build_constraints(c, x0, p.dhat, p.dmin));
         rigc_barrier_out bo;
         RIGC_TRY(barrier_term_impl(c, x0, p.dhat, p.dmin, RIGC_GRAD, &bo));
@@ -2551,8 +2545,7 @@ int adjoint_step(Ctx& c, Sim& S, const double* pre, const double* xs, double kap
         const double kbar = -dk / M * host_dot(c, S, lam, O.bo.grad);
         if (kbar != 0) {
             rigc_body_state bs = state_of(S);
-            double E;
-            RIGC_TRY(body_energy(c, bs, x0, p.gravity, h, &E, S.gE.as<double>(), S.hE.as<double>()));
+            RIGC_TRY(body_energy(c, bs, x0, p.gravity, h, nullptr, S.gE.as<double>(), S.hE.as<double>()));
             RIGC_TRY(build_constraints(c, x0, p.dhat, p.dmin));
             rigc_barrier_out bo;
             RIGC_TRY(barrier_term_impl(c, x0, p.dhat, p.dmin, RIGC_GRAD | RIGC_HESS, &bo));
