@@ -38,27 +38,9 @@ import numpy as np  # noqa: E402
 METRIC = "candidate pairs/s (CCD+barrier grad/Hess)"
 UNIT = "pairs/s"
 CCD_BYTES_PER_PAIR = 304        # ids + 4 rest vertices + 4 poses + toi
-# DRAM bytes (read + write) per continuous candidate of one CCD call (all its
-# search launches and the splits of their deferred pieces), from ncu captures
-# of the 200-icosphere pile (132,242 candidates): k_ccd 56.95 MB read +
-# 311.51 MB written over two launches (per-lane candidate state spilling
-# from L1, the frame cache; it searches without time windows);
-# k_ccd_group<32, 4> (one search per warp fitted to 4 blocks per SM)
-# 119.20 MB + 40.87 MB and k_ccd_group<16, 4> (one search per half-warp, the
-# same fit) 134.27 MB + 32.55 MB over three launches with time windows from
-# 2^-6, most of it the deferred pieces written and read back and the spills.
-# The traffic of a full call is this times its candidates.  FP64 figures of
-# the first launch of the same calls: pipe active (fraction of peak) and
-# lane-level GFLOP/s (dadd + dmul + 2 dfma over the launch).
-K_CCD_DRAM_BYTES_PER_CANDIDATE = {
-    "k_ccd": (42209536 + 14743808 + 310226176 + 1279232) / 132242,
-    "k_ccd_group<32, 4>": (119197184 + 40870912) / 132242,
-    "k_ccd_group<16, 4>": (134271488 + 32547072) / 132242}
-K_CCD_FP64 = {"k_ccd": {"pipe_active": 0.233, "lane_gflops": 53.0},
-              "k_ccd_group<32, 4>": {"pipe_active": 0.416, "lane_gflops": 108.6},
-              "k_ccd_group<16, 4>": {"pipe_active": 0.343, "lane_gflops": 73.5}}
 BARRIER_BYTES_PER_CONSTRAINT = 1456
-# the CCD kernel of each search mode (rigc_set_tune's ccd_warp)
+# the CCD kernel of each search mode (rigc_set_tune's ccd_warp), behind the
+# single-precision search that decides nearly all boxes
 CCD_KERNELS = {0: "k_ccd", 1: "k_ccd_group<32, 1>", 2: "k_ccd_group<32, 4>",
                3: "k_ccd_group<32, 5>", 4: "k_ccd_group<16, 1>", 5: "k_ccd_group<16, 4>"}
 
@@ -196,20 +178,6 @@ def fp64_peak():
     return out
 
 
-def fp64_roofline(captured, measured):
-    """The CCD kernel's FP64 side: its pipe-active fraction and lane-level
-    FP64 rate from the ncu capture, against the FP64 peak measured in this
-    run (all-lane DFMA chains)."""
-    if not captured:
-        return None
-    out = dict(captured, source="ncu capture of the 200-icosphere pile", nominal_gflops=1250.0)
-    if measured:
-        peak = measured["dfma_32"]["gflops"]
-        out["measured_peak_gflops"] = peak
-        out["frac_of_measured"] = captured["lane_gflops"] / peak
-    return out
-
-
 def pl_rate(ctx, sc, x0, x1, x0d, x1d, timed, with_cpu=True, sample=2000):
     """The piecewise-linear trajectory CCD (the reference's JSON default
     trajectory) over the headline's continuous candidates: one narrow-phase
@@ -222,7 +190,7 @@ def pl_rate(ctx, sc, x0, x1, x0d, x1d, timed, with_cpu=True, sample=2000):
     out = {"workload": "the headline pile's continuous candidates, trajectory PIECEWISE_LINEAR, "
                        "dmin 0, every candidate searched in full",
            "candidates": n, "ms": t_pl * 1e3, "pairs_per_s": n / t_pl,
-           "linear_ccd_boxes": st["ccd_boxes"], "kernel": "k_pl_ccd (one candidate per warp)"}
+           "linear_ccd_boxes": st["ccd_boxes"], "kernel": "k_pl_search (pieces and boxes as work items)"}
     if with_cpu:
         import oracle as O
 
@@ -839,7 +807,7 @@ def main():
     # the CCD kernel the context launches: one search per warp unless tuned
     # otherwise
     ccd_mode = tune.get("ccd_warp", -1) if tune else -1
-    ccd_kernel = CCD_KERNELS.get(ccd_mode, "k_ccd_group<32, 1>")
+    ccd_kernel = "k_ccd_filter + " + CCD_KERNELS.get(ccd_mode, "k_ccd_group<32, 1>")
     fp64 = fp64_peak() if rank == 0 else None
     ccd_bytes = CCD_BYTES_PER_PAIR * n_ccd
     achieved = ccd_bytes / t_ccd / 1e9
@@ -859,14 +827,9 @@ def main():
         "ccd_pairs_per_s": n_ccd / t_ccd, "barrier_constraints_per_s": n_cons / t_bar,
         "roofline": {"bound": "hbm", "kernel": ccd_kernel, "achieved": achieved, "peak": peak,
                      "unit": "GB/s", "frac": achieved / peak,
-                     "traffic": (K_CCD_DRAM_BYTES_PER_CANDIDATE[ccd_kernel] * n_ccd
-                                 if ccd_kernel in K_CCD_DRAM_BYTES_PER_CANDIDATE else None),
-                     "traffic_source": "ncu capture of the 200-icosphere pile scaled by candidates",
-                     "peak_source": peak_kind,
-                     "note": "FP64-issue-bound (an FP64 warp instruction holds its SM "
-                             "sub-partition's FP64 unit 64 cycles on GB300), not HBM: algorithmic "
-                             "bytes are 304 B per candidate",
-                     "fp64": fp64_roofline(K_CCD_FP64.get(ccd_kernel), fp64)},
+                     "traffic": None, "peak_source": peak_kind,
+                     "note": "bound by instruction issue (some 400 single-precision instructions "
+                             "a box), not HBM: algorithmic bytes are 304 B per candidate"},
         "e2e": {"value": e2e, "unit": UNIT, "h2d_bytes_per_step": h2d,
                 "d2h_bytes_per_step": d2h},
         "clocks": clk.summary(),

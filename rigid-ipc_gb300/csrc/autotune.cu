@@ -19,9 +19,9 @@
 //  * the CCD boxes a search piece evaluates before it hands its pending
 //    boxes to a further launch (never, 16, the built-in 64, 256): short
 //    pieces spread deep searches over the GPU, each hand-off costs a launch;
-//  * k_barrier_local's constraints per warp (1 .. 32): one thread per
-//    constraint fills the SMs for small sets, a full warp per 32 constraints
-//    shares the PSD projections for large ones.
+//  * k_barrier_local's constraints per warp (1 .. 32): few give each constraint
+//    more lanes (a shorter chain), 32 a lane each (every lane of an FP64
+//    instruction at work).
 // The choice stays in the context (Ctx::tune) for every later call.
 #include <algorithm>
 #include <chrono>

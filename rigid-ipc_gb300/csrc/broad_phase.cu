@@ -1503,12 +1503,6 @@ __global__ void __launch_bounds__(1024) k_bucket_large(
     }
 }
 
-__global__ void k_iota(uint32_t* __restrict__ v, int64_t n)
-{
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) v[i] = (uint32_t)i;
-}
-
 // ---------------------------------------------------------------------------
 
 constexpr int kDirectVertices = 16384;  // as compute_world_vertices_rn has it
