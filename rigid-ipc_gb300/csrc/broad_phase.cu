@@ -477,6 +477,14 @@ __global__ void __launch_bounds__(kVBThreads) k_vertex_hulls(HullList list, cons
 // (included body, slot).
 constexpr int kBPTableNodes = 127;  // slots 0 .. 126: depths 0 .. 6
 
+__device__ __forceinline__ void slot_interval(int slot, double toi_tol, double& t0, double& t1)
+{
+    const int d = 31 - __clz(slot + 1);
+    const int k = slot + 1 - (1 << d);
+    t0 = slot == kBPTableNodes ? 0.0 : ldexp((double)k, -d);
+    t1 = slot == kBPTableNodes ? toi_tol : ldexp((double)(k + 1), -d);
+}
+
 __global__ void k_bp_frames(const double* __restrict__ x0, const double* __restrict__ x1,
                             const int* __restrict__ body_in, int nb, double toi_tol,
                             double* __restrict__ table)
@@ -485,11 +493,45 @@ __global__ void k_bp_frames(const double* __restrict__ x0, const double* __restr
     if (i >= (int64_t)nb * kRotTableSlots) return;
     const int b = (int)(i / kRotTableSlots), slot = (int)(i % kRotTableSlots);
     if (!body_in[b]) return;
-    const int d = 31 - __clz(slot + 1);
-    const int k = slot + 1 - (1 << d);
+    double t0, t1;
+    slot_interval(slot, toi_tol, t0, t1);
+    body_time_frame(x0, x1, b, t0, t1, table + ((size_t)b * kRotTableSlots + slot) * kRotTableEntry);
+}
+
+// Four lanes per frame, for few bodies: a frame's chain of FP64 instructions
+// (some 460 by a thread) is what the kernel takes until its warps fill the 608
+// sub-partitions a few times: 27 cubes 69 -> 19 us, 131 icospheres 69 -> 45.  The
+// four lanes issue 1.4 times a thread's instructions, so more bodies stay with it.
+constexpr int kQuadFrames = 152;  // bodies up to which (16 warps each: four a sub-partition)
+
+__global__ void __launch_bounds__(128) k_bp_frames_quad(const double* __restrict__ x0, const double* __restrict__ x1,
+                                                        const int* __restrict__ body_in, int nb, double toi_tol,
+                                                        double* __restrict__ table)
+{
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 2, q = threadIdx.x & 3;
+    const int b = i / kRotTableSlots, slot = i % kRotTableSlots;
+    if (b >= nb || !body_in[b]) return;  // uniform over the warp
+    double t0, t1;
+    slot_interval(slot, toi_tol, t0, t1);
+    const Itv t { t0, t1 };
     double* out = table + ((size_t)b * kRotTableSlots + slot) * kRotTableEntry;
-    if (slot == kBPTableNodes) body_time_frame(x0, x1, b, 0.0, toi_tol, out);
-    else body_time_frame(x0, x1, b, ldexp((double)k, -d), ldexp((double)(k + 1), -d), out);
+    auto at = [&](int k) {
+        const double a = x0[6 * b + k], c = x1[6 * b + k];
+        return iadd(imul(Itv { sub_dn(c, a), sub_up(c, a) }, t), pt(a));
+    };
+    auto put = [&](int k, const Itv& x) {
+        out[2 * k] = x.lo;
+        out[2 * k + 1] = x.hi;
+    };
+    const Itv r[3] = { at(3), at(4), at(5) };
+    Itv diag, neg, pos;
+    irotation_quad(r, q, &diag, &neg, &pos);
+    if (q < 3) {
+        put(4 * q, diag);
+        put(q == 0 ? 5 : q == 1 ? 6 : 1, neg);
+        put(q == 0 ? 7 : q == 1 ? 2 : 3, pos);
+        put(9 + q, at(q));
+    }
 }
 
 // One thread per vertex: its interval positions over the two forced halves,
@@ -1639,8 +1681,12 @@ int detect_pairs(Ctx& c, const double* x0, const double* x1, bool continuous, do
         RIGC_COUNT_LAUNCH();
         k_scene_box<<<1, 256, 0, st>>>(c.body_box.as<double>(), c.body_in.as<int>(), s.nb, d_domain);
         RIGC_COUNT_LAUNCH();
-        k_bp_frames<<<grid_for((int64_t)s.nb * kRotTableSlots, 128), 128, 0, st>>>(
-            x0, x1, c.body_in.as<int>(), s.nb, kDefaultToiTol, table);
+        if (s.nb <= kQuadFrames)
+            k_bp_frames_quad<<<grid_for((int64_t)s.nb * kRotTableSlots * 4, 128), 128, 0, st>>>(
+                x0, x1, c.body_in.as<int>(), s.nb, kDefaultToiTol, table);
+        else
+            k_bp_frames<<<grid_for((int64_t)s.nb * kRotTableSlots, 128), 128, 0, st>>>(
+                x0, x1, c.body_in.as<int>(), s.nb, kDefaultToiTol, table);
         RIGC_CUDA(cudaMemsetAsync(c.bp_deeper.ptr, 0, deeper_bytes, st));
         RIGC_COUNT_LAUNCH();
         k_vertex_boxes_half<<<grid_for(s.nv, 128), 128, 0, st>>>(

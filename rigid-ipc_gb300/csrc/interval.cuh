@@ -295,17 +295,18 @@ static __device__ __noinline__ double sinc_bound(double xd, bool upper)
     return upper ? t.hi : t.lo;
 }
 
+constexpr double kSincMono = 4.4934094579;  // sinc decreases up to here
+
 // sinc over a non-negative interval (sinc.cpp:49-101; the input is a norm)
 static __device__ __noinline__ Itv isinc_nonneg(const Itv& x)
 {
-    const double kMono = 4.4934094579;
     Itv y = iempty();
     Itv x_gt = x;
-    if (x.lo <= kMono) {
+    if (x.lo <= kSincMono) {
         Itv x_mono = x;
-        if (x_mono.hi > kMono) {
-            x_mono = Itv { x_mono.lo, kMono };
-            x_gt = Itv { kMono, x.hi };
+        if (x_mono.hi > kSincMono) {
+            x_mono = Itv { x_mono.lo, kSincMono };
+            x_gt = Itv { kSincMono, x.hi };
         } else {
             x_gt = iempty();
         }
@@ -315,12 +316,24 @@ static __device__ __noinline__ Itv isinc_nonneg(const Itv& x)
     return y;
 }
 
-__device__ __forceinline__ Itv isinc_norm(const Itv r[3])
+// one bound of it
+__device__ __forceinline__ double isinc_nonneg_bound(const Itv& x, bool upper)
+{
+    if (x.lo <= kSincMono && x.hi <= kSincMono) {
+        const double b = sinc_bound(upper ? x.lo : x.hi, upper);
+        return upper ? smin(b, 1.0) : smax(b, -0.271724);
+    }
+    const Itv y = isinc_nonneg(x);
+    return upper ? y.hi : y.lo;
+}
+
+__device__ __forceinline__ Itv inorm(const Itv r[3])
 {
     Itv a0 = iabs(r[0]), a1 = iabs(r[1]), a2 = iabs(r[2]);
-    Itv d = iadd(iadd(imul(a0, a0), imul(a1, a1)), imul(a2, a2));
-    return isinc_nonneg(isqrt(d));
+    return isqrt(iadd(iadd(imul(a0, a0), imul(a1, a1)), imul(a2, a2)));
 }
+
+__device__ __forceinline__ Itv isinc_norm(const Itv r[3]) { return isinc_nonneg(inorm(r)); }
 
 // 0 + x: the bounds one step outward
 __device__ __forceinline__ Itv istep(const Itv& x)
@@ -361,6 +374,28 @@ static __device__ __noinline__ void irotation(const Itv r[3], Itv R[9])
     R[6] = iadd(ineg(s[1]), m02);
     R[5] = iadd(ineg(s[0]), m12);
     R[7] = iadd(s[0], m12);
+}
+
+// The same by four lanes (q = 0 .. 3): a bound of the two sinc each, then lane k
+// < 3 the entries of R's diagonal and of K at index k
+__device__ __forceinline__ void irotation_quad(const Itv r[3], int q, Itv* diag, Itv* neg, Itv* pos)
+{
+    Itv x[3];
+#pragma unroll
+    for (int k = 0; k < 3; k++) x[k] = q < 2 ? r[k] : Itv { mul_dn(r[k].lo, 0.5), mul_up(r[k].hi, 0.5) };
+    const double b = isinc_nonneg_bound(inorm(x), q & 1);
+    const Itv sa { __shfl_sync(0xffffffffu, b, 0, 4), __shfl_sync(0xffffffffu, b, 1, 4) };
+    const Itv sh { __shfl_sync(0xffffffffu, b, 2, 4), __shfl_sync(0xffffffffu, b, 3, 4) };
+    const Itv c = imul(imul(0.5, sh), sh);
+    const Itv ru = q == 2 ? r[1] : r[2], rv = q == 0 ? r[1] : r[0], rk = q == 0 ? r[0] : q == 1 ? r[1] : r[2];
+    const Itv nu = imul(ineg(ru), ru), nv = imul(ineg(rv), rv);
+    const Itv d = q == 0 ? istep(iadd(nu, nv)) : iadd(nu, istep(nv));
+    *diag = iadd(istep(imul(c, d)), pt(1.0));
+    Itv t = istep(imul(ru, rv));
+    if (q > 0) t = istep(t);
+    const Itv m = imul(c, t), s = imul(sa, rk);
+    *neg = iadd(ineg(s), m);
+    *pos = iadd(s, m);
 }
 
 // world vertex over intervals: ((v0 R_j0 + v1 R_j1) + v2 R_j2) + p_j

@@ -138,3 +138,28 @@ def test_constraint_sets(oracle, n):
         np.add.at(ref, g["bodies"][:, i], gl[:, 6 * i:6 * i + 6])
         np.add.at(mag, g["bodies"][:, i], np.abs(gl[:, 6 * i:6 * i + 6]))
     assert (np.abs(G.reshape(2, 6) - ref) <= 1e-12 * mag).all()
+
+
+@pytest.mark.parametrize("turn", [0.0, 0.3, 3.0, 9.0])
+def test_frames_by_four_lanes(turn):
+    """152 bodies (frames by four lanes) and one more far away, in no pair
+    (frames by a thread): the same candidates and times of impact, for small
+    turns, turns beyond the sinc's decrease (4.49) and none."""
+    import rigc
+
+    rng = np.random.default_rng(11)
+    M = [_hull(rng, 8 + i % 9) for i in range(153)]
+    P = np.concatenate([rng.uniform(-3.0, 3.0, (152, 3)), [[1e3, 0, 0]]])
+    dx = np.concatenate([rng.normal(0, 0.3, (153, 3)), rng.normal(0, turn, (153, 3))], 1)
+    res = []
+    for n in (152, 153):
+        sc = _scene(M[:n], P[:n])
+        x0 = sc.poses()
+        x1 = (x0.reshape(-1, 6) + dx[:n]).reshape(-1)
+        ctx = rigc.Context(sc)
+        ee, fv = ctx.detect_collision_candidates_rigid(x0, x1, True, 0.0)
+        assert len(ee) > 0
+        ctx.set_candidates(ee[::97], fv[::97])
+        res.append((ee, fv, ctx.earliest_toi(x0, x1), ctx.compute_earliest_toi(x0, x1)))
+    for a, b in zip(*res):
+        assert np.array_equal(a, b)
