@@ -1717,6 +1717,7 @@ int detect_pairs(Ctx& c, const double* x0, const double* x1, bool continuous, do
     const int64_t tiles = tiles_of(s.nv) + tiles_of(s.ne) + tiles_of(s.nf);
     const int64_t tile_pairs = tile_pairs_of(s, kind);
     const bool all_pairs = tile_pairs <= kAllPairsTiles;
+    const bool any_pairs = tile_pairs > 0;  // none: a scene without faces, or of vertices alone
     // patches wherever they are built, until their lists run over: a discrete and
     // a continuous call by the grid and by patches, 54 hulls 1025 and 366 us, 28
     // icospheres 1169 and 611, 1000 icospheres 4603 and 2413; beyond some 32
@@ -1730,7 +1731,7 @@ int detect_pairs(Ctx& c, const double* x0, const double* x1, bool continuous, do
     const uint64_t nslots = filter_slots(ntot);
     ElemBox* elem_boxes = nullptr;
     float* tile_boxes = nullptr;
-    if (all_pairs) {
+    if (all_pairs && any_pairs) {
         RIGC_TRY(c.bp_f32.reserve((size_t)ntot * sizeof(ElemBox) + (size_t)tiles * 6 * sizeof(float) + 8));
         elem_boxes = c.bp_f32.as<ElemBox>();
         tile_boxes = reinterpret_cast<float*>(elem_boxes + ntot);
@@ -1842,7 +1843,7 @@ int detect_pairs(Ctx& c, const double* x0, const double* x1, bool continuous, do
         PairOut o { c.pair_out.as<unsigned long long>(), c.pair_out.as<unsigned long long>() + cap_ee,
                     cap_ee, cap_fv, pn, pn + 1 };
         RIGC_CUDA(cudaMemsetAsync(pn, 0, 2 * sizeof(unsigned long long), st));
-        if (all_pairs) {
+        if (all_pairs && any_pairs) {
             RIGC_COUNT_LAUNCH();
             k_all_pairs<<<(unsigned)(tile_pairs * kTileParts), kTile, 0, st>>>(E, kind, elem_boxes, tile_boxes, o);
         }
