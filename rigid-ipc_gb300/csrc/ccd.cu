@@ -107,6 +107,8 @@ struct CCDArgs {
     // records for the single-precision front of the search (ccd_filter.cuh),
     // written by the set-up kernel; null: none
     struct FilterRec* rec;
+    unsigned long long* fstate;  // its candidates' states (the launch behind it)
+    unsigned long long* flat;    // set to 1 when some are flat
     const double* ref;
     const float* frames32;
     const float* bodies32;
@@ -715,6 +717,8 @@ __global__ void __launch_bounds__(128) k_ccd_prepare(CCDArgs a)
     if (a.rec) {
         filter_levels(tol, r);
         a.rec[i] = r;
+        a.fstate[i] = 0;
+        if (r.lev & kRecFlat) *a.flat = 1;
     }
 }
 
@@ -830,8 +834,16 @@ static __device__ __noinline__ double earliest_unexplored(const Node& cn, u128 m
 // work items of a launch: pieces, or the candidates' seeds
 __device__ __forceinline__ int64_t work_items(const CCDArgs& a)
 {
-    if (a.n_pieces_dev) return (int64_t)(*a.n_pieces_dev < a.out_cap ? *a.n_pieces_dev : a.out_cap);
+    // (more pieces than the buffer holds: the call is redone)
+    if (a.n_pieces_dev) return *a.n_pieces_dev <= a.out_cap ? (int64_t)*a.n_pieces_dev : 0;
     return a.pieces_in ? a.n_pieces : ((a.nee + a.nfv) << a.seeds_log2);
+}
+
+// a piece of the filter whose candidate was handed on as a whole later (that
+// one's pieces, its seeds, have 0 boxes)
+__device__ __forceinline__ bool superseded(const CCDArgs& a, const Piece& pc)
+{
+    return a.n_pieces_dev && pc.boxes != 0 && (a.fstate[pc.cand] & kHandedOn);
 }
 
 // Persistent kernel: each lane takes the next unprocessed candidate from a
@@ -1017,6 +1029,7 @@ k_ccd(CCDArgs a)
                     // the piece's node is popped (and tested) in the next iteration
                     const Piece pc = a.pieces_in[w];
                     cur = pc.cand;
+                    if (cur >= 0 && superseded(a, pc)) cur = -1;
                     if (cur >= 0) {
                         load_candidate(a, cur, q);
                         tol[0] = a.ctol[3 * cur];
@@ -1333,6 +1346,7 @@ k_ccd_group(CCDArgs a)
             if (a.pieces_in) {
                 const Piece pc = a.pieces_in[w];
                 cur = pc.cand;
+                if (cur >= 0 && superseded(a, pc)) cur = -1;
                 if (cur < 0) continue;
                 if (a.prune && !a.scene_gmin) {
                     // the group's first lane's copy of the running minimum
@@ -1647,8 +1661,8 @@ int reserve_rot_table(Ctx& c)
 // [0] gmin bits, [1] boxes, [2] hits, [3] status, [4] next work item,
 // [5] search pieces handed off, [6] pieces of the next launch, [7] / [8] of
 // later windows, [9] the filter's next work item, [10] the pieces of the
-// launch behind it
-constexpr int kCCDCounters = 11;
+// launch behind it, [11] whether some candidates are flat
+constexpr int kCCDCounters = 12;
 
 // filter: with the single-precision front; *redo is set (and no result
 // given) when its pieces did not fit their buffers
@@ -1728,6 +1742,8 @@ static int run_search(Ctx& c, const double* x0, const double* x1, double toi_tol
         a.fvals = c.frame_vals.as<double>();
         a.fmask = slots - 1;
         a.rec = nullptr;
+        a.fstate = nullptr;
+        a.flat = cnt + 11;
         a.ref = nullptr;
         a.frames32 = nullptr;
         a.bodies32 = nullptr;
@@ -1736,8 +1752,9 @@ static int run_search(Ctx& c, const double* x0, const double* x1, double toi_tol
             const size_t body_bytes = (size_t)c.s.nb * kBody32 * sizeof(float);
             RIGC_TRY(c.ccd_frames32.reserve(ref_bytes + body_bytes
                                             + (size_t)c.s.nb * kTableSlots * kFrame32 * sizeof(float)));
-            RIGC_TRY(c.ccd_rec.reserve((size_t)n * sizeof(FilterRec)));
+            RIGC_TRY(c.ccd_rec.reserve((size_t)n * (sizeof(FilterRec) + sizeof(unsigned long long))));
             a.rec = c.ccd_rec.as<FilterRec>();
+            a.fstate = reinterpret_cast<unsigned long long*>(a.rec + n);
             a.ref = c.ccd_frames32.as<double>();
             a.bodies32 = reinterpret_cast<const float*>(c.ccd_frames32.as<char>() + ref_bytes);
             a.frames32 = reinterpret_cast<const float*>(c.ccd_frames32.as<char>() + ref_bytes + body_bytes);
@@ -1821,7 +1838,10 @@ static int run_search(Ctx& c, const double* x0, const double* x1, double toi_tol
         int later = 2;
         // the filter appends its pieces to the first launch's
         FilterArgs f;
+        f.d = a;
         f.rec = a.rec;
+        f.state = a.fstate;
+        f.flat = a.flat;
         f.frames = a.frames32;
         f.bodies = a.bodies32;
         f.n = n;
@@ -1851,7 +1871,9 @@ static int run_search(Ctx& c, const double* x0, const double* x1, double toi_tol
                 RIGC_TRY(c.ccd_later.reserve((size_t)blocks * kFilterLists * f.later_cap * sizeof(FNode)));
                 f.later = c.ccd_later.as<FNode>();
                 RIGC_COUNT_LAUNCH();
-                k_ccd_filter<<<blocks, kFilterThreads, 0, st>>>(f);
+                k_ccd_filter<false><<<blocks, kFilterThreads, 0, st>>>(f);
+                RIGC_COUNT_LAUNCH();
+                k_ccd_filter<true><<<blocks, kFilterThreads, 0, st>>>(f);
                 RIGC_CUDA(cudaGetLastError());
                 a.n_pieces_dev = n_now_dev;
                 want = full;

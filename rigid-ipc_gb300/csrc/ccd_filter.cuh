@@ -11,6 +11,16 @@
 //    beyond kFilterLevel, is written out as a search piece, and the
 //    double-precision kernels decide it;
 //  * any other box is split by the search's own rule.
+// What single precision cannot decide is bounded: where the bodies do not move
+// along an axis and the offset there is 0 (a box landing on or sliding along
+// another, parallel edges), that axis's bounds are within E whatever the box's
+// size, no box is ever a root, and at gaps below E none is dropped either.  So a
+// candidate with kUndecidedLimit undecided boxes goes to the double-precision
+// search from its seeds, and its other boxes and pieces are dropped; a launch
+// whose pieces run over their buffer ends (the call is redone without it).
+// Parallel 1 m edges, 0.1 m along one another at a gap of 1e-7 m: above 2^28
+// boxes without the limit, 9000 with it (a block's boxes in flight when the first
+// reach the tolerance).
 // A box kept here that double precision would have dropped only costs its
 // subtree: the interval operations are inclusion isotonic, so the boxes
 // inside it are not roots.
@@ -77,6 +87,12 @@ constexpr int kBody32 = 24;          // deep_frame's body: theta, dtheta, dp (3 
 constexpr int kTaylor = 6;           // terms of S and C about the start pose
 constexpr int kSeries = 20;
 constexpr float kMaxTheta = 4.4f;    // S decreases up to 4.493
+// a candidate's state: undecided boxes from bit 32 on (kUndecidedLeaf for one
+// within tolerance, 1 for one at the limit of the levels, a subtree), bit 63 set
+// once it is handed on.  The limit: over piles, cubes and chains (tilted
+// contacts) a candidate has at most 20 within tolerance, nearly all none.
+constexpr unsigned kUndecidedLeaf = 16, kUndecidedLimit = 64 * kUndecidedLeaf;
+constexpr unsigned long long kHandedOn = 1ull << 63;
 
 struct alignas(16) FilterRec {
     float v[4][3];                   // rest vertices
@@ -91,6 +107,10 @@ static_assert(sizeof(FilterRec) == 128, "one 128-byte line per candidate");
 constexpr unsigned kRecFV = 1u << 18;       // face-vertex
 constexpr unsigned kRecDouble = 1u << 19;   // searched in double alone
 constexpr unsigned kRecShallow = 1u << 20;  // in double from time depth 7 on
+// f stays within E on an axis: no box is surely a root, those within tolerance
+// are decided in double where they are met; on two axes: next to none is dropped,
+// the candidate is searched in double alone, from its seeds
+constexpr unsigned kRecFlat = 1u << 21, kRecFlat2 = 1u << 22;
 
 // candidate; index (24 bits) and level (5 bits) of time, alpha and beta
 struct FNode {
@@ -100,7 +120,10 @@ __device__ __forceinline__ int fn_level(const FNode& n, int d) { return (int)(n.
 __device__ __forceinline__ unsigned fn_index(const FNode& n, int d) { return n.x[d] & 0xffffffu; }
 
 struct FilterArgs {
+    CCDArgs d;                       // the double-precision search's
     const FilterRec* rec;
+    unsigned long long* state;       // per candidate
+    const unsigned long long* flat;  // not 0: some candidates are flat
     const float* frames;             // nb x kTableSlots x kFrame32
     const float* bodies;             // nb x kBody32
     int64_t n;                       // candidates
@@ -291,6 +314,7 @@ __device__ __forceinline__ void filter_record(const Query& q, const double* __re
     const int na = q.fv ? 1 : 2;
     double X[4][3];
     float D = 0.0f, W = 0.0f, Tv = 0.0f, m = 0.0f;
+    float Dc[3] = { 0.0f, 0.0f, 0.0f };
     const float Ta = bodies[(size_t)q.body_a * kBody32 + 21], Tb = bodies[(size_t)q.body_b * kBody32 + 21];
     const bool deep = Ta < INFINITY && Tb < INFINITY;
 #pragma unroll
@@ -313,6 +337,7 @@ __device__ __forceinline__ void filter_record(const Query& q, const double* __re
 #pragma unroll
             for (int k = 0; k < 3; k++)
                 d = fmaf(fabsf(r.v[v][k]), fabsf(root[3 * c + k]) + root[9 + 3 * c + k], d);
+            Dc[c] = fmaxf(Dc[c], d);
             D = fmaxf(D, d);
             W = fmaxf(W, fabsf((float)X[v][c]));
         }
@@ -331,6 +356,10 @@ __device__ __forceinline__ void filter_record(const Query& q, const double* __re
     r.body_a = q.body_a;
     r.body_b = q.body_b;
     r.lev = (q.fv ? kRecFV : 0u) | (deep ? 0u : kRecShallow);
+    int flat = 0;
+#pragma unroll
+    for (int c = 0; c < 3; c++) flat += fabsf(r.Z[c]) + fabsf(r.A[c]) + fabsf(r.B[c]) + 6.0f * Dc[c] <= r.E;
+    r.lev |= (flat > 0 ? kRecFlat : 0u) | (flat > 1 ? kRecFlat2 : 0u);
     // finite bounds and tolerances whose keys order the splits; anything
     // else is left to the double-precision search from its root
     if (!(r.E < 1e18f) || !(m < 1e18f)) r.lev |= kRecDouble;
@@ -516,13 +545,104 @@ __device__ __forceinline__ bool filter_defer(const FilterArgs& a, FNode* later, 
     return true;
 }
 
+// Node j at depth seeds_log2 of a candidate's tree (seed_node); a candidate
+// left to the double-precision search, or within tolerance above that depth,
+// has one for all j below its node: false for the others
+__device__ __forceinline__ bool filter_seed(const FilterRec& r, int seeds_log2, unsigned j, FNode& x)
+{
+    int l = seeds_log2 - 1;
+    for (; l >= 0; l--) {
+        const int s = (r.lev & kRecDouble) ? -1 : filter_split(r, x);
+        if (s < 0) break;
+        x = filter_half(x, s, (j >> l) & 1u);
+    }
+    return l < 0 || (j & ((2u << l) - 1u)) == 0;
+}
+
+__device__ __forceinline__ Piece filter_piece(const FNode& x, unsigned long long boxes)
+{
+    Piece pc;
+    pc.cand = x.cand;
+    pc.earliest = INFINITY;
+    pc.depth = 0;
+    for (int d = 0; d < 3; d++) {
+        pc.ix[d] = fn_index(x, d);
+        pc.lv[d] = fn_level(x, d);
+        pc.depth += pc.lv[d];
+    }
+    pc.boxes = boxes;
+    return pc;
+}
+
+// f_zero of a box in double precision
+static __device__ __noinline__ bool filter_exact(const CCDArgs& a, const FNode& x)
+{
+    Query q;
+    load_candidate(a, x.cand, q);
+    Node n { { 0, 0, 0 }, { 0ull, 0ull, 0ull }, 0 };
+    for (int d = 0; d < 3; d++) {
+        n.lv[d] = fn_level(x, d);
+        n.ix[d] = fn_index(x, d);
+    }
+    const Box b = node_box(n);
+    const int na = q.fv ? 1 : 2;
+    Itv R[9], p[3];
+    frame_compute(a, q.body_a, Itv { b.t0, b.t1 }, R, p);
+    for (int v = 0; v < na; v++) iworld_vertex(R, p, q.v[v], q.P[v]);
+    frame_compute(a, q.body_b, Itv { b.t0, b.t1 }, R, p);
+    for (int v = na; v < 4; v++) iworld_vertex(R, p, q.v[v], q.P[v]);
+    return f_zero(q, b);
+}
+
+// one more undecided box of a candidate (weight k): its state
+__device__ __forceinline__ unsigned long long filter_undecided(const FilterArgs& a, unsigned cand, unsigned k)
+{
+    return atomicAdd(a.state + cand, (unsigned long long)k << 32) + ((unsigned long long)k << 32);
+}
+__device__ __forceinline__ bool past_limit(unsigned long long state)
+{
+    return (unsigned)((state & ~kHandedOn) >> 32) >= kUndecidedLimit;
+}
+
+__device__ __forceinline__ void record_root(const FilterArgs& a, const FNode& x)
+{
+    const unsigned long long t0 = (unsigned long long)dbits(dyadic(fn_index(x, 0), fn_level(x, 0)));
+    atomicMin(a.gmin, t0);
+    if (a.scene_gmin) atomicMin(a.scene_gmin + a.bscene[a.rec[x.cand].body_a], t0);
+}
+
+// a handed-on candidate's seeds as pieces (told from its earlier ones by 0
+// boxes); false: they did not fit
+static __device__ __noinline__ bool filter_hand_on(const FilterArgs& a, unsigned cand)
+{
+    const unsigned n = 1u << a.seeds_log2;
+    const unsigned long long o = atomicAdd(a.n_out, (unsigned long long)n);
+    if (o + n > a.cap) return false;
+    for (unsigned j = 0; j < n; j++) {
+        FNode x { cand, { 0, 0, 0 } };
+        const bool own = filter_seed(a.rec[cand], a.seeds_log2, j, x);
+        Piece pc = filter_piece(x, 0);
+        if (!own) pc.cand = -1;
+        a.out[o + j] = pc;
+    }
+    return true;
+}
+
+// kExact: for calls with flat candidates, whose boxes within tolerance are
+// decided here, in double, so that the running minimum falls in this launch (a
+// slab of 36 x 36 quads landing on another, aligned: 14.9 -> 1.5 ms); the call
+// costs registers (spills: a pile of 1000 icospheres 3 % slower), so both are
+// launched and the wrong one ends at once.
+template <bool kExact>
 __global__ void __launch_bounds__(kFilterThreads, kFilterBlocks)
 k_ccd_filter(FilterArgs a)
 {
+    if ((*a.flat != 0) != kExact) return;
     __shared__ FNode stack[kFilterStack];
     __shared__ int pushes[2][kFilterThreads / 32];  // per warp: lower halves | upper halves << 16
     __shared__ int later_cnt[kFilterLists];
     __shared__ unsigned long long batch, gmin_seen;
+    __shared__ bool full, over;      // the pieces have run over their buffer: seen by this block, by any
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const unsigned below = (1u << lane) - 1u;
     FNode* later = a.later + (size_t)blockIdx.x * kFilterLists * a.later_cap;
@@ -535,37 +655,30 @@ k_ccd_filter(FilterArgs a)
     int cnt = 0;                     // pending boxes (the same in every thread)
     int cur = -1;                    // the list being searched
     if (tid < kFilterLists) later_cnt[tid] = 0;
+    if (tid == 0) full = false;
     __syncthreads();
     for (int turn = 0;; turn ^= 1) {
         bool mine = false;
         FNode x { 0, { 0, 0, 0 } };
         if (cnt < kFilterThreads / 2 && more) {
             // a batch of new work items, one per thread, and nothing from the stack
-            if (tid == 0) batch = atomicAdd(a.next, 1ull);
+            if (tid == 0) {
+                batch = atomicAdd(a.next, 1ull);
+                over = *(volatile unsigned long long*)a.n_out > a.cap;
+            }
             __syncthreads();
             unsigned long long w = batch;
+            const bool stop = over;
             __syncthreads();
+            if (stop) break;
             if (w >= batches) {
                 more = false;
                 continue;
             }
             w += (unsigned long long)tid * batches;
             if (w < nwork) {
-                mine = true;
-                // seed j of the candidate: the node of its tree at depth
-                // seeds_log2 (seed_node); a candidate left to the
-                // double-precision search, or within tolerance above that
-                // depth, has one seed only
-                const unsigned j = (unsigned)(w / (unsigned long long)a.n);
                 x.cand = (unsigned)(w % (unsigned long long)a.n);
-                const FilterRec& r = a.rec[x.cand];
-                int l = a.seeds_log2 - 1;
-                for (; l >= 0; l--) {
-                    const int s = (r.lev & kRecDouble) ? -1 : filter_split(r, x);
-                    if (s < 0) break;
-                    x = filter_half(x, s, (j >> l) & 1u);
-                }
-                if (l >= 0) mine = (j & ((2u << l) - 1u)) == 0;
+                mine = filter_seed(a.rec[x.cand], a.seeds_log2, (unsigned)(w / (unsigned long long)a.n), x);
             }
         } else if (cnt > 0) {
             const int n = min(cnt, kFilterThreads);
@@ -600,10 +713,11 @@ k_ccd_filter(FilterArgs a)
         }
         const int lt = fn_level(x, 0), la = fn_level(x, 1), lb = fn_level(x, 2);
         const unsigned it = fn_index(x, 0), ia = fn_index(x, 1), ib = fn_index(x, 2);
-        bool emit = false, split = false, low = false;
+        bool emit = false, split = false, low = false, hand_on = false, exact = false;
         int s = 0;
         FNode up = x;                // the upper half
         bool high = false;
+        unsigned long long piece_boxes = 1;
         if (mine) {
             const unsigned long long t0 = (unsigned long long)dbits(dyadic(it, lt));
             // integers on 2^-24: a0 + b0 <= 1 (add_dn rounds exact sums, so
@@ -611,7 +725,7 @@ k_ccd_filter(FilterArgs a)
             const unsigned fa = ia << (kFilterLevel - la), fb = ib << (kFilterLevel - lb);
             const FilterRec& r = a.rec[x.cand];
             const unsigned lev = r.lev;
-            const bool fv = (lev & kRecFV) != 0;
+            const bool fv = (lev & kRecFV) != 0, searched = !(lev & (kRecDouble | kRecFlat2));
             unsigned long long* g = a.scene_gmin ? a.scene_gmin + a.bscene[r.body_a] : a.gmin;
             bool keep = t0 < *(volatile unsigned long long*)g && !(fv && fa + fb > (1u << kFilterLevel));
             // a seed of a later window, or a box its list had no room for
@@ -623,11 +737,15 @@ k_ccd_filter(FilterArgs a)
                 tot++;
                 int in = 0;
                 s = -1;
-                if (!(lev & kRecDouble)) {
+                unsigned long long seen = 0;
+                if (searched) {
+                    // (every fourth level: the memory's latency is 2 % of a call)
+                    if ((lt + la + lb) % 4 == 0) seen = *(volatile unsigned long long*)(a.state + x.cand);
                     in = filter_test(r, fv, a.frames, a.bodies, lt < kTableDepth ? (1 << lt) - 1 + (int)it : -1,
                                      (float)it * wt, (float)(it + 1) * wt, (float)ia * wa, wa, (float)ib * wb, wb);
                     s = filter_split(r, x);
                 }
+                if (seen & kHandedOn) in = -1;
                 if (in >= 0) {
                     // split: not within tolerance, and the halves have frames
                     // and exact levels
@@ -638,11 +756,21 @@ k_ccd_filter(FilterArgs a)
                         up = filter_half(x, s, 1u);
                     } else if (s < 0 && in > 0 && it > 0) {
                         // a root: within tolerance, after t = 0, zero inside
-                        atomicMin(g, t0);
-                        if (a.scene_gmin) atomicMin(a.gmin, t0);
+                        record_root(a, x);
                         hits++;
                     } else {
-                        emit = true;
+                        // (a flat candidate's boxes within tolerance are decided below)
+                        exact = kExact && searched && s < 0 && it > 0 && (lev & kRecFlat);
+                        if (!exact) {
+                            emit = true;
+                            piece_boxes = 0;
+                            if (searched) {
+                                const unsigned long long u = filter_undecided(a, x.cand, s < 0 ? kUndecidedLeaf : 1u);
+                                emit = !(u & kHandedOn);
+                                hand_on = past_limit(u);
+                                piece_boxes = 1;
+                            }
+                        }
                     }
                 }
             }
@@ -668,27 +796,25 @@ k_ccd_filter(FilterArgs a)
             if (low) stack[cnt + nh + nl - 1 - (before & 0xffff) - __popc(ml & below)] = filter_half(x, s, 0u);
             cnt += nl + nh;
         }
+        if (kExact && exact) {
+            if (filter_exact(a.d, x)) {
+                record_root(a, x);
+                hits++;
+            } else {
+                hand_on = past_limit(filter_undecided(a, x.cand, kUndecidedLeaf));
+            }
+        }
         const unsigned e = __ballot_sync(0xffffffffu, emit);
         if (e) {
             unsigned long long o = 0;
             if (lane == 0) o = atomicAdd(a.n_out, (unsigned long long)__popc(e));
             o = __shfl_sync(0xffffffffu, o, 0) + __popc(e & below);
-            if (emit && o < a.cap) {
-                Piece pc;
-                pc.cand = x.cand;
-                pc.earliest = INFINITY;
-                pc.ix[0] = it;
-                pc.ix[1] = ia;
-                pc.ix[2] = ib;
-                pc.lv[0] = lt;
-                pc.lv[1] = la;
-                pc.lv[2] = lb;
-                pc.depth = lt + la + lb;
-                pc.boxes = (unsigned long long)pc.depth;  // the boxes on its path
-                a.out[o] = pc;
-            }
+            if (emit && o < a.cap) a.out[o] = filter_piece(x, piece_boxes);
+            if (emit && o >= a.cap) full = true;
         }
-        __syncthreads();             // the pushed boxes are written
+        if (hand_on && !(atomicOr(a.state + x.cand, kHandedOn) & kHandedOn) && !filter_hand_on(a, x.cand)) full = true;
+        __syncthreads();             // the pushed boxes and full are written
+        if (full) break;
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
