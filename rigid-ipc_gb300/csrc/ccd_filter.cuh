@@ -305,6 +305,20 @@ __device__ __forceinline__ float split_pair(double x, unsigned short& rest)
 }
 __device__ __forceinline__ float pair_rest(unsigned short b) { return __uint_as_float((unsigned)b << 16); }
 
+// bound of the displacements along axis c over [0, 1] (rarely asked for)
+static __device__ __noinline__ float filter_axis_motion(const FilterRec& r, const Query& q,
+                                                        const float* __restrict__ frames, int c)
+{
+    float D = 0.0f;
+    for (int v = 0; v < 4; v++) {
+        const float* root = frames + (size_t)(v < (q.fv ? 1 : 2) ? q.body_a : q.body_b) * kTableSlots * kFrame32;
+        float d = fabsf(root[18 + c]) + root[21 + c];
+        for (int k = 0; k < 3; k++) d = fmaf(fabsf(r.v[v][k]), fabsf(root[3 * c + k]) + root[9 + 3 * c + k], d);
+        D = fmaxf(D, d);
+    }
+    return D;
+}
+
 // the record of a candidate (rest vertices and bodies in q) without its
 // tolerances' part
 __device__ __forceinline__ void filter_record(const Query& q, const double* __restrict__ ref,
@@ -314,7 +328,6 @@ __device__ __forceinline__ void filter_record(const Query& q, const double* __re
     const int na = q.fv ? 1 : 2;
     double X[4][3];
     float D = 0.0f, W = 0.0f, Tv = 0.0f, m = 0.0f;
-    float Dc[3] = { 0.0f, 0.0f, 0.0f };
     const float Ta = bodies[(size_t)q.body_a * kBody32 + 21], Tb = bodies[(size_t)q.body_b * kBody32 + 21];
     const bool deep = Ta < INFINITY && Tb < INFINITY;
 #pragma unroll
@@ -337,7 +350,6 @@ __device__ __forceinline__ void filter_record(const Query& q, const double* __re
 #pragma unroll
             for (int k = 0; k < 3; k++)
                 d = fmaf(fabsf(r.v[v][k]), fabsf(root[3 * c + k]) + root[9 + 3 * c + k], d);
-            Dc[c] = fmaxf(Dc[c], d);
             D = fmaxf(D, d);
             W = fmaxf(W, fabsf((float)X[v][c]));
         }
@@ -358,7 +370,10 @@ __device__ __forceinline__ void filter_record(const Query& q, const double* __re
     r.lev = (q.fv ? kRecFV : 0u) | (deep ? 0u : kRecShallow);
     int flat = 0;
 #pragma unroll
-    for (int c = 0; c < 3; c++) flat += fabsf(r.Z[c]) + fabsf(r.A[c]) + fabsf(r.B[c]) + 6.0f * Dc[c] <= r.E;
+    for (int c = 0; c < 3; c++) {
+        const float w = fabsf(r.Z[c]) + fabsf(r.A[c]) + fabsf(r.B[c]);
+        if (w <= r.E && w + 6.0f * filter_axis_motion(r, q, frames, c) <= r.E) flat++;
+    }
     r.lev |= (flat > 0 ? kRecFlat : 0u) | (flat > 1 ? kRecFlat2 : 0u);
     // finite bounds and tolerances whose keys order the splits; anything
     // else is left to the double-precision search from its root
@@ -559,7 +574,8 @@ __device__ __forceinline__ bool filter_seed(const FilterRec& r, int seeds_log2, 
     return l < 0 || (j & ((2u << l) - 1u)) == 0;
 }
 
-__device__ __forceinline__ Piece filter_piece(const FNode& x, unsigned long long boxes)
+// (its budget starts with the boxes on its path)
+__device__ __forceinline__ Piece filter_piece(const FNode& x)
 {
     Piece pc;
     pc.cand = x.cand;
@@ -570,7 +586,7 @@ __device__ __forceinline__ Piece filter_piece(const FNode& x, unsigned long long
         pc.lv[d] = fn_level(x, d);
         pc.depth += pc.lv[d];
     }
-    pc.boxes = boxes;
+    pc.boxes = (unsigned long long)pc.depth;
     return pc;
 }
 
@@ -621,7 +637,8 @@ static __device__ __noinline__ bool filter_hand_on(const FilterArgs& a, unsigned
     for (unsigned j = 0; j < n; j++) {
         FNode x { cand, { 0, 0, 0 } };
         const bool own = filter_seed(a.rec[cand], a.seeds_log2, j, x);
-        Piece pc = filter_piece(x, 0);
+        Piece pc = filter_piece(x);
+        pc.boxes = 0;
         if (!own) pc.cand = -1;
         a.out[o + j] = pc;
     }
@@ -717,7 +734,6 @@ k_ccd_filter(FilterArgs a)
         int s = 0;
         FNode up = x;                // the upper half
         bool high = false;
-        unsigned long long piece_boxes = 1;
         if (mine) {
             const unsigned long long t0 = (unsigned long long)dbits(dyadic(it, lt));
             // integers on 2^-24: a0 + b0 <= 1 (add_dn rounds exact sums, so
@@ -763,12 +779,10 @@ k_ccd_filter(FilterArgs a)
                         exact = kExact && searched && s < 0 && it > 0 && (lev & kRecFlat);
                         if (!exact) {
                             emit = true;
-                            piece_boxes = 0;
                             if (searched) {
                                 const unsigned long long u = filter_undecided(a, x.cand, s < 0 ? kUndecidedLeaf : 1u);
                                 emit = !(u & kHandedOn);
                                 hand_on = past_limit(u);
-                                piece_boxes = 1;
                             }
                         }
                     }
@@ -809,7 +823,7 @@ k_ccd_filter(FilterArgs a)
             unsigned long long o = 0;
             if (lane == 0) o = atomicAdd(a.n_out, (unsigned long long)__popc(e));
             o = __shfl_sync(0xffffffffu, o, 0) + __popc(e & below);
-            if (emit && o < a.cap) a.out[o] = filter_piece(x, piece_boxes);
+            if (emit && o < a.cap) a.out[o] = filter_piece(x);
             if (emit && o >= a.cap) full = true;
         }
         if (hand_on && !(atomicOr(a.state + x.cand, kHandedOn) & kHandedOn) && !filter_hand_on(a, x.cand)) full = true;
