@@ -183,10 +183,15 @@ int rigc_detect_candidates(rigc_ctx* ctx, const double* x0, const double* x1,
 int rigc_set_candidates(rigc_ctx* ctx, int64_t num_ee, const int32_t* ee,
                         int64_t num_fv, const int32_t* fv);
 
-/* Per-candidate cap on the boxes one CCD search may evaluate (default
+/* Cap on the boxes one double-precision CCD search may evaluate (default
  * 2^22; the reference has none).  A search that reaches it reports the
  * smallest t.lo still unexplored, a conservative time of impact, and
- * RIGC_ERR_ITER_LIMIT. */
+ * RIGC_ERR_ITER_LIMIT.  A search is a candidate's; in the pruned calls (the
+ * earliest time alone), whose searches are spread over the GPU in pieces, a
+ * piece's, with the boxes on the way to it.  The pruned calls with a cap of
+ * 2^22 or more search in single precision first; those boxes are not counted,
+ * and a candidate that single precision cannot decide within 64 boxes at the
+ * tolerance goes to the double-precision search. */
 int rigc_set_ccd_budget(rigc_ctx* ctx, int64_t max_boxes_per_candidate);
 
 /* ---- narrow phase CCD: compute_earliest_toi_narrow_phase
