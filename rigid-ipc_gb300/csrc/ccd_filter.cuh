@@ -328,6 +328,7 @@ __device__ __forceinline__ void filter_record(const Query& q, const double* __re
     const int na = q.fv ? 1 : 2;
     double X[4][3];
     float D = 0.0f, W = 0.0f, Tv = 0.0f, m = 0.0f;
+    float all = 0.0f;  // NaN when a position or displacement is (the maxima pass over NaN)
     const float Ta = bodies[(size_t)q.body_a * kBody32 + 21], Tb = bodies[(size_t)q.body_b * kBody32 + 21];
     const bool deep = Ta < INFINITY && Tb < INFINITY;
 #pragma unroll
@@ -352,6 +353,7 @@ __device__ __forceinline__ void filter_record(const Query& q, const double* __re
                 d = fmaf(fabsf(r.v[v][k]), fabsf(root[3 * c + k]) + root[9 + 3 * c + k], d);
             D = fmaxf(D, d);
             W = fmaxf(W, fabsf((float)X[v][c]));
+            all += 0.0f * (d + (float)X[v][c]);
         }
     }
 #pragma unroll
@@ -377,7 +379,7 @@ __device__ __forceinline__ void filter_record(const Query& q, const double* __re
     r.lev |= (flat > 0 ? kRecFlat : 0u) | (flat > 1 ? kRecFlat2 : 0u);
     // finite bounds and tolerances whose keys order the splits; anything
     // else is left to the double-precision search from its root
-    if (!(r.E < 1e18f) || !(m < 1e18f)) r.lev |= kRecDouble;
+    if (!(r.E < 1e18f) || !(m < 1e18f) || !(all == 0.0f)) r.lev |= kRecDouble;
 }
 
 // the tolerances' part

@@ -101,3 +101,23 @@ def test_batched_aligned():
         alone.append(one.earliest_toi(X0[12 * k:12 * k + 12], X1[12 * k:12 * k + 12], prune=False))
     ctx.compute_earliest_toi(X0, X1)
     assert np.array_equal(ctx.scene_tois(), np.array(alone))
+
+
+def test_pose_not_finite():
+    """Poses on the device are not checked: the search with a NaN among them ends
+    with the double-precision search's answer."""
+    import rigc
+
+    sc = _stack("cubes", 1e-3)
+    x0 = sc.poses()
+    x1 = x0.copy()
+    x1[7] -= 0.01
+    ctx = rigc.Context(sc)
+    ee, fv = ctx.detect_collision_candidates_rigid(x0, x1, True, 0.0)
+    for k in range(3):
+        y1 = x1.copy()
+        y1[6 + k] = np.nan
+        ctx.set_candidates(ee, fv)
+        (t, boxes), (t64, boxes64) = _searches(ctx, x0, y1)
+        assert t == t64
+        assert boxes <= boxes64 + 2 * (len(ee) + len(fv))  # one each, then from the root in double
