@@ -769,7 +769,8 @@ constexpr int kBlockSlices = 16, kGradSlices = 64;
 // Blocks over the unique Hessian blocks.  A diagonal block's segment lists
 // its body's constraints (slot 4 c: its first body, 4 c + 3: its second) in the
 // order of the gradient's own segment, so its block sums the body's gradient
-// too.
+// too.  (A constraint between vertices of one body, which a caller may set, has
+// all four slots there: 4 c + 1 and 4 c + 2 add nothing to the gradient.)
 __global__ void __launch_bounds__(36 * kBlockSlices) k_block_sums(
     const uint64_t* __restrict__ keys, const uint32_t* __restrict__ slots, const int32_t* __restrict__ seg_start,
     const int32_t* __restrict__ nseg_ptr, int64_t m, const double* __restrict__ blocks,
@@ -786,8 +787,8 @@ __global__ void __launch_bounds__(36 * kBlockSlices) k_block_sums(
         const uint32_t row = (uint32_t)(k / (uint64_t)nb);
         if (k != (uint64_t)row * (uint64_t)nb + row) continue;  // uniform over the block
         const double g = segment_sum<6, kGradSlices>(s0, s1, part, [&](int64_t i, int e) {
-            const uint32_t slot = slots[i];
-            return cgrad[(size_t)(slot >> 2) * 12 + 6 * ((slot & 3) == 3) + e];
+            const uint32_t slot = slots[i], q = slot & 3;
+            return q == 1 || q == 2 ? 0.0 : cgrad[(size_t)(slot >> 2) * 12 + 6 * (q == 3) + e];
         });
         if (threadIdx.x < 6) grad[(size_t)row * 6 + threadIdx.x] = g;
     }
