@@ -138,16 +138,6 @@ __device__ __forceinline__ void add_curvature(SMat H, const double* const* frame
 // -> 3.1 ms (FP64 issue), 98 k friction constraints 25.9 -> 1.4 ms, 338 barrier
 // constraints (16 lanes each) 0.50 -> 0.17 ms (the chain of one matrix).
 
-// 1 / sqrt(h) for normal h: the hardware approximation (about 20 bits) and one
-// third-order step
-__device__ __forceinline__ double rsqrt_refined(double h)
-{
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(h));
-    const double e = fma(-h * y, y, 1.0);
-    return fma(y * e, fma(0.375, e, 0.5), y);
-}
-
 template <int W>
 __device__ __forceinline__ void group_sync(unsigned mask)
 {
@@ -189,7 +179,7 @@ static __device__ void psd_project(SMat H, int g, unsigned mask)
             group_sync<W>(mask);
             continue;
         }
-        const double r = __dmul_rn(h, rsqrt_refined(h));
+        const double r = __dmul_rn(h, rsqrt(h));
         e[k] = x1 > 0 ? -r : r;
         const double v1 = x1 - e[k];
         const double beta = 1.0 / fma(fabs(x1), r, h);
@@ -288,7 +278,7 @@ static __device__ void psd_project(SMat H, int g, unsigned mask)
             const double h = fma(x, x, z * z);
             double c = 1, s = 0;
             if (h > 1e-290) {
-                const double ir = rsqrt_refined(h);
+                const double ir = rsqrt(h);
                 c = x * ir;
                 s = z * ir;
                 if (k > p) {

@@ -465,15 +465,7 @@ __global__ void k_dense_fill(HessView H, const int* __restrict__ free_idx, int n
 // one fused multiply-add per term: 17, 5 and 46 us (the back substitution alone).
 constexpr int kPanel = 32;
 
-// 1 / d for normal d: the hardware approximation (about 20 bits) and one
-// third-order step
-__device__ __forceinline__ double reciprocal(double d)
-{
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
-    const double e = fma(-d, y, 1.0);
-    return fma(y, fma(e, e, e), y);
-}
+static __device__ __noinline__ double quotient(double a, double d) { return a / d; }
 
 // Warps 0-3: the panel's diagonal block, lane = row, warp q taking columns
 // q, q + 4, ...; warps 4-7: the block's own rows j0 + w + 32 blockIdx.x + lane
@@ -504,7 +496,7 @@ __global__ void __launch_bounds__(256) k_ldlt_panel(double* __restrict__ A, int 
             col[b][half][lane] = v[c >> 2];
             if (half == 0 && lane == c) {
                 pivot = v[c >> 2];
-                inv[b] = reciprocal(pivot);
+                inv[b] = 1.0 / pivot;
             }
         }
         __syncthreads();
@@ -513,7 +505,9 @@ __global__ void __launch_bounds__(256) k_ldlt_panel(double* __restrict__ A, int 
             bad = true;  // the same in every thread
             break;
         }
-        const double l = __dmul_rn(col[b][half][lane], inv[b]);
+        // (the reciprocal of a subnormal pivot is infinite)
+        const double l = fabs(d) >= 2.2250738585072014e-308 ? __dmul_rn(col[b][half][lane], inv[b])
+                                                            : quotient(col[b][half][lane], d);
         if ((c & 3) == q) v[c >> 2] = l;
 #pragma unroll
         for (int k = 0; k < kPanel / 4; k++)
