@@ -475,7 +475,8 @@ __global__ void __launch_bounds__(256) k_ldlt_panel(double* __restrict__ A, int 
 {
     __shared__ double col[2][2][kPanel];  // [column parity][half][row]: the column before scaling
     __shared__ double inv[2];
-    if (flags[0]) return;
+    // (a block that fails sets the flag: one answer for all threads of this one)
+    if (__syncthreads_or(flags[0])) return;
     const int w = min(kPanel, n - j0);
     const int lane = threadIdx.x & 31, half = threadIdx.x >> 7, q = (threadIdx.x >> 5) & 3;
     const int row = half ? j0 + w + 32 * (int)blockIdx.x + lane : j0 + lane;
