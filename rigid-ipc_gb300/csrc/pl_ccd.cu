@@ -1264,12 +1264,9 @@ int run_pl_ccd(Ctx& c, const double* x0, const double* x1, double dmin, double* 
             s.hard = s.nboxes + n;
             s.n_hard = cnt + 5;
             s.per_batch = per_batch;
-            static bool attr = false;
-            if (!attr) {
-                RIGC_CUDA(cudaFuncSetAttribute(k_pl_search, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)search_smem_bytes()));
-                attr = true;
-            }
+            // (the device's own attribute: set on each call, whichever device that is for)
+            RIGC_CUDA(cudaFuncSetAttribute(k_pl_search, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)search_smem_bytes()));
             RIGC_COUNT_LAUNCH();
             k_pl_init<<<grid_for(n, 256), 256, 0, st>>>(s, n);
             RIGC_COUNT_LAUNCH();
