@@ -484,7 +484,8 @@ int rigc_sim_set_kinematic(rigc_ctx* ctx, int32_t body, double max_time, int64_t
  * candidates of x0 -> x1 and the constraint set at x0 (device poses), and
  * keeps the fastest in the context for every later call.  rigc_set_tune
  * sets them directly: for ccd_blocks_per_sm, cache_slots_per_body and
- * barrier_per_warp 0 is the built-in choice; for ccd_seeds_log2,
+ * barrier_per_warp 0 is the built-in choice (barrier_per_warp is rounded up
+ * to a power of two of at least 2); for ccd_seeds_log2,
  * ccd_hand_off and ccd_warp the built-in choice is -1 (0 means something
  * else there: one seed, never hand off, one search per lane). */
 typedef struct rigc_tune_report {

@@ -19,7 +19,7 @@
 //  * the CCD boxes a search piece evaluates before it hands its pending
 //    boxes to a further launch (never, 16, the built-in 64, 256): short
 //    pieces spread deep searches over the GPU, each hand-off costs a launch;
-//  * k_barrier_local's constraints per warp (1 .. 32): few give each constraint
+//  * k_barrier_local's constraints per warp (2 .. 32): few give each constraint
 //    more lanes (a shorter chain), 32 a lane each (every lane of an FP64
 //    instruction at work).
 // The choice stays in the context (Ctx::tune) for every later call.
@@ -159,7 +159,7 @@ int autotune(Ctx& c, const double* x0, const double* x1, double dhat, double dmi
     RIGC_TRY(median_ms(barrier, &r.barrier_ms_default));
     best = r.barrier_ms_default;
     int best_pw = 0;
-    for (int pw : { 1, 2, 4, 8, 16, 32 }) {
+    for (int pw : { 2, 4, 8, 16, 32 }) {
         c.tune.barrier_per_warp = pw;
         double ms;
         RIGC_TRY(median_ms(barrier, &ms));

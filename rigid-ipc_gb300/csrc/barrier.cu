@@ -515,7 +515,7 @@ size_t local_terms_smem_bytes(int per_warp)
 
 // Constraints per warp: a thread per constraint (32) once they give every SM
 // eight warps, fewer for small sets, down to 2 (16 lanes to each).  A power of
-// two; tuned > 0: at most that.
+// two; tuned > 0: the next one from it, at least 2.
 int local_terms_per_warp(int64_t n, int tuned)
 {
     const int64_t w = tuned > 0 ? tuned : (n + kNumSMs * 8 - 1) / (kNumSMs * 8);
