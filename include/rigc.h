@@ -244,8 +244,9 @@ int rigc_set_pl_search(rigc_ctx* ctx, int32_t per_lane);
  * that start before 2^-window_log2 and defers the others, each later launch
  * doubles the window, so the boxes of all candidates are searched roughly in
  * time order and the running minimum, once found, skips every later box.
- * -1 the built-in choice (2^-6 from 65,536 candidates on, else none), 0 no
- * windows.  The earliest time of impact
+ * -1 the built-in choice (2^-6 for the calls that search in single precision
+ * first, see rigc_set_ccd_budget, whose windows are lists within one launch; for
+ * the others 2^-6 from 65,536 candidates on, below that none), 0 no windows.  The earliest time of impact
  * is the same bits either way; only the work differs. */
 int rigc_set_ccd_window(rigc_ctx* ctx, int32_t window_log2);
 

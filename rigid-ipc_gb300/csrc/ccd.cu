@@ -53,7 +53,8 @@ constexpr int kHandOff = 64;
 constexpr unsigned long long kPiecesCap = 1ull << 18;
 constexpr int kMaxLaunches = 32;
 // time windows (search groups, prune mode): the first window 2^-k (built-in
-// k, from kWindowMinCandidates candidates on: below, the launches they add
+// k; without the single-precision front, whose windows are lists within its
+// launch, from kWindowMinCandidates candidates on: below, the launches they add
 // cost more than the boxes they skip), each later launch's twice the last
 // one's, none from 1 on; slots per piece buffer at most kWindowCap
 constexpr int kWindowLog2 = 6;
