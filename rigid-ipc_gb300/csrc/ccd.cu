@@ -1973,10 +1973,15 @@ int run_ccd(Ctx& c, const double* x0, const double* x1, double toi_tol, int flag
 {
     const bool filter = !(flags & RIGC_TOI_NO_PRUNE) && !per && c.ccd_max_boxes >= kFilterMinBudget
         && c.cand.num_ee + c.cand.num_fv < (int64_t(1) << 31);
-    bool redo = false;
-    const int s = run_search(c, x0, x1, toi_tol, flags, toi_host, per, filter, &redo);
-    if (!redo) return s;
-    return run_search(c, x0, x1, toi_tol, flags, toi_host, per, false, &redo);
+    if (filter) {
+        bool redo = false;
+        const int s = run_search(c, x0, x1, toi_tol, flags, toi_host, per, true, &redo);
+        if (s != RIGC_ERR_OOM && !redo) return s;
+        // no memory for its records and lists: given back, the search goes without
+        if (s == RIGC_ERR_OOM)
+            for (DevBuf* b : { &c.ccd_rec, &c.ccd_frames32, &c.ccd_later }) b->release();
+    }
+    return run_search(c, x0, x1, toi_tol, flags, toi_host, per, false, nullptr);
 }
 
 } // namespace rigc

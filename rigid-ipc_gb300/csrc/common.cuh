@@ -74,6 +74,8 @@ struct DevBuf {
         size_t want = n + n / 4 + 256;
         cudaError_t e = cudaMalloc(&ptr, want);
         if (e != cudaSuccess) {
+            ptr = nullptr;
+            cudaGetLastError();  // a caller may do without
             set_error(RIGC_ERR_OOM, cudaGetErrorString(e), __FILE__, __LINE__);
             return RIGC_ERR_OOM;
         }

@@ -1242,19 +1242,20 @@ int run_pl_ccd(Ctx& c, const double* x0, const double* x1, double dmin, double* 
         RIGC_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
         // pieces and boxes as work items unless tuned to one candidate per
         // warp (slower on every workload measured: k_pl_search's header)
-        const bool search = c.tune.pl_per_lane != 0 && n < (int64_t(1) << 31);
+        bool search = c.tune.pl_per_lane != 0 && n < (int64_t(1) << 31);
         a.list = nullptr;
         a.n_list = nullptr;
         int blocks = 0;
         RIGC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k_pl_ccd, kPLThreads, 0));
         const unsigned full = (unsigned)(sms * std::max(1, blocks));
         unsigned grid = (unsigned)std::min<int64_t>((n + 3) / 4, full);
+        // few candidates spread over all blocks, four or more to each
+        const int per_batch = (int)std::max<int64_t>(4, std::min<int64_t>(kSearchThreads, (n + 2 * sms - 1) / (2 * sms)));
+        const unsigned sblocks = (unsigned)std::min<int64_t>((n + per_batch - 1) / per_batch, 2 * sms);
+        const size_t job_bytes = (size_t)sblocks * kJobs * sizeof(Job);
+        // no memory for their state: one candidate per warp
+        if (search) search = c.pl_work.reserve(job_bytes + (size_t)n * (2 * sizeof(double) + 3 * sizeof(int))) == RIGC_OK;
         if (search) {
-            // few candidates spread over all blocks, four or more to each
-            const int per_batch = (int)std::max<int64_t>(4, std::min<int64_t>(kSearchThreads, (n + 2 * sms - 1) / (2 * sms)));
-            const unsigned sblocks = (unsigned)std::min<int64_t>((n + per_batch - 1) / per_batch, 2 * sms);
-            const size_t job_bytes = (size_t)sblocks * kJobs * sizeof(Job);
-            RIGC_TRY(c.pl_work.reserve(job_bytes + (size_t)n * (2 * sizeof(double) + 3 * sizeof(int))));
             SearchArgs s;
             s.jobs = c.pl_work.as<Job>();
             s.d0 = reinterpret_cast<double*>(c.pl_work.as<char>() + job_bytes);
