@@ -28,7 +28,9 @@
 // What bounds it: an FP64 warp instruction takes 64 cycles of its
 // sub-partition on this GPU, a single-precision one 1, so the ~260 FP64
 // operations of a box (or the ~900 warp instructions that spread them over a
-// warp) become ~400 single-precision ones of a thread, a box per thread.
+// warp) become ~400 single-precision ones of a thread, a box per thread.  What is
+// left is the latency of a block's turns: 16 to 23 % of the issue slots are used, the
+// warps wait at the two barriers of a turn and for records and frames.
 // Measured (device time of the search, double-precision kernels alone and
 // with this one in front): a pile of 1000 icospheres, 709 k candidates, 20.4
 // -> 0.84 ms (5.4 M boxes); a 200-link chain in contact, 41 k candidates, 6 ->
@@ -629,10 +631,11 @@ __device__ __forceinline__ void record_root(const FilterArgs& a, const FNode& x)
     if (a.scene_gmin) atomicMin(a.scene_gmin + a.bscene[a.rec[x.cand].body_a], t0);
 }
 
-// a handed-on candidate's seeds as pieces (told from its earlier ones by 0
-// boxes); false: they did not fit
+// A candidate is handed on: its seeds as pieces (told from its earlier ones by 0
+// boxes), once; false: they did not fit
 static __device__ __noinline__ bool filter_hand_on(const FilterArgs& a, unsigned cand)
 {
+    if (atomicOr(a.state + cand, kHandedOn) & kHandedOn) return true;
     const unsigned n = 1u << a.seeds_log2;
     const unsigned long long o = atomicAdd(a.n_out, (unsigned long long)n);
     if (o + n > a.cap) return false;
@@ -649,9 +652,9 @@ static __device__ __noinline__ bool filter_hand_on(const FilterArgs& a, unsigned
 
 // kExact: for calls with flat candidates, whose boxes within tolerance are
 // decided here, in double, so that the running minimum falls in this launch (a
-// slab of 36 x 36 quads landing on another, aligned: 14.9 -> 1.5 ms); the call
-// costs registers (spills: a pile of 1000 icospheres 3 % slower), so both are
-// launched and the wrong one ends at once.
+// slab of 36 x 36 quads landing on another, aligned: 14.9 -> 1.4 ms).  It is done between the turns, which the call would otherwise cost
+// registers (a 200-link chain in line, without a box to decide, 1.40 -> 1.54 ms;
+// so 1.45); both are launched, and the wrong one ends at once.
 template <bool kExact>
 __global__ void __launch_bounds__(kFilterThreads, kFilterBlocks)
 k_ccd_filter(FilterArgs a)
@@ -673,165 +676,189 @@ k_ccd_filter(FilterArgs a)
     bool more = true;
     int cnt = 0;                     // pending boxes (the same in every thread)
     int cur = -1;                    // the list being searched
+    // kExact: the turns stop when boxes are to be decided in double (a call
+    // within them would cost every turn its registers)
+    __shared__ FNode exact_box[kExact ? kFilterThreads : 1];
+    __shared__ int n_exact;
+    __shared__ bool exact_full;
+    bool pause = false;
+    int turn = 0;
     if (tid < kFilterLists) later_cnt[tid] = 0;
-    if (tid == 0) full = false;
+    if (tid == 0) {
+        full = exact_full = false;
+        n_exact = 0;
+    }
     __syncthreads();
-    for (int turn = 0;; turn ^= 1) {
-        bool mine = false;
-        FNode x { 0, { 0, 0, 0 } };
-        if (cnt < kFilterThreads / 2 && more) {
-            // a batch of new work items, one per thread, and nothing from the stack
-            if (tid == 0) {
-                batch = atomicAdd(a.next, 1ull);
-                over = *(volatile unsigned long long*)a.n_out > a.cap;
-            }
-            __syncthreads();
-            unsigned long long w = batch;
-            const bool stop = over;
-            __syncthreads();
-            if (stop) break;
-            if (w >= batches) {
-                more = false;
-                continue;
-            }
-            w += (unsigned long long)tid * batches;
-            if (w < nwork) {
-                x.cand = (unsigned)(w % (unsigned long long)a.n);
-                mine = filter_seed(a.rec[x.cand], a.seeds_log2, (unsigned)(w / (unsigned long long)a.n), x);
-            }
-        } else if (cnt > 0) {
-            const int n = min(cnt, kFilterThreads);
-            mine = tid < n;
-            if (mine) x = stack[cnt - 1 - tid];
-            cnt -= n;
-        } else {
-            // the next list; a list after a single scene's first impact and
-            // all later ones are dropped
-            if (cur >= 0) {
-                const int left = later_cnt[cur];
-                __syncthreads();
-                if (left > 0) {
-                    const int n = min(left, kFilterThreads);
-                    mine = tid < n;
-                    if (mine) x = later[(size_t)cur * a.later_cap + left - 1 - tid];
-                    if (tid == 0) later_cnt[cur] = left - n;
+    do {
+        pause = false;
+        for (;; turn ^= 1) {
+            bool mine = false;
+            FNode x { 0, { 0, 0, 0 } };
+            if (cnt < kFilterThreads / 2 && more) {
+                // a batch of new work items, one per thread, and nothing from the stack
+                if (tid == 0) {
+                    batch = atomicAdd(a.next, 1ull);
+                    over = *(volatile unsigned long long*)a.n_out > a.cap;
                 }
-                if (left == 0) {
-                    if (++cur >= kFilterLists) break;
+                __syncthreads();
+                unsigned long long w = batch;
+                const bool stop = over;
+                __syncthreads();
+                if (stop) break;
+                if (w >= batches) {
+                    more = false;
                     continue;
                 }
-            } else {
-                cur = 0;
-                continue;
-            }
-            if (!a.scene_gmin) {
-                if (tid == 0) gmin_seen = *(volatile unsigned long long*)a.gmin;
-                __syncthreads();
-                if (gmin_seen <= (unsigned long long)(1023 + cur - a.window_log2) << 52) break;
-            }
-        }
-        const int lt = fn_level(x, 0), la = fn_level(x, 1), lb = fn_level(x, 2);
-        const unsigned it = fn_index(x, 0), ia = fn_index(x, 1), ib = fn_index(x, 2);
-        bool emit = false, split = false, low = false, hand_on = false, exact = false;
-        int s = 0;
-        FNode up = x;                // the upper half
-        bool high = false;
-        if (mine) {
-            const unsigned long long t0 = (unsigned long long)dbits(dyadic(it, lt));
-            // integers on 2^-24: a0 + b0 <= 1 (add_dn rounds exact sums, so
-            // its test is this one), and the upper sum is never negative
-            const unsigned fa = ia << (kFilterLevel - la), fb = ib << (kFilterLevel - lb);
-            const FilterRec& r = a.rec[x.cand];
-            const unsigned lev = r.lev;
-            const bool fv = (lev & kRecFV) != 0, searched = !(lev & (kRecDouble | kRecFlat2));
-            unsigned long long* g = a.scene_gmin ? a.scene_gmin + a.bscene[r.body_a] : a.gmin;
-            bool keep = t0 < *(volatile unsigned long long*)g && !(fv && fa + fb > (1u << kFilterLevel));
-            // a seed of a later window, or a box its list had no room for
-            if (keep) keep = !filter_defer(a, later, later_cnt, cur, x);
-            if (keep) {
-                // exact: integers up to 2^24 times a power of two
-                const float wt = __int_as_float((127 - lt) << 23);
-                const float wa = __int_as_float((127 - la) << 23), wb = __int_as_float((127 - lb) << 23);
-                tot++;
-                int in = 0;
-                s = -1;
-                unsigned long long seen = 0;
-                if (searched) {
-                    // (every fourth level: the memory's latency is 2 % of a call)
-                    if ((lt + la + lb) % 4 == 0) seen = *(volatile unsigned long long*)(a.state + x.cand);
-                    in = filter_test(r, fv, a.frames, a.bodies, lt < kTableDepth ? (1 << lt) - 1 + (int)it : -1,
-                                     (float)it * wt, (float)(it + 1) * wt, (float)ia * wa, wa, (float)ib * wb, wb);
-                    s = filter_split(r, x);
+                w += (unsigned long long)tid * batches;
+                if (w < nwork) {
+                    x.cand = (unsigned)(w % (unsigned long long)a.n);
+                    mine = filter_seed(a.rec[x.cand], a.seeds_log2, (unsigned)(w / (unsigned long long)a.n), x);
                 }
-                if (seen & kHandedOn) in = -1;
-                if (in >= 0) {
-                    // split: not within tolerance, and the halves have frames
-                    // and exact levels
-                    const int limit = s == 0 && (lev & kRecShallow) ? kTableDepth - 1 : kFilterLevel - 1;
-                    split = s >= 0 && (s == 0 ? lt : s == 1 ? la : lb) < limit;
-                    if (split) {
-                        low = high = true;
-                        up = filter_half(x, s, 1u);
-                    } else if (s < 0 && in > 0 && it > 0) {
-                        // a root: within tolerance, after t = 0, zero inside
-                        record_root(a, x);
-                        hits++;
-                    } else {
-                        // (a flat candidate's boxes within tolerance are decided below)
-                        exact = kExact && searched && s < 0 && it > 0 && (lev & kRecFlat);
-                        if (!exact) {
-                            emit = true;
-                            if (searched) {
-                                const unsigned long long u = filter_undecided(a, x.cand, s < 0 ? kUndecidedLeaf : 1u);
-                                emit = !(u & kHandedOn);
-                                hand_on = past_limit(u);
+            } else if (cnt > 0) {
+                const int n = min(cnt, kFilterThreads);
+                mine = tid < n;
+                if (mine) x = stack[cnt - 1 - tid];
+                cnt -= n;
+            } else {
+                // the next list; a list after a single scene's first impact and
+                // all later ones are dropped
+                if (cur >= 0) {
+                    const int left = later_cnt[cur];
+                    __syncthreads();
+                    if (left > 0) {
+                        const int n = min(left, kFilterThreads);
+                        mine = tid < n;
+                        if (mine) x = later[(size_t)cur * a.later_cap + left - 1 - tid];
+                        if (tid == 0) later_cnt[cur] = left - n;
+                    }
+                    if (left == 0) {
+                        if (++cur >= kFilterLists) break;
+                        continue;
+                    }
+                } else {
+                    cur = 0;
+                    continue;
+                }
+                if (!a.scene_gmin) {
+                    if (tid == 0) gmin_seen = *(volatile unsigned long long*)a.gmin;
+                    __syncthreads();
+                    if (gmin_seen <= (unsigned long long)(1023 + cur - a.window_log2) << 52) break;
+                }
+            }
+            const int lt = fn_level(x, 0), la = fn_level(x, 1), lb = fn_level(x, 2);
+            const unsigned it = fn_index(x, 0), ia = fn_index(x, 1), ib = fn_index(x, 2);
+            bool emit = false, split = false, low = false, hand_on = false, exact = false;
+            int s = 0;
+            FNode up = x;                // the upper half
+            bool high = false;
+            if (mine) {
+                const unsigned long long t0 = (unsigned long long)dbits(dyadic(it, lt));
+                // integers on 2^-24: a0 + b0 <= 1 (add_dn rounds exact sums, so
+                // its test is this one), and the upper sum is never negative
+                const unsigned fa = ia << (kFilterLevel - la), fb = ib << (kFilterLevel - lb);
+                const FilterRec& r = a.rec[x.cand];
+                const unsigned lev = r.lev;
+                const bool fv = (lev & kRecFV) != 0, searched = !(lev & (kRecDouble | kRecFlat2));
+                unsigned long long* g = a.scene_gmin ? a.scene_gmin + a.bscene[r.body_a] : a.gmin;
+                bool keep = t0 < *(volatile unsigned long long*)g && !(fv && fa + fb > (1u << kFilterLevel));
+                // a seed of a later window, or a box its list had no room for
+                if (keep) keep = !filter_defer(a, later, later_cnt, cur, x);
+                if (keep) {
+                    // exact: integers up to 2^24 times a power of two
+                    const float wt = __int_as_float((127 - lt) << 23);
+                    const float wa = __int_as_float((127 - la) << 23), wb = __int_as_float((127 - lb) << 23);
+                    tot++;
+                    int in = 0;
+                    s = -1;
+                    unsigned long long seen = 0;
+                    if (searched) {
+                        // (every fourth level: the memory's latency is 2 % of a call)
+                        if ((lt + la + lb) % 4 == 0) seen = *(volatile unsigned long long*)(a.state + x.cand);
+                        in = filter_test(r, fv, a.frames, a.bodies, lt < kTableDepth ? (1 << lt) - 1 + (int)it : -1,
+                                         (float)it * wt, (float)(it + 1) * wt, (float)ia * wa, wa, (float)ib * wb, wb);
+                        s = filter_split(r, x);
+                    }
+                    if (seen & kHandedOn) in = -1;
+                    if (in >= 0) {
+                        // split: not within tolerance, and the halves have frames
+                        // and exact levels
+                        const int limit = s == 0 && (lev & kRecShallow) ? kTableDepth - 1 : kFilterLevel - 1;
+                        split = s >= 0 && (s == 0 ? lt : s == 1 ? la : lb) < limit;
+                        if (split) {
+                            low = high = true;
+                            up = filter_half(x, s, 1u);
+                        } else if (s < 0 && in > 0 && it > 0) {
+                            // a root: within tolerance, after t = 0, zero inside
+                            record_root(a, x);
+                            hits++;
+                        } else {
+                            // (a flat candidate's boxes within tolerance are decided below)
+                            exact = kExact && searched && s < 0 && it > 0 && (lev & kRecFlat);
+                            if (!exact) {
+                                emit = true;
+                                if (searched) {
+                                    const unsigned long long u = filter_undecided(a, x.cand, s < 0 ? kUndecidedLeaf : 1u);
+                                    emit = !(u & kHandedOn);
+                                    hand_on = past_limit(u);
+                                }
                             }
                         }
                     }
                 }
+                if (high) high = !filter_defer(a, later, later_cnt, cur, up);
             }
-            if (high) high = !filter_defer(a, later, later_cnt, cur, up);
-        }
-        // halves: the lower ones on top; without room the box itself goes on
-        const unsigned ml = __ballot_sync(0xffffffffu, low), mh = __ballot_sync(0xffffffffu, high);
-        if (lane == 0) pushes[turn][warp] = __popc(ml) | __popc(mh) << 16;
-        __syncthreads();             // the boxes popped are read, the counts written
-        if (tid < kFilterLists && later_cnt[tid] > a.later_cap) later_cnt[tid] = a.later_cap;
-        int all = 0, before = 0;
+            // halves: the lower ones on top; without room the box itself goes on
+            const unsigned ml = __ballot_sync(0xffffffffu, low), mh = __ballot_sync(0xffffffffu, high);
+            if (lane == 0) pushes[turn][warp] = __popc(ml) | __popc(mh) << 16;
+            __syncthreads();             // the boxes popped are read, the counts written
+            if (tid < kFilterLists && later_cnt[tid] > a.later_cap) later_cnt[tid] = a.later_cap;
+            int all = 0, before = 0;
 #pragma unroll
-        for (int k = 0; k < kFilterThreads / 32; k++) {
-            const int q = pushes[turn][k];
-            all += q;
-            if (k < warp) before += q;
-        }
-        const int nl = all & 0xffff, nh = all >> 16;
-        if (cnt + nl + nh > kFilterStack) {
-            emit = emit || split;
-        } else {
-            if (high) stack[cnt + nh - 1 - (before >> 16) - __popc(mh & below)] = up;
-            if (low) stack[cnt + nh + nl - 1 - (before & 0xffff) - __popc(ml & below)] = filter_half(x, s, 0u);
-            cnt += nl + nh;
-        }
-        if (kExact && exact) {
-            if (filter_exact(a.d, x)) {
-                record_root(a, x);
-                hits++;
+            for (int k = 0; k < kFilterThreads / 32; k++) {
+                const int q = pushes[turn][k];
+                all += q;
+                if (k < warp) before += q;
+            }
+            const int nl = all & 0xffff, nh = all >> 16;
+            if (cnt + nl + nh > kFilterStack) {
+                emit = emit || split;
             } else {
-                hand_on = past_limit(filter_undecided(a, x.cand, kUndecidedLeaf));
+                if (high) stack[cnt + nh - 1 - (before >> 16) - __popc(mh & below)] = up;
+                if (low) stack[cnt + nh + nl - 1 - (before & 0xffff) - __popc(ml & below)] = filter_half(x, s, 0u);
+                cnt += nl + nh;
+            }
+            if (kExact && exact) exact_box[atomicAdd(&n_exact, 1)] = x;
+            const unsigned e = __ballot_sync(0xffffffffu, emit);
+            if (e) {
+                unsigned long long o = 0;
+                if (lane == 0) o = atomicAdd(a.n_out, (unsigned long long)__popc(e));
+                o = __shfl_sync(0xffffffffu, o, 0) + __popc(e & below);
+                if (emit && o < a.cap) a.out[o] = filter_piece(x);
+                if (emit && o >= a.cap) full = true;
+            }
+            if (hand_on && !filter_hand_on(a, x.cand)) full = true;
+            __syncthreads();             // the pushed boxes and full are written
+            if (full) break;
+            if (kExact && n_exact > 0) {
+                pause = true;
+                break;
             }
         }
-        const unsigned e = __ballot_sync(0xffffffffu, emit);
-        if (e) {
-            unsigned long long o = 0;
-            if (lane == 0) o = atomicAdd(a.n_out, (unsigned long long)__popc(e));
-            o = __shfl_sync(0xffffffffu, o, 0) + __popc(e & below);
-            if (emit && o < a.cap) a.out[o] = filter_piece(x);
-            if (emit && o >= a.cap) full = true;
+        if (kExact && pause) {
+            if (tid < n_exact) {
+                const FNode x = exact_box[tid];
+                if (filter_exact(a.d, x)) {
+                    record_root(a, x);
+                    hits++;
+                } else if (past_limit(filter_undecided(a, x.cand, kUndecidedLeaf)) && !filter_hand_on(a, x.cand)) {
+                    exact_full = true;
+                }
+            }
+            __syncthreads();             // the boxes are read, exact_full is written
+            if (tid == 0) n_exact = 0;
+            pause = !exact_full;
         }
-        if (hand_on && !(atomicOr(a.state + x.cand, kHandedOn) & kHandedOn) && !filter_hand_on(a, x.cand)) full = true;
-        __syncthreads();             // the pushed boxes and full are written
-        if (full) break;
-    }
+    } while (kExact && pause);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         tot += __shfl_down_sync(0xffffffffu, tot, o);
