@@ -828,8 +828,8 @@ def main():
         "roofline": {"bound": "hbm", "kernel": ccd_kernel, "achieved": achieved, "peak": peak,
                      "unit": "GB/s", "frac": achieved / peak,
                      "traffic": None, "peak_source": peak_kind,
-                     "note": "bound by instruction issue (some 400 single-precision instructions "
-                             "a box), not HBM: algorithmic bytes are 304 B per candidate"},
+                     "note": "bound by the latency of the search's turns (a quarter of the issue slots "
+                             "used at most), not HBM: algorithmic bytes are 304 B per candidate"},
         "e2e": {"value": e2e, "unit": UNIT, "h2d_bytes_per_step": h2d,
                 "d2h_bytes_per_step": d2h},
         "clocks": clk.summary(),

@@ -399,7 +399,8 @@ static __device__ __noinline__ double barrier_coord(const BarrierBase& o, const 
     st[13 * stride] = E;
     st[14 * stride] = D;
     // by the forces on A .. W (the scalars' parts, N' and D' of a shallow angle
-    // above all, cancel in them before they are rounded)
+    // above all, cancel in them before they are rounded; by the scalars, in three
+    // orders, the converged run of 27 landing cubes ends 1e-8 from the oracle's)
     double G = fdot(o.f[1], d[1], fdot(o.f[0], d[0], 0.0));
     if (o.cross2) G = fdot(o.f[3], d[3], fdot(o.f[2], d[2], G));
     return fdot(o.f[4], d[4], G);

@@ -48,7 +48,7 @@ constexpr int kLargeCells = 64;
 // 1. body boxes and inclusion
 
 // A block per body.  Bound by the chain of one warp's vertices when a warp took a
-// body (18 FP64 instructions of 64 cycles for every 32 vertices): 32 slabs of 3.4 k
+// body (18 FP64 instructions of 64 cycles for every 32 vertices): 32 slabs of 2562
 // vertices 113 -> 39 us, 200 links of 1152 49 -> 23, 417 icospheres 25 -> 19.
 constexpr int kBodyThreads = 128;
 

