@@ -90,9 +90,10 @@ constexpr int kTaylor = 6;           // terms of S and C about the start pose
 constexpr int kSeries = 20;
 constexpr float kMaxTheta = 4.4f;    // S decreases up to 4.493
 // a candidate's state: undecided boxes from bit 32 on (kUndecidedLeaf for one
-// within tolerance, 1 for one at the limit of the levels, a subtree), bit 63 set
-// once it is handed on.  The limit: over piles, cubes and chains (tilted
-// contacts) a candidate has at most 20 within tolerance, nearly all none.
+// within tolerance, 1 for a subtree: at the limit of the levels, or without room
+// on the stack), bit 63 set once it is handed on.  The limit: over piles, cubes
+// and chains (tilted contacts) a candidate has at most 20 within tolerance, nearly
+// all none.
 constexpr unsigned kUndecidedLeaf = 16, kUndecidedLimit = 64 * kUndecidedLeaf;
 constexpr unsigned long long kHandedOn = 1ull << 63;
 
@@ -821,7 +822,12 @@ k_ccd_filter(FilterArgs a)
             }
             const int nl = all & 0xffff, nh = all >> 16;
             if (cnt + nl + nh > kFilterStack) {
-                emit = emit || split;
+                // (counted: a search that fills the stack without deciding is handed on)
+                if (split) {
+                    const unsigned long long u = filter_undecided(a, x.cand, 1u);
+                    emit = !(u & kHandedOn);
+                    hand_on = past_limit(u);
+                }
             } else {
                 if (high) stack[cnt + nh - 1 - (before >> 16) - __popc(mh & below)] = up;
                 if (low) stack[cnt + nh + nl - 1 - (before & 0xffff) - __popc(ml & below)] = filter_half(x, s, 0u);
