@@ -191,7 +191,7 @@ int rigc_set_candidates(rigc_ctx* ctx, int64_t num_ee, const int32_t* ee,
  * piece's, with the boxes on the way to it.  The pruned calls with a cap of
  * 2^22 or more search in single precision first; those boxes are not counted,
  * and a candidate that single precision cannot decide within 64 boxes at the
- * tolerance goes to the double-precision search. */
+ * tolerance (1,024 subtrees above it) goes to the double-precision search. */
 int rigc_set_ccd_budget(rigc_ctx* ctx, int64_t max_boxes_per_candidate);
 
 /* ---- narrow phase CCD: compute_earliest_toi_narrow_phase
